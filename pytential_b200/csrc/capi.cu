@@ -1261,9 +1261,9 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
   // The stage graph of drive_fmm (fmm.py:436-588) on four streams.  Every buffer
   // that several stages add into is written by one stream at a time:
   //   caller's stream: strengths, P2M, M2M | M2L, L2L | L2P | L2QBXL, QBXL2P, assembly
-  //   side[0]:         P2P, target-specific near field | M2P
+  //   side[0]:         P2P, target-specific near field | M2T, M2P
   //   side[1]:         P2L
-  //   side[2]:         P2QBXL | M2QBXL
+  //   side[2]:         P2QBXL | M2QBXL (unless M2T takes its place)
   // with events: fork after the strengths; M2P and M2QBXL wait for M2M; M2L waits
   // for P2L (both add into the locals); L2P and QBXL2P wait for side[0]
   // (pot_nonqbx, pot_tree); L2QBXL waits for side[2] (the QBX expansions).  Every
@@ -1274,6 +1274,8 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
   void* s3 = p->side[2];
   cudaStream_t side1 = p->side[0], side2 = p->side[1], side3 = p->side[2];
   const bool tsqbx = p->kern.target_specific_qbx != 0;
+  // 3D Helmholtz in FP64: the list-3 multipoles go straight to the QBX targets
+  const bool m2t = p->h3 && !p->mixed && tsqbx && h3_m2t_wins(p->geo);
   bool forked = false;
   // on an error, join the side streams before returning, so that a stream capture
   // of the caller's stream stays well formed
@@ -1313,10 +1315,16 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
   QBX_STEP(m2m());
   QBX_CUDA_STEP(cudaEventRecord(p->ev_mpoles, st), "apply: multipole event");
   QBX_CUDA_STEP(cudaStreamWaitEvent(side3, p->ev_mpoles, 0), "apply: multipole event");
-  QBX_STEP(qbxfmm_translate_box_multipoles_to_qbx_local(p, ws->mpoles, ws->qbx_exps,
-                                                        ws->error_word, s3));
+  if (!m2t)
+    QBX_STEP(qbxfmm_translate_box_multipoles_to_qbx_local(p, ws->mpoles, ws->qbx_exps,
+                                                          ws->error_word, s3));
   QBX_CUDA_STEP(cudaEventRecord(p->ev_qbx, side3), "apply: QBX-expansion event");
   QBX_CUDA_STEP(cudaStreamWaitEvent(side1, p->ev_mpoles, 0), "apply: multipole event");
+  if (m2t)
+    QBX_CUDA_STEP(h3_launch_m2t(p->geo, p->hc, p->kern.fmm_order, p->kern.qbx_order, p->kern.nrhs,
+                                (const double2*)ws->mpoles, (double2*)ws->pot_tree,
+                                ws->error_word, side1),
+                  "apply: multipoles to QBX targets");
   QBX_STEP(qbxfmm_eval_multipoles(p, ws->mpoles, ws->pot_nonqbx, ws->error_word, s1));
   QBX_CUDA_STEP(cudaEventRecord(p->ev_near, side1), "apply: near-field event");
   QBX_CUDA_STEP(cudaStreamWaitEvent(st, p->ev_p2l, 0), "apply: join P2L");

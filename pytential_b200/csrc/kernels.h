@@ -192,6 +192,11 @@ cudaError_t h3_launch_m2l_rot(const qbxfmm_geometry& g, int pf, int nrhs, const 
 cudaError_t h3_launch_m2qbxl(const qbxfmm_geometry& g, HelmCoeffs hc, int pf, int q, int nrhs,
                              const double2* mp, const double* rot, double2* qe, int32_t* err,
                              cudaStream_t st, bool fp32 = false);
+// list-3 multipoles straight to the QBX targets (M2QBXL and QBXL2P in one, added into
+// pot_tree); h3_m2t_wins: whether that is less work than the expansions
+cudaError_t h3_launch_m2t(const qbxfmm_geometry& g, HelmCoeffs hc, int pf, int q, int nrhs,
+                          const double2* mp, double2* pot_tree, int32_t* err, cudaStream_t st);
+bool h3_m2t_wins(const qbxfmm_geometry& g);
 cudaError_t h3_launch_l2qbxl(const qbxfmm_geometry& g, HelmCoeffs hc, int pf, int q, int nrhs,
                              const double2* lo, const double* rot, double2* qe, int32_t* err,
                              cudaStream_t st);

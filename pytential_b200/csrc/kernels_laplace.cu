@@ -11,6 +11,7 @@
 #include <cooperative_groups.h>
 
 #include "laplace.cuh"
+#include "near_poly.cuh"
 #include "kernels.h"
 
 namespace cg = cooperative_groups;
@@ -1451,15 +1452,129 @@ k_m2qbxl(qbxfmm_geometry g, int pf, int ncf, int nrhs, const double2* __restrict
 // reference native code pytential/qbx/target_specific/impl.pyx:222-362, 566-785).
 // For a QBX target t with center c and a list-1 source s, a = t - c, b = s - c:
 //   3D: 1/|t-s| ~ sum_{n<=Q} |a|^n / |b|^{n+1} P_n(cos g),  cos g = a.b / (|a||b|),
-//       double layer d.grad_s = sum_n |a|^n/|b|^{n+2} [-(n+1)(d.b^) P_n + (d.a^ - cos g d.b^) P_n']
+//       and its derivative along the source normal (near_poly.cuh)
 //   2D: log|t-s| ~ log|b| - Re sum_{n=1..Q} (a/b)^n / n,
 //       double layer Re(nu / b sum_{n=0..Q} (a/b)^n)      (nu = n_x + i n_y)
 // the same truncation as forming the order-Q QBX local from the list-1 sources and
 // evaluating it at t.  CTA = 4 warps over a chunk of <= 32 (target, center) pairs of
-// one target box (lane = pair); warps split the list-1 source tiles.
-template <int DIM, int Q, bool CHG, bool DIP>
+// one target box; the warps split the list-1 source tiles.
+//
+// 3D: bound by the FP64 pipe.  A lane holds up to four targets (lane % 8 of each octet
+// of the chunk) and every fourth source: a chunk of cnt targets costs ceil(cnt / 8)
+// octets instead of a full warp (chunks hold 22 targets on average), one load of a
+// source serves the octets, and the octets are independent chains.
+template <int Q, bool CHG, bool DIP>
 __global__ void __launch_bounds__(NT)
-k_tsqbx(qbxfmm_geometry g, SourceCoeffs sc, int nrhs, const double* __restrict__ strengths,
+k_tsqbx3(qbxfmm_geometry g, SourceCoeffs sc, int nrhs, const double* __restrict__ strengths,
+         double* __restrict__ pot_tree, int32_t* err)
+{
+  constexpr bool BOTH = CHG && DIP;
+  // (y0, y1), (y2, charge or m2), (m0, m1), m2: m = cd q nu
+  __shared__ double2 s_a[NT], s_b[NT], s_c[DIP ? NT : 1];
+  __shared__ double s_d[BOTH ? NT : 1];
+  __shared__ int s_pref[MAXB + 1], s_start[MAXB];
+  __shared__ double s_red[NW - 1][32];
+  const int chunk = blockIdx.x, r = blockIdx.y;
+  const int itb = g.tsqbx_chunk_target_box[chunk];
+  const int i0 = g.tsqbx_chunk_start[chunk], cnt = g.tsqbx_chunk_count[chunk];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int noct = (cnt + 7) >> 3;
+  double cc[4][3], a[4][3], aa[4], acc[4];
+  int tt[4];
+#pragma unroll
+  for (int o = 0; o < 4; ++o) {
+    const int ti = 8 * o + (lane & 7);
+    const int pi = i0 + max(0, min(ti, cnt - 1));
+    int t = g.tsqbx_targets[pi], ctr = g.tsqbx_centers[pi];
+    tt[o] = ti < cnt ? t : -1;
+    if ((unsigned)ctr >= (unsigned)g.ncenters || (unsigned)t >= (unsigned)g.ntargets) {
+      report(err, QBX_DEVERR_BAD_CENTER);
+      tt[o] = -1;
+      t = ctr = 0;
+    }
+    load_point<3>(g.centers, g.ncenters, ctr, cc[o]);
+    load_point<3>(g.targets, g.ntargets, t, a[o]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) a[o][d] -= cc[o][d];
+    aa[o] = a[o][0] * a[o][0] + a[o][1] * a[o][1] + a[o][2] * a[o][2];
+    acc[o] = 0.0;
+  }
+  const double* st = strengths + (size_t)r * g.nsources;
+  const int l0 = g.list1_starts[itb], l1 = g.list1_starts[itb + 1];
+  for (int gb = l0; gb < l1; gb += MAXB) {
+    const int nb = min(MAXB, l1 - gb);
+    __syncthreads();
+    list_prefix(g, g.list1_lists, gb, nb, s_pref, s_start, err);
+    __syncthreads();
+    const int total = s_pref[nb];
+    for (int base = 0; base < total; base += NT) {
+      const int v = base + threadIdx.x;
+      if (v < total) {
+        const int s = stream_source(v, nb, s_pref, s_start);
+        double y[3], m[3] = {0.0, 0.0, 0.0};
+        load_point<3>(g.sources, g.nsources, s, y);
+        const double q = __ldg(st + s);
+        if (DIP) {
+          load_point<3>(g.source_normals, g.nsources, s, m);
+#pragma unroll
+          for (int d = 0; d < 3; ++d) m[d] *= sc.cd * q;
+        }
+        s_a[threadIdx.x] = c2(y[0], y[1]);
+        s_b[threadIdx.x] = c2(y[2], CHG ? sc.cq * q : m[2]);
+        if (DIP) s_c[threadIdx.x] = c2(m[0], m[1]);
+        if (BOTH) s_d[threadIdx.x] = m[2];
+      }
+      __syncthreads();
+      const int jend = min(warp * 32 + 32, total - base);
+      for (int j = warp * 32 + (lane >> 3); j < jend; j += 4) {
+        const double2 ya = s_a[j], yb = s_b[j];
+        const double2 mc = DIP ? s_c[j] : c2(0.0);
+        const double m2 = BOTH ? s_d[j] : yb.y;
+#pragma unroll
+        for (int o = 0; o < 4; ++o) {
+          if (o >= noct) break;
+          const double b0 = ya.x - cc[o][0], b1 = ya.y - cc[o][1], b2 = yb.x - cc[o][2];
+          const double rho = rsqrt_h(b0 * b0 + b1 * b1 + b2 * b2);
+          const double rho2 = rho * rho;
+          const double x = (a[o][0] * b0 + a[o][1] * b1 + a[o][2] * b2) * rho2;
+          const double y = aa[o] * rho2;
+          double v = 0.0;
+          if (CHG) v = yb.y * near_f<Q>(x, y);
+          if (DIP) {
+            const double bn = b0 * mc.x + b1 * mc.y + b2 * m2;
+            double u = -bn * near_h<Q>(x, y);
+            if (Q > 0)
+              u = fma(a[o][0] * mc.x + a[o][1] * mc.y + a[o][2] * m2, near_dx<Q>(x, y), u);
+            v = CHG ? fma(rho2, u, v) : rho2 * u;
+          }
+          acc[o] = fma(rho, v, acc[o]);
+        }
+      }
+      __syncthreads();
+    }
+  }
+#pragma unroll
+  for (int o = 0; o < 4; ++o) {
+    acc[o] += __shfl_xor_sync(0xffffffffu, acc[o], 8);
+    acc[o] += __shfl_xor_sync(0xffffffffu, acc[o], 16);
+    if (warp > 0 && lane < 8) s_red[warp - 1][8 * o + lane] = acc[o];
+  }
+  __syncthreads();
+  if (warp == 0 && lane < 8) {
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {
+      if (tt[o] < 0) continue;
+      double v = acc[o];
+      for (int w = 1; w < NW; ++w) v += s_red[w - 1][8 * o + lane];
+      pot_tree[(size_t)r * g.ntargets + tt[o]] += v;
+    }
+  }
+}
+
+// 2D (lane = target)
+template <int Q, bool CHG, bool DIP>
+__global__ void __launch_bounds__(NT)
+k_tsqbx2(qbxfmm_geometry g, SourceCoeffs sc, int nrhs, const double* __restrict__ strengths,
         double* __restrict__ pot_tree, int32_t* err)
 {
   __shared__ double s_y[3][NT];
@@ -1480,13 +1595,10 @@ k_tsqbx(qbxfmm_geometry g, SourceCoeffs sc, int nrhs, const double* __restrict__
     active = false;
     t = ctr = 0;
   }
-  double cc[3] = {0, 0, 0}, x[3] = {0, 0, 0};
-  load_point<DIM>(g.centers, g.ncenters, ctr, cc);
-  load_point<DIM>(g.targets, g.ntargets, t, x);
-  double a[3] = {x[0] - cc[0], x[1] - cc[1], DIM == 3 ? x[2] - cc[2] : 0.0};
-  double alen = sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
-  double ainv = alen > 0.0 ? 1.0 / alen : 0.0;
-  double ah[3] = {a[0] * ainv, a[1] * ainv, a[2] * ainv};
+  double cc[2], x[2];
+  load_point<2>(g.centers, g.ncenters, ctr, cc);
+  load_point<2>(g.targets, g.ntargets, t, x);
+  const double a[2] = {x[0] - cc[0], x[1] - cc[1]};
   const double* st = strengths + (size_t)r * g.nsources;
   double acc = 0.0;
   int l0 = g.list1_starts[itb], l1 = g.list1_starts[itb + 1];
@@ -1497,76 +1609,31 @@ k_tsqbx(qbxfmm_geometry g, SourceCoeffs sc, int nrhs, const double* __restrict__
     __syncthreads();
     int total = s_pref[nb];
     for (int base = 0; base < total; base += NT) {
-      load_stream_tile<DIM, DIP>(g, st, total, nb, base, s_pref, s_start, s_y, s_n, s_q);
+      load_stream_tile<2, DIP>(g, st, total, nb, base, s_pref, s_start, s_y, s_n, s_q);
       __syncthreads();
       int jbeg = warp * 32, jend = min(jbeg + 32, total - base);
       if (active) {
         for (int j = jbeg; j < jend; ++j) {
           double q = s_q[j];
-          if (DIM == 3) {
-            double b0 = s_y[0][j] - cc[0], b1 = s_y[1][j] - cc[1], b2 = s_y[2][j] - cc[2];
-            double b2s = b0 * b0 + b1 * b1 + b2 * b2;
-            double binv = rsqrt(b2s);
-            double cg = (ah[0] * b0 + ah[1] * b1 + ah[2] * b2) * binv;   // cos g
-            double ratio = alen * binv;                                  // |a| / |b|
-            // Legendre P_n, P_n' by recurrence; R_n = ratio^n / |b|
-            double pm1 = 1.0, pm2 = 0.0, dm1 = 0.0, dm2 = 0.0;
-            double rn = binv;
-            double sS = 0.0, sA = 0.0, sB = 0.0;
+          double2 bb = c2(s_y[0][j] - cc[0], s_y[1][j] - cc[1]);
+          double2 binv = cinv(bb);
+          double2 w = cmul(c2(a[0], a[1]), binv);   // a / b
+          double2 pw = w;
+          double2 sl = c2(0.0);   // sum_{n>=1} w^n / n
+          double2 sd = c2(1.0);   // sum_{n>=0} w^n
 #pragma unroll
-            for (int n = 0; n <= Q; ++n) {
-              double pn, dn;
-              if (n == 0) {
-                pn = 1.0;
-                dn = 0.0;
-              } else if (n == 1) {
-                pn = cg;
-                dn = 1.0;
-              } else {
-                pn = ((2.0 * n - 1) * cg * pm1 - (n - 1.0) * pm2) * (1.0 / n);
-                dn = n * pm1 + cg * dm1;
-              }
-              if (CHG) sS = fma(rn, pn, sS);
-              if (DIP) {
-                sA = fma(-(n + 1.0) * rn, pn, sA);
-                sB = fma(rn, dn, sB);
-              }
-              pm2 = pm1;
-              pm1 = pn;
-              dm2 = dm1;
-              dm1 = dn;
-              rn *= ratio;
-            }
-            double v = 0.0;
-            if (CHG) v = sc.cq * sS;
-            if (DIP) {
-              double db = (s_n[0][j] * b0 + s_n[1][j] * b1 + s_n[2][j] * b2) * binv;
-              double da = s_n[0][j] * ah[0] + s_n[1][j] * ah[1] + s_n[2][j] * ah[2];
-              v += sc.cd * binv * (sA * db + sB * (da - cg * db));
-            }
-            acc = fma(q, v, acc);
-            (void)dm2;
-          } else {
-            double2 bb = c2(s_y[0][j] - cc[0], s_y[1][j] - cc[1]);
-            double2 binv = cinv(bb);
-            double2 w = cmul(c2(a[0], a[1]), binv);   // a / b
-            double2 pw = w;
-            double2 sl = c2(0.0);   // sum_{n>=1} w^n / n
-            double2 sd = c2(1.0);   // sum_{n>=0} w^n
-#pragma unroll
-            for (int n = 1; n <= Q; ++n) {
-              if (CHG) sl = caxpy(1.0 / n, pw, sl);
-              if (DIP) sd = cadd(sd, pw);
-              pw = cmul(pw, w);
-            }
-            double v = 0.0;
-            if (CHG) v = sc.cq * (0.5 * log(bb.x * bb.x + bb.y * bb.y) - sl.x);
-            if (DIP) {
-              double2 f = cmul(cmul(c2(s_n[0][j], s_n[1][j]), binv), sd);
-              v += sc.cd * f.x;
-            }
-            acc = fma(q, v, acc);
+          for (int n = 1; n <= Q; ++n) {
+            if (CHG) sl = caxpy(1.0 / n, pw, sl);
+            if (DIP) sd = cadd(sd, pw);
+            pw = cmul(pw, w);
           }
+          double v = 0.0;
+          if (CHG) v = sc.cq * (0.5 * log(bb.x * bb.x + bb.y * bb.y) - sl.x);
+          if (DIP) {
+            double2 f = cmul(cmul(c2(s_n[0][j], s_n[1][j]), binv), sd);
+            v += sc.cd * f.x;
+          }
+          acc = fma(q, v, acc);
         }
       }
       __syncthreads();
@@ -2036,9 +2103,15 @@ static cudaError_t tsqbx_q(const qbxfmm_geometry& g, SourceCoeffs sc, int nrhs, 
                            double* pt, int32_t* err, cudaStream_t st)
 {
   dim3 grid(g.ntsqbx_chunks, grid_y(nrhs));
-  if (sc.cq != 0.0 && sc.cd != 0.0) k_tsqbx<DIM, Q, true, true><<<grid, NT, 0, st>>>(g, sc, nrhs, s, pt, err);
-  else if (sc.cd != 0.0) k_tsqbx<DIM, Q, false, true><<<grid, NT, 0, st>>>(g, sc, nrhs, s, pt, err);
-  else k_tsqbx<DIM, Q, true, false><<<grid, NT, 0, st>>>(g, sc, nrhs, s, pt, err);
+  if constexpr (DIM == 3) {
+    if (sc.cq != 0.0 && sc.cd != 0.0) k_tsqbx3<Q, true, true><<<grid, NT, 0, st>>>(g, sc, nrhs, s, pt, err);
+    else if (sc.cd != 0.0) k_tsqbx3<Q, false, true><<<grid, NT, 0, st>>>(g, sc, nrhs, s, pt, err);
+    else k_tsqbx3<Q, true, false><<<grid, NT, 0, st>>>(g, sc, nrhs, s, pt, err);
+  } else {
+    if (sc.cq != 0.0 && sc.cd != 0.0) k_tsqbx2<Q, true, true><<<grid, NT, 0, st>>>(g, sc, nrhs, s, pt, err);
+    else if (sc.cd != 0.0) k_tsqbx2<Q, false, true><<<grid, NT, 0, st>>>(g, sc, nrhs, s, pt, err);
+    else k_tsqbx2<Q, true, false><<<grid, NT, 0, st>>>(g, sc, nrhs, s, pt, err);
+  }
   return cudaGetLastError();
 }
 

@@ -28,6 +28,7 @@
 // depend on scheduling.  The box stages of the transpose are the library's own P2M / M2M /
 // M2L / M2P / P2L / L2L / L2P / P2P on the exchanged-role geometry.
 #include "laplace.cuh"
+#include "near_poly.cuh"
 #include "kernels.h"
 
 #include <algorithm>
@@ -379,7 +380,8 @@ k_tr_tsqbx(qbxfmm_geometry g, qbxfmm_transpose_index ix, int nrhs, double cq,
            const double* __restrict__ tvals, double* __restrict__ vals,
            double* __restrict__ grads, int32_t* err)
 {
-  __shared__ double s_c[3][TR_PB], s_ah[3][TR_PB], s_al[TR_PB], s_w[TR_PB];
+  // (c0, c1), (c2, w), (a0, a1), (a2, |a|^2)
+  __shared__ double2 s_c01[TR_PB], s_c2w[TR_PB], s_a01[TR_PB], s_a2s[TR_PB];
   __shared__ double s_part[TR_KS][DIP ? 4 : 1][NT];
   const int row = blockIdx.x / CL, part = blockIdx.x - row * CL;
   cg::cluster_group cl = cg::this_cluster();
@@ -423,52 +425,34 @@ k_tr_tsqbx(qbxfmm_geometry g, qbxfmm_transpose_index ix, int nrhs, double cq,
           } else if ((unsigned)t >= (unsigned)g.ntargets) {
             report(err, QBX_DEVERR_BAD_CENTER);
           }
-          double al = sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
-          double ainv = al > 0.0 ? 1.0 / al : 0.0;
-          for (int d = 0; d < 3; ++d) {
-            s_c[d][threadIdx.x] = cc[d];
-            s_ah[d][threadIdx.x] = a[d] * ainv;
-          }
-          s_al[threadIdx.x] = al;
-          s_w[threadIdx.x] = w;
+          s_c01[threadIdx.x] = c2(cc[0], cc[1]);
+          s_c2w[threadIdx.x] = c2(cc[2], w);
+          s_a01[threadIdx.x] = c2(a[0], a[1]);
+          s_a2s[threadIdx.x] = c2(a[2], a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
         }
         __syncthreads();
         for (int pi = 0; pi < np; ++pi) {
-          double w = s_w[pi];
+          const double2 cw = s_c2w[pi];
+          const double w = cw.y;
           if (w == 0.0) continue;
-          double cx = s_c[0][pi], cy = s_c[1][pi], cz = s_c[2][pi];
-          double hx = s_ah[0][pi], hy = s_ah[1][pi], hz = s_ah[2][pi], al = s_al[pi];
+          const double2 c01 = s_c01[pi], a01 = s_a01[pi], a2s = s_a2s[pi];
 #pragma unroll
           for (int k = 0; k < TR_KS; ++k) {
             if (g0 + threadIdx.x + k * NT >= ns) break;
-            double b0 = y[k][0] - cx, b1 = y[k][1] - cy, b2 = y[k][2] - cz;
-            double binv = rsqrt(b0 * b0 + b1 * b1 + b2 * b2);
-            double cg = (hx * b0 + hy * b1 + hz * b2) * binv;
-            double ratio = al * binv;
-            double pm1 = 1.0, pm2 = 0.0, dm1 = 0.0, rn = binv, sum = 0.0, sa = 0.0, sb = 0.0;
-#pragma unroll
-            for (int n = 0; n <= Q; ++n) {
-              double pn = n == 0 ? 1.0
-                        : n == 1 ? cg
-                                 : ((2.0 * n - 1) * cg * pm1 - (n - 1.0) * pm2) * (1.0 / n);
-              sum = fma(rn, pn, sum);
-              if (DIP) {
-                double dn = n == 0 ? 0.0 : n * pm1 + cg * dm1;
-                sa = fma(-(n + 1.0) * rn, pn, sa);
-                sb = fma(rn, dn, sb);
-                dm1 = dn;
-              }
-              pm2 = pm1;
-              pm1 = pn;
-              rn *= ratio;
-            }
-            acc[k] = fma(w, sum, acc[k]);
+            const double b0 = y[k][0] - c01.x, b1 = y[k][1] - c01.y, b2 = y[k][2] - cw.x;
+            const double rho = rsqrt_h(b0 * b0 + b1 * b1 + b2 * b2);
+            const double rho2 = rho * rho, wr = w * rho;
+            const double xx = (a01.x * b0 + a01.y * b1 + a2s.x * b2) * rho2;
+            const double yy = a2s.y * rho2;
+            acc[k] = fma(wr, near_f<Q>(xx, yy), acc[k]);
             if (DIP) {
-              // grad_b K = (sa b^ + sb (a^ - cos g b^)) / |b|
-              double fb = w * binv * (sa - sb * cg), fa = w * binv * sb;
-              gacc[DIP ? k : 0][0] += fb * b0 * binv + fa * hx;
-              gacc[DIP ? k : 0][1] += fb * b1 * binv + fa * hy;
-              gacc[DIP ? k : 0][2] += fb * b2 * binv + fa * hz;
+              // grad_b K = rho^3 (a dF/dx - b H)
+              const double wr3 = wr * rho2, fb = -wr3 * near_h<Q>(xx, yy);
+              const double fa = Q > 0 ? wr3 * near_dx<Q>(xx, yy) : 0.0;
+              double* G = gacc[DIP ? k : 0];
+              G[0] = fma(fa, a01.x, fma(fb, b0, G[0]));
+              G[1] = fma(fa, a01.y, fma(fb, b1, G[1]));
+              G[2] = fma(fa, a2s.x, fma(fb, b2, G[2]));
             }
           }
         }

@@ -1,0 +1,55 @@
+"""3D Laplace stage kernels at the edges of their orders, against the checker's stages."""
+
+import functools
+
+import numpy as np
+import pytest
+import torch
+
+from oracle.oracle import Oracle
+from pytential_b200 import fmm
+from pytential_b200.discretization import make_ellipsoid
+from pytential_b200.geometry import QBXFMMGeometryData
+
+pytestmark = pytest.mark.gpu
+
+# float64 sums of at most a few thousand terms per output, as for every stage
+TOL = 1e-12
+
+
+@functools.lru_cache(maxsize=None)
+def _geometry():
+    d = make_ellipsoid(1)
+    rng = np.random.default_rng(2)
+    v = rng.normal(size=(3, 45))
+    far = 3.0 * v / np.linalg.norm(v, axis=0)
+    return d, QBXFMMGeometryData(d, [(d.nodes, +1), (far, 0)], max_leaf_refine_weight=64)
+
+
+def _setup(q, p, cq, cd, nrhs=1, tsqbx=False):
+    d, geo = _geometry()
+    spec = fmm.SourceKernelSpec(fmm.LaplaceKernel(3), charge_coeff=cq, dipole_coeff=cd)
+    w = fmm.B200QBXExpansionWrangler(
+        fmm.B200TreeIndependentDataForWrangler(spec), geo, np.float64, q,
+        lambda kern, args, tree, lev: p, _use_target_specific_qbx=tsqbx, nrhs=nrhs)
+    o = Oracle(geo, dim=3, qbx_order=q, fmm_order=p, nrhs=nrhs, charge_coeff=cq, dipole_coeff=cd)
+    s = o.tree_strengths(np.random.default_rng(3).normal(size=(nrhs, d.nquad)))
+    return w, o, s
+
+
+def _close(got, want):
+    got = got.cpu().numpy()
+    assert np.abs(want).max() > 0
+    assert np.abs(got - want).max() <= TOL * np.abs(want).max()
+
+
+@pytest.mark.parametrize("q", range(9))
+@pytest.mark.parametrize("cq,cd", [(1.0, 0.0), (0.0, 1.0), (0.7, -1.3)])
+def test_target_specific_near_field(q, cq, cd):
+    """The polynomial form against the expansions formed from the same sources."""
+    w, o, s = _setup(q, 5, cq, cd, nrhs=2, tsqbx=True)
+    got = w.eval_target_specific_qbx_locals(None, [torch.from_numpy(s).cuda()])
+    qe, want = o.zeros_qbx_exps(), o.zeros_tree_pot()
+    o.stage("form_global_qbx_locals", s, qe)
+    o.stage("eval_qbx_expansions", qe, want)
+    _close(got, want)

@@ -569,205 +569,33 @@ k_m2l2(qbxfmm_geometry g, int p, int ncf, int nrhs, const double2* __restrict__ 
 
 // {{{ P2L (form_locals, list 4, fmm.py:502-510)
 
-// One CTA per target-or-parent box; its list-4 sources stream through shared memory
-// in sub-tiles of SUB; per sub-tile each source's singular-harmonic table (orders
-// 0..p+1) is built by one thread per (source, column), then each thread accumulates
-// its coefficient(s) with precomputed table offsets.  The tables are stored
-// entry-major, tab[entry * P2L_TS + source], so the lanes of a warp building one
-// column write consecutive words, and the lanes reading different entries of one
-// source are spread over the banks by the padded stride.
+// One CTA per target-or-parent box; its list-4 sources stream through shared memory.
+
+// 2D: per sub-tile of SUB sources one thread per source builds the table of its inverse
+// powers, then each thread accumulates its coefficient.  Entry-major, padded stride.
 constexpr int P2L_SUB = 32;
 constexpr int P2L_TS = P2L_SUB + 1;
 
-template <int DIM>
 __global__ void __launch_bounds__(NT)
-k_p2l(qbxfmm_geometry g, SourceCoeffs sc, int p, int ncf, int nrhs,
-      const double* __restrict__ strengths, double2* __restrict__ locals, int32_t* err)
+k_p2l2(qbxfmm_geometry g, SourceCoeffs sc, int p, int ncf, int nrhs,
+       const double* __restrict__ strengths, double2* __restrict__ locals, int32_t* err)
 {
   constexpr int SUB = P2L_SUB;
   constexpr int TS = P2L_TS;
   extern __shared__ double2 smem2[];
-  double2* tab = smem2;   // [nct][TS]
-  __shared__ double s_u[SUB][3], s_n[SUB][3], s_q[SUB];
+  double2* tab = smem2;   // [p + 3][TS]
+  __shared__ double s_u[SUB][2], s_n[SUB][2], s_q[SUB];
   __shared__ int s_pref[MAXB + 1], s_start[MAXB];
   int i = blockIdx.x;
   int tb = g.target_or_target_parent_boxes[i];
   int r = blockIdx.y;
   double rho = level_width(g, g.box_levels[tb]);
   double rinv = 1.0 / rho;
-  double c[3];
-  load_point<DIM>(g.box_centers, g.nboxes, tb, c);
+  double c[2];
+  load_point<2>(g.box_centers, g.nboxes, tb, c);
   const double* st = strengths + (size_t)r * g.nsources;
   const bool dip = sc.cd != 0.0;
-
-  // per-thread coefficient bookkeeping (3D): table offsets of S_n^m and the
-  // dipole neighbours S_{n+1}^{m-1}, S_{n+1}^m, S_{n+1}^{m+1}
-  int o_nm[2], o_a[2], o_b[2], o_c[2];
-  double sb_sign[2];
-  bool valid[2];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    int ci = threadIdx.x + h * NT;
-    valid[h] = ci < ncf;
-    o_nm[h] = o_a[h] = o_b[h] = o_c[h] = 0;
-    sb_sign[h] = 1.0;
-    if (DIM == 3 && valid[h]) {
-      int n, m;
-      decode3(ci, n, m);
-      o_nm[h] = idx3(n, m) * TS;
-      o_a[h] = idx3(n + 1, m) * TS;
-      o_b[h] = idx3(n + 1, m > 0 ? m - 1 : 1) * TS;   // m = 0: S_{n+1}^{-1} = -conj(S_{n+1}^1)
-      sb_sign[h] = m > 0 ? 1.0 : -1.0;
-      o_c[h] = idx3(n + 1, m + 1) * TS;
-    }
-  }
-
-  double2 acc[2] = {c2(0.0), c2(0.0)};
-  int l0 = g.list4_starts[i], l1 = g.list4_starts[i + 1];
-  for (int gb = l0; gb < l1; gb += MAXB) {
-    int nb = min(MAXB, l1 - gb);
-    __syncthreads();
-    list_prefix(g, g.list4_lists, gb, nb, s_pref, s_start, err);
-    __syncthreads();
-    int total = s_pref[nb];
-    for (int base = 0; base < total; base += SUB) {
-      int cnt = min(SUB, total - base);
-      if (threadIdx.x < cnt) {
-        int s = stream_source(base + threadIdx.x, nb, s_pref, s_start);
-        double y[3];
-        load_point<DIM>(g.sources, g.nsources, s, y);
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) s_u[threadIdx.x][d] = (y[d] - c[d]) * rinv;
-        if (dip) {
-          double nv[3];
-          load_point<DIM>(g.source_normals, g.nsources, s, nv);
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) s_n[threadIdx.x][d] = nv[d];
-        }
-        s_q[threadIdx.x] = __ldg(st + s);
-      }
-      __syncthreads();
-      if (DIM == 3) {
-        for (int w = threadIdx.x; w < cnt * (p + 2); w += NT) {
-          int m = w / cnt, j = w - m * cnt;
-          double x = s_u[j][0], y = s_u[j][1], z = s_u[j][2];
-          double rinv2 = 1.0 / (x * x + y * y + z * z);
-          double2 a = c2(sqrt(rinv2));
-          for (int k = 1; k <= m; ++k) a = cscale((2.0 * k - 1) * rinv2, cmul(a, c2(x, y)));
-          double2* T = tab + j;
-          T[idx3(m, m) * TS] = a;
-          double2 prev = c2(0.0);
-          for (int n = m + 1; n <= p + 1; ++n) {
-            double2 bb = cscale(rinv2, csub(cscale((2.0 * n - 1) * z, a),
-                                            cscale((double)(n + m - 1) * (n - m - 1), prev)));
-            T[idx3(n, m) * TS] = bb;
-            prev = a;
-            a = bb;
-          }
-        }
-      } else {
-        for (int j = threadIdx.x; j < cnt; j += NT) {
-          double2 tinv = cinv(c2(s_u[j][0], s_u[j][1]));
-          double2* T = tab + j;
-          double2 a = c2(1.0);
-          for (int k = 0; k <= p + 1; ++k) {
-            T[k * TS] = a;   // tau^-k
-            a = cmul(a, tinv);
-          }
-          T[(p + 2) * TS] =
-              c2(0.5 * log((s_u[j][0] * s_u[j][0] + s_u[j][1] * s_u[j][1]) * rho * rho));
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (!valid[h]) continue;
-        int ci = threadIdx.x + h * NT;
-        double2 a = acc[h];
-        for (int j = 0; j < cnt; ++j) {
-          const double2* T = tab + j;
-          double q = s_q[j];
-          if (DIM == 3) {
-            a = caxpy(sc.cq * q * rinv, T[o_nm[h]], a);
-            if (dip) {
-              double f = sc.cd * q * rinv * rinv;
-              double dx = s_n[j][0], dy = s_n[j][1], dz = s_n[j][2];
-              double2 tb_ = T[o_b[h]];
-              if (sb_sign[h] < 0) tb_ = c2(-tb_.x, tb_.y);
-              double2 v = cscale(-dz, T[o_a[h]]);
-              v = cfma(c2(0.5 * dx, 0.5 * dy), tb_, v);
-              v = cfma(c2(-0.5 * dx, 0.5 * dy), T[o_c[h]], v);
-              a = caxpy(f, v, a);
-            }
-          } else {
-            int l = ci;
-            if (l == 0) a.x += sc.cq * q * T[(p + 2) * TS].x;
-            else a = caxpy(-sc.cq * q * rcp(l), T[l * TS], a);
-            if (dip) {
-              double2 nu = c2(s_n[j][0], s_n[j][1]);
-              a = cfma(cscale(sc.cd * q * rinv, nu), T[(l + 1) * TS], a);
-            }
-          }
-        }
-        acc[h] = a;
-      }
-      __syncthreads();
-    }
-  }
-  double2* L = locals + ((size_t)tb * nrhs + r) * ncf;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    int o = threadIdx.x + h * NT;
-    if (o < ncf) L[o] = cadd(L[o], acc[h]);
-  }
-}
-
-// }}}
-
-// 3D P2L with every coefficient split over two threads: a block of
-// P2L3_SPLIT x ncf threads (rounded up to whole warps) takes, per 32-source tile, the
-// sources [0, 16) in the first half of the threads and [16, 32) in the second, so no
-// thread waits idle through the accumulation (with one thread per coefficient, 62 of
-// 128 threads had nothing to accumulate at p = 10).  All threads build the tile's
-// harmonic tables; the halves are added in shared memory at the end.
-constexpr int P2L3_SPLIT = 2;
-constexpr int P2L3_MAXT = 256;
-
-__global__ void __launch_bounds__(P2L3_MAXT)
-k_p2l3s(qbxfmm_geometry g, SourceCoeffs sc, int p, int ncf, int nrhs,
-        const double* __restrict__ strengths, double2* __restrict__ locals, int32_t* err)
-{
-  constexpr int SUB = P2L_SUB;
-  constexpr int TS = P2L_TS;
-  constexpr int HALF = SUB / P2L3_SPLIT;
-  extern __shared__ double2 smem2[];
-  double2* tab = smem2;   // [nct][TS]
-  __shared__ double s_u[SUB][3], s_n[SUB][3], s_q[SUB];
-  __shared__ int s_pref[MAXB + 1], s_start[MAXB];
-  const int nthr = blockDim.x;
-  int i = blockIdx.x;
-  int tb = g.target_or_target_parent_boxes[i];
-  int r = blockIdx.y;
-  double rho = level_width(g, g.box_levels[tb]);
-  double rinv = 1.0 / rho;
-  double c[3];
-  load_point<3>(g.box_centers, g.nboxes, tb, c);
-  const double* st = strengths + (size_t)r * g.nsources;
-  const bool dip = sc.cd != 0.0;
-
-  // this thread's coefficient (n, m) and source half; table offsets of S_n^m and of
-  // the dipole neighbours S_{n+1}^{m-1}, S_{n+1}^m, S_{n+1}^{m+1}
-  const bool active = (int)threadIdx.x < P2L3_SPLIT * ncf;
-  const int ci = active ? (int)threadIdx.x % ncf : 0;
-  const int half = active ? (int)threadIdx.x / ncf : 0;
-  int n, m;
-  decode3(ci, n, m);
-  const int o_nm = idx3(n, m) * TS;
-  const int o_a = idx3(n + 1, m) * TS;
-  const int o_b = idx3(n + 1, m > 0 ? m - 1 : 1) * TS;   // m = 0: S_{n+1}^{-1} = -conj(S_{n+1}^1)
-  const double sb_sign = m > 0 ? 1.0 : -1.0;
-  const int o_c = idx3(n + 1, m + 1) * TS;
-
+  const int l = threadIdx.x;
   double2 acc = c2(0.0);
   int l0 = g.list4_starts[i], l1 = g.list4_starts[i + 1];
   for (int gb = l0; gb < l1; gb += MAXB) {
@@ -778,68 +606,192 @@ k_p2l3s(qbxfmm_geometry g, SourceCoeffs sc, int p, int ncf, int nrhs,
     int total = s_pref[nb];
     for (int base = 0; base < total; base += SUB) {
       int cnt = min(SUB, total - base);
-      if ((int)threadIdx.x < cnt) {
-        int s = stream_source(base + threadIdx.x, nb, s_pref, s_start);
-        double y[3];
-        load_point<3>(g.sources, g.nsources, s, y);
+      if (threadIdx.x < cnt) {
+        const int j = threadIdx.x;
+        int s = stream_source(base + j, nb, s_pref, s_start);
+        double y[2];
+        load_point<2>(g.sources, g.nsources, s, y);
 #pragma unroll
-        for (int d = 0; d < 3; ++d) s_u[threadIdx.x][d] = (y[d] - c[d]) * rinv;
+        for (int d = 0; d < 2; ++d) s_u[j][d] = (y[d] - c[d]) * rinv;
         if (dip) {
-          double nv[3];
-          load_point<3>(g.source_normals, g.nsources, s, nv);
+          double nv[2];
+          load_point<2>(g.source_normals, g.nsources, s, nv);
 #pragma unroll
-          for (int d = 0; d < 3; ++d) s_n[threadIdx.x][d] = nv[d];
+          for (int d = 0; d < 2; ++d) s_n[j][d] = nv[d];
         }
-        s_q[threadIdx.x] = __ldg(st + s);
-      }
-      __syncthreads();
-      for (int w = threadIdx.x; w < cnt * (p + 2); w += nthr) {
-        int mm = w / cnt, j = w - mm * cnt;
-        double x = s_u[j][0], yy = s_u[j][1], z = s_u[j][2];
-        double rinv2 = 1.0 / (x * x + yy * yy + z * z);
-        double2 a = c2(sqrt(rinv2));
-        for (int k = 1; k <= mm; ++k) a = cscale((2.0 * k - 1) * rinv2, cmul(a, c2(x, yy)));
+        s_q[j] = __ldg(st + s);
+        double2 tinv = cinv(c2(s_u[j][0], s_u[j][1]));
         double2* T = tab + j;
-        T[idx3(mm, mm) * TS] = a;
-        double2 prev = c2(0.0);
-        for (int nn = mm + 1; nn <= p + 1; ++nn) {
-          double2 bb = cscale(rinv2, csub(cscale((2.0 * nn - 1) * z, a),
-                                          cscale((double)(nn + mm - 1) * (nn - mm - 1), prev)));
-          T[idx3(nn, mm) * TS] = bb;
-          prev = a;
-          a = bb;
+        double2 a = c2(1.0);
+        for (int k = 0; k <= p + 1; ++k) {
+          T[k * TS] = a;   // tau^-k
+          a = cmul(a, tinv);
         }
+        T[(p + 2) * TS] =
+            c2(0.5 * log((s_u[j][0] * s_u[j][0] + s_u[j][1] * s_u[j][1]) * rho * rho));
       }
       __syncthreads();
-      if (active) {
-        int jend = min(cnt, (half + 1) * HALF);
-        for (int j = half * HALF; j < jend; ++j) {
+      if (l < ncf) {
+        for (int j = 0; j < cnt; ++j) {
           const double2* T = tab + j;
           double q = s_q[j];
-          acc = caxpy(sc.cq * q * rinv, T[o_nm], acc);
+          if (l == 0) acc.x += sc.cq * q * T[(p + 2) * TS].x;
+          else acc = caxpy(-sc.cq * q * rcp(l), T[l * TS], acc);
           if (dip) {
-            double f = sc.cd * q * rinv * rinv;
-            double dx = s_n[j][0], dy = s_n[j][1], dz = s_n[j][2];
-            double2 tb_ = T[o_b];
-            if (sb_sign < 0) tb_ = c2(-tb_.x, tb_.y);
-            double2 v = cscale(-dz, T[o_a]);
-            v = cfma(c2(0.5 * dx, 0.5 * dy), tb_, v);
-            v = cfma(c2(-0.5 * dx, 0.5 * dy), T[o_c], v);
-            acc = caxpy(f, v, acc);
+            double2 nu = c2(s_n[j][0], s_n[j][1]);
+            acc = cfma(cscale(sc.cd * q * rinv, nu), T[(l + 1) * TS], acc);
           }
         }
       }
       __syncthreads();
     }
   }
-  // the second half's sums through the (now free) table space
-  if (active && half == 1) tab[ci] = acc;
-  __syncthreads();
-  if (active && half == 0) {
+  if (l < ncf) {
     double2* L = locals + ((size_t)tb * nrhs + r) * ncf;
-    L[ci] = cadd(L[ci], cadd(acc, tab[ci]));
+    L[l] = cadd(L[l], acc);
   }
 }
+
+// 3D: harmonics and sums in registers.  G = p / 2 + 1 lanes share a source: lane l runs the
+// recurrence along n down the column m = l (p - l + 1 entries) and then the column
+// m = p - l (l + 1 entries), p + 2 entries for every lane, each added into an
+// accumulator of its own (index = step), so no table is written or read; a warp takes
+// 32 / G sources at a time.  In inverted coordinates v = u / |u|^2, the recurrence is
+//   S_{n+1} = (2n + 1) v_z S_n - (n^2 - m^2) |v|^2 S_{n-1},
+// started at S_m^m (one thread per source, in shared memory).  DIP: c = cq S + cd nu.grad S
+// is carried beside S by differentiating the recurrence.  2n + 1 and n^2 - m^2 are
+// exact running sums.  T >= p + 2 bounds the steps (register accumulators).
+template <int T, bool DIP>
+__global__ void __launch_bounds__(NT)
+k_p2l3(qbxfmm_geometry g, SourceCoeffs sc, int p, int ncf, int nrhs,
+       const double* __restrict__ strengths, double2* __restrict__ locals, int32_t* err)
+{
+  constexpr int SW = NT + 1;
+  extern __shared__ double2 smem2[];
+  double2* s_s = smem2;                                  // [p + 1][SW]: q S_m^m
+  double2* s_c = s_s + (DIP ? (size_t)(p + 1) * SW : 0);  // [p + 1][SW]: q c_m^m
+  __shared__ double2 s_v[NT], s_dv[DIP ? NT : 1];        // (v_z, |v|^2), cd times derivatives
+  __shared__ int s_pref[MAXB + 1], s_start[MAXB];
+  const int i = blockIdx.x, r = blockIdx.y;
+  const int l0 = g.list4_starts[i], l1 = g.list4_starts[i + 1];
+  if (l1 <= l0) return;
+  const int tb = g.target_or_target_parent_boxes[i];
+  const double rinv = 1.0 / level_width(g, g.box_levels[tb]);
+  double c[3];
+  load_point<3>(g.box_centers, g.nboxes, tb, c);
+  const double* st = strengths + (size_t)r * g.nsources;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int G = p / 2 + 1, SPW = 32 / G;
+  const int grp = lane / G, m1 = lane - grp * G, m2 = p - m1;
+  const bool lane_on = grp < SPW;
+
+  double2 acc[T];
+#pragma unroll
+  for (int t = 0; t < T; ++t) acc[t] = c2(0.0);
+
+  for (int gb = l0; gb < l1; gb += MAXB) {
+    const int nb = min(MAXB, l1 - gb);
+    __syncthreads();
+    list_prefix(g, g.list4_lists, gb, nb, s_pref, s_start, err);
+    __syncthreads();
+    const int total = s_pref[nb];
+    for (int base = 0; base < total; base += NT) {
+      const int j0 = threadIdx.x;
+      if (base + j0 < total) {
+        const int s = stream_source(base + j0, nb, s_pref, s_start);
+        double u[3];
+        load_point<3>(g.sources, g.nsources, s, u);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) u[d] = (u[d] - c[d]) * rinv;
+        const double q = __ldg(st + s) * rinv;
+        const double ri = rsqrt_h(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+        const double r2 = ri * ri;
+        const double2 X = c2(u[0] * r2, u[1] * r2);
+        const double vz = u[2] * r2;
+        s_v[j0] = c2(vz, r2);
+        double2 a = c2(DIP ? q * ri : sc.cq * q * ri);
+        double2 b = c2(0.0), dX = c2(0.0);
+        if (DIP) {
+          double nv[3];
+          load_point<3>(g.source_normals, g.nsources, s, nv);
+#pragma unroll
+          for (int d = 0; d < 3; ++d) nv[d] *= sc.cd * rinv;
+          const double du = nv[0] * u[0] + nv[1] * u[1] + nv[2] * u[2];
+          dX = c2(r2 * (nv[0] - 2.0 * X.x * du), r2 * (nv[1] - 2.0 * X.y * du));
+          s_dv[j0] = c2(r2 * (nv[2] - 2.0 * vz * du), -2.0 * du * r2 * r2);
+          b = c2(a.x * (sc.cq - du * r2));
+        }
+        for (int m = 0;; ++m) {
+          s_s[m * SW + j0] = a;
+          if (DIP) s_c[m * SW + j0] = b;
+          if (m == p) break;
+          const double f = 2.0 * m + 1.0;
+          if (DIP) b = cscale(f, cfma(X, b, cmul(dX, a)));
+          a = cscale(f, cmul(X, a));
+        }
+      }
+      __syncthreads();
+      const int jend = min(warp * 32 + 32, total - base);
+      for (int j = warp * 32 + grp; lane_on && j < jend; j += SPW) {
+        const double2 v = s_v[j], dv = DIP ? s_dv[j] : c2(0.0);
+        double2 a = s_s[m1 * SW + j], pa = c2(0.0);
+        double2 b = DIP ? s_c[m1 * SW + j] : c2(0.0), pb = c2(0.0);
+        double al = 2.0 * m1 + 1.0, be = 0.0;
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+          if (t > p + 1) break;
+          acc[t] = cadd(acc[t], DIP ? b : a);
+          const double az = al * v.x, bz = be * v.y;
+          double2 na = c2(fma(az, a.x, -bz * pa.x), fma(az, a.y, -bz * pa.y));
+          if (DIP) {
+            const double ad = al * dv.x, bd = be * dv.y;
+            double2 nb2 = c2(fma(az, b.x, -bz * pb.x), fma(az, b.y, -bz * pb.y));
+            nb2 = c2(fma(ad, a.x, nb2.x), fma(ad, a.y, nb2.y));
+            nb2 = c2(fma(-bd, pa.x, nb2.x), fma(-bd, pa.y, nb2.y));
+            pb = b;
+            b = nb2;
+          }
+          pa = a;
+          a = na;
+          be += al;
+          al += 2.0;
+          if (t == m2) {             // the column m = m1 ends at n = p
+            a = s_s[m2 * SW + j];
+            pa = c2(0.0);
+            if (DIP) {
+              b = s_c[m2 * SW + j];
+              pb = c2(0.0);
+            }
+            al = 2.0 * m2 + 1.0;
+            be = 0.0;
+          }
+        }
+      }
+      __syncthreads();
+    }
+  }
+  // sum over the lane groups and warps (the start tables are free)
+  double2* red = smem2;              // [NW * SPW][ncf]
+  __syncthreads();
+  if (lane_on) {
+    double2* R = red + (size_t)(warp * SPW + grp) * ncf;
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      if (t > p + 1) break;
+      if (t <= m2) R[idx3(m1 + t, m1)] = acc[t];
+      else if (m2 != m1) R[idx3(t - 1, m2)] = acc[t];     // n = m2 + t - (m2 + 1)
+    }
+  }
+  __syncthreads();
+  double2* L = locals + ((size_t)tb * nrhs + r) * ncf;
+  for (int o = threadIdx.x; o < ncf; o += NT) {
+    double2 v = red[o];
+    for (int k = 1; k < NW * SPW; ++k) v = cadd(v, red[(size_t)k * ncf + o]);
+    L[o] = cadd(L[o], v);
+  }
+}
+
+// }}}
 
 // {{{ L2L (refine_locals, fmm.py:519-523), one launch per child level
 
@@ -1895,29 +1847,48 @@ cudaError_t launch_m2l(const qbxfmm_geometry& g, int p, int nrhs, const double2*
   return cudaGetLastError();
 }
 
-template <int DIM>
-static cudaError_t p2l_(const qbxfmm_geometry& g, SourceCoeffs sc, int p, int nrhs,
+template <int T, bool DIP>
+static cudaError_t p2l3_t(const qbxfmm_geometry& g, SourceCoeffs sc, int p, int nrhs,
+                          const double* s, double2* lo, int32_t* err, cudaStream_t st)
+{
+  const int ncf = (int)ncoef_dim(3, p);
+  const size_t start = (size_t)(DIP ? 2 : 1) * (p + 1) * (NT + 1);
+  const size_t red = (size_t)NW * (32 / (p / 2 + 1)) * ncf;
+  const size_t sh = std::max(start, red) * sizeof(double2);
+  cudaError_t e = cudaFuncSetAttribute(k_p2l3<T, DIP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sh);
+  if (e != cudaSuccess) return e;
+  k_p2l3<T, DIP><<<dim3(g.nttp_boxes, grid_y(nrhs)), NT, sh, st>>>(g, sc, p, ncf, nrhs, s, lo, err);
+  return cudaGetLastError();
+}
+
+template <bool DIP>
+static cudaError_t p2l3(const qbxfmm_geometry& g, SourceCoeffs sc, int p, int nrhs,
                         const double* s, double2* lo, int32_t* err, cudaStream_t st)
 {
-  if (g.nttp_boxes == 0) return cudaSuccess;
-  int ncf = (int)ncoef_dim(DIM, p);
-  int nct = DIM == 3 ? (p + 2) * (p + 3) / 2 : p + 3;
-  size_t sh = (size_t)P2L_TS * nct * sizeof(double2);
-  int nthr = (P2L3_SPLIT * ncf + 31) / 32 * 32;
-  if (DIM == 3 && nthr <= P2L3_MAXT) {
-    cudaFuncSetAttribute(k_p2l3s, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    k_p2l3s<<<dim3(g.nttp_boxes, grid_y(nrhs)), nthr, sh, st>>>(g, sc, p, ncf, nrhs, s, lo, err);
-    return cudaGetLastError();
-  }
-  cudaFuncSetAttribute(k_p2l<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-  k_p2l<DIM><<<dim3(g.nttp_boxes, grid_y(nrhs)), NT, sh, st>>>(g, sc, p, ncf, nrhs, s, lo, err);
+  // the accumulators' register count by order
+  if (p <= 6) return p2l3_t<8, DIP>(g, sc, p, nrhs, s, lo, err, st);
+  if (p <= 10) return p2l3_t<12, DIP>(g, sc, p, nrhs, s, lo, err, st);
+  if (p <= 13) return p2l3_t<15, DIP>(g, sc, p, nrhs, s, lo, err, st);
+  return p2l3_t<22, DIP>(g, sc, p, nrhs, s, lo, err, st);
+}
+
+static cudaError_t p2l2(const qbxfmm_geometry& g, SourceCoeffs sc, int p, int nrhs,
+                        const double* s, double2* lo, int32_t* err, cudaStream_t st)
+{
+  int ncf = (int)ncoef_dim(2, p);
+  size_t sh = (size_t)P2L_TS * (p + 3) * sizeof(double2);
+  k_p2l2<<<dim3(g.nttp_boxes, grid_y(nrhs)), NT, sh, st>>>(g, sc, p, ncf, nrhs, s, lo, err);
   return cudaGetLastError();
 }
 
 cudaError_t launch_p2l(const qbxfmm_geometry& g, SourceCoeffs sc, int p, int nrhs,
                        const double* s, double2* lo, int32_t* err, cudaStream_t st)
 {
-  return g.dim == 3 ? p2l_<3>(g, sc, p, nrhs, s, lo, err, st) : p2l_<2>(g, sc, p, nrhs, s, lo, err, st);
+  if (g.nttp_boxes == 0) return cudaSuccess;
+  if (g.dim == 2) return p2l2(g, sc, p, nrhs, s, lo, err, st);
+  return sc.cd != 0.0 ? p2l3<true>(g, sc, p, nrhs, s, lo, err, st)
+                      : p2l3<false>(g, sc, p, nrhs, s, lo, err, st);
 }
 
 template <int DIM>

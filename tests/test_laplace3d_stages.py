@@ -53,3 +53,13 @@ def test_target_specific_near_field(q, cq, cd):
     o.stage("form_global_qbx_locals", s, qe)
     o.stage("eval_qbx_expansions", qe, want)
     _close(got, want)
+
+
+@pytest.mark.parametrize("p", [1, 2, 5, 6, 7, 10, 11, 13, 14, 19, 20])
+@pytest.mark.parametrize("cq,cd", [(1.0, 0.0), (0.7, -1.3)])
+def test_form_locals(p, cq, cd):
+    w, o, s = _setup(2, p, cq, cd)
+    got = w.form_locals(None, None, None, None, None, [torch.from_numpy(s).cuda()])
+    want = o.zeros_box_exps()
+    o.stage("form_locals", s, want)
+    _close(got, want)

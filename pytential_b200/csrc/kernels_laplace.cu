@@ -1205,36 +1205,183 @@ k_p2qbxl(qbxfmm_geometry g, SourceCoeffs sc, int nrhs, const double* __restrict_
 }
 
 // M2QBXL (translate_box_multipoles_to_qbx_local, fmm.py:267-312;
-// interactions.py:196-235), all source levels in one launch.  A cluster of MZ CTAs
-// x 4 warps per chunk of <= 32 centers (lane = center); the MZ * 4 warps split the
-// list-3 boxes, and the partial sums meet in CTA 0 of the cluster in a fixed order
-// (warps through shared memory, CTAs through distributed shared memory), so the
-// result does not depend on scheduling.  Splitting a chunk over MZ CTAs evens out
-// chunks with long list-3 runs.
-// 3D: each warp expands the source multipole into a zero-padded dense table
-// Mpad[k][l] (rows k in [-Q, pf+Q], columns l in [-(pf+2Q), pf+Q]); each lane runs the
-// singular-harmonic recurrence for its center column by column and scatters every
-// S_{n'}^{m'} into its register-resident coefficients (j, i) through
-// Mpad[n'-j][m'-i]: one broadcast shared load and one complex FMA per term, no
-// branches.
-template <int DIM, int Q, int MZ>
+// interactions.py:196-235), all source levels in one launch.
+//
+// 3D, L_j^i(center) = (-rho_t)^j sum_nm M_n^m S_{n+j}^{m+i}(c - c_s), bound by the FP64
+// pipe.  With the columns -m' folded onto m' (S^{-m'} = (-1)^m' conj S^m'),
+//   L_j^i += T1_i[n][m'] Re S_{n+j}^{m'} + T2_i[n][m'] Im S_{n+j}^{m'},
+//   T1 = M_n^{m'-i} + s M_n^{-m'-i}, T2 = i (M_n^{m'-i} - s M_n^{-m'-i}), s = (-1)^m'
+// (m' = 0: T1 = M_n^{-i}, T2 = 0): four real multiply-adds per (n, m', j, i), for
+// m' <= n + Q only.  A CTA holds one chunk of <= 32 centers (lane = center); per list-3
+// box it builds the T tables in shared memory once, and its four warps
+// split the columns m' (dealt 0 1 2 3 3 2 1 0 ..: the long ones are the small m').  Down
+// a column a lane keeps the window S_n .. S_{n+Q} in registers, so the 2 (Q + 1) table
+// entries of (n, m') feed the 2 (Q + 1)(Q + 2) multiply-adds of all (j, i).  A cluster of
+// MZ CTAs splits the boxes of a chunk where there are too few chunks to fill the GPU
+// or to even out long list-3 runs; fixed-order sums (warps, then CTAs through
+// distributed shared memory).
+template <int Q, int MZ>
 __global__ void __launch_bounds__(NT)
-k_m2qbxl(qbxfmm_geometry g, int pf, int ncf, int nrhs, const double2* __restrict__ mpoles,
+k_m2qbxl3(qbxfmm_geometry g, int pf, int ncf, int nrhs, const double2* __restrict__ mpoles,
+          double2* __restrict__ qbx_exps, int32_t* err)
+{
+  constexpr int NC = (Q + 1) * (Q + 2) / 2;
+  extern __shared__ double2 smem2[];
+  const int NMP = pf + Q + 1;                          // columns m'
+  const int TSZ = NMP * (pf + 1) * (Q + 1) * 2;        // [m'][n][i]{T1, T2}
+  double2* Ms = smem2;                                 // [ncf] the box's multipole, rho_s^n
+  double2* T = Ms + ncf;                               // [TSZ]
+  double2* red = T;                                    // [NW][32][NC] after the last box
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int chunk = blockIdx.x / MZ, zpart = blockIdx.x - chunk * MZ;
+  const int r = blockIdx.y;
+  const int itb = g.qbx_chunk_target_box[chunk];
+  bool has_center = lane < g.qbx_chunk_count[chunk];
+  int ctr = has_center ? g.centers_by_target_box[g.qbx_chunk_start[chunk] + lane] : 0;
+  if ((unsigned)ctr >= (unsigned)g.ncenters) {
+    report(err, QBX_DEVERR_BAD_CENTER);
+    has_center = false;
+    ctr = 0;
+  }
+  double cc[3];
+  load_point<3>(g.centers, g.ncenters, ctr, cc);
+  double2 acc[NC];
+#pragma unroll
+  for (int i = 0; i < NC; ++i) acc[i] = c2(0.0);
+
+  const int l0 = g.list3_starts[itb], l1 = g.list3_starts[itb + 1];
+  for (int li = l0 + zpart; li < l1; li += MZ) {
+    const int sb = g.list3_lists[li];
+    if ((unsigned)sb >= (unsigned)g.nboxes) {
+      report(err, QBX_DEVERR_BAD_BOX);
+      continue;                                        // uniform over the CTA
+    }
+    const double2* src = mpoles + ((size_t)sb * nrhs + r) * ncf;
+    const double rho_s = level_width(g, g.box_levels[sb]);
+    // rows scaled by rho_s^n: the harmonics are taken at the unscaled offset
+    for (int q = threadIdx.x; q < ncf; q += NT) {
+      int n, m;
+      decode3(q, n, m);
+      double sc = 1.0;
+      for (int u = 0; u < n; ++u) sc *= rho_s;
+      Ms[q] = cscale(sc, src[q]);
+    }
+    __syncthreads();
+    for (int w = threadIdx.x; w < NMP * (pf + 1); w += NT) {
+      const int n = w % (pf + 1), mp = w / (pf + 1);
+      if (n < mp - Q) continue;                        // never read
+      double2* Tw = T + (size_t)w * (Q + 1) * 2;
+#pragma unroll
+      for (int i = 0; i <= Q; ++i) {
+        const double2 u = sh3_get(Ms, n, mp - i);
+        double2 t1 = u, t2 = c2(0.0);
+        if (mp > 0) {
+          double2 v = sh3_get(Ms, n, -mp - i);
+          if (mp & 1) v = c2(-v.x, -v.y);
+          t1 = cadd(u, v);
+          t2 = c2(v.y - u.y, u.x - v.x);
+        }
+        Tw[2 * i] = t1;
+        Tw[2 * i + 1] = t2;
+      }
+    }
+    __syncthreads();
+    if (!has_center) continue;
+    double cs[3];
+    load_point<3>(g.box_centers, g.nboxes, sb, cs);
+    const double d0 = cc[0] - cs[0], d1 = cc[1] - cs[1], d2 = cc[2] - cs[2];
+    const double rinv2 = 1.0 / (d0 * d0 + d1 * d1 + d2 * d2);
+    const double vz = d2 * rinv2;
+    const double2 X = c2(d0 * rinv2, d1 * rinv2);
+    double2 mm = c2(sqrt(rinv2));
+    for (int mp = 0; mp < NMP; ++mp) {
+      if (mp > 0) mm = cscale(2.0 * mp - 1.0, cmul(X, mm));
+      const int deal = mp & 7;
+      if ((deal < 4 ? deal : 7 - deal) != warp) continue;
+      double2 win[Q + 1];                              // S_n .. S_{n+Q}
+#pragma unroll
+      for (int j = 0; j <= Q; ++j) win[j] = c2(0.0);
+      win[Q] = mm;
+      double2 prev = c2(0.0);                          // S_{n+Q-1} once that exists
+      double al = 2.0 * mp + 1.0, be = 0.0;
+      const double2* Tn = T + (size_t)mp * (pf + 1) * (Q + 1) * 2 + (mp - Q) * (Q + 1) * 2;
+#pragma unroll (Q + 1)
+      for (int n = mp - Q; n <= pf; ++n) {
+        if (n >= 0) {
+#pragma unroll
+          for (int i = 0; i <= Q; ++i) {
+            const double2 t1 = Tn[2 * i], t2 = Tn[2 * i + 1];
+#pragma unroll
+            for (int j = i; j <= Q; ++j) {
+              double2& A = acc[idx3(j, i)];
+              A = caxpy(win[j].x, t1, A);
+              A = caxpy(win[j].y, t2, A);
+            }
+          }
+        }
+        Tn += (Q + 1) * 2;
+        const double az = al * vz, bz = be * rinv2;
+        const double2 top = win[Q];
+        const double2 nx = c2(fma(az, top.x, -bz * prev.x), fma(az, top.y, -bz * prev.y));
+        prev = top;
+        be += al;
+        al += 2.0;
+#pragma unroll
+        for (int j = 0; j < Q; ++j) win[j] = win[j + 1];
+        win[Q] = nx;
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < NC; ++i) red[((size_t)warp * NC + i) * 32 + lane] = acc[i];
+  __syncthreads();
+  // thread: coefficients tid / 32, tid / 32 + 4, .. of center lane, summed over the warps
+  // into the first warp's block
+  for (int i = warp; i < NC; i += NW) {
+    double2 v = red[(size_t)i * 32 + lane];
+    for (int w = 1; w < NW; ++w) v = cadd(v, red[((size_t)w * NC + i) * 32 + lane]);
+    red[(size_t)i * 32 + lane] = v;
+  }
+  if (MZ > 1) {
+    cg::cluster_group cl = cg::this_cluster();
+    cl.sync();
+    if (zpart == 0) {
+      for (int i = warp; i < NC; i += NW) {
+        double2 v = red[(size_t)i * 32 + lane];
+        for (unsigned z = 1; z < MZ; ++z) v = cadd(v, cl.map_shared_rank(red, z)[(size_t)i * 32 + lane]);
+        red[(size_t)i * 32 + lane] = v;
+      }
+    }
+    cl.sync();
+  }
+  if (zpart == 0 && has_center) {
+    const double rho_t = g.expansion_radii[ctr];
+    double2* out = qbx_exps + ((size_t)ctr * nrhs + r) * NC;
+    for (int i = warp; i < NC; i += NW) {              // the entries this thread summed
+      int j, ii;
+      decode3(i, j, ii);
+      double f = 1.0;
+      for (int u = 0; u < j; ++u) f *= -rho_t;
+      out[i] = caxpy(f, red[(size_t)i * 32 + lane], out[i]);
+    }
+  }
+}
+
+// 2D: CTA per chunk (lane = center), the warps split the list-3 boxes, each staging the
+// box's multipole in its own shared slice; fixed-order sum over the warps.
+template <int Q>
+__global__ void __launch_bounds__(NT)
+k_m2qbxl2(qbxfmm_geometry g, int pf, int ncf, int nrhs, const double2* __restrict__ mpoles,
          double2* __restrict__ qbx_exps, int32_t* err)
 {
-  constexpr int NC = (DIM == 3) ? (Q + 1) * (Q + 2) / 2 : Q + 1;
+  constexpr int NC = Q + 1;
   extern __shared__ double2 smem2[];
-  const int MW = 2 * pf + 3 * Q + 1;      // columns l + (pf + 2Q)
-  const int MR = pf + 2 * Q + 1;          // rows k + Q
-  const int MSZ = (DIM == 3) ? MR * MW : ncf;
-  const int loff = pf + 2 * Q;
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double2* Mw = smem2 + (size_t)warp * MSZ;
-  double2* red = smem2 + (size_t)NW * MSZ;   // [NW-1][32][NC]
-  double2* cpart = red + (NW - 1) * 32 * NC;  // [32][NC]: this CTA's sum (MZ > 1)
+  double2* Mw = smem2 + (size_t)warp * ncf;
+  double2* red = smem2 + (size_t)NW * ncf;   // [NW-1][32][NC]
 
-  int chunk = blockIdx.x / MZ;
-  int zpart = blockIdx.x - chunk * MZ;
+  int chunk = blockIdx.x;
   int r = blockIdx.y;
   int itb = g.qbx_chunk_target_box[chunk];
   bool has_center = lane < g.qbx_chunk_count[chunk];
@@ -1244,17 +1391,15 @@ k_m2qbxl(qbxfmm_geometry g, int pf, int ncf, int nrhs, const double2* __restrict
     has_center = false;
     ctr = 0;
   }
-  double cc[3] = {0, 0, 0};
-  load_point<DIM>(g.centers, g.ncenters, ctr, cc);
+  double cc[2];
+  load_point<2>(g.centers, g.ncenters, ctr, cc);
   double rho_t = g.expansion_radii[ctr];
-  if (DIM == 3)
-    for (int q = lane; q < MSZ; q += 32) Mw[q] = c2(0.0);
   double2 acc[NC];
 #pragma unroll
   for (int i = 0; i < NC; ++i) acc[i] = c2(0.0);
 
   int l0 = g.list3_starts[itb], l1 = g.list3_starts[itb + 1];
-  for (int li = l0 + zpart * NW + warp; li < l1; li += MZ * NW) {
+  for (int li = l0 + warp; li < l1; li += NW) {
     int sb = g.list3_lists[li];
     if ((unsigned)sb >= (unsigned)g.nboxes) {
       report(err, QBX_DEVERR_BAD_BOX);
@@ -1263,97 +1408,45 @@ k_m2qbxl(qbxfmm_geometry g, int pf, int ncf, int nrhs, const double2* __restrict
     __syncwarp();
     const double2* src = mpoles + ((size_t)sb * nrhs + r) * ncf;
     double rho_s = level_width(g, g.box_levels[sb]);
-    if (DIM == 3) {
-      // rows scaled by rho_s^k: with the harmonics taken at the unscaled offset
-      // c - c_s, the per-box factor rho_s^-(j+1) of the scaled form moves into the
-      // table and the boxes' terms add into acc directly
-      for (int q = lane; q < ncf; q += 32) {
-        int k, l;
-        decode3(q, k, l);
-        double sc = 1.0;
-        for (int u = 0; u < k; ++u) sc *= rho_s;
-        double2 v = cscale(sc, src[q]);
-        Mw[(k + Q) * MW + loff + l] = v;
-        if (l > 0) Mw[(k + Q) * MW + loff - l] = (l & 1) ? c2(-v.x, v.y) : c2(v.x, -v.y);
-      }
-    } else {
-      for (int q = lane; q < ncf; q += 32) Mw[q] = src[q];
-    }
+    for (int q = lane; q < ncf; q += 32) Mw[q] = src[q];
     __syncwarp();
     if (!has_center) continue;
-    double cs[3];
-    load_point<DIM>(g.box_centers, g.nboxes, sb, cs);
+    double cs[2];
+    load_point<2>(g.box_centers, g.nboxes, sb, cs);
     double ratio = rho_t / rho_s;
-    if (DIM == 3) {
-      double d0 = cc[0] - cs[0], d1 = cc[1] - cs[1], d2 = cc[2] - cs[2];
-      double rinv2 = 1.0 / (d0 * d0 + d1 * d1 + d2 * d2);
-      int nmax = pf + Q;
-      double2* part = acc;
-      double2 mm = c2(sqrt(rinv2));
-      for (int mp = 0; mp <= nmax; ++mp) {
-        if (mp > 0) mm = cscale((2.0 * mp - 1) * rinv2, cmul(mm, c2(d0, d1)));
-        double2 a = mm, prev = c2(0.0);
-        const double2* bpos = Mw + (mp + Q) * MW + loff + mp;   // row n'=mp, column m'
-        const double2* bneg = Mw + (mp + Q) * MW + loff - mp;   // column -m'
-        for (int np = mp; np <= nmax; ++np) {
-          if (np > mp) {
-            double2 bb = cscale(rinv2, csub(cscale((2.0 * np - 1) * d2, a),
-                                            cscale((double)(np + mp - 1) * (np - mp - 1), prev)));
-            prev = a;
-            a = bb;
-          }
+    const double2* M = Mw;
+    double2 tau = c2((cc[0] - cs[0]) / rho_s, (cc[1] - cs[1]) / rho_s);
+    double2 tinv = cinv(tau);
+    double2 t = c2(cc[0] - cs[0], cc[1] - cs[1]);
+    double2 s0 = cmul(M[0], clog_(t));
+    double2 sl[Q + 1];
+    double bin[Q + 1];
 #pragma unroll
-          for (int j = 0; j <= Q; ++j)
-#pragma unroll
-            for (int ii = 0; ii <= j; ++ii)
-              part[idx3(j, ii)] = cfma(bpos[-j * MW - ii], a, part[idx3(j, ii)]);
-          if (mp > 0) {
-            double2 aneg = (mp & 1) ? c2(-a.x, a.y) : c2(a.x, -a.y);
-#pragma unroll
-            for (int j = 0; j <= Q; ++j)
-#pragma unroll
-              for (int ii = 0; ii <= j; ++ii)
-                part[idx3(j, ii)] = cfma(bneg[-j * MW - ii], aneg, part[idx3(j, ii)]);
-          }
-          bpos += MW;
-          bneg += MW;
-        }
-      }
-    } else {
-      const double2* M = Mw;
-      double2 tau = c2((cc[0] - cs[0]) / rho_s, (cc[1] - cs[1]) / rho_s);
-      double2 tinv = cinv(tau);
-      double2 t = c2(cc[0] - cs[0], cc[1] - cs[1]);
-      double2 s0 = cmul(M[0], clog_(t));
-      double2 sl[Q + 1];
-      double bin[Q + 1];
-#pragma unroll
-      for (int l = 0; l <= Q; ++l) {
-        sl[l] = c2(0.0);
-        bin[l] = 1.0;
-      }
-      double2 pw = tinv;
-      for (int k = 1; k <= pf; ++k) {
-        double2 mk = cmul(M[k], pw);
-        s0 = cadd(s0, mk);
-#pragma unroll
-        for (int l = 1; l <= Q; ++l) {
-          sl[l] = caxpy(bin[l], mk, sl[l]);
-          bin[l] = bin[l] * (k + l) * rcp(k);
-        }
-        pw = cmul(pw, tinv);
-      }
-      acc[0] = cadd(acc[0], s0);
-      double2 tl = tinv;
-      double rl = ratio;
+    for (int l = 0; l <= Q; ++l) {
+      sl[l] = c2(0.0);
+      bin[l] = 1.0;
+    }
+    double2 pw = tinv;
+    for (int k = 1; k <= pf; ++k) {
+      double2 mk = cmul(M[k], pw);
+      s0 = cadd(s0, mk);
 #pragma unroll
       for (int l = 1; l <= Q; ++l) {
-        double2 v = cscale(((l & 1) ? 1.0 : -1.0) * rcp(l), M[0]);
-        v = cadd(v, cscale((l & 1) ? -1.0 : 1.0, sl[l]));
-        acc[l] = cadd(acc[l], cscale(rl, cmul(v, tl)));
-        tl = cmul(tl, tinv);
-        rl *= ratio;
+        sl[l] = caxpy(bin[l], mk, sl[l]);
+        bin[l] = bin[l] * (k + l) * rcp(k);
       }
+      pw = cmul(pw, tinv);
+    }
+    acc[0] = cadd(acc[0], s0);
+    double2 tl = tinv;
+    double rl = ratio;
+#pragma unroll
+    for (int l = 1; l <= Q; ++l) {
+      double2 v = cscale(((l & 1) ? 1.0 : -1.0) * rcp(l), M[0]);
+      v = cadd(v, cscale((l & 1) ? -1.0 : 1.0, sl[l]));
+      acc[l] = cadd(acc[l], cscale(rl, cmul(v, tl)));
+      tl = cmul(tl, tinv);
+      rl *= ratio;
     }
   }
   __syncthreads();
@@ -1367,34 +1460,8 @@ k_m2qbxl(qbxfmm_geometry g, int pf, int ncf, int nrhs, const double2* __restrict
     for (int i = 0; i < NC; ++i)
       for (int w = 1; w < NW; ++w) acc[i] = cadd(acc[i], red[((w - 1) * 32 + lane) * NC + i]);
   }
-  if (MZ > 1) {
-    cg::cluster_group cl = cg::this_cluster();
-    if (warp == 0) {
-#pragma unroll
-      for (int i = 0; i < NC; ++i) cpart[lane * NC + i] = acc[i];
-    }
-    cl.sync();
-    if (zpart == 0 && warp == 0) {
-      for (unsigned q = 1; q < MZ; ++q) {
-        const double2* rp = cl.map_shared_rank(cpart, q) + lane * NC;
-#pragma unroll
-        for (int i = 0; i < NC; ++i) acc[i] = cadd(acc[i], rp[i]);
-      }
-    }
-    cl.sync();
-  }
-  if (zpart == 0 && warp == 0 && has_center) {
+  if (warp == 0 && has_center) {
     double2* out = qbx_exps + ((size_t)ctr * nrhs + r) * NC;
-    if (DIM == 3) {
-      // (-1)^j rho_t^j of the local coefficient of order j
-      double f = 1.0;
-#pragma unroll
-      for (int j = 0; j <= Q; ++j) {
-#pragma unroll
-        for (int ii = 0; ii <= j; ++ii) acc[idx3(j, ii)] = cscale(f, acc[idx3(j, ii)]);
-        f *= -rho_t;
-      }
-    }
 #pragma unroll
     for (int i = 0; i < NC; ++i) out[i] = cadd(out[i], acc[i]);
   }
@@ -1967,26 +2034,20 @@ static cudaError_t p2qbxl_q(const qbxfmm_geometry& g, SourceCoeffs sc, int nrhs,
   return cudaGetLastError();
 }
 
-// CTAs per chunk in the 3D M2QBXL cluster launch
-constexpr int M2QBXL_Z = 4;
+// clusters of 4 CTAs per chunk below this many chunks (boxes of a chunk dealt round-robin)
+constexpr int M2QBXL_SPLIT_BELOW = 4096;
 
-template <int DIM, int Q>
-static cudaError_t m2qbxl_q(const qbxfmm_geometry& g, int pf, int nrhs, const double2* mp,
-                            double2* qe, int32_t* err, cudaStream_t st)
+template <int Q, int MZ>
+static cudaError_t m2qbxl3_launch(const qbxfmm_geometry& g, int pf, int nrhs, const double2* mp,
+                                  double2* qe, int32_t* err, cudaStream_t st)
 {
-  int ncf = (int)ncoef_dim(DIM, pf);
-  constexpr int NC = (DIM == 3) ? (Q + 1) * (Q + 2) / 2 : Q + 1;
-  size_t msz = DIM == 3 ? (size_t)(pf + 2 * Q + 1) * (2 * pf + 3 * Q + 1) : (size_t)ncf;
-  size_t sh = (NW * msz + (size_t)NW * 32 * NC) * sizeof(double2);
-  if constexpr (DIM == 2) {
-    cudaFuncSetAttribute(k_m2qbxl<DIM, Q, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    k_m2qbxl<DIM, Q, 1><<<dim3(g.nqbx_chunks, grid_y(nrhs)), NT, sh, st>>>(g, pf, ncf, nrhs, mp, qe,
-                                                                          err);
-    return cudaGetLastError();
-  } else {
-  // 3D: clusters of M2QBXL_Z CTAs per chunk
-  constexpr int MZ = M2QBXL_Z;
-  cudaFuncSetAttribute(k_m2qbxl<DIM, Q, MZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+  const int ncf = (int)ncoef_dim(3, pf);
+  const size_t tab = (size_t)(pf + Q + 1) * (pf + 1) * (Q + 1) * 2;
+  const size_t red = (size_t)NW * 32 * (Q + 1) * (Q + 2) / 2;
+  const size_t sh = (ncf + std::max(tab, red)) * sizeof(double2);
+  cudaError_t e = cudaFuncSetAttribute(k_m2qbxl3<Q, MZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sh);
+  if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(g.nqbx_chunks * MZ, grid_y(nrhs));
   cfg.blockDim = dim3(NT);
@@ -1999,7 +2060,22 @@ static cudaError_t m2qbxl_q(const qbxfmm_geometry& g, int pf, int nrhs, const do
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_m2qbxl<DIM, Q, MZ>, g, pf, ncf, nrhs, mp, qe, err);
+  return cudaLaunchKernelEx(&cfg, k_m2qbxl3<Q, MZ>, g, pf, ncf, nrhs, mp, qe, err);
+}
+
+template <int DIM, int Q>
+static cudaError_t m2qbxl_q(const qbxfmm_geometry& g, int pf, int nrhs, const double2* mp,
+                            double2* qe, int32_t* err, cudaStream_t st)
+{
+  if constexpr (DIM == 2) {
+    const int ncf = (int)ncoef_dim(2, pf);
+    const size_t sh = (NW * (size_t)ncf + (size_t)NW * 32 * (Q + 1)) * sizeof(double2);
+    cudaFuncSetAttribute(k_m2qbxl2<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+    k_m2qbxl2<Q><<<dim3(g.nqbx_chunks, grid_y(nrhs)), NT, sh, st>>>(g, pf, ncf, nrhs, mp, qe, err);
+    return cudaGetLastError();
+  } else {
+    if (g.nqbx_chunks < M2QBXL_SPLIT_BELOW) return m2qbxl3_launch<Q, 4>(g, pf, nrhs, mp, qe, err, st);
+    return m2qbxl3_launch<Q, 1>(g, pf, nrhs, mp, qe, err, st);
   }
 }
 

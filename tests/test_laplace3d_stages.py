@@ -63,3 +63,16 @@ def test_form_locals(p, cq, cd):
     want = o.zeros_box_exps()
     o.stage("form_locals", s, want)
     _close(got, want)
+
+
+@pytest.mark.parametrize("q,p", [(0, 1), (0, 20), (1, 7), (2, 2), (3, 10), (4, 12), (5, 3),
+                                 (6, 15), (7, 5), (8, 20)])
+def test_multipoles_to_qbx_locals(q, p):
+    w, o, s = _setup(q, p, 1.0, 0.5, nrhs=2)
+    mp = o.zeros_box_exps()
+    o.stage("form_multipoles", s, mp)
+    o.stage("coarsen_multipoles", mp)
+    got = w.translate_box_multipoles_to_qbx_local(None, torch.from_numpy(mp).cuda())
+    want = o.zeros_qbx_exps()
+    o.stage("translate_box_multipoles_to_qbx_local", mp, want)
+    _close(got, want)

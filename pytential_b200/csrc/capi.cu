@@ -126,9 +126,11 @@ void h3_layout(const qbxfmm_plan* p, size_t o[8])
   o[0] = p->tc.nmatrices * p->tc.rp * p->tc.kp;
   o[1] = o[0] + p->h3gaunt.size();
   o[2] = (o[1] + p->h3rot.size() + 1) & ~(size_t)1;
-  o[3] = (o[2] + p->h3m2l.size() + 1) & ~(size_t)1;    // 16-byte aligned for bulk copies
-  o[4] = o[3] + (size_t)p->h3_ndir * h3_m2l_dsize(p->kern.fmm_order);
-  o[5] = (o[4] + 2 * (size_t)p->h3_ncoax * h3_m2l_csize(p->kern.fmm_order) + 1) & ~(size_t)1;
+  o[3] = (o[2] + p->h3m2l.size() + 1) & ~(size_t)1;    // 16-byte aligned for the copies
+  const int pf = p->kern.fmm_order;
+  o[4] = o[3] + (size_t)p->h3_ndir * (p->mixed ? h3_m2l_dsize(pf) : h3_m2l_mma_dsize(pf));
+  o[5] = (o[4] + (size_t)p->h3_ncoax * (p->mixed ? 2 * h3_m2l_csize(pf) : h3_m2l_mma_csize(pf)) +
+          1) & ~(size_t)1;
   o[6] = o[5] + 2 * p->h3tp.G0.size();
   o[7] = o[6] + 2 * p->h3tq.Ginv.size();
 }
@@ -690,11 +692,17 @@ int qbxfmm_multipole_to_local(const qbxfmm_plan* p, const void* mpoles, void* lo
     const int nm = 2 * p->kern.fmm_order + 1;
     const double* clsmap = p->trans_dev + o[2] + (size_t)nm * nm * 4 + 4 * (size_t)p->h3_ndir +
                            2 * (size_t)p->h3_ncoax;
-    QBX_TRY(h3_launch_m2l_rot(p->geo, p->kern.fmm_order, p->kern.nrhs, (const double2*)mpoles,
-                              (double2*)locals, p->trans_dev + o[3],
-                              reinterpret_cast<const double2*>(p->trans_dev + o[4]), clsmap,
-                              error_word, S(stream), p->mixed, p->hc.rb_m2l),
-            "multipole_to_local");
+    if (p->mixed)
+      QBX_TRY(h3_launch_m2l_rot_f32(p->geo, p->kern.fmm_order, p->kern.nrhs, (const double2*)mpoles,
+                                    (double2*)locals, p->trans_dev + o[3],
+                                    reinterpret_cast<const double2*>(p->trans_dev + o[4]), clsmap,
+                                    error_word, S(stream), p->hc.rb_m2l),
+              "multipole_to_local");
+    else
+      QBX_TRY(h3_launch_m2l_mma(p->geo, p->kern.fmm_order, p->kern.nrhs, (const double2*)mpoles,
+                                (double2*)locals, p->trans_dev + o[3], p->trans_dev + o[4], clsmap,
+                                error_word, S(stream), p->hc.rb_m2l),
+              "multipole_to_local");
     return mask_all_levels(p, locals, S(stream));
   }
   if (p->helm)
@@ -1126,9 +1134,14 @@ int qbxfmm_precompute_translations(const qbxfmm_plan* p, const qbxfmm_workspace*
     const double* rt = isq + (size_t)(pf + 2) * (pf + 1);
     const double* dirs = H + (size_t)nm * nm * 4;
     const double* coaxp = dirs + 4 * (size_t)p->h3_ndir;
-    QBX_TRY(h3_launch_m2l_tables(pf, p->h3_ndir, p->h3_ncoax, dirs, coaxp, H, isq, rt, G, T + o[3],
-                                 reinterpret_cast<double2*>(T + o[4]), S(stream)),
-            "precompute_translations: M2L tables");
+    if (p->mixed)
+      QBX_TRY(h3_launch_m2l_tables(pf, p->h3_ndir, p->h3_ncoax, dirs, coaxp, H, isq, rt, G, T + o[3],
+                                   reinterpret_cast<double2*>(T + o[4]), S(stream)),
+              "precompute_translations: M2L tables");
+    else
+      QBX_TRY(h3_launch_m2l_mma_tables(pf, p->h3_ndir, p->h3_ncoax, dirs, coaxp, H, isq, rt, G,
+                                       T + o[3], T + o[4], S(stream)),
+              "precompute_translations: M2L tables");
     p->trans_dev = T;
     p->scratch_dev = (double*)ws->pair_scratch;
     return QBXFMM_OK;

@@ -130,6 +130,17 @@ QBX_D void h3_sph_h(int N, double x, double2* hv)
 
 QBX_D double h3_scale(double k, double rho) { return fmin(1.0, k * rho); }
 
+// i^e for integer e
+QBX_D double2 ipow(int e)
+{
+  switch (e & 3) {
+    case 0: return c2(1.0, 0.0);
+    case 1: return c2(0.0, 1.0);
+    case 2: return c2(-1.0, 0.0);
+    default: return c2(0.0, -1.0);
+  }
+}
+
 // D (8x8, two per lane: row lane/4, columns 2 (lane%4) + {0,1}) += A (8x4, row major,
 // element (lane/4, lane%4)) B (4x8, column major, element (lane%4, lane/4)), FP64
 QBX_D void h3_dmma(double& d0, double& d1, double a, double b)

@@ -172,20 +172,29 @@ cudaError_t h3_launch_eval_locals(const qbxfmm_geometry& g, HelmCoeffs hc, int p
                                   const double2* lo, double2* pot, cudaStream_t st);
 cudaError_t h3_launch_p2qbxl(const qbxfmm_geometry& g, HelmCoeffs hc, int q, int nrhs,
                              const double2* s, double2* qe, int32_t* err, cudaStream_t st);
-// 3D Helmholtz M2L by rotation: per-direction rotation tables (Dtab, h3_m2l_dsize
-// doubles each) and per-(length, level) coaxial tables (Ctab, h3_m2l_csize complex
-// each) built by h3_launch_m2l_tables; clsmap[2 c] / [2 c + 1] = direction / coaxial
-// table of M2L class c.
+// 3D Helmholtz M2L by rotation: per-direction rotation tables (Dtab) and per-(length,
+// level) coaxial tables (Ctab); clsmap[2 c] / [2 c + 1] = direction / coaxial table of M2L
+// class c.  FP64: h3_m2l_mma_dsize / _csize doubles each, tensor-core products of
+// rb densities per CTA (0: by their number).
+size_t h3_m2l_mma_dsize(int p);
+size_t h3_m2l_mma_csize(int p);
+cudaError_t h3_launch_m2l_mma_tables(int pf, int ndir, int ncoax, const double* dirs,
+                                     const double* coaxp, const double* start, const double* isq,
+                                     const double* rt, const double* gaunt, double* Dtab,
+                                     double* Ctab, cudaStream_t st);
+cudaError_t h3_launch_m2l_mma(const qbxfmm_geometry& g, int p, int nrhs, const double2* mp,
+                              double2* lo, const double* Dtab, const double* Ctab,
+                              const double* clsmap, int32_t* err, cudaStream_t st, int rb);
+// FP32 arithmetic (the mixed form): h3_m2l_dsize doubles and h3_m2l_csize complex each
 __host__ __device__ size_t h3_m2l_dsize(int pf);
 __host__ __device__ size_t h3_m2l_csize(int pf);
 cudaError_t h3_launch_m2l_tables(int pf, int ndir, int ncoax, const double* dirs,
                                  const double* coaxp, const double* start, const double* isq,
                                  const double* rt, const double* gaunt, double* Dtab,
                                  double2* Ctab, cudaStream_t st);
-cudaError_t h3_launch_m2l_rot(const qbxfmm_geometry& g, int pf, int nrhs, const double2* mp,
-                              double2* lo, const double* Dtab, const double2* Ctab,
-                              const double* clsmap, int32_t* err, cudaStream_t st,
-                              bool fp32 = false, int rb = 0);
+cudaError_t h3_launch_m2l_rot_f32(const qbxfmm_geometry& g, int pf, int nrhs, const double2* mp,
+                                  double2* lo, const double* Dtab, const double2* Ctab,
+                                  const double* clsmap, int32_t* err, cudaStream_t st, int rb);
 // rot: rotation tables of h3_rotation_tables (start values, recurrence factors,
 // lambda = 0 Gaunt slice)
 // fp32: the mixed-precision form (FP32 arithmetic, FP64 expansions in and out)

@@ -103,17 +103,6 @@ QBX_D void h3_wave_column(int m, int N, double t, double2 w, const double2* rec,
   }
 }
 
-// i^e for integer e
-QBX_D double2 ipow(int e)
-{
-  switch (e & 3) {
-    case 0: return c2(1.0, 0.0);
-    case 1: return c2(0.0, 1.0);
-    case 2: return c2(-1.0, 0.0);
-    default: return c2(0.0, -1.0);
-  }
-}
-
 // list helpers (as in the Laplace kernels)
 QBX_D void h3_list_prefix(const qbxfmm_geometry& g, const int32_t* __restrict__ lists, int gb,
                           int nb, int* s_pref, int* s_start, int32_t* err)
@@ -2004,336 +1993,6 @@ k_h3_m2l_rot(qbxfmm_geometry g, int pf, int nrhs, const double2* __restrict__ mp
   }
 }
 
-// {{{ M2L with the pair tables brought in by bulk copies
-
-QBX_D unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-QBX_D void mbar_init(uint64_t* mb)
-{
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_addr(mb)) : "memory");
-}
-
-// one arrival that also expects `bytes` of copy completion on the barrier
-QBX_D void mbar_expect(uint64_t* mb, unsigned bytes)
-{
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n"
-               ::"r"(smem_addr(mb)), "r"(bytes) : "memory");
-}
-
-// global -> this CTA's shared memory, completion counted on mb (16-byte aligned
-// addresses, size a multiple of 16)
-QBX_D void bulk_copy(void* dst, const void* src, unsigned bytes, uint64_t* mb)
-{
-  asm volatile("fence.proxy.async.shared::cta;\n"
-               "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
-               ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(mb)) : "memory");
-}
-
-// bounded wait for the phase of the given parity; false if it did not complete
-QBX_D bool mbar_wait(uint64_t* mb, unsigned parity)
-{
-  for (int it = 0; it < (1 << 22); ++it) {
-    unsigned done;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                 " selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(done) : "r"(smem_addr(mb)), "r"(parity) : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-
-// The FP64 M2L of k_h3_m2l_rot with its pair tables brought in by bulk copies
-// (cp.async.bulk, completion on an mbarrier) into buffers of their own: the rotation
-// table once per pair (the register-staged form copies it twice, before the rotation
-// and again before the back rotation, because it shares one buffer with the coaxial
-// table) and the coaxial table of pair q + 1 while pair q's back rotation runs.  One
-// thread issues the copies; waits are bounded: a copy that does not arrive sets the
-// error word, the CTA waits (bounded) for the copies it issued and stops.  With ND = 2
-// the rotation table has two buffers: pair q + 1's is requested as soon as pair q's
-// has arrived (into the buffer pair q - 1 used), so its copy runs under all of pair
-// q's work instead of between the pairs.
-template <int RB, int NTHR = H3M2L_NT, int ND = 1>
-__global__ void __launch_bounds__(NTHR, NTHR == H3M2L_NT ? 2 : 1)
-k_h3_m2l_bulk(qbxfmm_geometry g, int pf, int nrhs, const double2* __restrict__ mp,
-              double2* __restrict__ lo, const double* __restrict__ Dtab,
-              const double2* __restrict__ Ctab, const double* __restrict__ clsmap,
-              int32_t* err)
-{
-  static_assert(ND == 1 || ND == 2, "one or two rotation-table buffers");
-  extern __shared__ double2 smem2[];
-  __shared__ uint64_t mbD[ND], mbC;
-  __shared__ int s_gn[H3M2L_NG], s_gm0[H3M2L_NG];
-  __shared__ int s_cmu[H3M2L_NCG], s_cnu0[H3M2L_NCG];
-  __shared__ int s_ng, s_ncg;
-  __shared__ unsigned char s_nof[(H3_MAXP + 1) * (H3_MAXP + 1)];
-  constexpr int KMAX = (H3M2L_NG * RB + NTHR - 1) / NTHR;
-  const int ncf = (pf + 1) * (pf + 1), XS = ncf + 1, nm = 2 * pf + 1;
-  const size_t dsz = h3_m2l_dsize(pf), csz = h3_m2l_csize(pf);
-  double2* X = smem2;                                              // [RB][ncf + 1]
-  double2* A = X + (size_t)RB * XS;                                // [RB][ncf + 1]
-  double* Db0 = reinterpret_cast<double*>(A + (size_t)RB * XS);    // [ND][dsz]
-  double2* Cb = reinterpret_cast<double2*>(Db0 + ND * dsz);         // [csz]
-  if (threadIdx.x == 0) {
-    int ng = 0;
-    for (int n = 0; n <= pf; ++n)
-      for (int m0 = -n; m0 <= n; m0 += 4) {
-        s_gn[ng] = n;
-        s_gm0[ng] = m0;
-        ++ng;
-      }
-    s_ng = ng;
-    int ncg = 0;
-    for (int mu = -pf; mu <= pf; ++mu)
-      for (int nu0 = abs(mu); nu0 <= pf; nu0 += 4) {
-        s_cmu[ncg] = mu;
-        s_cnu0[ncg] = nu0;
-        ++ncg;
-      }
-    s_ncg = ncg;
-    for (int b = 0; b < ND; ++b) mbar_init(&mbD[b]);
-    mbar_init(&mbC);
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  for (int n = 0; n <= pf; ++n)
-    for (int x = n * n + threadIdx.x; x < (n + 1) * (n + 1); x += NTHR) s_nof[x] = (unsigned char)n;
-  __syncthreads();
-  const int i = blockIdx.x;
-  const int r0 = blockIdx.y * RB;
-  const int q0 = g.m2l_tgt_pair_starts[i], q1 = g.m2l_tgt_pair_starts[i + 1];
-  if (q1 <= q0) return;                    // before any copy is issued
-  const int ng = s_ng, ncg = s_ncg;
-  const unsigned dbytes = (unsigned)(dsz * sizeof(double)), cbytes = (unsigned)(csz * sizeof(double2));
-  auto cls_of = [&](int q) {
-    const int pr = g.m2l_tgt_pairs[q];
-    int lo_c = 0, hi_c = g.m2l_nclasses - 1;
-    while (lo_c < hi_c) {
-      const int mid = (lo_c + hi_c + 1) >> 1;
-      if (g.m2l_class_starts[mid] <= pr) lo_c = mid;
-      else hi_c = mid - 1;
-    }
-    return lo_c;
-  };
-  // copies issued / completed-and-waited per barrier (the phase parity of the next
-  // wait is the completed count's)
-  int nd_issued[ND], nd_done[ND], nc_issued = 0, nc_done = 0;
-#pragma unroll
-  for (int b = 0; b < ND; ++b) nd_issued[b] = nd_done[b] = 0;
-  auto issue_D = [&](int q, int b) {
-    if (threadIdx.x == 0) {
-      const int c = cls_of(q);
-      mbar_expect(&mbD[b], dbytes);
-      bulk_copy(Db0 + b * dsz, Dtab + (size_t)clsmap[2 * c] * dsz, dbytes, &mbD[b]);
-    }
-    ++nd_issued[b];
-  };
-  auto issue_C = [&](int q) {
-    if (threadIdx.x == 0) {
-      const int c = cls_of(q);
-      mbar_expect(&mbC, cbytes);
-      bulk_copy(Cb, Ctab + (size_t)clsmap[2 * c + 1] * csz, cbytes, &mbC);
-    }
-    ++nc_issued;
-  };
-  auto wait_D = [&](int b) {
-    if (!mbar_wait(&mbD[b], nd_done[b] & 1)) return 1;
-    ++nd_done[b];
-    return 0;
-  };
-  auto wait_C = [&]() {
-    if (!mbar_wait(&mbC, nc_done & 1)) return 1;
-    ++nc_done;
-    return 0;
-  };
-  // after a copy that did not arrive: report, then wait (bounded) for the copies
-  // still in flight so that none outlives the CTA
-  auto drain = [&]() {
-    if (threadIdx.x == 0) report(err, QBX_DEVERR_COPY_TIMEOUT);
-#pragma unroll
-    for (int b = 0; b < ND; ++b)
-      for (; nd_done[b] < nd_issued[b]; ++nd_done[b]) mbar_wait(&mbD[b], nd_done[b] & 1);
-    for (; nc_done < nc_issued; ++nc_done) mbar_wait(&mbC, nc_done & 1);
-  };
-
-  double2 acc[KMAX][4];
-#pragma unroll
-  for (int k = 0; k < KMAX; ++k)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[k][j] = c2(0.0);
-
-  issue_D(q0, 0);
-  issue_C(q0);
-  for (int q = q0; q < q1; ++q) {
-    const int buf = ND == 2 ? ((q - q0) & 1) : 0;
-    const double* Db = Db0 + buf * dsz;
-    const int src = g.m2l_pair_src[g.m2l_tgt_pairs[q]];
-    const bool bad = (unsigned)src >= (unsigned)g.nboxes;
-    if (bad && threadIdx.x == 0) report(err, QBX_DEVERR_BAD_BOX);
-    int fail = wait_D(buf);
-    // the other buffer was last read by pair q - 1, before the barrier that ended it
-    if (ND == 2 && q + 1 < q1) issue_D(q + 1, buf ^ 1);
-    const double2* ph = reinterpret_cast<const double2*>(Db);
-    const double* blocks = Db + 2 * nm;
-    // X = e^{i m alpha} M
-    for (int e = threadIdx.x; e < RB * ncf; e += NTHR) {
-      const int r = e / ncf, ci = e - r * ncf;
-      const int n = s_nof[ci];
-      double2 v = c2(0.0);
-      if (!fail && !bad && r0 + r < nrhs)
-        v = cmul(ph[ci - n * n - n + pf], mp[((size_t)src * nrhs + r0 + r) * ncf + ci]);
-      X[r * XS + ci] = v;
-    }
-    if (__syncthreads_or(fail)) {
-      drain();
-      return;
-    }
-    // A[(n, mu)] = sum_m T^n[m][mu] X[(n, m)]
-    for (int t = threadIdx.x; t < ng * RB; t += NTHR) {
-      const int grp = t / RB, r = t - grp * RB;
-      const int n = s_gn[grp], mu0 = s_gm0[grp];
-      const double* Tn = blocks + h3_dblock(n);
-      const int w = 2 * n + 1, nv = min(4, n - mu0 + 1);
-      double2 o[4] = {c2(0.0), c2(0.0), c2(0.0), c2(0.0)};
-      const double2* Xr = X + r * XS + n * n;
-      for (int m = 0; m < w; ++m) {
-        const double2 x = Xr[m];
-        const int ma = m - n;
-        const double* row = ma >= 0 ? Tn + ma * w + (mu0 + n) : Tn + (-ma) * w + (n - mu0);
-        const int step = ma >= 0 ? 1 : -1;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (j < nv) o[j] = caxpy(row[step * j], x, o[j]);
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (j < nv) A[r * XS + n * n + n + mu0 + j] = o[j];
-    }
-    fail = wait_C();
-    if (__syncthreads_or(fail)) {
-      drain();
-      return;
-    }
-    // B[(nu, mu)] = sum_{n >= |mu|} C^mu[n][nu] A[(n, mu)]   (into X)
-    for (int t = threadIdx.x; t < ncg * RB; t += NTHR) {
-      const int grp = t / RB, r = t - grp * RB;
-      const int mu = s_cmu[grp], nu0 = s_cnu0[grp];
-      const int am = abs(mu), w = pf + 1 - am, nv = min(4, pf - nu0 + 1);
-      const double2* Cq = Cb + h3_cblock(pf, am) + (nu0 - am);
-      double2 o[4] = {c2(0.0), c2(0.0), c2(0.0), c2(0.0)};
-      const double2* Ar = A + r * XS;
-      for (int n = am; n <= pf; ++n) {
-        const double2 a = Ar[n * n + n + mu];
-        const double2* row = Cq + (n - am) * w;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (j < nv) o[j] = cfma(row[j], a, o[j]);
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int nu = nu0 + j;
-        if (j < nv) X[r * XS + nu * nu + nu + mu] = o[j];
-      }
-    }
-    __syncthreads();
-    // the coaxial buffer is free: the next pair's table lands during the back rotation
-    if (q + 1 < q1) issue_C(q + 1);
-    // L[(nu, m2)] += e^{-i m2 alpha} sum_mu T^nu[m2][mu] B[(nu, mu)]
-#pragma unroll
-    for (int k = 0; k < KMAX; ++k) {
-      const int t = threadIdx.x + k * NTHR;
-      if (t >= ng * RB) break;
-      const int grp = t / RB, r = t - grp * RB;
-      const int nu = s_gn[grp], m20 = s_gm0[grp];
-      const int w = 2 * nu + 1, nv = min(4, nu - m20 + 1);
-      const double* Tn = blocks + h3_dblock(nu);
-      const double* pj[4];
-      int sj[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int m2 = m20 + j;
-        pj[j] = m2 >= 0 ? Tn + m2 * w : Tn + (-m2) * w + 2 * nu;
-        sj[j] = m2 >= 0 ? 1 : -1;
-      }
-      double2 o[4] = {c2(0.0), c2(0.0), c2(0.0), c2(0.0)};
-      const double2* Br = X + r * XS + nu * nu;
-      for (int mu = 0; mu < w; ++mu) {
-        const double2 bb = Br[mu];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (j < nv) o[j] = caxpy(pj[j][sj[j] * mu], bb, o[j]);
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (j < nv) acc[k][j] = cfma(cconj(ph[m20 + j + pf]), o[j], acc[k][j]);
-    }
-    __syncthreads();
-    // the rotation buffer is free
-    if (ND == 1 && q + 1 < q1) issue_D(q + 1, 0);
-  }
-  const int tb = g.target_or_target_parent_boxes[i];
-  if ((unsigned)tb >= (unsigned)g.nboxes) {
-    if (threadIdx.x == 0) report(err, QBX_DEVERR_BAD_BOX);
-    return;
-  }
-#pragma unroll
-  for (int k = 0; k < KMAX; ++k) {
-    const int t = threadIdx.x + k * NTHR;
-    if (t >= ng * RB) break;
-    const int grp = t / RB, r = t - grp * RB;
-    if (r0 + r >= nrhs) continue;
-    const int nu = s_gn[grp], m20 = s_gm0[grp];
-    const int nv = min(4, nu - m20 + 1);
-    double2* out = lo + ((size_t)tb * nrhs + r0 + r) * ncf + nu * nu + nu + m20;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (j < nv) out[j] = cadd(out[j], acc[k][j]);
-  }
-}
-
-// }}}
-
-// dynamic shared memory of k_h3_m2l_bulk: the X and A blocks, nd rotation tables,
-// the coaxial table
-static size_t h3_m2l_bulk_smem(int rb, int pf, int nd)
-{
-  return 2 * (size_t)rb * ((pf + 1) * (pf + 1) + 1) * sizeof(double2) +
-         nd * h3_m2l_dsize(pf) * sizeof(double) + h3_m2l_csize(pf) * sizeof(double2);
-}
-
-// dynamic shared memory a CTA may use beside the kernels' static arrays (227 KB less
-// a margin for them)
-constexpr size_t H3M2L_SMEM_MAX = 227 * 1024 - 4 * 1024;
-
-template <int RB, int NTHR = H3M2L_NT, int ND = 1>
-static cudaError_t h3_m2l_bulk_launch(const qbxfmm_geometry& g, int pf, int nrhs, const double2* mp,
-                                      double2* lo, const double* Dtab, const double2* Ctab,
-                                      const double* clsmap, int32_t* err, cudaStream_t st)
-{
-  // bulk copies need 16-byte aligned tables
-  if ((reinterpret_cast<uintptr_t>(Dtab) | reinterpret_cast<uintptr_t>(Ctab)) & 15)
-    return cudaErrorInvalidValue;
-  const size_t sh = h3_m2l_bulk_smem(RB, pf, ND);
-  if (sh > H3M2L_SMEM_MAX) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(k_h3_m2l_bulk<RB, NTHR, ND>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-  if (e != cudaSuccess) return e;
-  dim3 grid(g.nttp_boxes, (nrhs + RB - 1) / RB);
-  k_h3_m2l_bulk<RB, NTHR, ND><<<grid, NTHR, sh, st>>>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err);
-  return cudaGetLastError();
-}
-
-// 16 densities per CTA (512 threads, one CTA per SM): two rotation-table buffers where
-// they fit, else one, else 8 densities per CTA
-static cudaError_t h3_m2l_bulk16(const qbxfmm_geometry& g, int pf, int nrhs, const double2* mp,
-                                 double2* lo, const double* Dtab, const double2* Ctab,
-                                 const double* clsmap, int32_t* err, cudaStream_t st)
-{
-  if (h3_m2l_bulk_smem(16, pf, 2) <= H3M2L_SMEM_MAX)
-    return h3_m2l_bulk_launch<16, 2 * H3M2L_NT, 2>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-  if (h3_m2l_bulk_smem(16, pf, 1) <= H3M2L_SMEM_MAX)
-    return h3_m2l_bulk_launch<16, 2 * H3M2L_NT, 1>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-  return h3_m2l_bulk_launch<8>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-}
-
 template <typename R, int RB>
 static cudaError_t h3_m2l_rot_launch(const qbxfmm_geometry& g, int pf, int nrhs, const double2* mp,
                                      double2* lo, const double* Dtab, const double2* Ctab,
@@ -2348,39 +2007,23 @@ static cudaError_t h3_m2l_rot_launch(const qbxfmm_geometry& g, int pf, int nrhs,
   return cudaGetLastError();
 }
 
-cudaError_t h3_launch_m2l_rot(const qbxfmm_geometry& g, int pf, int nrhs, const double2* mp,
-                              double2* lo, const double* Dtab, const double2* Ctab,
-                              const double* clsmap, int32_t* err, cudaStream_t st, bool fp32,
-                              int rb)
+cudaError_t h3_launch_m2l_rot_f32(const qbxfmm_geometry& g, int pf, int nrhs, const double2* mp,
+                                  double2* lo, const double* Dtab, const double2* Ctab,
+                                  const double* clsmap, int32_t* err, cudaStream_t st, int rb)
 {
   if (g.nttp_boxes == 0 || g.m2l_nclasses == 0) return cudaSuccess;
   if (pf > H3_MAXP) return cudaErrorInvalidValue;
   switch (rb) {   // the plan's tuning
-    case 1:
-      return fp32 ? h3_m2l_rot_launch<float, 1>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st)
-                  : h3_m2l_rot_launch<double, 1>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-    case 4:
-      return fp32 ? h3_m2l_rot_launch<float, 4>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st)
-                  : h3_m2l_rot_launch<double, 4>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-    case 8:
-      return fp32 ? h3_m2l_rot_launch<float, 8>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st)
-                  : h3_m2l_bulk_launch<8>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-    case 16:
-      if (fp32) return h3_m2l_rot_launch<float, 16>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-      return h3_m2l_bulk16(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
+    case 1: return h3_m2l_rot_launch<float, 1>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
+    case 4: return h3_m2l_rot_launch<float, 4>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
+    case 8: return h3_m2l_rot_launch<float, 8>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
+    case 16: return h3_m2l_rot_launch<float, 16>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
     default: break;
   }
-  if (fp32) {   // mixed form: FP32 arithmetic, all 16 densities of a pair's tables at once
-    if (nrhs >= 16) return h3_m2l_rot_launch<float, 16>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-    if (nrhs >= 8) return h3_m2l_rot_launch<float, 8>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-    return h3_m2l_rot_launch<float, 4>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-  }
-  // 16 densities per CTA (512 threads) when there are as many: at the 3D Helmholtz
-  // benchmark size the autotuner measured 158 ms against 162 ms for 8
-  if (nrhs >= 16) return h3_m2l_bulk16(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-  if (nrhs >= 8) return h3_m2l_bulk_launch<8>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-  if (nrhs >= 2) return h3_m2l_rot_launch<double, 4>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-  return h3_m2l_rot_launch<double, 1>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
+  // all 16 densities of a pair's tables at once
+  if (nrhs >= 16) return h3_m2l_rot_launch<float, 16>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
+  if (nrhs >= 8) return h3_m2l_rot_launch<float, 8>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
+  return h3_m2l_rot_launch<float, 4>(g, pf, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
 }
 
 cudaError_t h3_launch_m2l_tables(int pf, int ndir, int ncoax, const double* dirs,

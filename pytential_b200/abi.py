@@ -140,6 +140,27 @@ class QBXFMMWorkspace(ctypes.Structure):
                 ("pair_scratch", ctypes.c_void_p)]
 
 
+#: list-1 sources that cost as much as one list-3 box in the QBX stages (in 3D a
+#: target's near-field term takes about 35 FP64 instructions, a list-3 multipole about 8000)
+LIST3_BOX_COST = 200
+
+
+def longest_chunks_first(arrays: dict, prefix: str) -> dict:
+    """The chunk arrays ``<prefix>_chunk_*`` in order of decreasing work: (list-1 sources +
+    LIST3_BOX_COST x list-3 boxes) of the target box per octet of the chunk, so that no
+    long chunk starts last (list 3 holds 12 to 23 boxes on average, several hundred at
+    most)."""
+    tb = arrays[prefix + "_chunk_target_box"]
+    cnt = arrays["box_source_counts_nonchild"].astype(np.int64)[arrays["list1_lists"]]
+    csum = np.concatenate([[0], np.cumsum(cnt)])
+    l1s = arrays["list1_starts"]
+    work = (csum[l1s[1:]] - csum[l1s[:-1]]
+            + LIST3_BOX_COST * np.diff(arrays["list3_starts"].astype(np.int64)))
+    order = np.argsort(-work[tb] * ((arrays[prefix + "_chunk_count"] + 7) // 8), kind="stable")
+    return {prefix + name: arrays[prefix + name][order]
+            for name in ("_chunk_target_box", "_chunk_start", "_chunk_count")}
+
+
 def qbx_center_schedule(global_qbx_centers, qbx_center_to_target_box, list1_starts,
                         list1_lists, box_source_counts_nonchild, chunk: int = CENTER_CHUNK):
     """Global QBX centers grouped by target box and cut into chunks of at most
@@ -393,6 +414,8 @@ def geometry_arrays(geo, per_level_classes: bool = False) -> tuple[dict, dict]:
                         arrays["center_to_targets_starts"], arrays["center_to_targets_lists"])
     arrays.update(dict(zip(["tsqbx_chunk_target_box", "tsqbx_chunk_start", "tsqbx_chunk_count",
                             "tsqbx_targets", "tsqbx_centers"], ts)))
+    for prefix in ("qbx", "tsqbx"):
+        arrays.update(longest_chunks_first(arrays, prefix))
     tc = translation_classes(tree, trav, per_level=per_level_classes)
     arrays.update({k_: np.ascontiguousarray(v, np.int32) for k_, v in tc.items()
                    if not k_.endswith(("nclasses", "npairs"))})

@@ -1259,7 +1259,12 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
   cudaStream_t st = S(stream);
   QBX_TRY(cudaMemsetAsync(ws->mpoles, 0, sz[1], st), "apply: clear");
   QBX_TRY(cudaMemsetAsync(ws->locals, 0, sz[2], st), "apply: clear");
-  QBX_TRY(cudaMemsetAsync(ws->qbx_exps, 0, sz[3], st), "apply: clear");
+  // 3D Helmholtz in FP64 with the target-specific near field: the list-3 multipoles go
+  // straight to the QBX targets and, in the compressed-Taylor truncation, the box locals
+  // too (then no QBX expansions are formed)
+  const bool m2t = p->h3 && !p->mixed && p->kern.target_specific_qbx != 0 && h3_m2t_wins(p->geo);
+  const bool l2t = m2t && p->hc.taylor;
+  if (!l2t) QBX_TRY(cudaMemsetAsync(ws->qbx_exps, 0, sz[3], st), "apply: clear");
   QBX_TRY(cudaMemsetAsync(ws->pot_nonqbx, 0, sz[4], st), "apply: clear");
   QBX_TRY(cudaMemsetAsync(ws->pot_tree, 0, sz[5], st), "apply: clear");
   if (ws->error_word) QBX_TRY(cudaMemsetAsync(ws->error_word, 0, sizeof(int32_t), st), "apply: clear");
@@ -1287,8 +1292,6 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
   void* s3 = p->side[2];
   cudaStream_t side1 = p->side[0], side2 = p->side[1], side3 = p->side[2];
   const bool tsqbx = p->kern.target_specific_qbx != 0;
-  // 3D Helmholtz in FP64: the list-3 multipoles go straight to the QBX targets
-  const bool m2t = p->h3 && !p->mixed && tsqbx && h3_m2t_wins(p->geo);
   bool forked = false;
   // on an error, join the side streams before returning, so that a stream capture
   // of the caller's stream stays well formed
@@ -1349,8 +1352,18 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
   forked = false;
 #undef QBX_STEP
 #undef QBX_CUDA_STEP
-  if ((rc = qbxfmm_translate_box_local_to_qbx_local(p, ws->locals, ws->qbx_exps, stream))) return rc;
-  if ((rc = qbxfmm_eval_qbx_expansions(p, ws->qbx_exps, ws->pot_tree, stream))) return rc;
+  if (l2t) {
+    size_t o[8];
+    h3_layout(p, o);
+    QBX_TRY(h3_launch_l2t_taylor(p->geo, p->hc, p->kern.fmm_order, p->kern.qbx_order, p->kern.nrhs,
+                                 (const double2*)ws->locals,
+                                 reinterpret_cast<const double2*>(p->trans_dev + o[5]),
+                                 (double2*)ws->pot_tree, ws->error_word, st),
+            "apply: locals to QBX targets");
+  } else {
+    if ((rc = qbxfmm_translate_box_local_to_qbx_local(p, ws->locals, ws->qbx_exps, stream))) return rc;
+    if ((rc = qbxfmm_eval_qbx_expansions(p, ws->qbx_exps, ws->pot_tree, stream))) return rc;
+  }
   return qbxfmm_assemble(p, ws->pot_nonqbx, ws->pot_tree, out, stream);
 }
 

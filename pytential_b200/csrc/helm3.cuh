@@ -141,6 +141,104 @@ QBX_D double2 ipow(int e)
   }
 }
 
+// list helpers (as in the Laplace kernels)
+constexpr int MAXB = 128;       // list boxes staged per pass
+
+QBX_D void h3_list_prefix(const qbxfmm_geometry& g, const int32_t* __restrict__ lists, int gb,
+                          int nb, int* s_pref, int* s_start, int32_t* err)
+{
+  if (threadIdx.x >= 32) return;
+  int lane = threadIdx.x;
+  int cnt[4], loc = 0;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    int k = lane * 4 + u;
+    cnt[u] = 0;
+    if (k < nb) {
+      int sb = lists[gb + k];
+      int s0 = 0;
+      if ((unsigned)sb < (unsigned)g.nboxes) {
+        s0 = g.box_source_starts[sb];
+        cnt[u] = g.box_source_counts_nonchild[sb];
+      } else {
+        report(err, QBX_DEVERR_BAD_BOX);
+      }
+      s_start[k] = s0;
+    }
+    loc += cnt[u];
+  }
+  int incl = loc;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    int v = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += v;
+  }
+  int run = incl - loc;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    int k = lane * 4 + u;
+    if (k < nb) s_pref[k] = run;
+    run += cnt[u];
+  }
+  if (lane == 31) s_pref[nb] = incl;
+}
+
+QBX_D int h3_stream_source(int v, int nb, const int* s_pref, const int* s_start)
+{
+  int lo = 0, hi = nb - 1;
+  while (lo < hi) {
+    int mid = (lo + hi + 1) >> 1;
+    if (s_pref[mid] <= v) lo = mid;
+    else hi = mid - 1;
+  }
+  return s_start[lo] + (v - s_pref[lo]);
+}
+
+// Weights g_t of the Taylor coefficients b_t along a line of length |a| (x = k|a|) that
+// give the order-Q expansion's value: 1 where j_n is cut to its power series (cut), else
+// sum_n j_n Lambda_n with b_t = sum_{n + 2j = t} alpha_nj x^t Lambda_n, from the highest
+// order down
+template <int Q>
+QBX_D void m2t_taylor_weights(bool cut, double x, double* gw)
+{
+#pragma unroll
+  for (int n = 0; n <= Q; ++n) gw[n] = 1.0;
+  if (cut) return;
+  // jh_n = j_n(x) (2n+1)!! / x^n: by its series for small x, else from j_n
+  double jh[Q + 1];
+  const double mx2 = -0.5 * x * x;
+  if (x < 2.0) {
+#pragma unroll
+    for (int n = 0; n <= Q; ++n) {
+      double t = 1.0, acc = 0.0;
+      for (int j = 0; j < 16; ++j) {
+        acc += t;
+        t *= mx2 * rcp(j + 1) * rcp(2 * n + 2 * j + 3);
+      }
+      jh[n] = acc;
+    }
+  } else {
+    double jv[H3_LMAX + 2];
+    h3_sph_j(Q, x, jv);
+    double f = 1.0;
+#pragma unroll
+    for (int n = 0; n <= Q; ++n) {
+      jh[n] = jv[n] * f;
+      f *= (2.0 * n + 3.0) / x;
+    }
+  }
+#pragma unroll
+  for (int n = Q; n >= 0; --n) {
+    double t = 1.0, v = jh[n];
+#pragma unroll
+    for (int j = 1; n + 2 * j <= Q; ++j) {
+      t *= mx2 * rcp(j) * rcp(2 * n + 2 * j + 1);
+      v -= gw[n + 2 * j] * t;
+    }
+    gw[n] = v;
+  }
+}
+
 // D (8x8, two per lane: row lane/4, columns 2 (lane%4) + {0,1}) += A (8x4, row major,
 // element (lane/4, lane%4)) B (4x8, column major, element (lane%4, lane/4)), FP64
 QBX_D void h3_dmma(double& d0, double& d1, double a, double b)

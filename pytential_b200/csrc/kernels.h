@@ -206,6 +206,11 @@ cudaError_t h3_launch_m2qbxl(const qbxfmm_geometry& g, HelmCoeffs hc, int pf, in
 cudaError_t h3_launch_m2t(const qbxfmm_geometry& g, HelmCoeffs hc, int pf, int q, int nrhs,
                           const double2* mp, double2* pot_tree, int32_t* err, cudaStream_t st);
 bool h3_m2t_wins(const qbxfmm_geometry& g);
+// box locals straight to the QBX targets in the compressed-Taylor truncation (L2QBXL and
+// QBXL2P in one, added into pot_tree); G0: monomial table of the order-p locals
+cudaError_t h3_launch_l2t_taylor(const qbxfmm_geometry& g, HelmCoeffs hc, int p, int q, int nrhs,
+                                 const double2* lo, const double2* G0, double2* pot_tree,
+                                 int32_t* err, cudaStream_t st);
 cudaError_t h3_launch_l2qbxl(const qbxfmm_geometry& g, HelmCoeffs hc, int pf, int q, int nrhs,
                              const double2* lo, const double* rot, double2* qe, int32_t* err,
                              cudaStream_t st);

@@ -34,7 +34,6 @@ namespace {
 
 constexpr int NT = 128;
 constexpr int NW = NT / 32;
-constexpr int MAXB = 128;
 
 // Ladder terms of nu . grad F_n^mm (mm = -m for the source coefficient (n, m)):
 // six table entries with real weights (0 where the entry is outside the table).
@@ -103,229 +102,7 @@ QBX_D void h3_wave_column(int m, int N, double t, double2 w, const double2* rec,
   }
 }
 
-// list helpers (as in the Laplace kernels)
-QBX_D void h3_list_prefix(const qbxfmm_geometry& g, const int32_t* __restrict__ lists, int gb,
-                          int nb, int* s_pref, int* s_start, int32_t* err)
-{
-  if (threadIdx.x >= 32) return;
-  int lane = threadIdx.x;
-  int cnt[4], loc = 0;
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    int k = lane * 4 + u;
-    cnt[u] = 0;
-    if (k < nb) {
-      int sb = lists[gb + k];
-      int s0 = 0;
-      if ((unsigned)sb < (unsigned)g.nboxes) {
-        s0 = g.box_source_starts[sb];
-        cnt[u] = g.box_source_counts_nonchild[sb];
-      } else {
-        report(err, QBX_DEVERR_BAD_BOX);
-      }
-      s_start[k] = s0;
-    }
-    loc += cnt[u];
-  }
-  int incl = loc;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    int v = __shfl_up_sync(0xffffffffu, incl, off);
-    if (lane >= off) incl += v;
-  }
-  int run = incl - loc;
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    int k = lane * 4 + u;
-    if (k < nb) s_pref[k] = run;
-    run += cnt[u];
-  }
-  if (lane == 31) s_pref[nb] = incl;
-}
-
-QBX_D int h3_stream_source(int v, int nb, const int* s_pref, const int* s_start)
-{
-  int lo = 0, hi = nb - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (s_pref[mid] <= v) lo = mid;
-    else hi = mid - 1;
-  }
-  return s_start[lo] + (v - s_pref[lo]);
-}
-
 }  // namespace
-
-// {{{ P2M / P2L
-
-// One CTA per box (P2M: source boxes, own sources; P2L: target-or-parent boxes, list-4
-// sources) and group of RB densities.  Sources in sub-tiles of SUB: one thread per
-// source computes the radial values (j_n for P2M, h_n for P2L, n <= p + 1), one thread
-// per (column, source) fills the wave table (entry-major, padded stride), then one
-// thread per coefficient forms the source's kernel row cq F_n^-m + cd nu . grad F_n^-m
-// (precomputed ladder offsets) once and adds density x row for each of the RB
-// densities, so the table and the row serve all densities of the group.
-constexpr int H3_SUB = 16;
-constexpr int H3_TS = H3_SUB + 1;
-constexpr int H3_NH = 3;          // coefficients per thread: (p+1)^2 <= 3 * 128
-
-// TH threads per CTA, NH coefficients per thread ((p+1)^2 <= NH x TH): 128 x 3 with up
-// to 8 densities, or 256 x 1 with 16 (the wave tables of a source serve all 16)
-template <bool LOCAL, int RB, int TH = NT, int NH = H3_NH>
-__global__ void __launch_bounds__(TH, TH == NT ? 1 : 2)
-k_h3_p2e(qbxfmm_geometry g, HelmCoeffs hc, int p, int nrhs, const double2* __restrict__ strengths,
-         double2* __restrict__ exps, int32_t* err)
-{
-  constexpr int SUB = H3_SUB, TS = H3_TS;
-  extern __shared__ double2 smem2[];
-  const int N = p + 1;
-  const int ncf = (p + 1) * (p + 1);
-  double2* tab = smem2;                              // [(N+1)^2][TS]
-  double2* rec = smem2 + (size_t)(N + 1) * (N + 1) * TS;   // [(N+1)(N+2)/2]
-  __shared__ double2 s_rad[SUB][H3_LMAX + 2];
-  __shared__ double s_t[SUB];
-  __shared__ double2 s_w[SUB], s_sig[SUB][RB], s_np[SUB], s_nm[SUB];
-  __shared__ double s_nz[SUB];
-  __shared__ int s_pref[MAXB + 1], s_start[MAXB];
-
-  int b, l0 = 0, l1 = 0;
-  if (LOCAL) {
-    int i = blockIdx.x;
-    b = g.target_or_target_parent_boxes[i];
-    l0 = g.list4_starts[i];
-    l1 = g.list4_starts[i + 1];
-    if (l1 <= l0) return;
-  } else {
-    b = g.source_boxes[blockIdx.x];
-  }
-  int r0 = blockIdx.y * RB;
-  double rho = level_width(g, g.box_levels[b]);
-  double sc = h3_scale(hc.k, rho);
-  double c[3];
-  load_point<3>(g.box_centers, g.nboxes, b, c);
-  const bool dip = hc.cd.x != 0.0 || hc.cd.y != 0.0;
-  // the reference's default multipoles (moments of degree <= p): the charge row from
-  // j_n^[p], the normal derivative from j_n^[p-1] (a second table)
-  const bool two = !LOCAL && hc.taylor && dip;
-  double2* tab2 = two ? rec + (size_t)(N + 1) * (N + 2) / 2 : tab;   // [(N+1)^2][TS]
-  double2* rad2 = two ? tab2 + (size_t)(N + 1) * (N + 1) * TS : nullptr;   // [SUB][N+2]
-  h3_rec_table(N, rec, threadIdx.x, TH);
-
-  int o_c[NH];
-  Ladder lad[NH];
-  bool valid[NH];
-#pragma unroll
-  for (int h = 0; h < NH; ++h) {
-    int ci = threadIdx.x + h * TH;
-    valid[h] = ci < ncf;
-    int n = 0, m = 0;
-    if (valid[h]) hq_decode(ci, n, m);
-    o_c[h] = hq(n, -m) * TS;
-    lad[h] = h3_ladder(n, -m, hc.k);
-#pragma unroll
-    for (int u = 0; u < 6; ++u) lad[h].o[u] *= TS;
-  }
-  double2 acc[NH][RB];
-#pragma unroll
-  for (int h = 0; h < NH; ++h)
-#pragma unroll
-    for (int rr = 0; rr < RB; ++rr) acc[h][rr] = c2(0.0);
-
-  // one stream over the box's own sources (P2M) or the list-4 boxes' sources (P2L)
-  for (int gb = l0; gb < (LOCAL ? l1 : 1); gb += MAXB) {
-    int nb = 0, total;
-    __syncthreads();
-    if (LOCAL) {
-      nb = min(MAXB, l1 - gb);
-      h3_list_prefix(g, g.list4_lists, gb, nb, s_pref, s_start, err);
-      __syncthreads();
-      total = s_pref[nb];
-    } else {
-      total = g.box_source_counts_nonchild[b];
-    }
-    int s0 = LOCAL ? 0 : g.box_source_starts[b];
-    for (int base = 0; base < total; base += SUB) {
-      int cnt = min(SUB, total - base);
-      __syncthreads();
-      if (threadIdx.x < cnt) {
-        int j = threadIdx.x;
-        int s = LOCAL ? h3_stream_source(base + j, nb, s_pref, s_start) : s0 + base + j;
-        double y[3], u[3], rr;
-        load_point<3>(g.sources, g.nsources, s, y);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) u[d] = y[d] - c[d];
-        double2 w;
-        s_t[j] = h3_dir(u, w, rr);
-        s_w[j] = w;
-        double x = hc.k * rr;
-        if (LOCAL) {
-          h3_sph_h(N, x, s_rad[j]);
-        } else {
-          double jv[H3_LMAX + 2];
-          h3_sph_j_cut(N, x, hc.taylor ? p : -1, jv);
-          for (int n = 0; n <= N; ++n) s_rad[j][n] = c2(jv[n]);
-          if (two) {
-            h3_sph_j_cut(N, x, p - 1, jv);
-            for (int n = 0; n <= N; ++n) rad2[j * (N + 2) + n] = c2(jv[n]);
-          }
-        }
-#pragma unroll
-        for (int rr = 0; rr < RB; ++rr)
-          s_sig[j][rr] = r0 + rr < nrhs ? strengths[(size_t)(r0 + rr) * g.nsources + s] : c2(0.0);
-        if (dip) {
-          double nv[3];
-          load_point<3>(g.source_normals, g.nsources, s, nv);
-          s_np[j] = c2(0.5 * nv[0], -0.5 * nv[1]);
-          s_nm[j] = c2(0.5 * nv[0], 0.5 * nv[1]);
-          s_nz[j] = nv[2];
-        }
-      }
-      __syncthreads();
-      for (int wk = threadIdx.x; wk < cnt * (N + 1); wk += TH) {
-        int m = wk / cnt, j = wk - m * cnt;
-        h3_wave_column(m, N, s_t[j], s_w[j], rec, s_rad[j], tab + j, TS);
-        if (two) h3_wave_column(m, N, s_t[j], s_w[j], rec, rad2 + j * (N + 2), tab2 + j, TS);
-      }
-      __syncthreads();
-#pragma unroll
-      for (int h = 0; h < NH; ++h) {
-        if (!valid[h]) continue;
-        for (int j = 0; j < cnt; ++j) {
-          const double2* T = tab + j;
-          double2 kr = cmul(hc.cq, T[o_c[h]]);
-          if (dip) {
-            T = tab2 + j;
-            const Ladder& L = lad[h];
-            double2 vz = caxpy(L.w[0], T[L.o[0]], cscale(L.w[1], T[L.o[1]]));
-            double2 vp = caxpy(L.w[2], T[L.o[2]], cscale(L.w[3], T[L.o[3]]));
-            double2 vm = caxpy(L.w[4], T[L.o[4]], cscale(L.w[5], T[L.o[5]]));
-            double2 v = cfma(s_np[j], vp, cfma(s_nm[j], vm, cscale(s_nz[j], vz)));
-            kr = cfma(hc.cd, v, kr);
-          }
-#pragma unroll
-          for (int rr = 0; rr < RB; ++rr) acc[h][rr] = cfma(s_sig[j][rr], kr, acc[h][rr]);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int h = 0; h < NH; ++h) {
-    if (!valid[h]) continue;
-    int ci = threadIdx.x + h * TH;
-    int n, m;
-    hq_decode(ci, n, m);
-    double f = FOUR_PI * hc.k * (LOCAL ? pow(sc, (double)n) : pow(sc, -(double)n));
-#pragma unroll
-    for (int rr = 0; rr < RB; ++rr) {
-      if (r0 + rr >= nrhs) break;
-      // 4 pi i k f acc
-      double2* E = exps + ((size_t)b * nrhs + r0 + rr) * ncf + ci;
-      *E = cadd(*E, c2(-f * acc[h][rr].y, f * acc[h][rr].x));
-    }
-  }
-}
-
-// }}}
 
 // {{{ point evaluations at non-QBX targets
 
@@ -1403,154 +1180,6 @@ k_h3_qbxl2p(qbxfmm_geometry g, HelmCoeffs hc, int q, int nrhs, const double2* __
   }
 }
 
-// Target-specific near field (eval_target_specific_qbx_locals, pytential/qbx/fmm.py:391-394;
-// the reference's native module pytential/qbx/target_specific/impl.pyx:363-563):
-// per (target t, its center c, list-1 source y), with a = t - c, b = y - c,
-//   K_S = ik sum_{n<=Q} (2n+1) j_n(k|a|) h_n(k|b|) P_n(cos g),
-//   K_D = ik sum (2n+1) j_n(k|a|) (k h_n'(k|b|) P_n nu.bh + h_n P_n' (nu.ah - cos g nu.bh) / |b|),
-// the order-Q spherical-wave QBX expansion evaluated without forming it.  The kernel
-// value K = cq K_S + cd K_D is computed once per pair and applied to RB densities at
-// a time (lane = target; 4 warps split each 128-source tile; strengths of the tile's
-// sources for the RB densities staged in shared memory).
-template <int Q, int RB>
-__global__ void __launch_bounds__(NT)
-k_h3_tsqbx(qbxfmm_geometry g, HelmCoeffs hc, int nrhs, const double2* __restrict__ strengths,
-           double2* __restrict__ pot_tree, int32_t* err)
-{
-  __shared__ double s_y[3][NT], s_n[3][NT];
-  __shared__ double2 s_q[RB][NT];
-  __shared__ int s_pref[MAXB + 1], s_start[MAXB];
-  extern __shared__ double2 smem2[];
-  double2* s_red = smem2;   // [NW-1][32][RB]
-  int chunk = blockIdx.x;
-  int r0 = blockIdx.y * RB;
-  int itb = g.tsqbx_chunk_target_box[chunk];
-  int i0 = g.tsqbx_chunk_start[chunk];
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  bool active = lane < g.tsqbx_chunk_count[chunk];
-  int t = active ? g.tsqbx_targets[i0 + lane] : 0;
-  int ctr = active ? g.tsqbx_centers[i0 + lane] : 0;
-  if ((unsigned)ctr >= (unsigned)g.ncenters || (unsigned)t >= (unsigned)g.ntargets) {
-    report(err, QBX_DEVERR_BAD_CENTER);
-    active = false;
-    t = ctr = 0;
-  }
-  double cc[3], x[3];
-  load_point<3>(g.centers, g.ncenters, ctr, cc);
-  load_point<3>(g.targets, g.ntargets, t, x);
-  double a[3] = {x[0] - cc[0], x[1] - cc[1], x[2] - cc[2]};
-  double alen = sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
-  double ainv = alen > 0.0 ? 1.0 / alen : 0.0;
-  double ah[3] = {a[0] * ainv, a[1] * ainv, a[2] * ainv};
-  double jn[Q + 1];
-  {
-    double jv[H3_LMAX + 2];
-    h3_sph_j_cut(Q, hc.k * alen, hc.taylor ? Q : -1, jv);
-#pragma unroll
-    for (int n = 0; n <= Q; ++n) jn[n] = (2.0 * n + 1.0) * jv[n];
-  }
-  const bool chg = hc.cq.x != 0.0 || hc.cq.y != 0.0;
-  const bool dip = hc.cd.x != 0.0 || hc.cd.y != 0.0;
-  // ik cq, ik cd
-  const double2 kq = c2(-hc.k * hc.cq.y, hc.k * hc.cq.x), kd = c2(-hc.k * hc.cd.y, hc.k * hc.cd.x);
-  double2 acc[RB];
-#pragma unroll
-  for (int i = 0; i < RB; ++i) acc[i] = c2(0.0);
-  int l0 = g.list1_starts[itb], l1 = g.list1_starts[itb + 1];
-  for (int gb = l0; gb < l1; gb += MAXB) {
-    int nb = min(MAXB, l1 - gb);
-    __syncthreads();
-    h3_list_prefix(g, g.list1_lists, gb, nb, s_pref, s_start, err);
-    __syncthreads();
-    int total = s_pref[nb];
-    for (int base = 0; base < total; base += NT) {
-      int v = base + threadIdx.x;
-      if (v < total) {
-        int s = h3_stream_source(v, nb, s_pref, s_start);
-        double y[3], nv[3] = {0, 0, 0};
-        load_point<3>(g.sources, g.nsources, s, y);
-        if (dip) load_point<3>(g.source_normals, g.nsources, s, nv);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          s_y[d][threadIdx.x] = y[d];
-          s_n[d][threadIdx.x] = nv[d];
-        }
-#pragma unroll
-        for (int i = 0; i < RB; ++i)
-          s_q[i][threadIdx.x] = (r0 + i < nrhs) ? strengths[(size_t)(r0 + i) * g.nsources + s] : c2(0.0);
-      }
-      __syncthreads();
-      int jbeg = warp * 32, jend = min(jbeg + 32, total - base);
-      if (active) {
-        for (int j = jbeg; j < jend; ++j) {
-          double b0 = s_y[0][j] - cc[0], b1 = s_y[1][j] - cc[1], b2 = s_y[2][j] - cc[2];
-          double b2s = b0 * b0 + b1 * b1 + b2 * b2;
-          if (b2s == 0.0) continue;
-          double binv = rsqrt(b2s);
-          double blen = b2s * binv;
-          double cg = (ah[0] * b0 + ah[1] * b1 + ah[2] * b2) * binv;
-          double2 h[Q + 2];
-          h3_sph_h(Q + 1, hc.k * blen, h);
-          double xinv = 1.0 / (hc.k * blen);
-          double pm1 = 1.0, pm2 = 0.0, dm1 = 0.0;
-          double2 sS = c2(0.0), sA = c2(0.0), sB = c2(0.0);
-#pragma unroll
-          for (int n = 0; n <= Q; ++n) {
-            double pn, dn;
-            if (n == 0) {
-              pn = 1.0;
-              dn = 0.0;
-            } else if (n == 1) {
-              pn = cg;
-              dn = 1.0;
-            } else {
-              pn = ((2.0 * n - 1) * cg * pm1 - (n - 1.0) * pm2) * (1.0 / n);
-              dn = n * pm1 + cg * dm1;
-            }
-            if (chg) sS = caxpy(jn[n] * pn, h[n], sS);
-            if (dip) {
-              // h_n'(x) = h_{n-1} - (n+1)/x h_n  (n >= 1), h_0' = -h_1
-              double2 hd = (n == 0) ? c2(-h[1].x, -h[1].y)
-                                    : caxpy(-(n + 1.0) * xinv, h[n], h[n - 1]);
-              sA = caxpy(jn[n] * pn * hc.k, hd, sA);
-              sB = caxpy(jn[n] * dn, h[n], sB);
-            }
-            pm2 = pm1;
-            pm1 = pn;
-            dm1 = dn;
-          }
-          double2 K = c2(0.0);
-          if (chg) K = cmul(kq, sS);
-          if (dip) {
-            double db = (s_n[0][j] * b0 + s_n[1][j] * b1 + s_n[2][j] * b2) * binv;
-            double da = s_n[0][j] * ah[0] + s_n[1][j] * ah[1] + s_n[2][j] * ah[2];
-            double2 vd = caxpy(db, sA, cscale((da - cg * db) * binv, sB));
-            K = cfma(kd, vd, K);
-          }
-#pragma unroll
-          for (int i = 0; i < RB; ++i) acc[i] = cfma(K, s_q[i][j], acc[i]);
-        }
-      }
-      __syncthreads();
-    }
-  }
-  if (warp > 0) {
-#pragma unroll
-    for (int i = 0; i < RB; ++i) s_red[((warp - 1) * 32 + lane) * RB + i] = acc[i];
-  }
-  __syncthreads();
-  if (warp == 0 && active) {
-#pragma unroll
-    for (int i = 0; i < RB; ++i) {
-      if (r0 + i >= nrhs) continue;
-      double2 v = acc[i];
-      for (int w = 1; w < NW; ++w) v = cadd(v, s_red[((w - 1) * 32 + lane) * RB + i]);
-      double2* P = pot_tree + (size_t)(r0 + i) * g.ntargets + t;
-      *P = cadd(*P, v);
-    }
-  }
-}
-
 // }}}
 
 // {{{ translation matrices
@@ -2045,58 +1674,6 @@ cudaError_t h3_launch_m2l_tables(int pf, int ndir, int ncoax, const double* dirs
 static int gridy(int nrhs) { return nrhs; }
 
 // densities per CTA: 8, 4 or 1
-template <bool LOCAL>
-static cudaError_t h3_p2e_launch(int nbox, size_t sh, const qbxfmm_geometry& g, HelmCoeffs hc, int p,
-                                 int nrhs, const double2* s, double2* e, int32_t* err,
-                                 cudaStream_t st)
-{
-#define QBX_H3_P2E(RB)                                                                          \
-  {                                                                                             \
-    cudaFuncSetAttribute(k_h3_p2e<LOCAL, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
-                         (int)sh);                                                              \
-    k_h3_p2e<LOCAL, RB><<<dim3(nbox, (nrhs + RB - 1) / RB), NT, sh, st>>>(g, hc, p, nrhs, s, e, \
-                                                                          err);                 \
-    return cudaGetLastError();                                                                  \
-  }
-  // 16 densities: 256 threads, one coefficient each
-  const bool wide = (p + 1) * (p + 1) <= 2 * NT;
-  if (hc.rb_p2e == 16 || (hc.rb_p2e == 0 && nrhs > 8 && wide)) {
-    if (!wide) return cudaErrorInvalidValue;
-    cudaFuncSetAttribute(k_h3_p2e<LOCAL, 16, 2 * NT, 1>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    k_h3_p2e<LOCAL, 16, 2 * NT, 1><<<dim3(nbox, (nrhs + 15) / 16), 2 * NT, sh, st>>>(
-        g, hc, p, nrhs, s, e, err);
-    return cudaGetLastError();
-  }
-  if (hc.rb_p2e == 8) QBX_H3_P2E(8)   // the plan's tuning
-  if (hc.rb_p2e == 4) QBX_H3_P2E(4)
-  if (hc.rb_p2e == 1) QBX_H3_P2E(1)
-  if (nrhs >= 8) QBX_H3_P2E(8)
-  if (nrhs >= 3) QBX_H3_P2E(4)
-  QBX_H3_P2E(1)
-#undef QBX_H3_P2E
-}
-
-cudaError_t h3_launch_p2m(const qbxfmm_geometry& g, HelmCoeffs hc, int p, int nrhs,
-                          const double2* s, double2* mp, cudaStream_t st)
-{
-  if (g.nsource_boxes == 0) return cudaSuccess;
-  int N = p + 1;
-  size_t sh = ((size_t)(N + 1) * (N + 1) * H3_TS + (size_t)(N + 1) * (N + 2) / 2) * sizeof(double2);
-  if (hc.taylor && (hc.cd.x != 0.0 || hc.cd.y != 0.0))   // second (dipole) table
-    sh += ((size_t)(N + 1) * (N + 1) * H3_TS + (size_t)H3_SUB * (N + 2)) * sizeof(double2);
-  return h3_p2e_launch<false>(g.nsource_boxes, sh, g, hc, p, nrhs, s, mp, nullptr, st);
-}
-
-cudaError_t h3_launch_p2l(const qbxfmm_geometry& g, HelmCoeffs hc, int p, int nrhs,
-                          const double2* s, double2* lo, int32_t* err, cudaStream_t st)
-{
-  if (g.nttp_boxes == 0) return cudaSuccess;
-  int N = p + 1;
-  size_t sh = ((size_t)(N + 1) * (N + 1) * H3_TS + (size_t)(N + 1) * (N + 2) / 2) * sizeof(double2);
-  return h3_p2e_launch<true>(g.nttp_boxes, sh, g, hc, p, nrhs, s, lo, err, st);
-}
-
 cudaError_t h3_launch_eval_direct(const qbxfmm_geometry& g, HelmCoeffs hc, int nrhs,
                                   const double2* s, double2* pot, int32_t* err, cudaStream_t st)
 {
@@ -2150,47 +1727,6 @@ cudaError_t h3_launch_p2qbxl(const qbxfmm_geometry& g, HelmCoeffs hc, int q, int
     case 3: return h3_p2qbxl_q<3>(g, hc, nrhs, s, qe, err, st);
     case 4: return h3_p2qbxl_q<4>(g, hc, nrhs, s, qe, err, st);
     case 5: return h3_p2qbxl_q<5>(g, hc, nrhs, s, qe, err, st);
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-template <int Q, int RB>
-static cudaError_t h3_tsqbx_qr(const qbxfmm_geometry& g, HelmCoeffs hc, int nrhs, const double2* s,
-                               double2* pt, int32_t* err, cudaStream_t st)
-{
-  size_t sh = (size_t)(NW - 1) * 32 * RB * sizeof(double2);
-  dim3 grid(g.ntsqbx_chunks, (nrhs + RB - 1) / RB);
-  cudaFuncSetAttribute(k_h3_tsqbx<Q, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-  k_h3_tsqbx<Q, RB><<<grid, NT, sh, st>>>(g, hc, nrhs, s, pt, err);
-  return cudaGetLastError();
-}
-
-template <int Q>
-static cudaError_t h3_tsqbx_q(const qbxfmm_geometry& g, HelmCoeffs hc, int nrhs, const double2* s,
-                              double2* pt, int32_t* err, cudaStream_t st)
-{
-  switch (hc.rb_ts) {   // the plan's tuning
-    case 1: return h3_tsqbx_qr<Q, 1>(g, hc, nrhs, s, pt, err, st);
-    case 4: return h3_tsqbx_qr<Q, 4>(g, hc, nrhs, s, pt, err, st);
-    case 16: return h3_tsqbx_qr<Q, 16>(g, hc, nrhs, s, pt, err, st);
-    default: break;
-  }
-  if (nrhs == 1) return h3_tsqbx_qr<Q, 1>(g, hc, nrhs, s, pt, err, st);
-  if (nrhs <= 4) return h3_tsqbx_qr<Q, 4>(g, hc, nrhs, s, pt, err, st);
-  return h3_tsqbx_qr<Q, 16>(g, hc, nrhs, s, pt, err, st);
-}
-
-cudaError_t h3_launch_tsqbx(const qbxfmm_geometry& g, HelmCoeffs hc, int q, int nrhs,
-                            const double2* s, double2* pt, int32_t* err, cudaStream_t st)
-{
-  if (g.ntsqbx_chunks == 0) return cudaSuccess;
-  switch (q) {
-    case 0: return h3_tsqbx_q<0>(g, hc, nrhs, s, pt, err, st);
-    case 1: return h3_tsqbx_q<1>(g, hc, nrhs, s, pt, err, st);
-    case 2: return h3_tsqbx_q<2>(g, hc, nrhs, s, pt, err, st);
-    case 3: return h3_tsqbx_q<3>(g, hc, nrhs, s, pt, err, st);
-    case 4: return h3_tsqbx_q<4>(g, hc, nrhs, s, pt, err, st);
-    case 5: return h3_tsqbx_q<5>(g, hc, nrhs, s, pt, err, st);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -38,48 +38,8 @@ __host__ __device__ constexpr size_t m2t_warp_smem(int pf, int q)
   return (size_t)M2T_TG * (pf + q + 1 + (pf + 1) * (q + 1) + (q + 1)) + 32 * (q + 1);
 }
 
-// weights g of the Taylor coefficients, from the highest order down
-template <int Q>
-QBX_D void m2t_taylor_weights(bool cut, double x, double* gw)
-{
-#pragma unroll
-  for (int n = 0; n <= Q; ++n) gw[n] = 1.0;
-  if (cut) return;
-  // jh_n = j_n(x) (2n+1)!! / x^n: by its series for small x, else from j_n
-  double jh[Q + 1];
-  const double mx2 = -0.5 * x * x;
-  if (x < 2.0) {
-#pragma unroll
-    for (int n = 0; n <= Q; ++n) {
-      double t = 1.0, acc = 0.0;
-      for (int j = 0; j < 16; ++j) {
-        acc += t;
-        t *= mx2 * rcp(j + 1) * rcp(2 * n + 2 * j + 3);
-      }
-      jh[n] = acc;
-    }
-  } else {
-    double jv[H3_LMAX + 2];
-    h3_sph_j(Q, x, jv);
-    double f = 1.0;
-#pragma unroll
-    for (int n = 0; n <= Q; ++n) {
-      jh[n] = jv[n] * f;
-      f *= (2.0 * n + 3.0) / x;
-    }
-  }
-#pragma unroll
-  for (int n = Q; n >= 0; --n) {
-    double t = 1.0, v = jh[n];
-#pragma unroll
-    for (int j = 1; n + 2 * j <= Q; ++j) {
-      t *= mx2 * rcp(j) * rcp(2 * n + 2 * j + 1);
-      v -= gw[n + 2 * j] * t;
-    }
-    gw[n] = v;
-  }
-}
-
+// A CTA holds one octet of a chunk's targets; its four warps split the list-3 boxes
+// (fixed-order sum at the end), so that one long list is spread over four warps.
 // A warp holds 8 targets x 4 lanes: lane l carries target l / 4 and the columns
 // m = 4 j + l % 4 (both signs).  At each (j, n) a lane's weights w_{n,m} and w_{n,-m} are,
 // as they stand, the A fragment of an 8 x 4 FP64 tensor-core product (row = target,
@@ -101,15 +61,16 @@ k_h3_m2t(qbxfmm_geometry g, HelmCoeffs hc, int pf, int nrhs, const double2* __re
   double2* Phi = H + (size_t)M2T_TG * (pf + Q + 1);              // [n][i][target]
   double2* P4 = Phi + (size_t)M2T_TG * (pf + 1) * (Q + 1) + tg;  // [i][target]
   double2* E = P4 - tg + M2T_TG * (Q + 1) + lane;                // [i][lane]
-  const int chunk = blockIdx.x;
+  constexpr int NWARP = M2T_NT / 32, OCT = QBXFMM_CENTER_CHUNK / M2T_TG;
+  const int chunk = blockIdx.x / OCT, oct = blockIdx.x - chunk * OCT;
   const int itb = g.tsqbx_chunk_target_box[chunk];
   const int cnt = g.tsqbx_chunk_count[chunk];
+  if (oct * M2T_TG >= cnt) return;
   const int l0 = g.list3_starts[itb], l1 = g.list3_starts[itb + 1];
   if (l1 <= l0) return;
   h3_rec_table(pf, rec, threadIdx.x, M2T_NT);
   __syncthreads();
-  if (warp * M2T_TG >= cnt) return;
-  const int ti = warp * M2T_TG + tg;
+  const int ti = oct * M2T_TG + tg;
   const int pi = g.tsqbx_chunk_start[chunk] + min(ti, cnt - 1);
   bool active = ti < cnt;
   int t = g.tsqbx_targets[pi], ctr = g.tsqbx_centers[pi];
@@ -131,7 +92,7 @@ k_h3_m2t(qbxfmm_geometry g, HelmCoeffs hc, int pf, int nrhs, const double2* __re
 #pragma unroll
   for (int d = 0; d < DG; ++d) vre[d][0] = vre[d][1] = vim[d][0] = vim[d][1] = 0.0;
 
-  for (int li = l0; li < l1; ++li) {
+  for (int li = l0 + warp; li < l1; li += NWARP) {
     const int sb = g.list3_lists[li];
     if ((unsigned)sb >= (unsigned)g.nboxes) {
       report(err, QBX_DEVERR_BAD_BOX);
@@ -324,31 +285,30 @@ k_h3_m2t(qbxfmm_geometry g, HelmCoeffs hc, int pf, int nrhs, const double2* __re
       }
     }
   }
-  if constexpr (!MMA) {
+  // sum over the warps (the warps' scratch is free)
+  __syncthreads();
+  double2* red = smem2 + nrec;                 // [NWARP][2 DG or DG][32]
+  constexpr int NV = MMA ? 2 * DG : DG;
 #pragma unroll
-    for (int d = 0; d < DG; ++d) {
-      double2 v = c2(vre[d][0], vim[d][0]);
+  for (int d = 0; d < NV; ++d) {
+    double2 v = MMA ? c2(vre[d / 2][d & 1], vim[d / 2][d & 1]) : c2(vre[d % DG][0], vim[d % DG][0]);
+    if constexpr (!MMA) {                      // and over the four lanes of a target
 #pragma unroll
       for (int o = 1; o < 4; o <<= 1) {
         v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
         v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
       }
-      if (active && kq == 0 && r0 + d < nrhs) {
-        double2* P = pot_tree + (size_t)(r0 + d) * g.ntargets + t;
-        *P = cadd(*P, v);
-      }
     }
-  } else {
-#pragma unroll
-    for (int d = 0; d < DG; ++d)
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int r = r0 + 8 * d + 2 * kq + u;
-        if (active && r < nrhs) {
-          double2* P = pot_tree + (size_t)r * g.ntargets + t;
-          *P = cadd(*P, c2(vre[d][u], vim[d][u]));
-        }
-      }
+    red[(warp * NV + d) * 32 + lane] = v;
+  }
+  __syncthreads();
+  for (int d = warp; d < NV; d += NWARP) {
+    const int r = MMA ? r0 + 8 * (d / 2) + 2 * kq + (d & 1) : r0 + d;
+    if (!active || r >= nrhs || (!MMA && kq != 0)) continue;
+    double2 v = red[d * 32 + lane];
+    for (int w = 1; w < NWARP; ++w) v = cadd(v, red[(w * NV + d) * 32 + lane]);
+    double2* P = pot_tree + (size_t)r * g.ntargets + t;
+    *P = cadd(*P, v);
   }
 }
 
@@ -357,12 +317,12 @@ cudaError_t m2t_launch(const qbxfmm_geometry& g, HelmCoeffs hc, int pf, int nrhs
                        const double2* mp, double2* pot, int32_t* err, cudaStream_t st)
 {
   constexpr int ND = MMA ? 8 * DG : DG;
-  const size_t sh = ((size_t)(pf + 1) * (pf + 2) / 2 +
-                     (M2T_NT / 32) * m2t_warp_smem(pf, Q)) * sizeof(double2);
+  const size_t scratch = std::max(m2t_warp_smem(pf, Q), (size_t)(MMA ? 2 * DG : DG) * 32);
+  const size_t sh = ((size_t)(pf + 1) * (pf + 2) / 2 + (M2T_NT / 32) * scratch) * sizeof(double2);
   cudaError_t e = cudaFuncSetAttribute(k_h3_m2t<Q, DG, MMA>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
   if (e != cudaSuccess) return e;
-  dim3 grid(g.ntsqbx_chunks, (nrhs + ND - 1) / ND);
+  dim3 grid(g.ntsqbx_chunks * (QBXFMM_CENTER_CHUNK / M2T_TG), (nrhs + ND - 1) / ND);
   k_h3_m2t<Q, DG, MMA><<<grid, M2T_NT, sh, st>>>(g, hc, pf, nrhs, mp, pot, err);
   return cudaGetLastError();
 }

@@ -7,6 +7,7 @@
 // that share a target box, holds each center's coefficients in registers and
 // streams that box's list-1 sources through shared memory in tiles of 128.
 #include <algorithm>
+#include <type_traits>
 
 #include <cooperative_groups.h>
 
@@ -1545,29 +1546,38 @@ k_tsqbx3(qbxfmm_geometry g, SourceCoeffs sc, int nrhs, const double* __restrict_
       }
       __syncthreads();
       const int jend = min(warp * 32 + 32, total - base);
-      for (int j = warp * 32 + (lane >> 3); j < jend; j += 4) {
-        const double2 ya = s_a[j], yb = s_b[j];
-        const double2 mc = DIP ? s_c[j] : c2(0.0);
-        const double m2 = BOTH ? s_d[j] : yb.y;
+      // straight-line code per number of octets, so that their chains interleave
+      auto run = [&](auto octets) {
+        constexpr int NO = decltype(octets)::value;
+        for (int j = warp * 32 + (lane >> 3); j < jend; j += 4) {
+          const double2 ya = s_a[j], yb = s_b[j];
+          const double2 mc = DIP ? s_c[j] : c2(0.0);
+          const double m2 = BOTH ? s_d[j] : yb.y;
 #pragma unroll
-        for (int o = 0; o < 4; ++o) {
-          if (o >= noct) break;
-          const double b0 = ya.x - cc[o][0], b1 = ya.y - cc[o][1], b2 = yb.x - cc[o][2];
-          const double rho = rsqrt_h(b0 * b0 + b1 * b1 + b2 * b2);
-          const double rho2 = rho * rho;
-          const double x = (a[o][0] * b0 + a[o][1] * b1 + a[o][2] * b2) * rho2;
-          const double y = aa[o] * rho2;
-          double v = 0.0;
-          if (CHG) v = yb.y * near_f<Q>(x, y);
-          if (DIP) {
-            const double bn = b0 * mc.x + b1 * mc.y + b2 * m2;
-            double u = -bn * near_h<Q>(x, y);
-            if (Q > 0)
-              u = fma(a[o][0] * mc.x + a[o][1] * mc.y + a[o][2] * m2, near_dx<Q>(x, y), u);
-            v = CHG ? fma(rho2, u, v) : rho2 * u;
+          for (int o = 0; o < NO; ++o) {
+            const double b0 = ya.x - cc[o][0], b1 = ya.y - cc[o][1], b2 = yb.x - cc[o][2];
+            const double rho = rsqrt_h(b0 * b0 + b1 * b1 + b2 * b2);
+            const double rho2 = rho * rho;
+            const double x = (a[o][0] * b0 + a[o][1] * b1 + a[o][2] * b2) * rho2;
+            const double y = aa[o] * rho2;
+            double v = 0.0;
+            if (CHG) v = yb.y * near_f<Q>(x, y);
+            if (DIP) {
+              const double bn = b0 * mc.x + b1 * mc.y + b2 * m2;
+              double u = -bn * near_h<Q>(x, y);
+              if (Q > 0)
+                u = fma(a[o][0] * mc.x + a[o][1] * mc.y + a[o][2] * m2, near_dx<Q>(x, y), u);
+              v = CHG ? fma(rho2, u, v) : rho2 * u;
+            }
+            acc[o] = fma(rho, v, acc[o]);
           }
-          acc[o] = fma(rho, v, acc[o]);
         }
+      };
+      switch (noct) {
+        case 1: run(std::integral_constant<int, 1>()); break;
+        case 2: run(std::integral_constant<int, 2>()); break;
+        case 3: run(std::integral_constant<int, 3>()); break;
+        default: run(std::integral_constant<int, 4>()); break;
       }
       __syncthreads();
     }

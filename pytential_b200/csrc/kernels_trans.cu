@@ -262,116 +262,168 @@ k_trans_gemm(int ncf, int rp, int kp, int nrhs, int nwm, const double* __restric
   }
 }
 
-// Tiled form for large matrices (rp >= 256): CTA tile of 64 rows x 64 columns
-// (pair x rhs), K streamed in chunks of 32; warp (wm, wn) owns 32 x 32 of the tile
-// as 4 x 4 m8n8 accumulators.  Groups g0 .. g0 + gridDim.z - 1 (blockIdx.z).  The
-// result is added (x scale) into pair_dst's expansion when given (the caller
-// guarantees each destination occurs once per launch), else stored per pair.
-constexpr int GT_M = 64, GT_N = 64, GT_K = 32;
-constexpr int GT_AS = GT_K + 4;      // A row stride (doubles)
-constexpr int GT_BS = GT_N + 8;      // B row stride (doubles)
+// Tiled form for large matrices (3D Helmholtz M2M / L2L): CTA tile of 64 rows x 64 columns
+// (box x rhs), K streamed in chunks of 16 through a cp.async pipeline of GT_ST stages (the
+// synchronous form waited for two rounds of global loads per chunk: 8.8 us of 140 us a
+// launch); warp (wm, wn) owns 32 x 32 of the tile as 4 x 4 m8n8 accumulators.  Both
+// operands are staged k-contiguous with a row stride of 20 doubles (4 mod 16), free of
+// bank conflicts as fragments.
+//   L2L (SUM false): blockIdx.z = one of the level's eight groups; a group's children are
+//   distinct, so each column is added into its child.
+//   M2M (SUM true): a cluster of eight CTAs along z, one per child position of the
+//   parents of the column tile; the eight products are summed in a fixed order through
+//   distributed shared memory (rank q sums the rows 8 q .. 8 q + 7) and added into the
+//   parents: one launch per level instead of eight that follow one another.
+constexpr int GT_M = 64, GT_N = 64, GT_K = 16, GT_ST = 4;
+constexpr int GT_S = GT_K + 4;               // row stride of a staged operand (doubles)
+constexpr int GT_STAGE = (GT_M + GT_N) * GT_S;
+constexpr int GT_CS = GT_N + 4;              // row stride of the result tile (doubles)
 
-__global__ void __launch_bounds__(NT)
-k_trans_gemm_tiled(int ncf, int rp, int kp, int nrhs, const double* __restrict__ T, int mat_mod,
-                   const int32_t* __restrict__ group_starts, int g0,
-                   const int32_t* __restrict__ pair_src, const int32_t* __restrict__ pair_dst,
-                   const double2* __restrict__ ein, double2* __restrict__ eout, double scale,
-                   double* __restrict__ cpair, int32_t* err, int nboxes)
+QBX_D void cp_async16_zfill(void* dst, const void* src, bool on)
 {
-  __shared__ __align__(16) double As[GT_M][GT_AS];
-  __shared__ __align__(16) double Bs[GT_K][GT_BS];
-  __shared__ int s_src[GT_N];
-  int grp = g0 + blockIdx.z;
-  int p0 = group_starts[grp], p1 = group_starts[grp + 1];
-  int ncol = (p1 - p0) * nrhs;
-  int c0 = blockIdx.x * GT_N;
-  int m0 = blockIdx.y * GT_M;
-  if (c0 >= ncol || m0 >= rp) return;
-  int mat = mat_mod > 0 ? (grp % mat_mod) : grp;
-  const double* Tg = T + (size_t)mat * rp * kp;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(on ? 16 : 0)
+               : "memory");
+}
+
+template <bool SUM>
+__global__ void __launch_bounds__(NT)
+k_trans_gemm_pipe(qbxfmm_geometry g, int ncf, int rp, int kp, int nrhs,
+                  const double* __restrict__ T, int mat_mod, int g0, int i0, int i1,
+                  double2* __restrict__ exps, int32_t* err)
+{
+  extern __shared__ double2 smem2[];
+  double* sm = reinterpret_cast<double*>(smem2);
+  __shared__ int s_src[GT_N], s_dst[GT_N];
+  const int grp = g0 + blockIdx.z;
+  const int p0 = SUM ? i0 : g.l2l_group_starts[grp], p1 = SUM ? i1 : g.l2l_group_starts[grp + 1];
+  const int ncol = (p1 - p0) * nrhs;
+  const int c0 = blockIdx.x * GT_N, m0 = blockIdx.y * GT_M;
+  if (!SUM && c0 >= ncol) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int R = 2 * ncf;
-  for (int j = threadIdx.x; j < GT_N; j += NT) {
-    int c = c0 + j;
-    int src = -1;
+  bool any = false;
+  for (int j = tid; j < GT_N; j += NT) {
+    const int c = c0 + j;
+    int src = -1, dst = -1;
     if (c < ncol) {
-      src = pair_src[p0 + c / nrhs];
-      if ((unsigned)src >= (unsigned)nboxes) {
-        report(err, QBX_DEVERR_BAD_BOX);
-        src = -1;
+      const int q = p0 + c / nrhs;
+      if (SUM) {
+        dst = g.source_parent_boxes[q];
+        if ((unsigned)dst < (unsigned)g.nboxes) {
+          src = g.box_child_ids[(size_t)blockIdx.z * g.nboxes + dst];
+          if (src == 0) src = -1;                        // no such child
+          else if ((unsigned)src >= (unsigned)g.nboxes) report(err, QBX_DEVERR_BAD_BOX), src = -1;
+          else if (g.box_source_counts_cumul[src] == 0) src = -1;
+        }
+      } else {
+        src = g.l2l_pair_src[q];
+        dst = g.l2l_pair_dst[q];
+        if ((unsigned)src >= (unsigned)g.nboxes) report(err, QBX_DEVERR_BAD_BOX), src = -1;
       }
+      if ((unsigned)dst >= (unsigned)g.nboxes) report(err, QBX_DEVERR_BAD_BOX), dst = -1;
     }
     s_src[j] = src;
+    s_dst[j] = dst;
+    any |= src >= 0;
   }
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int g = lane >> 2, tq = lane & 3;
-  int wm = warp & 1, wn = warp >> 1;
+  any = __syncthreads_or(any);
+  const double* Tg = T + (size_t)(mat_mod > 0 ? grp % mat_mod : grp) * rp * kp;
+  // this thread's 16-byte pieces of a chunk: rows / columns tid / 8 + 16 i, k = 2 (tid % 8)
+  const int kk = 2 * (tid & 7), rb = tid >> 3;
+  const double* ap[4];
+  const double* bp[4];
+  bool aon[4], bon[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = m0 + rb + 16 * i, src = s_src[rb + 16 * i];
+    aon[i] = row < rp;
+    ap[i] = Tg + (size_t)(aon[i] ? row : 0) * kp + kk;
+    bon[i] = src >= 0;
+    bp[i] = reinterpret_cast<const double*>(
+                exps + ((size_t)(bon[i] ? src : 0) * nrhs + (c0 + rb + 16 * i) % nrhs) * ncf) + kk;
+  }
+  const int nk = any ? (R + GT_K - 1) / GT_K : 0;
+  auto fetch = [&](int ck) {
+    if (ck < nk) {
+      double* A = sm + (ck % GT_ST) * GT_STAGE;
+      double* B = A + GT_M * GT_S;
+      const bool in = ck * GT_K + kk < R;                // kp >= R; the rest is zero
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const bool a = aon[i] && in, b = bon[i] && in;
+        cp_async16_zfill(A + (rb + 16 * i) * GT_S + kk, a ? ap[i] + ck * GT_K : Tg, a);
+        cp_async16_zfill(B + (rb + 16 * i) * GT_S + kk, b ? bp[i] + ck * GT_K : Tg, b);
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  const int row = lane >> 2, tq = lane & 3, wm = warp & 1, wn = warp >> 1;
   double acc[4][4][2];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  for (int kc = 0; kc < kp; kc += GT_K) {
+  for (int i = 0; i < GT_ST - 1; ++i) fetch(i);
+  for (int ck = 0; ck < nk; ++ck) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(GT_ST - 2) : "memory");
     __syncthreads();
-    // 16-byte loads and stores (kp, kc, GT_AS, R and the matrix offsets are even)
-    constexpr int KH = GT_K / 2;
-    for (int e = threadIdx.x; e < GT_M * KH; e += NT) {
-      const int row = e / KH, k = 2 * (e - row * KH);
-      const double2 v = (m0 + row < rp && kc + k < kp)
-          ? __ldg(reinterpret_cast<const double2*>(Tg + (size_t)(m0 + row) * kp + kc + k)) : c2(0.0);
-      *reinterpret_cast<double2*>(&As[row][k]) = v;
-    }
-    for (int e = threadIdx.x; e < GT_N * KH; e += NT) {
-      const int j = e / KH, k = 2 * (e - j * KH);
-      const int src = s_src[j];
-      double2 v = c2(0.0);
-      if (src >= 0 && kc + k < R)
-        v = __ldg(ein + ((size_t)src * nrhs + (c0 + j) % nrhs) * ncf + ((kc + k) >> 1));
-      Bs[k][j] = v.x;
-      Bs[k + 1][j] = v.y;
-    }
-    __syncthreads();
+    fetch(ck + GT_ST - 1);                               // into the stage read last round
+    const double* A = sm + (ck % GT_ST) * GT_STAGE + (wm * 32 + row) * GT_S + tq;
+    const double* B = sm + (ck % GT_ST) * GT_STAGE + (GT_M + wn * 32 + row) * GT_S + tq;
 #pragma unroll
     for (int k0 = 0; k0 < GT_K; k0 += 4) {
       double a[4], b[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[wm * 32 + i * 8 + g][k0 + tq];
+      for (int i = 0; i < 4; ++i) a[i] = A[i * 8 * GT_S + k0];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[k0 + tq][wn * 32 + j * 8 + g];
+      for (int j = 0; j < 4; ++j) b[j] = B[j * 8 * GT_S + k0];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
     }
   }
-  // epilogue: acc[i][j][v] = C[row = m0 + wm*32 + i*8 + g][col = c0 + wn*32 + j*8 + 2 tq + v]
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  // acc[i][j][v] = C[row m0 + wm 32 + 8 i + row][column c0 + wn 32 + 8 j + 2 tq + v]
+  if constexpr (!SUM) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < 4; ++j)
 #pragma unroll
-    for (int v = 0; v < 2; ++v) {
-      int c = c0 + wn * 32 + j * 8 + 2 * tq + v;
-      if (c >= ncol) continue;
-      int pr = p0 + c / nrhs, r = c % nrhs;
-      if (pair_dst) {
-        int dst = pair_dst[pr];
-        if ((unsigned)dst >= (unsigned)nboxes) {
-          report(err, QBX_DEVERR_BAD_BOX);
-          continue;
-        }
-        double* y = reinterpret_cast<double*>(eout + ((size_t)dst * nrhs + r) * ncf);
+      for (int v = 0; v < 2; ++v) {
+        const int jc = wn * 32 + j * 8 + 2 * tq + v, dst = s_dst[jc];
+        if (dst < 0) continue;
+        double* y = reinterpret_cast<double*>(exps + ((size_t)dst * nrhs + (c0 + jc) % nrhs) * ncf);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          int row = m0 + wm * 32 + i * 8 + g;
-          if (row < R) y[row] += scale * acc[i][j][v];
-        }
-      } else {
-        double* y = cpair + ((size_t)pr * nrhs + r) * rp;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          int row = m0 + wm * 32 + i * 8 + g;
-          if (row < rp) y[row] = acc[i][j][v];
+          const int rr = m0 + wm * 32 + i * 8 + row;
+          if (rr < R) y[rr] += acc[i][j][v];
         }
       }
+  } else {
+    cg::cluster_group cl = cg::this_cluster();
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int v = 0; v < 2; ++v)
+          sm[(wm * 32 + i * 8 + row) * GT_CS + wn * 32 + j * 8 + 2 * tq + v] = acc[i][j][v];
+    cl.sync();
+    const int rank = blockIdx.z;
+    for (int e = tid; e < 8 * GT_N; e += NT) {
+      const int jc = e >> 3, rl = 8 * rank + (e & 7), rr = m0 + rl;
+      double v = 0.0;
+      for (int z = 0; z < 8; ++z) v += cl.map_shared_rank(sm, z)[rl * GT_CS + jc];
+      const int dst = s_dst[jc];
+      if (dst < 0 || rr >= R) continue;
+      double* y = reinterpret_cast<double*>(exps + ((size_t)dst * nrhs + (c0 + jc) % nrhs) * ncf);
+      y[rr] += v;
     }
+    cl.sync();
+  }
 }
 
 // out box o (o = boxes[obase + blockIdx.x]): eout[o][r] += scale(o) sum_{pairs} cpair[pair][r]
@@ -766,36 +818,43 @@ cudaError_t launch_trans_reduce_m2m(const qbxfmm_geometry& g, const TransHost& t
   return cudaGetLastError();
 }
 
-static cudaError_t gemm_tiled_launch(const qbxfmm_geometry& g, const TransCfg& c, int nrhs,
-                                     const double* T, size_t mat_base, int mat_mod,
-                                     const int32_t* group_starts_dev, int g0, int ngroups,
-                                     int maxcols, const int32_t* pair_src, const int32_t* pair_dst,
-                                     const double2* ein, double2* eout, double scale,
-                                     double* cpair, int32_t* err, cudaStream_t st)
+template <bool SUM>
+static cudaError_t gemm_pipe_launch(const qbxfmm_geometry& g, const TransCfg& c, int nrhs,
+                                    const double* T, size_t mat_base, int g0, int i0, int i1,
+                                    int maxcols, double2* exps, int32_t* err, cudaStream_t st)
 {
-  if (ngroups <= 0 || maxcols <= 0) return cudaSuccess;
-  dim3 grid((maxcols + GT_N - 1) / GT_N, (c.rp + GT_M - 1) / GT_M, ngroups);
-  k_trans_gemm_tiled<<<grid, NT, 0, st>>>(c.ncf, c.rp, c.kp, nrhs, T + mat_base * (size_t)c.rp * c.kp,
-                                          mat_mod, group_starts_dev, g0, pair_src, pair_dst, ein,
-                                          eout, scale, cpair, err, g.nboxes);
-  return cudaGetLastError();
+  if (maxcols <= 0) return cudaSuccess;
+  const size_t sh = (size_t)std::max(GT_ST * GT_STAGE, GT_M * GT_CS) * sizeof(double);
+  cudaError_t e = cudaFuncSetAttribute(k_trans_gemm_pipe<SUM>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((maxcols + GT_N - 1) / GT_N, (2 * c.ncf + GT_M - 1) / GT_M, 8);
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = sh;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = SUM ? 8 : 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_trans_gemm_pipe<SUM>, g, c.ncf, c.rp, c.kp, nrhs,
+                            T + mat_base * (size_t)c.rp * c.kp, c.m2m_mat_mod, g0, i0, i1, exps,
+                            err);
 }
 
-// M2M without pair scratch: one launch per (parent level, child position) group,
-// whose parents are distinct.
+// M2M without pair scratch: one launch per parent level
 cudaError_t launch_m2m_direct(const qbxfmm_geometry& g, const TransHost& th, const TransCfg& c,
                               int nrhs, const double* T, double2* mp, int32_t* err, cudaStream_t st)
 {
-  const int nch = 8;
   for (int lev = g.nlevels - 2; lev >= 0; --lev) {
-    int maxp = th.m2m_level_max_group[lev];
-    if (maxp == 0) continue;
-    for (int ci = 0; ci < nch; ++ci) {
-      cudaError_t e = gemm_tiled_launch(g, c, nrhs, T, c.m2m_base, c.m2m_mat_mod, g.m2m_group_starts,
-                                        lev * nch + ci, 1, maxp * nrhs, g.m2m_pair_src,
-                                        g.m2m_pair_dst, mp, mp, 1.0, nullptr, err, st);
-      if (e != cudaSuccess) return e;
-    }
+    if (th.m2m_level_max_group[lev] == 0) continue;
+    const int i0 = th.lvl_source_parent[lev], i1 = th.lvl_source_parent[lev + 1];
+    cudaError_t e = gemm_pipe_launch<true>(g, c, nrhs, T, c.m2m_base, lev * 8, i0, i1,
+                                           (i1 - i0) * nrhs, mp, err, st);
+    if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
@@ -804,13 +863,9 @@ cudaError_t launch_m2m_direct(const qbxfmm_geometry& g, const TransHost& th, con
 cudaError_t launch_l2l_direct(const qbxfmm_geometry& g, const TransHost& th, const TransCfg& c,
                               int nrhs, const double* T, double2* lo, int32_t* err, cudaStream_t st)
 {
-  const int nch = 8;
   for (int lev = 1; lev < g.nlevels; ++lev) {
-    int maxp = th.l2l_level_max_group[lev];
-    if (maxp == 0) continue;
-    cudaError_t e = gemm_tiled_launch(g, c, nrhs, T, c.l2l_base, c.m2m_mat_mod, g.l2l_group_starts,
-                                      lev * nch, nch, maxp * nrhs, g.l2l_pair_src, g.l2l_pair_dst,
-                                      lo, lo, 1.0, nullptr, err, st);
+    cudaError_t e = gemm_pipe_launch<false>(g, c, nrhs, T, c.l2l_base, lev * 8, 0, 0,
+                                            th.l2l_level_max_group[lev] * nrhs, lo, err, st);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

@@ -189,11 +189,12 @@ k_h3_near(qbxfmm_geometry g, HelmCoeffs hc, int nrhs, const double2* __restrict_
           if (dip) K = cfma(kD, cscale(rho, vD), K);
           if (j >= ns || bs == 0.0) K = c2(0.0);
           const double* B = S + j * SS;
-          const double sg = (row & 1) ? K.y : -K.y;
 #pragma unroll
           for (int n = 0; n < NT; ++n) {
+            // columns (density, part): i sigma has (-im, re) there
+            const double bx = B[8 * n + (row ^ 1)];
             h3_dmma(acc[n][0], acc[n][1], K.x, B[8 * n + row]);
-            h3_dmma(acc[n][0], acc[n][1], sg, B[8 * n + (row ^ 1)]);
+            h3_dmma(acc[n][0], acc[n][1], K.y, (row & 1) ? bx : -bx);
           }
         }
       }

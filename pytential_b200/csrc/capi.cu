@@ -1259,11 +1259,12 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
   cudaStream_t st = S(stream);
   QBX_TRY(cudaMemsetAsync(ws->mpoles, 0, sz[1], st), "apply: clear");
   QBX_TRY(cudaMemsetAsync(ws->locals, 0, sz[2], st), "apply: clear");
-  // 3D Helmholtz in FP64 with the target-specific near field: the list-3 multipoles go
-  // straight to the QBX targets and, in the compressed-Taylor truncation, the box locals
-  // too (then no QBX expansions are formed)
-  const bool m2t = p->h3 && !p->mixed && p->kern.target_specific_qbx != 0 && h3_m2t_wins(p->geo);
-  const bool l2t = m2t && p->hc.taylor;
+  // Helmholtz in FP64 with the target-specific near field: the list-3 multipoles go straight
+  // to the QBX targets, and the box locals too (then no QBX expansions are formed) except in
+  // the spherical-wave truncation in 3D
+  const bool direct = p->helm && !p->mixed && p->kern.target_specific_qbx != 0;
+  const bool m2t = direct && (p->h3 ? h3_m2t_wins(p->geo) : h2_e2t_wins(p->geo, p->kern.nrhs));
+  const bool l2t = m2t && (!p->h3 || p->hc.taylor);
   if (!l2t) QBX_TRY(cudaMemsetAsync(ws->qbx_exps, 0, sz[3], st), "apply: clear");
   QBX_TRY(cudaMemsetAsync(ws->pot_nonqbx, 0, sz[4], st), "apply: clear");
   QBX_TRY(cudaMemsetAsync(ws->pot_tree, 0, sz[5], st), "apply: clear");
@@ -1336,10 +1337,15 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
                                                           ws->error_word, s3));
   QBX_CUDA_STEP(cudaEventRecord(p->ev_qbx, side3), "apply: QBX-expansion event");
   QBX_CUDA_STEP(cudaStreamWaitEvent(side1, p->ev_mpoles, 0), "apply: multipole event");
-  if (m2t)
+  if (m2t && p->h3)
     QBX_CUDA_STEP(h3_launch_m2t(p->geo, p->hc, p->kern.fmm_order, p->kern.qbx_order, p->kern.nrhs,
                                 (const double2*)ws->mpoles, (double2*)ws->pot_tree,
                                 ws->error_word, side1),
+                  "apply: multipoles to QBX targets");
+  else if (m2t)
+    QBX_CUDA_STEP(h2_launch_e2t(p->geo, p->hc.k, p->kern.fmm_order, p->kern.qbx_order,
+                                p->kern.nrhs, false, (const double2*)ws->mpoles,
+                                (double2*)ws->pot_tree, ws->error_word, side1),
                   "apply: multipoles to QBX targets");
   QBX_STEP(qbxfmm_eval_multipoles(p, ws->mpoles, ws->pot_nonqbx, ws->error_word, s1));
   QBX_CUDA_STEP(cudaEventRecord(p->ev_near, side1), "apply: near-field event");
@@ -1352,7 +1358,11 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
   forked = false;
 #undef QBX_STEP
 #undef QBX_CUDA_STEP
-  if (l2t) {
+  if (l2t && !p->h3) {
+    QBX_TRY(h2_launch_e2t(p->geo, p->hc.k, p->kern.fmm_order, p->kern.qbx_order, p->kern.nrhs, true,
+                          (const double2*)ws->locals, (double2*)ws->pot_tree, ws->error_word, st),
+            "apply: locals to QBX targets");
+  } else if (l2t) {
     size_t o[8];
     h3_layout(p, o);
     QBX_TRY(h3_launch_l2t_taylor(p->geo, p->hc, p->kern.fmm_order, p->kern.qbx_order, p->kern.nrhs,

@@ -148,6 +148,13 @@ cudaError_t h2_launch_eval_locals(const qbxfmm_geometry& g, HelmCoeffs hc, int p
                                   const double2* lo, double2* pot, int32_t* err, cudaStream_t st);
 cudaError_t h2_launch_p2qbxl(const qbxfmm_geometry& g, HelmCoeffs hc, int q, int nrhs,
                              const double2* s, double2* qe, int32_t* err, cudaStream_t st);
+// list-3 multipoles (from_local false) or the target box's local straight to the QBX
+// targets (the expansions' stages in one, added into pot_tree); h2_e2t_wins: whether that
+// is less work than the expansions
+cudaError_t h2_launch_e2t(const qbxfmm_geometry& g, double k, int p, int q, int nrhs,
+                          bool from_local, const double2* exps, double2* pot_tree, int32_t* err,
+                          cudaStream_t st);
+bool h2_e2t_wins(const qbxfmm_geometry& g, int nrhs);
 cudaError_t h2_launch_m2qbxl(const qbxfmm_geometry& g, HelmCoeffs hc, int pf, int q, int nrhs,
                              const double2* mp, double2* qe, int32_t* err, cudaStream_t st);
 cudaError_t h2_launch_l2qbxl(const qbxfmm_geometry& g, HelmCoeffs hc, int pf, int q, int nrhs,

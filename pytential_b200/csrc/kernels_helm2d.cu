@@ -97,22 +97,36 @@ QBX_D double2 hbar(const double2* Z, int N, int m)
 
 // {{{ strengths (complex density)
 
+// One thread per tree source and up to FS_RB densities: a source's interpolation row (a
+// strided read of the matrix) serves all of them.
+constexpr int FS_RB = 8;
+
 __global__ void __launch_bounds__(256)
-k_h2_form_strengths(int nsources, int ndofs, int npe, int nqpe, const double* __restrict__ U,
-                    const double* __restrict__ qw, const int32_t* __restrict__ user_source_ids,
+k_h2_form_strengths(int nsources, int ndofs, int npe, int nqpe, int nrhs,
+                    const double* __restrict__ U, const double* __restrict__ qw,
+                    const int32_t* __restrict__ user_source_ids,
                     const double2* __restrict__ density, double2* __restrict__ out)
 {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  int r = blockIdx.y;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r0 = blockIdx.y * FS_RB, nr = min(FS_RB, nrhs - r0);
   if (t >= nsources) return;
-  int j = __ldg(user_source_ids + t);
-  int e = j / nqpe;
-  int jj = j - e * nqpe;
-  const double* u = U + (size_t)jj * npe;
-  const double2* d = density + (size_t)r * ndofs + (size_t)e * npe;
-  double2 acc = c2(0.0);
-  for (int i = 0; i < npe; ++i) acc = caxpy(__ldg(u + i), d[i], acc);
-  out[(size_t)r * nsources + t] = cscale(__ldg(qw + j), acc);
+  const int j = __ldg(user_source_ids + t);
+  const int e = j / nqpe;
+  const double* u = U + (size_t)(j - e * nqpe) * npe;
+  const double2* d = density + (size_t)r0 * ndofs + (size_t)e * npe;
+  double2 acc[FS_RB];
+#pragma unroll
+  for (int r = 0; r < FS_RB; ++r) acc[r] = c2(0.0);
+  for (int i = 0; i < npe; ++i) {
+    const double w = __ldg(u + i);
+#pragma unroll
+    for (int r = 0; r < FS_RB; ++r)
+      if (r < nr) acc[r] = caxpy(w, __ldg(d + (size_t)r * ndofs + i), acc[r]);
+  }
+  const double w = __ldg(qw + j);
+#pragma unroll
+  for (int r = 0; r < FS_RB; ++r)
+    if (r < nr) out[(size_t)(r0 + r) * nsources + t] = cscale(w, acc[r]);
 }
 
 // }}}
@@ -124,7 +138,8 @@ k_h2_form_strengths(int nsources, int ndofs, int npe, int nqpe, const double* __
 //   P2L: W(m) = cq Hb_m + kd (conj(nu) Hb_{m-1} - nu Hb_{m+1})
 // (kd = (k/2) cd) do not depend on the density, so a box is a (2p+1) x nsrc times
 // nsrc x rhs complex product.  One CTA per (box, tile of RW * TR right-hand sides),
-// thread layout as in k_h2_translate; SUB sources per stage: Bessel tables one per
+// thread t: right-hand sides rl + RW j
+// (rl = t % RW, j < TR) and coefficients mg + G i (mg = t / RW, G = NT / RW); SUB sources per stage: Bessel tables one per
 // thread, then W and the strengths tile in shared memory.
 template <bool LOCAL, int RW, int TR>
 __global__ void __launch_bounds__(NT)
@@ -241,142 +256,6 @@ k_h2_p2e(qbxfmm_geometry g, HelmCoeffs hc, int p, int nrhs, const double2* __res
       if (r < nr) E[(size_t)r * NC + m] = caxpy(sc, acc[a][jj], E[(size_t)r * NC + m]);
     }
   }
-}
-
-// }}}
-
-// {{{ translations: M2M, L2L (per level), M2L (list 2)
-
-// Eout_m[r] += fout(m) sum_n Z_{n-m}(d) fin(n) Ein_n[r] with Z = J (M2M, L2L) or H (M2L):
-// per source box a Toeplitz (2p+1) x (2p+1) matrix applied to a tile of right-hand
-// sides.  One CTA per (output box, tile of RW * TR right-hand sides); thread t takes
-// the right-hand sides rl + RW j (rl = t % RW, j < TR) and the coefficients
-// mg + G i (mg = t / RW, G = NT / RW, i < TM), all in registers.  The Z tables (order
-// 2p) of up to PB source boxes are built one per thread into shared memory, once for
-// the whole tile; each source box's coefficient block ([rhs][coef], contiguous in
-// global memory) is staged scaled by fin(n) into shared memory with coalesced loads.
-template <int KIND, int RW, int TR>   // KIND 0 = M2M, 1 = M2L, 2 = L2L
-__global__ void __launch_bounds__(NT)
-k_h2_translate(qbxfmm_geometry g, HelmCoeffs hc, int p, int nrhs, int i0,
-               const double2* __restrict__ ein, double2* __restrict__ eout, int32_t* err)
-{
-  constexpr int PB = 16;
-  constexpr int G = NT / RW;
-  constexpr int TM = (2 * 20 + 1 + G - 1) / G;
-  constexpr int RC = RW * TR;
-  extern __shared__ double2 smem2[];
-  const int NZ = 2 * p, ZW = 2 * NZ + 1, NC = 2 * p + 1;
-  double2* Z = smem2;                       // [PB][ZW]
-  double2* E = Z + (size_t)PB * ZW;         // [RC][NC]
-  __shared__ int s_src[PB];
-  __shared__ double s_fin[PB][2 * 20 + 1];
-  double Jb[ZMAX], Yb[ZMAX];
-  int ib = i0 + blockIdx.x;
-  int r0 = blockIdx.y * RC;
-  int nr = min(RC, nrhs - r0);
-  int tb;
-  int l0, l1;
-  if (KIND == 0) {
-    tb = g.source_parent_boxes[ib];
-    l0 = 0;
-    l1 = 4;     // children
-  } else if (KIND == 1) {
-    tb = g.target_or_target_parent_boxes[ib];
-    l0 = g.list2_starts[ib];
-    l1 = g.list2_starts[ib + 1];
-  } else {
-    tb = g.target_or_target_parent_boxes[ib];
-    l0 = 0;
-    l1 = 1;     // parent
-  }
-  double ct[2];
-  load_point<2>(g.box_centers, g.nboxes, tb, ct);
-  const int rl = threadIdx.x % RW, mg = threadIdx.x / RW;
-  double2 acc[TM][TR];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TR; ++j) acc[i][j] = c2(0.0);
-  for (int lb = l0; lb < l1; lb += PB) {
-    int nbat = min(PB, l1 - lb);
-    __syncthreads();
-    if (threadIdx.x < nbat) {
-      int sb;
-      if (KIND == 0) {
-        sb = g.box_child_ids[(size_t)(lb + threadIdx.x) * g.nboxes + tb];
-        if (sb == 0 || g.box_source_counts_cumul[sb] == 0) sb = -1;
-      } else if (KIND == 1) {
-        sb = g.list2_lists[lb + threadIdx.x];
-        if ((unsigned)sb >= (unsigned)g.nboxes) {
-          report(err, QBX_DEVERR_BAD_BOX);
-          sb = -1;
-        }
-      } else {
-        sb = g.box_parent_ids[tb];
-      }
-      s_src[threadIdx.x] = sb;
-      if (sb >= 0) {
-        double cs[2];
-        load_point<2>(g.box_centers, g.nboxes, sb, cs);
-        // d = c_out - c_in
-        h2_zfun(NZ, hc.k, ct[0] - cs[0], ct[1] - cs[1], Jb, Yb, Z + (size_t)threadIdx.x * ZW,
-                KIND == 1);
-      }
-    }
-    __syncthreads();
-    for (int w = threadIdx.x; w < nbat * NC; w += NT) {
-      int bb = w / NC, n = w - bb * NC - p;
-      int sb = s_src[bb];
-      if (sb >= 0) {
-        double rin = level_width(g, g.box_levels[sb]);
-        int an = n < 0 ? -n : n;
-        s_fin[bb][n + p] = (KIND == 2) ? pow(rin, -(double)an) : pow(rin, (double)an);
-      }
-    }
-    for (int bb = 0; bb < nbat; ++bb) {
-      int sb = s_src[bb];
-      if (sb < 0) continue;      // uniform over the CTA
-      __syncthreads();           // E free, s_fin written
-      const double2* src = ein + ((size_t)sb * nrhs + r0) * NC;
-      for (int w = threadIdx.x; w < nr * NC; w += NT) {
-        int n = w % NC;
-        E[w] = cscale(s_fin[bb][n], src[w]);
-      }
-      __syncthreads();
-      // Z_{n-m} for coefficient indices n, m in [0, 2p] at Zt[n - m]
-      const double2* Zt = Z + (size_t)bb * ZW + NZ;
-      for (int n = 0; n < NC; ++n) {
-        double2 e[TR];
-#pragma unroll
-        for (int j = 0; j < TR; ++j) e[j] = E[(rl + RW * j) * NC + n];
-#pragma unroll
-        for (int i = 0; i < TM; ++i) {
-          int m = min(mg + G * i, NC - 1);
-          double2 z = Zt[n - m];
-#pragma unroll
-          for (int j = 0; j < TR; ++j) acc[i][j] = cfma(z, e[j], acc[i][j]);
-        }
-      }
-    }
-  }
-  // the tile through shared memory, then one coalesced read-modify-write
-  double rho_t = level_width(g, g.box_levels[tb]);
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    int m = mg + G * i;
-    if (m >= NC) continue;
-    int am = m - p < 0 ? p - m : m - p;
-    double f = (KIND == 0) ? pow(rho_t, -(double)am) : pow(rho_t, (double)am);
-#pragma unroll
-    for (int j = 0; j < TR; ++j) {
-      int r = rl + RW * j;
-      if (r < nr) E[r * NC + m] = cscale(f, acc[i][j]);
-    }
-  }
-  __syncthreads();
-  double2* dst = eout + ((size_t)tb * nrhs + r0) * NC;
-  for (int w = threadIdx.x; w < nr * NC; w += NT) dst[w] = cadd(dst[w], E[w]);
 }
 
 // }}}
@@ -1179,9 +1058,9 @@ static size_t zsh(int p) { return (size_t)(2 * (p + 1) + 1); }
 cudaError_t h2_launch_form_strengths(const qbxfmm_geometry& g, const qbxfmm_upsample& up, int nrhs,
                                      const double2* density, double2* strengths, cudaStream_t st)
 {
-  dim3 grid((g.nsources + 255) / 256, nrhs);
+  dim3 grid((g.nsources + 255) / 256, (nrhs + FS_RB - 1) / FS_RB);
   k_h2_form_strengths<<<grid, 256, 0, st>>>(g.nsources, up.nelements * up.nodes_per_element,
-                                            up.nodes_per_element, up.quad_nodes_per_element,
+                                            up.nodes_per_element, up.quad_nodes_per_element, nrhs,
                                             up.matrix, up.quad_weights, g.user_source_ids, density,
                                             strengths);
   return cudaGetLastError();
@@ -1227,64 +1106,6 @@ cudaError_t h2_launch_p2l(const qbxfmm_geometry& g, HelmCoeffs hc, int p, int nr
 }
 
 // right-hand-side tiling of the translation kernels: (lanes over rhs, rhs per lane)
-template <int KIND, int RW, int TR>
-static cudaError_t h2_translate_rt(const qbxfmm_geometry& g, HelmCoeffs hc, int p, int nrhs,
-                                   int i0, int nb, const double2* ein, double2* eout, int32_t* err,
-                                   cudaStream_t st)
-{
-  size_t sh = ((size_t)16 * (4 * p + 1) + (size_t)RW * TR * (2 * p + 1)) * sizeof(double2);
-  cudaError_t e = cudaFuncSetAttribute(k_h2_translate<KIND, RW, TR>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-  if (e != cudaSuccess) return e;
-  dim3 grid(nb, (nrhs + RW * TR - 1) / (RW * TR));
-  k_h2_translate<KIND, RW, TR><<<grid, NT, sh, st>>>(g, hc, p, nrhs, i0, ein, eout, err);
-  return cudaGetLastError();
-}
-
-template <int KIND>
-static cudaError_t h2_translate(const qbxfmm_geometry& g, HelmCoeffs hc, int p, int nrhs, int i0,
-                                int nb, const double2* ein, double2* eout, int32_t* err,
-                                cudaStream_t st)
-{
-  if (p > 20) return cudaErrorInvalidValue;
-  if (nrhs == 1) return h2_translate_rt<KIND, 1, 1>(g, hc, p, nrhs, i0, nb, ein, eout, err, st);
-  if (nrhs <= 4) return h2_translate_rt<KIND, 4, 1>(g, hc, p, nrhs, i0, nb, ein, eout, err, st);
-  if (nrhs <= 16) return h2_translate_rt<KIND, 16, 1>(g, hc, p, nrhs, i0, nb, ein, eout, err, st);
-  if (nrhs <= 32) return h2_translate_rt<KIND, 32, 1>(g, hc, p, nrhs, i0, nb, ein, eout, err, st);
-  return h2_translate_rt<KIND, 32, 2>(g, hc, p, nrhs, i0, nb, ein, eout, err, st);
-}
-
-cudaError_t h2_launch_m2m(const qbxfmm_geometry& g, const int32_t* lvl_host, HelmCoeffs hc, int p,
-                          int nrhs, double2* mp, int32_t* err, cudaStream_t st)
-{
-  for (int lev = g.nlevels - 2; lev >= 0; --lev) {
-    int i0 = lvl_host[lev], i1 = lvl_host[lev + 1];
-    if (i1 <= i0) continue;
-    cudaError_t e = h2_translate<0>(g, hc, p, nrhs, i0, i1 - i0, mp, mp, err, st);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
-}
-
-cudaError_t h2_launch_m2l(const qbxfmm_geometry& g, HelmCoeffs hc, int p, int nrhs,
-                          const double2* mp, double2* lo, int32_t* err, cudaStream_t st)
-{
-  if (g.nttp_boxes == 0) return cudaSuccess;
-  return h2_translate<1>(g, hc, p, nrhs, 0, g.nttp_boxes, mp, lo, err, st);
-}
-
-cudaError_t h2_launch_l2l(const qbxfmm_geometry& g, const int32_t* lvl_host, HelmCoeffs hc, int p,
-                          int nrhs, double2* lo, int32_t* err, cudaStream_t st)
-{
-  for (int lev = 1; lev < g.nlevels; ++lev) {
-    int i0 = lvl_host[lev], i1 = lvl_host[lev + 1];
-    if (i1 <= i0) continue;
-    cudaError_t e = h2_translate<2>(g, hc, p, nrhs, i0, i1 - i0, lo, lo, err, st);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
-}
-
 cudaError_t h2_launch_eval_direct(const qbxfmm_geometry& g, HelmCoeffs hc, int nrhs,
                                   const double2* s, double2* pot, int32_t* err, cudaStream_t st)
 {

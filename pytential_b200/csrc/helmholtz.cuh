@@ -10,7 +10,8 @@
 // Coefficients are scaled by rscale^|m| (multipoles divided, locals multiplied).
 //
 // Bessel functions: J_0..J_N by Miller's backward recurrence normalized with
-// J_0 + 2 sum_k J_2k = 1; Y_0, Y_1 from the CUDA math library (y0, y1) and
+// J_0 + 2 sum_k J_2k = 1; Y_0, Y_1 from the CUDA math library (y0, y1) below x = 8 and
+// their Neumann series above, where the library's error is absolute (5e-12);
 // Y_{n+1} = (2n/x) Y_n - Y_{n-1} (stable upward).
 #pragma once
 
@@ -18,12 +19,53 @@
 
 namespace qbx {
 
+// first index of Miller's recurrence for orders up to nmax and arguments up to nmax
+QBX_D int miller_start(int nmax) { return 2 * ((nmax + 16 + (int)sqrt(40.0 * nmax)) / 2); }
+
+// Y_0 and Y_1 at x > 0; from x = 8 on by Abramowitz & Stegun 9.1.88 and 9.1.89 over Miller's
+// J_k: (pi/2) Y_0 = (ln(x/2) + gamma) J_0 - 2 sum_k (-1)^k J_2k / k, (pi/2) Y_1 = (ln(x/2) +
+// gamma - 1) J_1 - J_0 / x - sum_k (-1)^k (2k+1) J_{2k+1} / (k (k+1))
+QBX_D void bessel_y01(double x, double& Y0, double& Y1)
+{
+  if (x < 8.0) {
+    Y0 = y0(x);
+    Y1 = y1(x);
+    return;
+  }
+  const double xinv = 1.0 / x;
+  double fp1 = 0.0, f = 1e-200, sum = 0.0, a = 0.0, b = 0.0;
+  for (int k = miller_start((int)x); k > 0; --k) {
+    const int m = k >> 1;
+    const double t = m & 1 ? -f : f;
+    if (!(k & 1)) {
+      sum += 2.0 * f;
+      a += t / m;
+    } else if (m > 0) {
+      b += t * (2 * m + 1) / ((double)m * (m + 1));
+    }
+    const double fm1 = 2.0 * k * xinv * f - fp1;
+    fp1 = f;
+    f = fm1;
+    if (fabs(f) > 1e200) {
+      f *= 1e-200;
+      fp1 *= 1e-200;
+      sum *= 1e-200;
+      a *= 1e-200;
+      b *= 1e-200;
+    }
+  }
+  const double norm = 1.0 / (sum + f), J0 = f * norm, J1 = fp1 * norm;
+  const double L = log(0.5 * x) + 0.57721566490153286061, c = 0.63661977236758134308;  // 2 / pi
+  Y0 = c * (L * J0 - 2.0 * a * norm);
+  Y1 = c * ((L - 1.0) * J1 - xinv * J0 - b * norm);
+}
+
 // J[0..N], Y[0..N] (Y only if want_y) at x > 0.
 QBX_D void bessel_jy(int N, double x, double* J, double* Y, bool want_y)
 {
   double xinv = 1.0 / x;
   int nmax = N > (int)x ? N : (int)x;
-  int start = 2 * ((nmax + 16 + (int)sqrt(40.0 * nmax)) / 2);
+  int start = miller_start(nmax);
   double fp1 = 0.0, f = 1e-200, sum = 0.0;
   for (int j = 0; j <= N; ++j) J[j] = 0.0;
   for (int k = start; k > 0; --k) {
@@ -44,8 +86,9 @@ QBX_D void bessel_jy(int N, double x, double* J, double* Y, bool want_y)
   double norm = 1.0 / sum;
   for (int j = 0; j <= N; ++j) J[j] *= norm;
   if (want_y) {
-    Y[0] = y0(x);
-    if (N >= 1) Y[1] = y1(x);
+    double b;
+    bessel_y01(x, Y[0], b);
+    if (N >= 1) Y[1] = b;
     for (int j = 1; j < N; ++j) Y[j + 1] = 2.0 * j * xinv * Y[j] - Y[j - 1];
   }
 }

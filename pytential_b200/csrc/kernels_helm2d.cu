@@ -480,8 +480,7 @@ k_h2_p2qbxl(qbxfmm_geometry g, HelmCoeffs hc, int nrhs, const double2* __restric
           sum += f;
           double norm = 1.0 / sum;
           double Y[N + 1];
-          Y[0] = y0(x);
-          Y[1] = y1(x);
+          bessel_y01(x, Y[0], Y[1]);
 #pragma unroll
           for (int k = 1; k < N; ++k) Y[k + 1] = 2.0 * k * xinv * Y[k] - Y[k - 1];
           // Hb_m = H_m(kr) e^{-i m th} for m >= 0; Hb_{-m} = (-1)^m H_m(kr) e^{i m th}

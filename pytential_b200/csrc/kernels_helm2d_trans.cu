@@ -114,7 +114,8 @@ k_h2_translate(qbxfmm_geometry g, double k, int p, int nrhs, int i0,
         if (KIND == 1) {
           double* Y = Ys + (size_t)lane * (NZ + 1);
           const double x = k * r, xinv = 1.0 / x;
-          double a = r == 0.0 ? 0.0 : y0(x), b = r == 0.0 ? 0.0 : y1(x);
+          double a = 0.0, b = 0.0;
+            if (r != 0.0) bessel_y01(x, a, b);
           Y[0] = a;
           Y[1] = b;
           for (int j = 1; j < NZ; ++j) {

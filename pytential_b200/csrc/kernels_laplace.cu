@@ -373,7 +373,9 @@ k_m2m(qbxfmm_geometry g, int p, int ncf, int nrhs, int i0, double2* __restrict__
 // list-2 pairs: the singular-harmonic tables (rows 0..2p, columns -p..2p) and the
 // multipoles (rows 0..p, columns -p..p) are expanded into zero-padded dense arrays
 // in shared memory, so the inner product is branch-free.  Each output's sum is
-// split over two threads (k ranges with about equal term counts).
+// split over two threads (k ranges with about equal term counts); each thread takes up to
+// M2L3_H of the 2 ncf jobs (462 at order 20).
+constexpr int M2L3_H = 4;
 __global__ void __launch_bounds__(NT)
 k_m2l3(qbxfmm_geometry g, int p, int ncf, int nrhs, int pb_max, const double2* __restrict__ mpoles,
        double2* __restrict__ locals, int32_t* err)
@@ -402,7 +404,9 @@ k_m2l3(qbxfmm_geometry g, int p, int ncf, int nrhs, int pb_max, const double2* _
     int half = (p + 1) * (p + 1) / 2, cum = 0;
     while (ksplit <= p && cum + ksplit <= half) cum += 2 * ksplit + 1, ++ksplit;
   }
-  double2 acc[2] = {c2(0.0), c2(0.0)};
+  double2 acc[M2L3_H];
+#pragma unroll
+  for (int h = 0; h < M2L3_H; ++h) acc[h] = c2(0.0);
   int l0 = g.list2_starts[i], l1 = g.list2_starts[i + 1];
   for (int lb = l0; lb < l1; lb += pb_max) {
     int nbat = min(pb_max, l1 - lb);
@@ -461,7 +465,7 @@ k_m2l3(qbxfmm_geometry g, int p, int ncf, int nrhs, int pb_max, const double2* _
     }
     __syncthreads();
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < M2L3_H; ++h) {
       int job = threadIdx.x + h * NT;
       if (job >= 2 * ncf) break;
       int o = job >> 1, half = job & 1;
@@ -484,14 +488,14 @@ k_m2l3(qbxfmm_geometry g, int p, int ncf, int nrhs, int pb_max, const double2* _
   // combine the two halves of each output
   __syncthreads();
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int h = 0; h < M2L3_H; ++h) {
     int job = threadIdx.x + h * NT;
     if (job < 2 * ncf && (job & 1)) red[job >> 1] = acc[h];
   }
   __syncthreads();
   double2* L = locals + ((size_t)tb * nrhs + r) * ncf;
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int h = 0; h < M2L3_H; ++h) {
     int job = threadIdx.x + h * NT;
     if (job < 2 * ncf && !(job & 1)) {
       int o = job >> 1;

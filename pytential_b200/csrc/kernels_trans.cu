@@ -168,6 +168,7 @@ k_trans_gemm(int ncf, int rp, int kp, int nrhs, int nwm, const double* __restric
   int mt = rp / 8;
   int mtw = (mt + nwm - 1) / nwm;
   int mbeg = wm * mtw;
+  mt = min(mt, mbeg + mtw);                 // the rows from there on are the next group's
   double acc[MTW][2];
 #pragma unroll
   for (int i = 0; i < MTW; ++i) acc[i][0] = acc[i][1] = 0.0;

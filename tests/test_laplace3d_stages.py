@@ -76,3 +76,43 @@ def test_multipoles_to_qbx_locals(q, p):
     want = o.zeros_qbx_exps()
     o.stage("translate_box_multipoles_to_qbx_local", mp, want)
     _close(got, want)
+
+
+def _close_by_degree(got, want, p):
+    """Box expansions: every degree against its own largest coefficient."""
+    got = got.cpu().numpy()
+    for n in range(p + 1):
+        i = slice(n * (n + 1) // 2, (n + 1) * (n + 2) // 2)
+        scale = np.abs(want[..., i]).max()
+        assert scale > 0
+        assert np.abs(got[..., i] - want[..., i]).max() <= TOL * scale, n
+
+
+@pytest.mark.parametrize("p", [1, 10, 14, 15, 20])
+def test_translations_by_pair(p):
+    w, o, s = _setup(2, p, 1.0, 0.0)
+    mp = o.zeros_box_exps()
+    o.stage("form_multipoles", s, mp)
+    _close_by_degree(w.form_multipoles(None, None, None, [torch.from_numpy(s).cuda()]), mp, p)
+    x = torch.from_numpy(mp.copy()).cuda()
+    o.stage("coarsen_multipoles", mp)
+    _close_by_degree(w.coarsen_multipoles(None, None, None, x), mp, p)
+    lo = o.zeros_box_exps()
+    o.stage("multipole_to_local", mp, lo)
+    x = torch.from_numpy(mp).cuda()
+    _close_by_degree(w.multipole_to_local(None, None, None, None, None, x), lo, p)
+    x = torch.from_numpy(lo.copy()).cuda()
+    o.stage("refine_locals", lo)
+    _close_by_degree(w.refine_locals(None, None, None, x), lo, p)
+
+
+@pytest.mark.parametrize("p", range(11, 21))
+def test_apply_orders(p):
+    """The whole apply: translations by class matrices, whose row groups change with p."""
+    d = make_ellipsoid(1)
+    geo = QBXFMMGeometryData(d, [(d.nodes, +1)], max_leaf_refine_weight=64)
+    ap = fmm.QBXApply(geo, fmm.SourceKernelSpec(fmm.LaplaceKernel(3), charge_coeff=1.0), 2, p)
+    o = Oracle(geo, dim=3, qbx_order=2, fmm_order=p, nrhs=1, charge_coeff=1.0)
+    dens = np.random.default_rng(3).normal(size=(1, d.ndofs))
+    want = o.apply(o.tree_strengths(d.upsample_density(dens) * d.quad_weights))
+    _close(ap(torch.from_numpy(dens).cuda()), want)

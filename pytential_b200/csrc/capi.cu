@@ -120,8 +120,8 @@ size_t h3_rot_offset(const qbxfmm_plan* p);
 // the M2M / L2L matrices: [0] Gaunt table, [1] rotation tables, [2] host M2L tables,
 // [3] M2L direction tables, [4] M2L coaxial tables (complex), [5] G0 of the order-p
 // monomial tables and [6] Ginv of the order-q ones (complex; the reference's default
-// truncation only, else empty), [7] end.
-void h3_layout(const qbxfmm_plan* p, size_t o[8])
+// truncation only, else empty), [7] the tables of each M2L pair (int32; FP64 form), [8] end.
+void h3_layout(const qbxfmm_plan* p, size_t o[9])
 {
   o[0] = p->tc.nmatrices * p->tc.rp * p->tc.kp;
   o[1] = o[0] + p->h3gaunt.size();
@@ -133,11 +133,12 @@ void h3_layout(const qbxfmm_plan* p, size_t o[8])
           1) & ~(size_t)1;
   o[6] = o[5] + 2 * p->h3tp.G0.size();
   o[7] = o[6] + 2 * p->h3tq.Ginv.size();
+  o[8] = o[7] + (p->mixed ? 0 : (size_t)(p->th.m2l_npairs + 1) / 2);
 }
 
 size_t h3_rot_offset(const qbxfmm_plan* p)
 {
-  size_t o[8];
+  size_t o[9];
   h3_layout(p, o);
   return o[1];
 }
@@ -687,7 +688,7 @@ int qbxfmm_multipole_to_local(const qbxfmm_plan* p, const void* mpoles, void* lo
   if (p->h3) {
     if (!p->trans_dev)
       return fail(QBXFMM_ERR_ARG, "3D Helmholtz: call qbxfmm_precompute_translations first");
-    size_t o[8];
+    size_t o[9];
     h3_layout(p, o);
     const int nm = 2 * p->kern.fmm_order + 1;
     const double* clsmap = p->trans_dev + o[2] + (size_t)nm * nm * 4 + 4 * (size_t)p->h3_ndir +
@@ -700,8 +701,9 @@ int qbxfmm_multipole_to_local(const qbxfmm_plan* p, const void* mpoles, void* lo
               "multipole_to_local");
     else
       QBX_TRY(h3_launch_m2l_mma(p->geo, p->kern.fmm_order, p->kern.nrhs, (const double2*)mpoles,
-                                (double2*)locals, p->trans_dev + o[3], p->trans_dev + o[4], clsmap,
-                                error_word, S(stream), p->hc.rb_m2l),
+                                (double2*)locals, p->trans_dev + o[3], p->trans_dev + o[4],
+                                reinterpret_cast<const int32_t*>(p->trans_dev + o[7]), error_word,
+                                S(stream), p->hc.rb_m2l),
               "multipole_to_local");
     return mask_all_levels(p, locals, S(stream));
   }
@@ -886,7 +888,7 @@ int qbxfmm_translate_box_local_to_qbx_local(const qbxfmm_plan* p, const void* lo
     if (!p->trans_dev)
       return fail(QBXFMM_ERR_ARG, "3D Helmholtz: call qbxfmm_precompute_translations first");
     if (p->hc.taylor) {
-      size_t o[8];
+      size_t o[9];
       h3_layout(p, o);
       QBX_TRY(h3_launch_l2qbxl_taylor(p->geo, p->hc, p->kern.fmm_order, p->kern.qbx_order,
                                       p->kern.nrhs, (const double2*)locals,
@@ -1078,9 +1080,9 @@ int qbxfmm_workspace_sizes(const qbxfmm_plan* p, size_t* sizes6 /* 8 entries */)
   if (int rc = qbx::plan_base_workspace_sizes(p, sizes6)) return rc;
   if (p->trans_ok) {
     int npairs = std::max(p->th.m2l_npairs, g.m2m_npairs);
-    size_t o[8];
+    size_t o[9];
     h3_layout(p, o);
-    sizes6[6] = p->h3 ? o[7] * sizeof(double) : p->m2l_aux_off + p->m2l_aux.size();
+    sizes6[6] = p->h3 ? o[8] * sizeof(double) : p->m2l_aux_off + p->m2l_aux.size();
     sizes6[7] = p->h3 ? 0 : trans_scratch_bytes(p->tc, npairs, p->kern.nrhs);
   } else {
     sizes6[6] = sizes6[7] = 0;
@@ -1096,7 +1098,7 @@ int qbxfmm_precompute_translations(const qbxfmm_plan* p, const qbxfmm_workspace*
     if (!ws->translations)
       return fail(QBXFMM_ERR_ARG, "3D Helmholtz needs the translations buffer");
     double* T = (double*)ws->translations;
-    size_t o[8];
+    size_t o[9];
     h3_layout(p, o);
     const int pf = p->kern.fmm_order, q = p->kern.qbx_order, nm = 2 * pf + 1;
     double* G = T + o[0];
@@ -1140,7 +1142,9 @@ int qbxfmm_precompute_translations(const qbxfmm_plan* p, const qbxfmm_workspace*
               "precompute_translations: M2L tables");
     else
       QBX_TRY(h3_launch_m2l_mma_tables(pf, p->h3_ndir, p->h3_ncoax, dirs, coaxp, H, isq, rt, G,
-                                       T + o[3], T + o[4], S(stream)),
+                                       T + o[3], T + o[4], p->geo, coaxp + 2 * (size_t)p->h3_ncoax,
+                                       p->th.m2l_npairs, reinterpret_cast<int32_t*>(T + o[7]),
+                                       S(stream)),
               "precompute_translations: M2L tables");
     p->trans_dev = T;
     p->scratch_dev = (double*)ws->pair_scratch;
@@ -1363,7 +1367,7 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
                           (const double2*)ws->locals, (double2*)ws->pot_tree, ws->error_word, st),
             "apply: locals to QBX targets");
   } else if (l2t) {
-    size_t o[8];
+    size_t o[9];
     h3_layout(p, o);
     QBX_TRY(h3_launch_l2t_taylor(p->geo, p->hc, p->kern.fmm_order, p->kern.qbx_order, p->kern.nrhs,
                                  (const double2*)ws->locals,

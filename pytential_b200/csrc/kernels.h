@@ -182,16 +182,17 @@ cudaError_t h3_launch_p2qbxl(const qbxfmm_geometry& g, HelmCoeffs hc, int q, int
 // 3D Helmholtz M2L by rotation: per-direction rotation tables (Dtab) and per-(length,
 // level) coaxial tables (Ctab); clsmap[2 c] / [2 c + 1] = direction / coaxial table of M2L
 // class c.  FP64: h3_m2l_mma_dsize / _csize doubles each, tensor-core products of
-// rb densities per CTA (0: by their number).
+// rb densities per CTA (0: by their number); pairtab: both tables of each M2L pair.
 size_t h3_m2l_mma_dsize(int p);
 size_t h3_m2l_mma_csize(int p);
 cudaError_t h3_launch_m2l_mma_tables(int pf, int ndir, int ncoax, const double* dirs,
                                      const double* coaxp, const double* start, const double* isq,
                                      const double* rt, const double* gaunt, double* Dtab,
-                                     double* Ctab, cudaStream_t st);
+                                     double* Ctab, const qbxfmm_geometry& g, const double* clsmap,
+                                     int npairs, int32_t* pairtab, cudaStream_t st);
 cudaError_t h3_launch_m2l_mma(const qbxfmm_geometry& g, int p, int nrhs, const double2* mp,
                               double2* lo, const double* Dtab, const double* Ctab,
-                              const double* clsmap, int32_t* err, cudaStream_t st, int rb);
+                              const int32_t* pairtab, int32_t* err, cudaStream_t st, int rb);
 // FP32 arithmetic (the mixed form): h3_m2l_dsize doubles and h3_m2l_csize complex each
 __host__ __device__ size_t h3_m2l_dsize(int pf);
 __host__ __device__ size_t h3_m2l_csize(int pf);

@@ -103,20 +103,28 @@ k_h3_l2t(qbxfmm_geometry g, HelmCoeffs hc, int p, int nrhs, const double2* __res
   };
   // stored monomials: P_s = sum_nm G0[s][nm] b_nm over n <= a+b+c of its parity, |m| <= a+b
   // of the parity of a+b
-  for (int e = tid; e < ncf * L2T_RB; e += L2T_NT) {
-    const int s = e / L2T_RB, r = e - s * L2T_RB;
+  // (a thread per monomial, all densities: the table entries come from L2)
+  for (int s = tid; s < ncf; s += L2T_NT) {
     const int a = s_st[3 * s], b = s_st[3 * s + 1], c = s_st[3 * s + 2];
     const int D = a + b + c, ab = a + b;
-    double2 acc = c2(0.0);
+    double2 acc[L2T_RB];
+#pragma unroll
+    for (int r = 0; r < L2T_RB; ++r) acc[r] = c2(0.0);
     for (int n = D & 1; n <= D; n += 2) {
       const int mm = min(n, ab) - ((min(n, ab) + ab) & 1);
+      const double2* G = G0 + (size_t)s * ncf + n * n + n;
+#pragma unroll 4
       for (int m = -mm; m <= mm; m += 2) {
-        const int col = n * n + n + m;
-        const double2 v = *reinterpret_cast<const double2*>(P + l2t_at(ncf + col, 2 * r));
-        acc = cfma(__ldg(G0 + (size_t)s * ncf + col), v, acc);
+        const double2 gv = __ldg(G + m);
+        const int at = ncf + n * n + n + m;
+#pragma unroll
+        for (int r = 0; r < L2T_RB; ++r)
+          acc[r] = cfma(gv, *reinterpret_cast<const double2*>(P + l2t_at(at, 2 * r)), acc[r]);
       }
     }
-    *reinterpret_cast<double2*>(P + l2t_at(mono(a, b, c), 2 * r)) = acc;
+    const int to = mono(a, b, c);
+#pragma unroll
+    for (int r = 0; r < L2T_RB; ++r) *reinterpret_cast<double2*>(P + l2t_at(to, 2 * r)) = acc[r];
   }
   __syncthreads();
   // the others from the PDE (Delta u + u = 0), by increasing exponent of z

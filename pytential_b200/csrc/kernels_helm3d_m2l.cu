@@ -14,13 +14,14 @@
 //
 // One CTA (16 warps) per target-or-parent box and 4 NT densities: the columns of every
 // product are (density, re / im), 8 columns = 4 densities a tensor-core tile
-// (mma.m8n8k4), so a lane's two results are one complex value.  The tables of a pair come
-// by cp.async: U, V by direction (loaded while the next multipole is fetched), the
-// coaxial blocks by (length, level) during the rotation back.  They are stored zero
+// (mma.m8n8k4), so a lane's two results are one complex value.  A pair's coaxial table
+// (by (length, level)), phases and raw multipole come by cp.async under the rotation back
+// of the pair before it, U, V (by direction) while X is formed.  The tables are stored zero
 // padded to multiples of 4 in the inner index with row strides of 4, 12 or 20 doubles
 // (4 or 12 mod 16), which are free of bank conflicts read along rows (rotation back) and
 // along columns (rotation); X and A rows likewise (8 NT + 4 doubles).
 #include <algorithm>
+#include <type_traits>
 
 #include "../../include/qbxfmm_api.h"
 #include "helm3.cuh"
@@ -190,14 +191,32 @@ k_h3_m2l_mma_tables(int pf, int ndir, int ncoax, const double* __restrict__ dirs
   }
 }
 
-// tiles of 8 rows of the groups of orders a warp takes (order p - sub, then the rest)
-template <int P15, int SUBS>
+// the tables of each M2L pair: direction | coaxial << 16
+__global__ void k_h3_m2l_pair_tables(qbxfmm_geometry g, const double* __restrict__ clsmap,
+                                     int npairs, int32_t* __restrict__ out)
+{
+  const int pr = blockIdx.x * blockDim.x + threadIdx.x;
+  if (pr >= npairs) return;
+  // class of the pair: m2l_class_starts[c] <= pr < m2l_class_starts[c + 1]
+  int lo = 0, hi = g.m2l_nclasses - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (g.m2l_class_starts[mid] <= pr) lo = mid;
+    else hi = mid - 1;
+  }
+  out[pr] = (int)clsmap[2 * lo] | (int)clsmap[2 * lo + 1] << 16;
+}
+
+// orders (and columns) per warp: n_0 = p - sub, n_1 = sub + max(0, p - 15) and, past 15,
+// n_2 = sub (16 subs: n_0 = p - sub, n_1 = sub for the orders past 15).  A product of s
+// columns has ceil(s / 4) steps and ceil(s / 8) row tiles, so its code is straight-line for
+// each number of steps KS (row tiles (KS + 1) / 2)
+template <bool P15, int SUBS>
 struct M2LGroups {
-  // orders per warp: n_0 = p - sub, n_1 = sub + max(0, p - 15) and, past 15, n_2 = sub
-  // (16 subs: n_0 = p - sub, n_1 = sub for the orders past 15)
   static constexpr int NG = SUBS == 16 ? (P15 ? 1 : 2) : (P15 ? 2 : 3);
-  static constexpr int NTL = P15 ? 2 : 3;       // row tiles of n_0
-  static constexpr int tiles(int g) { return g == 0 ? NTL : (g == 1 && SUBS == 8 && !P15 ? 2 : 1); }
+  static constexpr int KS0 = P15 ? 4 : 5;          // most steps of group 0
+  static constexpr int ks(int g) { return g == 0 ? KS0 : (g == 1 && SUBS == 8 ? (P15 ? 2 : 3) : 1); }
+  static constexpr int tiles(int g) { return (ks(g) + 1) / 2; }
 };
 
 template <int SUBS>
@@ -219,39 +238,62 @@ QBX_D int m2l_column(int p, int sub, int g)     // mu of the coaxial step
   return mu <= p ? mu : -1;
 }
 
+// run f with the number of steps as a constant, 1 .. MAX
+template <int MAX, typename F>
+QBX_D void with_steps(int ks, F f)
+{
+  if constexpr (MAX == 1) {
+    f(std::integral_constant<int, 1>());
+  } else {
+    if (ks == MAX) f(std::integral_constant<int, MAX>());
+    else with_steps<MAX - 1>(ks, f);
+  }
+}
+
+// run f with the group index as a constant, 0 .. N - 1
+template <int N, typename F>
+QBX_D void for_groups(F f)
+{
+  f(std::integral_constant<int, 0>());
+  if constexpr (N > 1) f(std::integral_constant<int, 1>());
+  if constexpr (N > 2) f(std::integral_constant<int, 2>());
+}
+
+constexpr int ks_stride(int ks) { return ks == 1 ? 4 : ks <= 3 ? 12 : 20; }
+
 // NT tiles of 4 densities per CTA, NPW of them per warp: 16 warps = SUBS x NT / NPW.
 // P15: p <= 15 (else p <= 17)
 template <int NT, int NPW, bool P15>
 __global__ void __launch_bounds__(M2L_NTHR)
 k_h3_m2l_mma(qbxfmm_geometry g, int p, int nrhs, const double2* __restrict__ mp,
              double2* __restrict__ lo, const double* __restrict__ Dtab,
-             const double* __restrict__ Ctab, const double* __restrict__ clsmap, int32_t* err)
+             const double* __restrict__ Ctab, const int32_t* __restrict__ pairtab, int32_t* err)
 {
   constexpr int SUBS = 16 * NPW / NT;
   using G = M2LGroups<P15, SUBS>;
-  constexpr int XS = 8 * NT + 4;
+  constexpr int XS = 8 * NT + 4, NR = 4 * NT;
   constexpr int PM = P15 ? 15 : 17;
-  constexpr int KIT = ((PM + 1) * (PM + 2) / 2 * 4 * NT + M2L_NTHR - 1) / M2L_NTHR;
+  constexpr int PARTS = 16 / NR;            // warps per density when X is formed
   extern __shared__ double2 smem2[];
   const int ncf = (p + 1) * (p + 1), ntri = (p + 1) * (p + 2) / 2;
-  const int dsz = m2l_dsize(p), csz = m2l_csize(p);
-  double* Td = reinterpret_cast<double*>(smem2);       // [dsz]
-  double* Tc = Td + dsz;                               // [csz]
+  const int nph = 2 * (p + 1), dsz = m2l_dsize(p), csz = m2l_csize(p);
+  double* Td = reinterpret_cast<double*>(smem2);       // [dsz - nph]: U, V
+  double* Tc = Td + (dsz - nph);                       // [csz]
   double* X = Tc + csz;                                // [ncf + 4][XS]
-  double* A = X + (size_t)(ncf + 4) * XS;              // [ncf + 4][XS]
+  double* A = X + (size_t)(ncf + 4) * XS;              // [ncf + 4][XS]; raw multipole [NR][ncf]
+  double* Ph = A + (size_t)(ncf + 4) * XS;             // [2][nph]: e^{i a alpha}
   __shared__ int s_u[PM + 2], s_v[PM + 2], s_c[PM + 2], s_ae[PM + 2], s_ao[PM + 2];
   __shared__ unsigned char s_tn[(PM + 1) * (PM + 2) / 2], s_ta[(PM + 1) * (PM + 2) / 2];
-  __shared__ int s_cls;
 
-  const int i = blockIdx.x, r0 = blockIdx.y * 4 * NT;
+  const int i = blockIdx.x, r0 = blockIdx.y * NR;
   const int q0 = g.m2l_tgt_pair_starts[i], q1 = g.m2l_tgt_pair_starts[i + 1];
   if (q1 <= q0) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int row = lane >> 2, kq = lane & 3;
   const int sub = warp % SUBS, nt0 = (warp / SUBS) * NPW;
   if (tid <= p) {
-    s_u[tid] = 2 * (p + 1) + off_u(tid);
-    int v = 2 * (p + 1) + off_u(p + 1);
+    s_u[tid] = off_u(tid);
+    int v = off_u(p + 1);
     for (int n = 1; n < tid; ++n) v += blk_size(n);
     s_v[tid] = v;
     s_c[tid] = off_c(p, tid);
@@ -265,215 +307,229 @@ k_h3_m2l_mma(qbxfmm_geometry g, int p, int nrhs, const double2* __restrict__ mp,
     s_tn[c] = (unsigned char)n;
     s_ta[c] = (unsigned char)m;
   }
+  // rows past the end are read against zero table entries: finite, and never written
   for (int x = tid; x < 4 * XS; x += M2L_NTHR) X[(size_t)ncf * XS + x] = A[(size_t)ncf * XS + x] = 0.0;
 
-  auto find_class = [&](int q) {            // class of pair q into s_cls
-    const int pr = g.m2l_tgt_pairs[q];
-    for (int c = tid; c < g.m2l_nclasses; c += M2L_NTHR)
-      if (g.m2l_class_starts[c] <= pr && pr < g.m2l_class_starts[c + 1]) s_cls = c;
-  };
-  auto load_table = [&](double* dst, const double* src, int n) {
+  auto copy = [&](double* dst, const double* src, int n) {
     for (int x = 2 * tid; x < n; x += 2 * M2L_NTHR) cp_async16(dst + x, src + x);
+  };
+  // the coaxial table, the phases and the raw multipole of pair q
+  auto load_pair = [&](int q, int tab, int buf) {
+    copy(Tc, Ctab + (size_t)(tab >> 16) * csz, csz);
+    copy(Ph + buf * nph, Dtab + (size_t)(tab & 0xffff) * dsz, nph);
+    const int src = g.m2l_pair_src[g.m2l_tgt_pairs[q]];
+    const bool bad = (unsigned)src >= (unsigned)g.nboxes;
+    if (bad && tid == 0) report(err, QBX_DEVERR_BAD_BOX);
+    const double* M = reinterpret_cast<const double*>(mp + ((size_t)(bad ? 0 : src) * nrhs + r0) * ncf);
+    const int have = bad ? 0 : 2 * ncf * min(NR, nrhs - r0);
+    for (int x = 2 * tid; x < 2 * ncf * NR; x += 2 * M2L_NTHR) {
+      if (x < have) cp_async16(A + x, M + x);
+      else *reinterpret_cast<double2*>(A + x) = c2(0.0);
+    }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
-  double acc[G::NG][G::NTL][NPW][4];        // (row, density): L_a (re, im), L_-a (re, im)
+  auto load_rotation = [&](int tab) {
+    copy(Td, Dtab + (size_t)(tab & 0xffff) * dsz + nph, dsz - nph);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  double acc[G::NG][G::tiles(0)][NPW][4];   // (row, density): L_a (re, im), L_-a (re, im)
 #pragma unroll
   for (int gi = 0; gi < G::NG; ++gi)
 #pragma unroll
-    for (int tl = 0; tl < G::NTL; ++tl)
+    for (int tl = 0; tl < G::tiles(0); ++tl)
 #pragma unroll
       for (int w = 0; w < NPW; ++w)
 #pragma unroll
         for (int x = 0; x < 4; ++x) acc[gi][tl][w][x] = 0.0;
 
-  if (tid == 0) s_cls = 0;
-  __syncthreads();
-  find_class(q0);
-  __syncthreads();
-  int cls = s_cls;
-  load_table(Tc, Ctab + (size_t)clsmap[2 * cls + 1] * csz, csz);
+  int tab = pairtab[g.m2l_tgt_pairs[q0]];
+  load_pair(q0, tab, 0);
+  load_rotation(tab);
   for (int q = q0; q < q1; ++q) {
-    load_table(Td, Dtab + (size_t)clsmap[2 * cls] * dsz, dsz);
-    const int src = g.m2l_pair_src[g.m2l_tgt_pairs[q]];
-    const bool bad = (unsigned)src >= (unsigned)g.nboxes;
-    if (bad && tid == 0) report(err, QBX_DEVERR_BAD_BOX);
-    double2 mv[KIT][2];
-#pragma unroll
-    for (int k = 0; k < KIT; ++k) {
-      const int t = tid + k * M2L_NTHR, r = t / ntri, c = t - r * ntri;
-      mv[k][0] = mv[k][1] = c2(0.0);
-      if (r < 4 * NT && r0 + r < nrhs && !bad) {
-        const double2* M = mp + ((size_t)src * nrhs + r0 + r) * ncf;
+    const int buf = (q - q0) & 1;
+    const int next = q + 1 < q1 ? pairtab[g.m2l_tgt_pairs[q + 1]] : 0;
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");   // all but the rotation table
+    __syncthreads();
+    // X^e, X^o from the raw multipole
+    {
+      const int r = warp % NR;
+      const double2* M = reinterpret_cast<const double2*>(A) + (size_t)r * ncf;
+      const double2* ph = reinterpret_cast<const double2*>(Ph + buf * nph);
+      for (int c = lane + 32 * (warp / NR); c < ntri; c += 32 * PARTS) {
         const int n = s_tn[c], a = s_ta[c], o = n * n + n;
-        mv[k][0] = __ldg(M + o + a);
-        if (a > 0) mv[k][1] = __ldg(M + o - a);
+        double2* E = reinterpret_cast<double2*>(X + (size_t)(n * n + a) * XS) + r;
+        if (a == 0) {
+          *E = M[o];
+        } else {
+          const double2 f = cscale(0.5 * M2L_SQRT2, ph[a]);
+          const double2 u = cmul(f, M[o + a]), v = cmulc(M[o - a], f);
+          *E = cadd(u, v);
+          reinterpret_cast<double2*>(X + (size_t)(o + a) * XS)[r] = csub(u, v);
+        }
       }
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
-    // X^e, X^o
-#pragma unroll
-    for (int k = 0; k < KIT; ++k) {
-      const int t = tid + k * M2L_NTHR, r = t / ntri, c = t - r * ntri;
-      if (r >= 4 * NT) break;
-      const int n = s_tn[c], a = s_ta[c];
-      double2* E = reinterpret_cast<double2*>(X + (size_t)(n * n + a) * XS) + r;
-      if (a == 0) {
-        *E = mv[k][0];
-      } else {
-        const double2 ph = reinterpret_cast<const double2*>(Td)[a];
-        const double2 u = cmul(ph, mv[k][0]), v = cmulc(mv[k][1], ph);
-        *E = cscale(0.5 * M2L_SQRT2, cadd(u, v));
-        double2* O = reinterpret_cast<double2*>(X + (size_t)(n * n + n + a) * XS) + r;
-        *O = cscale(0.5 * M2L_SQRT2, csub(u, v));
-      }
-    }
-    if (q + 1 < q1) find_class(q + 1);
-    __syncthreads();
-    if (q + 1 < q1) cls = s_cls;
     // rotation: A^e_b = sum_a U[a][b] X^e_a, A^o_b = sum_a V[a][b] X^o_a
-#pragma unroll
-    for (int gi = 0; gi < G::NG; ++gi) {
+    for_groups<G::NG>([&](auto group) {
+      constexpr int gi = decltype(group)::value;
       const int n = m2l_order<SUBS>(p, sub, gi);
-      if (n < 0) continue;
+      if (n < 0) return;
 #pragma unroll
       for (int par = 0; par < 2; ++par) {
         const int s = n + 1 - par;
         if (s == 0) continue;
-        const int stride = blk_stride(s), ks = pad4(s) >> 2;
-        const double* T = Td + (par ? s_v[n] : s_u[n]) + kq * stride + row;
-        const double* B = X + (size_t)(n * n + par * (n + 1) + kq) * XS + 8 * nt0 + row;
-        double d[G::tiles(0)][NPW][2];
+        const double* Tn = Td + (par ? s_v[n] : s_u[n]) + row;
+        const double* Bn = X + (size_t)(n * n + par * (n + 1) + kq) * XS + 8 * nt0 + row;
+        with_steps<G::ks(gi)>((s + 3) >> 2, [&](auto steps) {
+          constexpr int KS = decltype(steps)::value, TL = (KS + 1) / 2, ST = ks_stride(KS);
+          double b[KS][NPW], a[KS][TL], d[TL][NPW][2];
 #pragma unroll
-        for (int tl = 0; tl < G::tiles(gi); ++tl)
+          for (int k = 0; k < KS; ++k) {
 #pragma unroll
-          for (int w = 0; w < NPW; ++w) d[tl][w][0] = d[tl][w][1] = 0.0;
-        for (int k = 0; k < ks; ++k) {
-          double b[NPW];
+            for (int w = 0; w < NPW; ++w) b[k][w] = Bn[4 * k * XS + 8 * w];
 #pragma unroll
-          for (int w = 0; w < NPW; ++w) b[w] = B[8 * w];
-#pragma unroll
-          for (int tl = 0; tl < G::tiles(gi); ++tl) {
-            if (8 * tl >= s) break;
-            const double a = T[8 * tl];
-#pragma unroll
-            for (int w = 0; w < NPW; ++w) h3_dmma(d[tl][w][0], d[tl][w][1], a, b[w]);
+            for (int tl = 0; tl < TL; ++tl) a[k][tl] = Tn[(4 * k + kq) * ST + 8 * tl];
           }
-          T += 4 * stride;
-          B += 4 * XS;
-        }
 #pragma unroll
-        for (int tl = 0; tl < G::tiles(gi); ++tl) {
-          const int b = 8 * tl + row + par;
-          if (b > n) continue;
-          double* out = A + (size_t)((par ? s_ao[b] : s_ae[b]) + n - b) * XS + 8 * nt0 + 2 * kq;
+          for (int tl = 0; tl < TL; ++tl)
 #pragma unroll
-          for (int w = 0; w < NPW; ++w)
-            *reinterpret_cast<double2*>(out + 8 * w) = c2(d[tl][w][0], d[tl][w][1]);
-        }
+            for (int w = 0; w < NPW; ++w) d[tl][w][0] = d[tl][w][1] = 0.0;
+#pragma unroll
+          for (int k = 0; k < KS; ++k)
+#pragma unroll
+            for (int tl = 0; tl < TL; ++tl)
+#pragma unroll
+              for (int w = 0; w < NPW; ++w) h3_dmma(d[tl][w][0], d[tl][w][1], a[k][tl], b[k][w]);
+#pragma unroll
+          for (int tl = 0; tl < TL; ++tl) {
+            const int bb = 8 * tl + row + par;
+            if (bb > n) continue;
+            double* out = A + (size_t)((par ? s_ao[bb] : s_ae[bb]) + n - bb) * XS + 8 * nt0 + 2 * kq;
+#pragma unroll
+            for (int w = 0; w < NPW; ++w)
+              *reinterpret_cast<double2*>(out + 8 * w) = c2(d[tl][w][0], d[tl][w][1]);
+          }
+        });
       }
-    }
+    });
     __syncthreads();
     // coaxial translation: B_{nu mu} = sum_n C^mu[n][nu] A_{n mu}, e and o alike, into X
-#pragma unroll
-    for (int gi = 0; gi < G::NG; ++gi) {
+    for_groups<G::NG>([&](auto group) {
+      constexpr int gi = decltype(group)::value;
       const int mu = m2l_column<SUBS>(p, sub, gi);
-      if (mu < 0) continue;
-      const int s = p + 1 - mu, stride = blk_stride(s), ks = pad4(s) >> 2, im = blk_size(s);
-      const double* C = Tc + s_c[mu] + kq * stride + row;
+      if (mu < 0) return;
+      const int s = p + 1 - mu, im = blk_size(s);
       // columns (density, part): the product with Im C takes the other part, -im for re
-      const int colx = 8 * nt0 + (row ^ 1);
+      const int col = 8 * nt0 + row, colx = 8 * nt0 + (row ^ 1);
       const double sg = (row & 1) ? 1.0 : -1.0;
-#pragma unroll
-      for (int par = 0; par < 2; ++par) {
-        if (par && mu == 0) continue;
-        const double* B = A + (size_t)((par ? s_ao[mu] : s_ae[mu]) + kq) * XS;
-        const double* Ck = C;
-        double d[G::NTL][NPW][2];
-#pragma unroll
-        for (int tl = 0; tl < G::NTL; ++tl)
-#pragma unroll
-          for (int w = 0; w < NPW; ++w) d[tl][w][0] = d[tl][w][1] = 0.0;
-        for (int k = 0; k < ks; ++k) {
-          double b[NPW], bx[NPW];
-#pragma unroll
-          for (int w = 0; w < NPW; ++w) {
-            b[w] = B[8 * nt0 + row + 8 * w];
-            bx[w] = sg * B[colx + 8 * w];
-          }
-#pragma unroll
-          for (int tl = 0; tl < G::NTL; ++tl) {
-            if (8 * tl >= s) break;
-            const double cr = Ck[8 * tl], ci = Ck[im + 8 * tl];
-#pragma unroll
-            for (int w = 0; w < NPW; ++w) {
-              h3_dmma(d[tl][w][0], d[tl][w][1], cr, b[w]);
-              h3_dmma(d[tl][w][0], d[tl][w][1], ci, bx[w]);
-            }
-          }
-          Ck += 4 * stride;
-          B += 4 * XS;
-        }
-#pragma unroll
-        for (int tl = 0; tl < G::NTL; ++tl) {
-          const int nu = mu + 8 * tl + row;
-          if (nu > p) continue;
-          double* out = X + (size_t)(nu * nu + par * nu + mu) * XS + 8 * nt0 + 2 * kq;
-#pragma unroll
-          for (int w = 0; w < NPW; ++w)
-            *reinterpret_cast<double2*>(out + 8 * w) = c2(d[tl][w][0], d[tl][w][1]);
-        }
-      }
-    }
-    __syncthreads();
-    if (q + 1 < q1) load_table(Tc, Ctab + (size_t)clsmap[2 * cls + 1] * csz, csz);
-    // rotation back: L^e_a = sum_b U[a][b] B^e_b, then e^{-+ i a alpha} (L^e +- L^o)
-#pragma unroll
-    for (int gi = 0; gi < G::NG; ++gi) {
-      const int n = m2l_order<SUBS>(p, sub, gi);
-      if (n < 0) continue;
-#pragma unroll
-      for (int tl = 0; tl < G::tiles(gi); ++tl) {
-        if (8 * tl > n) break;
-        double d[2][NPW][2];
-        // V has the rows a = 1 .. n: its tile is read one row up, so that a lane's rows
-        // agree (the row a = 0 of the odd part is not used)
+      with_steps<G::KS0>((s + 3) >> 2, [&](auto steps) {
+        constexpr int KS = decltype(steps)::value, TL = (KS + 1) / 2, ST = ks_stride(KS);
+        const double* C = Tc + s_c[mu] + kq * ST + row;
 #pragma unroll
         for (int par = 0; par < 2; ++par) {
-          const int s = n + 1 - par;
+          if (par && mu == 0) continue;
+          const double* B = A + (size_t)((par ? s_ao[mu] : s_ae[mu]) + kq) * XS;
+          double d[TL][NPW][2];
 #pragma unroll
-          for (int w = 0; w < NPW; ++w) d[par][w][0] = d[par][w][1] = 0.0;
-          if (s == 0) continue;
-          const int stride = blk_stride(s), ks = pad4(s) >> 2;
-          const int ra = 8 * tl + row - par;
-          const double* T = Td + (par ? s_v[n] : s_u[n]) + max(ra, 0) * stride + kq;
-          const double* B = X + (size_t)(n * n + par * (n + 1) + kq) * XS + 8 * nt0 + row;
-          for (int k = 0; k < ks; ++k) {
-            const double a = T[4 * k];
+          for (int tl = 0; tl < TL; ++tl)
 #pragma unroll
-            for (int w = 0; w < NPW; ++w) h3_dmma(d[par][w][0], d[par][w][1], a, B[8 * w]);
-            B += 4 * XS;
+            for (int w = 0; w < NPW; ++w) d[tl][w][0] = d[tl][w][1] = 0.0;
+#pragma unroll
+          for (int k = 0; k < KS; ++k) {
+            double b[NPW], bx[NPW];
+#pragma unroll
+            for (int w = 0; w < NPW; ++w) {
+              b[w] = B[4 * k * XS + col + 8 * w];
+              bx[w] = sg * B[4 * k * XS + colx + 8 * w];
+            }
+#pragma unroll
+            for (int tl = 0; tl < TL; ++tl) {
+              const double cr = C[4 * k * ST + 8 * tl], ci = C[im + 4 * k * ST + 8 * tl];
+#pragma unroll
+              for (int w = 0; w < NPW; ++w) h3_dmma(d[tl][w][0], d[tl][w][1], cr, b[w]);
+#pragma unroll
+              for (int w = 0; w < NPW; ++w) h3_dmma(d[tl][w][0], d[tl][w][1], ci, bx[w]);
+            }
+          }
+#pragma unroll
+          for (int tl = 0; tl < TL; ++tl) {
+            const int nu = mu + 8 * tl + row;
+            if (nu > p) continue;
+            double* out = X + (size_t)(nu * nu + par * nu + mu) * XS + 8 * nt0 + 2 * kq;
+#pragma unroll
+            for (int w = 0; w < NPW; ++w)
+              *reinterpret_cast<double2*>(out + 8 * w) = c2(d[tl][w][0], d[tl][w][1]);
           }
         }
-        const int a = 8 * tl + row;
-        if (a > n) continue;
-        const double2 ph = reinterpret_cast<const double2*>(Td)[a];
-#pragma unroll
-        for (int w = 0; w < NPW; ++w) {
-          const double2 e = c2(d[0][w][0], d[0][w][1]);
-          const double2 o = a > 0 ? c2(d[1][w][0], d[1][w][1]) : c2(0.0);
-          double* ac = acc[gi][tl][w];
-          const double2 lp = cmulc(cadd(e, o), ph), lm = cmul(csub(e, o), ph);
-          ac[0] += lp.x;
-          ac[1] += lp.y;
-          ac[2] += lm.x;
-          ac[3] += lm.y;
-        }
-      }
-    }
+      });
+    });
     __syncthreads();
+    // A and the coaxial table are free: the next pair's copies run under the rotation back
+    if (q + 1 < q1) load_pair(q + 1, next, buf ^ 1);
+    // rotation back: L^e_a = sum_b U[a][b] B^e_b, then e^{-+ i a alpha} (L^e +- L^o)
+    for_groups<G::NG>([&](auto group) {
+      constexpr int gi = decltype(group)::value;
+      const int n = m2l_order<SUBS>(p, sub, gi);
+      if (n < 0) return;
+      with_steps<G::ks(gi)>((n + 4) >> 2, [&](auto steps) {
+        constexpr int KS = decltype(steps)::value, TL = (KS + 1) / 2, ST = ks_stride(KS);
+        // the odd part has one column and row less (row a = 0 is not used): the tile is
+        // read one row up, so that a lane's rows agree
+        const int so = blk_stride(n);
+        const bool full = n > 4 * (KS - 1);            // the odd part's last step exists
+        const double* Te = Td + s_u[n] + row * ST + kq;
+        const double* To = Td + s_v[n] + kq;
+        const double* Be = X + (size_t)(n * n + kq) * XS + 8 * nt0 + row;
+        const double* Bo = Be + (size_t)(n + 1) * XS;
+        double e[TL][NPW][2], o[TL][NPW][2];
+#pragma unroll
+        for (int tl = 0; tl < TL; ++tl)
+#pragma unroll
+          for (int w = 0; w < NPW; ++w)
+            e[tl][w][0] = e[tl][w][1] = o[tl][w][0] = o[tl][w][1] = 0.0;
+#pragma unroll
+        for (int k = 0; k < KS; ++k) {
+          double be[NPW], bo[NPW];
+#pragma unroll
+          for (int w = 0; w < NPW; ++w) {
+            be[w] = Be[4 * k * XS + 8 * w];
+            bo[w] = (k < KS - 1 || full) ? Bo[4 * k * XS + 8 * w] : 0.0;
+          }
+#pragma unroll
+          for (int tl = 0; tl < TL; ++tl) {
+            const double ae = Te[8 * tl * ST + 4 * k];
+#pragma unroll
+            for (int w = 0; w < NPW; ++w) h3_dmma(e[tl][w][0], e[tl][w][1], ae, be[w]);
+            if (k < KS - 1 || full) {
+              const double ao = To[max(8 * tl + row - 1, 0) * so + 4 * k];
+#pragma unroll
+              for (int w = 0; w < NPW; ++w) h3_dmma(o[tl][w][0], o[tl][w][1], ao, bo[w]);
+            }
+          }
+        }
+#pragma unroll
+        for (int tl = 0; tl < TL; ++tl) {
+          const int a = 8 * tl + row;
+          if (a > n) continue;
+          const double2 ph = reinterpret_cast<const double2*>(Ph + buf * nph)[a];
+#pragma unroll
+          for (int w = 0; w < NPW; ++w) {
+            const double2 ve = c2(e[tl][w][0], e[tl][w][1]);
+            const double2 vo = a > 0 ? c2(o[tl][w][0], o[tl][w][1]) : c2(0.0);
+            double* ac = acc[gi][tl][w];
+            const double2 lp = cmulc(cadd(ve, vo), ph), lm = cmul(csub(ve, vo), ph);
+            ac[0] += lp.x;
+            ac[1] += lp.y;
+            ac[2] += lm.x;
+            ac[3] += lm.y;
+          }
+        }
+      });
+    });
+    __syncthreads();
+    if (q + 1 < q1) load_rotation(next);
   }
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   const int tb = g.target_or_target_parent_boxes[i];
   if ((unsigned)tb >= (unsigned)g.nboxes) {
     if (tid == 0) report(err, QBX_DEVERR_BAD_BOX);
@@ -503,21 +559,21 @@ k_h3_m2l_mma(qbxfmm_geometry g, int p, int nrhs, const double2* __restrict__ mp,
 
 size_t m2l_mma_smem(int nt, int p)
 {
-  return (m2l_dsize(p) + m2l_csize(p) + 2 * ((size_t)(p + 1) * (p + 1) + 4) * (8 * nt + 4)) *
-         sizeof(double);
+  return (m2l_dsize(p) + 2 * (p + 1) + m2l_csize(p) +
+          2 * ((size_t)(p + 1) * (p + 1) + 4) * (8 * nt + 4)) * sizeof(double);
 }
 
 template <int NT, int NPW, bool P15>
 cudaError_t m2l_mma_launch(const qbxfmm_geometry& g, int p, int nrhs, const double2* mp,
                            double2* lo, const double* Dtab, const double* Ctab,
-                           const double* clsmap, int32_t* err, cudaStream_t st)
+                           const int32_t* pairtab, int32_t* err, cudaStream_t st)
 {
   const size_t sh = m2l_mma_smem(NT, p);
   cudaError_t e = cudaFuncSetAttribute(k_h3_m2l_mma<NT, NPW, P15>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
   if (e != cudaSuccess) return e;
   dim3 grid(g.nttp_boxes, (nrhs + 4 * NT - 1) / (4 * NT));
-  k_h3_m2l_mma<NT, NPW, P15><<<grid, M2L_NTHR, sh, st>>>(g, p, nrhs, mp, lo, Dtab, Ctab, clsmap, err);
+  k_h3_m2l_mma<NT, NPW, P15><<<grid, M2L_NTHR, sh, st>>>(g, p, nrhs, mp, lo, Dtab, Ctab, pairtab, err);
   return cudaGetLastError();
 }
 
@@ -528,7 +584,7 @@ size_t h3_m2l_mma_csize(int p) { return m2l_csize(p); }
 
 cudaError_t h3_launch_m2l_mma(const qbxfmm_geometry& g, int p, int nrhs, const double2* mp,
                               double2* lo, const double* Dtab, const double* Ctab,
-                              const double* clsmap, int32_t* err, cudaStream_t st, int rb)
+                              const int32_t* pairtab, int32_t* err, cudaStream_t st, int rb)
 {
   if (g.nttp_boxes == 0 || g.m2l_nclasses == 0) return cudaSuccess;
   // cp.async needs 16-byte aligned tables
@@ -538,20 +594,24 @@ cudaError_t h3_launch_m2l_mma(const qbxfmm_geometry& g, int p, int nrhs, const d
   // 16 or more do not fit the shared memory
   const int want = rb > 0 ? rb : nrhs;
   if (p <= 15) {
-    if (want > 8) return m2l_mma_launch<4, 2, true>(g, p, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-    if (want > 4) return m2l_mma_launch<2, 1, true>(g, p, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-    return m2l_mma_launch<1, 1, true>(g, p, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
+    if (want > 8) return m2l_mma_launch<4, 2, true>(g, p, nrhs, mp, lo, Dtab, Ctab, pairtab, err, st);
+    if (want > 4) return m2l_mma_launch<2, 1, true>(g, p, nrhs, mp, lo, Dtab, Ctab, pairtab, err, st);
+    return m2l_mma_launch<1, 1, true>(g, p, nrhs, mp, lo, Dtab, Ctab, pairtab, err, st);
   }
-  if (want > 4) return m2l_mma_launch<2, 1, false>(g, p, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
-  return m2l_mma_launch<1, 1, false>(g, p, nrhs, mp, lo, Dtab, Ctab, clsmap, err, st);
+  if (want > 4) return m2l_mma_launch<2, 1, false>(g, p, nrhs, mp, lo, Dtab, Ctab, pairtab, err, st);
+  return m2l_mma_launch<1, 1, false>(g, p, nrhs, mp, lo, Dtab, Ctab, pairtab, err, st);
 }
 
 cudaError_t h3_launch_m2l_mma_tables(int pf, int ndir, int ncoax, const double* dirs,
                                      const double* coaxp, const double* start, const double* isq,
                                      const double* rt, const double* gaunt, double* Dtab,
-                                     double* Ctab, cudaStream_t st)
+                                     double* Ctab, const qbxfmm_geometry& g, const double* clsmap,
+                                     int npairs, int32_t* pairtab, cudaStream_t st)
 {
   if (ndir + ncoax == 0) return cudaSuccess;
+  if (ndir > 0xffff || ncoax > 0x7fff) return cudaErrorInvalidValue;
+  if (npairs > 0)
+    k_h3_m2l_pair_tables<<<(npairs + 255) / 256, 256, 0, st>>>(g, clsmap, npairs, pairtab);
   k_h3_m2l_mma_tables<<<ndir + ncoax, 128, 0, st>>>(pf, ndir, ncoax, dirs, coaxp, start, isq, rt,
                                                     gaunt, Dtab, Ctab);
   return cudaGetLastError();

@@ -32,10 +32,16 @@ namespace {
 constexpr int M2T_NT = 128;
 constexpr int M2T_TG = 8;     // targets per warp
 
-// shared memory of one warp (in double2): the radial values, Phi, the two power series
+// shared memory of one warp (in double2): Phi, the fourth power, and the radial values or,
+// once Phi is formed, the series E of each lane
+__host__ __device__ constexpr size_t m2t_he(int pf, int q)
+{
+  return M2T_TG * (pf + q + 1) > 32 * (q + 1) ? M2T_TG * (pf + q + 1) : 32 * (q + 1);
+}
+
 __host__ __device__ constexpr size_t m2t_warp_smem(int pf, int q)
 {
-  return (size_t)M2T_TG * (pf + q + 1 + (pf + 1) * (q + 1) + (q + 1)) + 32 * (q + 1);
+  return (size_t)M2T_TG * ((pf + 1) * (q + 1) + (q + 1)) + m2t_he(pf, q);
 }
 
 // A CTA holds one octet of a chunk's targets; its four warps split the list-3 boxes
@@ -57,10 +63,10 @@ k_h3_m2t(qbxfmm_geometry g, HelmCoeffs hc, int pf, int nrhs, const double2* __re
   const int tg = lane >> 2, kq = lane & 3;
   double2* rec = smem2;                                          // [(pf+1)(pf+2)/2]
   const int nrec = (pf + 1) * (pf + 2) / 2;
-  double2* H = smem2 + nrec + (size_t)warp * m2t_warp_smem(pf, Q);   // [n][target]
-  double2* Phi = H + (size_t)M2T_TG * (pf + Q + 1);              // [n][i][target]
+  double2* Phi = smem2 + nrec + (size_t)warp * m2t_warp_smem(pf, Q);   // [n][i][target]
   double2* P4 = Phi + (size_t)M2T_TG * (pf + 1) * (Q + 1) + tg;  // [i][target]
-  double2* E = P4 - tg + M2T_TG * (Q + 1) + lane;                // [i][lane]
+  double2* H = P4 - tg + M2T_TG * (Q + 1);                       // [n][target]
+  double2* E = H + lane;                                         // [i][lane]
   constexpr int NWARP = M2T_NT / 32, OCT = QBXFMM_CENTER_CHUNK / M2T_TG;
   const int chunk = blockIdx.x / OCT, oct = blockIdx.x - chunk * OCT;
   const int itb = g.tsqbx_chunk_target_box[chunk];

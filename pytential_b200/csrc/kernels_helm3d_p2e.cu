@@ -14,8 +14,9 @@
 // Tiles of 16 sources: (1) thread (source, column m) runs its column into the wave table
 // in shared memory; (2) the table times the densities on the FP64 tensor cores, 8
 // coefficients x 4 sources x (4 densities, re / im), the warps splitting the coefficients.
-// During (2) one warp, another for each tile, first prepares the next tile's radial factors
-// and densities: serial recurrences that kept the whole CTA at a barrier before.
+// During (2) one warp, another for each tile, first prepares the next tile's radial factors,
+// serial recurrences that kept the whole CTA at a barrier before, and every thread has the
+// load of one strength of that tile in flight.
 #include <algorithm>
 
 #include "../../include/qbxfmm_api.h"
@@ -72,20 +73,29 @@ k_h3_p2e_mma(qbxfmm_geometry g, HelmCoeffs hc, int p, int nrhs,
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   h3_rec_table(p, rec, tid, P2E_NTHR);
 
-  // tile [base, base + 16) of the stream into a staged buffer, by one warp
+  // this thread's strength of the tile [base, base + 16): source tid % 16, density tid / 16
+  auto load_strength = [&](int base, int total, int nb, int s0) {
+    const int j = tid & 15, r = tid >> 4;
+    double2 v = c2(0.0);
+    if (r < NR && base + j < total && r0 + r < nrhs) {
+      const int s = LOCAL ? h3_stream_source(base + j, nb, s_pref, s_start) : s0 + base + j;
+      v = __ldg(strengths + (size_t)(r0 + r) * g.nsources + s);
+    }
+    return v;
+  };
+  auto store_strength = [&](double2* st, double2 v) {
+    const int j = tid & 15, r = tid >> 4;
+    double* sig = reinterpret_cast<double*>(st + 2 * (p + 1) * P2E_SUB);   // [SUB][SS]
+    if (r < NR) *reinterpret_cast<double2*>(sig + j * SS + 2 * r) = v;
+  };
+  // the radial factors and directions of tile [base, base + 16), by one warp
   auto prepare = [&](double2* st, int base, int total, int nb, int s0) {
     double2* Phi = st;                                             // [n][2][SUB]
-    double* sig = reinterpret_cast<double*>(Phi + 2 * (p + 1) * P2E_SUB);   // [SUB][SS]
-    double* dir = sig + P2E_SUB * SS;                              // [8][SUB]
+    double* dir = reinterpret_cast<double*>(Phi + 2 * (p + 1) * P2E_SUB) + P2E_SUB * SS;  // [8][SUB]
     const int j = lane & 15;
     const bool on = base + j < total;
     int s = 0;
     if (on) s = LOCAL ? h3_stream_source(base + j, nb, s_pref, s_start) : s0 + base + j;
-    for (int r = lane >> 4; r < NR; r += 2) {
-      double2 v = c2(0.0);
-      if (on && r0 + r < nrhs) v = __ldg(strengths + (size_t)(r0 + r) * g.nsources + s);
-      *reinterpret_cast<double2*>(sig + j * SS + 2 * r) = v;
-    }
     if (lane >= 16) return;
     double u[3] = {0.0, 0.0, 1.0}, nv[3] = {0.0, 0.0, 0.0};
     if (on) {
@@ -174,7 +184,10 @@ k_h3_p2e_mma(qbxfmm_geometry g, HelmCoeffs hc, int p, int nrhs,
       total = g.box_source_counts_nonchild[b];
       s0 = g.box_source_starts[b];
     }
-    if (warp == 0 && total > 0) prepare(stage, 0, total, nb, s0);
+    if (total > 0) {
+      store_strength(stage, load_strength(0, total, nb, s0));
+      if (warp == 0) prepare(stage, 0, total, nb, s0);
+    }
     int buf = 0, turn = 0;
     for (int base = 0; base < total; base += P2E_SUB, buf ^= 1) {
       __syncthreads();         // this tile is staged; the table and the other buffer are free
@@ -215,8 +228,12 @@ k_h3_p2e_mma(qbxfmm_geometry g, HelmCoeffs hc, int p, int nrhs,
         }
       }
       __syncthreads();         // the table is complete
-      if (warp == turn && base + P2E_SUB < total)
-        prepare(stage + (buf ^ 1) * nst, base + P2E_SUB, total, nb, s0);
+      const bool more = base + P2E_SUB < total;
+      double2 nxt = c2(0.0);
+      if (more) {
+        nxt = load_strength(base + P2E_SUB, total, nb, s0);
+        if (warp == turn) prepare(stage + (buf ^ 1) * nst, base + P2E_SUB, total, nb, s0);
+      }
       turn = (turn + 1) & 7;
 #pragma unroll
       for (int ks = 0; ks < P2E_SUB / 4; ++ks) {
@@ -240,6 +257,7 @@ k_h3_p2e_mma(qbxfmm_geometry g, HelmCoeffs hc, int p, int nrhs,
           }
         }
       }
+      if (more) store_strength(stage + (buf ^ 1) * nst, nxt);
     }
   }
   const double sc = h3_scale(hc.k, rho);

@@ -49,6 +49,7 @@ struct qbxfmm_plan {
   // rotation tables; then the device-built direction and coaxial tables
   std::vector<double> h3m2l;
   int h3_ndir = 0, h3_ncoax = 0;
+  int h2_npairs = 0;                       // 2D Helmholtz: list-2 pairs with classes (0: no tables)
   // 3D Helmholtz in the reference's default truncation (hc.taylor): monomial tables
   // of the box (order p) and QBX (order q) expansions
   H3TaylorHost h3tp, h3tq;
@@ -477,6 +478,15 @@ int qbxfmm_plan_create(const qbxfmm_kernel* kernel, const qbxfmm_geometry* geome
   if (e == cudaSuccess) e = cudaGetDevice(&p->device);
   p->h3 = p->helm && k.dim == 3;
   p->mixed = k.precision == 1;
+  if (p->helm && k.dim == 2 && g.m2l_nclasses > 0 && g.nttp_boxes > 0 && e == cudaSuccess) {
+    // tables by class where the classes cover list 2
+    int32_t nl2 = 0, npr = 0;
+    e = cudaMemcpy(&nl2, g.list2_starts + g.nttp_boxes, sizeof(int32_t), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess)
+      e = cudaMemcpy(&npr, g.m2l_class_starts + g.m2l_nclasses, sizeof(int32_t),
+                     cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess && nl2 == npr) p->h2_npairs = npr;
+  }
   if (k.dim == 3 && !p->h3 && g.m2l_nclasses > 0 && e == cudaSuccess) {
     std::vector<int32_t> off(3 * (size_t)g.m2l_nclasses);
     e = cudaMemcpy(off.data(), g.m2l_class_offsets, sizeof(int32_t) * off.size(),
@@ -616,7 +626,8 @@ int qbxfmm_form_multipoles(const qbxfmm_plan* p, const void* strengths, void* mp
   return mask_all_levels(p, mpoles, S(stream));
 }
 
-int qbxfmm_coarsen_multipoles(const qbxfmm_plan* p, void* mpoles, void* stream)
+// translations: 2D Helmholtz's tables, or null
+static int coarsen(const qbxfmm_plan* p, const void* translations, void* mpoles, void* stream)
 {
   if (int rc = check_plan(p)) return rc;
   if (p->h3 && !p->trans_dev)
@@ -632,7 +643,7 @@ int qbxfmm_coarsen_multipoles(const qbxfmm_plan* p, void* mpoles, void* stream)
         std::vector<int32_t> lv = one_level(p->lvl_source_parent, lev);
         if (p->helm)
           QBX_TRY(h2_launch_m2m(p->geo, lv.data(), p->hc, p->kern.fmm_order, p->kern.nrhs,
-                                (double2*)mpoles, nullptr, S(stream)),
+                                translations, (double2*)mpoles, nullptr, S(stream)),
                   "coarsen_multipoles");
         else
           QBX_TRY(launch_m2m(p->geo, lv.data(), p->kern.fmm_order, p->kern.nrhs, (double2*)mpoles,
@@ -651,13 +662,18 @@ int qbxfmm_coarsen_multipoles(const qbxfmm_plan* p, void* mpoles, void* stream)
   }
   if (p->helm)
     QBX_TRY(h2_launch_m2m(p->geo, p->lvl_source_parent.data(), p->hc, p->kern.fmm_order,
-                          p->kern.nrhs, (double2*)mpoles, nullptr, S(stream)),
+                          p->kern.nrhs, translations, (double2*)mpoles, nullptr, S(stream)),
             "coarsen_multipoles");
   else
     QBX_TRY(launch_m2m(p->geo, p->lvl_source_parent.data(), p->kern.fmm_order, p->kern.nrhs,
                        (double2*)mpoles, S(stream)),
             "coarsen_multipoles");
   return QBXFMM_OK;
+}
+
+int qbxfmm_coarsen_multipoles(const qbxfmm_plan* p, void* mpoles, void* stream)
+{
+  return coarsen(p, nullptr, mpoles, stream);
 }
 
 int qbxfmm_eval_direct(const qbxfmm_plan* p, const void* strengths, void* pot_nonqbx,
@@ -681,8 +697,8 @@ int qbxfmm_eval_direct(const qbxfmm_plan* p, const void* strengths, void* pot_no
   return QBXFMM_OK;
 }
 
-int qbxfmm_multipole_to_local(const qbxfmm_plan* p, const void* mpoles, void* locals,
-                              int32_t* error_word, void* stream)
+static int multipole_to_local(const qbxfmm_plan* p, const void* translations, const void* mpoles,
+                              void* locals, int32_t* error_word, void* stream)
 {
   if (int rc = check_plan(p)) return rc;
   if (p->h3) {
@@ -708,14 +724,20 @@ int qbxfmm_multipole_to_local(const qbxfmm_plan* p, const void* mpoles, void* lo
     return mask_all_levels(p, locals, S(stream));
   }
   if (p->helm)
-    QBX_TRY(h2_launch_m2l(p->geo, p->hc, p->kern.fmm_order, p->kern.nrhs, (const double2*)mpoles,
-                          (double2*)locals, error_word, S(stream)),
+    QBX_TRY(h2_launch_m2l(p->geo, p->hc, p->kern.fmm_order, p->kern.nrhs, translations,
+                          (const double2*)mpoles, (double2*)locals, error_word, S(stream)),
             "multipole_to_local");
   else
     QBX_TRY(launch_m2l(p->geo, p->kern.fmm_order, p->kern.nrhs, (const double2*)mpoles,
                        (double2*)locals, error_word, S(stream)),
             "multipole_to_local");
   return mask_all_levels(p, locals, S(stream));
+}
+
+int qbxfmm_multipole_to_local(const qbxfmm_plan* p, const void* mpoles, void* locals,
+                              int32_t* error_word, void* stream)
+{
+  return multipole_to_local(p, nullptr, mpoles, locals, error_word, stream);
 }
 
 int qbxfmm_eval_multipoles(const qbxfmm_plan* p, const void* mpoles, void* pot_nonqbx,
@@ -766,7 +788,7 @@ int qbxfmm_form_locals(const qbxfmm_plan* p, const void* strengths, void* locals
   return mask_all_levels(p, locals, S(stream));
 }
 
-int qbxfmm_refine_locals(const qbxfmm_plan* p, void* locals, void* stream)
+static int refine(const qbxfmm_plan* p, const void* translations, void* locals, void* stream)
 {
   if (int rc = check_plan(p)) return rc;
   if (p->h3 && !p->trans_dev)
@@ -782,7 +804,7 @@ int qbxfmm_refine_locals(const qbxfmm_plan* p, void* locals, void* stream)
         std::vector<int32_t> lv = one_level(p->lvl_ttp, lev);
         if (p->helm)
           QBX_TRY(h2_launch_l2l(p->geo, lv.data(), p->hc, p->kern.fmm_order, p->kern.nrhs,
-                                (double2*)locals, nullptr, S(stream)),
+                                translations, (double2*)locals, nullptr, S(stream)),
                   "refine_locals");
         else
           QBX_TRY(launch_l2l(p->geo, lv.data(), p->kern.fmm_order, p->kern.nrhs, (double2*)locals,
@@ -801,13 +823,18 @@ int qbxfmm_refine_locals(const qbxfmm_plan* p, void* locals, void* stream)
   }
   if (p->helm)
     QBX_TRY(h2_launch_l2l(p->geo, p->lvl_ttp.data(), p->hc, p->kern.fmm_order, p->kern.nrhs,
-                          (double2*)locals, nullptr, S(stream)),
+                          translations, (double2*)locals, nullptr, S(stream)),
             "refine_locals");
   else
     QBX_TRY(launch_l2l(p->geo, p->lvl_ttp.data(), p->kern.fmm_order, p->kern.nrhs,
                        (double2*)locals, S(stream)),
             "refine_locals");
   return QBXFMM_OK;
+}
+
+int qbxfmm_refine_locals(const qbxfmm_plan* p, void* locals, void* stream)
+{
+  return refine(p, nullptr, locals, stream);
 }
 
 int qbxfmm_eval_locals(const qbxfmm_plan* p, const void* locals, void* pot_nonqbx, void* stream)
@@ -1085,7 +1112,8 @@ int qbxfmm_workspace_sizes(const qbxfmm_plan* p, size_t* sizes6 /* 8 entries */)
     sizes6[6] = p->h3 ? o[8] * sizeof(double) : p->m2l_aux_off + p->m2l_aux.size();
     sizes6[7] = p->h3 ? 0 : trans_scratch_bytes(p->tc, npairs, p->kern.nrhs);
   } else {
-    sizes6[6] = sizes6[7] = 0;
+    sizes6[6] = p->h2_npairs > 0 ? h2_translations_bytes(g, p->kern.fmm_order, p->h2_npairs) : 0;
+    sizes6[7] = 0;
   }
   return QBXFMM_OK;
 }
@@ -1150,6 +1178,12 @@ int qbxfmm_precompute_translations(const qbxfmm_plan* p, const qbxfmm_workspace*
     p->scratch_dev = (double*)ws->pair_scratch;
     return QBXFMM_OK;
   }
+  if (p->h2_npairs > 0 && ws->translations) {
+    QBX_TRY(h2_launch_translations(p->geo, p->hc.k, p->kern.fmm_order, p->h2_npairs,
+                                   ws->translations, S(stream)),
+            "precompute_translations");
+    return QBXFMM_OK;
+  }
   if (!p->trans_ok || !ws->translations) return QBXFMM_OK;
   const TransAux aux = trans_aux(p, ws->translations);
   if (!p->m2l_aux.empty())
@@ -1193,7 +1227,7 @@ int run_m2m(const qbxfmm_plan* p, const qbxfmm_workspace* ws, const uint32_t* T3
                             (double2*)ws->mpoles, (double*)ws->pair_scratch, ws->error_word, st),
             "coarsen_multipoles (matrix form)");
   else
-    return qbxfmm_coarsen_multipoles(p, ws->mpoles, stream);
+    return coarsen(p, p->h2_npairs > 0 ? ws->translations : nullptr, ws->mpoles, stream);
   return QBXFMM_OK;
 }
 
@@ -1212,7 +1246,8 @@ int run_m2l(const qbxfmm_plan* p, const qbxfmm_workspace* ws, const uint32_t* T3
                             (double*)ws->pair_scratch, ws->error_word, st),
             "multipole_to_local (matrix form)");
   else
-    return qbxfmm_multipole_to_local(p, ws->mpoles, ws->locals, ws->error_word, stream);
+    return multipole_to_local(p, p->h2_npairs > 0 ? ws->translations : nullptr, ws->mpoles,
+                              ws->locals, ws->error_word, stream);
   return QBXFMM_OK;
 }
 
@@ -1233,7 +1268,7 @@ int run_l2l(const qbxfmm_plan* p, const qbxfmm_workspace* ws, const uint32_t* T3
                             (double2*)ws->locals, ws->error_word, st),
             "refine_locals (matrix form)");
   else
-    return qbxfmm_refine_locals(p, ws->locals, stream);
+    return refine(p, p->h2_npairs > 0 ? ws->translations : nullptr, ws->locals, stream);
   return QBXFMM_OK;
 }
 

@@ -132,18 +132,24 @@ cudaError_t h2_launch_form_strengths(const qbxfmm_geometry& g, const qbxfmm_upsa
                                      const double2* density, double2* strengths, cudaStream_t st);
 cudaError_t h2_launch_p2m(const qbxfmm_geometry& g, HelmCoeffs hc, int p, int nrhs,
                           const double2* s, double2* mp, int32_t* err, cudaStream_t st);
+// M2M / M2L / L2L with the plan's tables (h2_translations_bytes, filled by
+// h2_launch_translations), or without (translations null: each CTA builds its own)
+size_t h2_translations_bytes(const qbxfmm_geometry& g, int p, int npairs);
+cudaError_t h2_launch_translations(const qbxfmm_geometry& g, double k, int p, int npairs,
+                                   void* translations, cudaStream_t st);
 cudaError_t h2_launch_m2m(const qbxfmm_geometry& g, const int32_t* lvl_host, HelmCoeffs hc, int p,
-                          int nrhs, double2* mp, int32_t* err, cudaStream_t st);
+                          int nrhs, const void* translations, double2* mp, int32_t* err,
+                          cudaStream_t st);
 cudaError_t h2_launch_eval_direct(const qbxfmm_geometry& g, HelmCoeffs hc, int nrhs,
                                   const double2* s, double2* pot, int32_t* err, cudaStream_t st);
 cudaError_t h2_launch_m2l(const qbxfmm_geometry& g, HelmCoeffs hc, int p, int nrhs,
-                          const double2* mp, double2* lo, int32_t* err, cudaStream_t st);
+                          const void* translations, const double2* mp, double2* lo, int32_t* err, cudaStream_t st);
 cudaError_t h2_launch_eval_multipoles(const qbxfmm_geometry& g, HelmCoeffs hc, int p, int nrhs,
                                       const double2* mp, double2* pot, int32_t* err, cudaStream_t st);
 cudaError_t h2_launch_p2l(const qbxfmm_geometry& g, HelmCoeffs hc, int p, int nrhs,
                           const double2* s, double2* lo, int32_t* err, cudaStream_t st);
 cudaError_t h2_launch_l2l(const qbxfmm_geometry& g, const int32_t* lvl_host, HelmCoeffs hc, int p,
-                          int nrhs, double2* lo, int32_t* err, cudaStream_t st);
+                          int nrhs, const void* translations, double2* lo, int32_t* err, cudaStream_t st);
 cudaError_t h2_launch_eval_locals(const qbxfmm_geometry& g, HelmCoeffs hc, int p, int nrhs,
                                   const double2* lo, double2* pot, int32_t* err, cudaStream_t st);
 cudaError_t h2_launch_p2qbxl(const qbxfmm_geometry& g, HelmCoeffs hc, int q, int nrhs,

@@ -44,11 +44,10 @@ constexpr int NT = 128;
 constexpr int TR_CL = 8;      // CTAs per row (a cluster) in M2QBXL^T and P2QBXL^T when
                               // the rows alone would not fill the GPU
 constexpr int TR_SPLIT_BELOW = 4 * 148;   // rows below which a row is split
-// M2QBXL^T: threads per CTA and accumulation tasks per thread (2 ncf <= TRM_H TRM_NT:
-// each output coefficient is split over the even and odd centers of a batch; fmm_order
-// <= 21)
-constexpr int TRM_NT = 192;
-constexpr int TRM_H = 3;
+// M2QBXL^T: warps per CTA; rows of the product (qbx_order <= 8)
+constexpr int TRM_NW = 8;
+constexpr int TRM_MAXROWS = 81;
+constexpr int TRM_MAXSLOTS = 465;            // S_N^M, 0 <= M <= N <= p + q <= 29
 
 QBX_D bool box_ok(const qbxfmm_geometry& g, int b, int32_t* err)
 {
@@ -224,135 +223,244 @@ k_tr_l2qbxl(qbxfmm_geometry g, qbxfmm_transpose_index ix, int p, int q, int ncf,
 // {{{ M2QBXL^T: center multipoles into the locals of the list-3 boxes (M2L from the center)
 
 // L_j^i += (-1)^j (rho_s / rho_c)^j / rho_c sum_{k <= q, |l| <= k} Mc_k^l S_{k+j}^{l+i}(d),
-// d = (box center - center) / rho_c: the entries of M2QBXL with the roles exchanged.
-// Batches of mb centers per barrier (one S column task per thread): their S tables
-// (rows 0..p+q, columns -q..p+q), multipoles (rows 0..q, columns -q..q) and
-// (-1)^j ratio^j / rho_c factors in zero-padded dense shared arrays, so the inner
-// sums are branch-free.
-template <int CL>
-__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(TRM_NT, 3)
+// d = (box center - center) / rho_c: the entries of M2QBXL with the roles exchanged.  S is
+// homogeneous, so with v = (box center - center) / rho_s the powers of rho_c leave j:
+//   L_j^i = (-1)^j sum_{k, l} sum_c a_k^l(c) S_{k+j}^{l+i}(v_c),  a_k^l = (rho_c / rho_s)^k
+//   Mc_k^l / rho_s,
+// and every term is an entry of the real product G = A S over the centers c: (q + 1)^2 rows
+// (k, l >= 0, part of a) by the parts of S_N^M, 0 <= M <= N <= p + q, read off at the end by
+// the symmetry in the sign of l and M.  G on the FP64 tensor cores: a warp owns RT tiles of
+// 8 rows and a task of at most LEN degrees N of four M (8 columns: M, part); each lane runs
+// the recurrence in N of its column's part at its center (4 of a fragment's) and feeds it to
+// the products as it goes, so S is never stored.  Tasks beyond TRM_NW warps, and rows
+// beyond 4 tiles, take further passes over the centers.  Batches of 32 centers: warp 0
+// forms the seeds S_M^M while the others bring in the rows of A.
+// QCOMMENT
+template <int RT>
+constexpr int TRM_LEN = RT <= 2 ? 8 : RT == 3 ? 5 : 4;   // 2 RT LEN <= 32 accumulators
+
+// number of tasks with up to LEN degrees for the degrees 4 g .. P of the four M of group g
+__host__ __device__ inline int trm_chunks(int P, int g, int len) { return (P - 4 * g) / len + 1; }
+
+QBX_D void trm_dmma(double& d0, double& d1, double a, double b)
+{
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+      : "+d"(d0), "+d"(d1)
+      : "d"(a), "d"(b));
+}
+
+template <int CL, int RT>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * TRM_NW, 2)
 k_tr_m2qbxl(qbxfmm_geometry g, qbxfmm_transpose_index ix, int p, int q, int ncf, int ncq,
-            int nrhs, int mb, const double2* __restrict__ cmp, double2* __restrict__ locals,
+            int nrhs, int ntask, const double2* __restrict__ cmp, double2* __restrict__ locals,
             int32_t* err)
 {
+  constexpr int LEN = TRM_LEN<RT>, AS = 8 * RT + 4;      // AS = 4 or 12 mod 16: no conflicts
   const int row = blockIdx.x / CL, part = blockIdx.x - row * CL;
+  const int P = p + q, NG = P / 4 + 1, SD = 8 * NG + 4, NQ = (q + 1) * (q + 1);
+  const int nw = blockDim.x >> 5, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   extern __shared__ double2 smem2[];
-  const int SW = p + 2 * q + 1, SS = (p + q + 1) * SW;   // S: rows 0..p+q, columns -q..p+q
-  const int MW = 2 * q + 1, MS = (q + 1) * MW;
-  double2* S = smem2;                                    // [mb][SS]
-  double2* Mp = S + (size_t)mb * SS;                     // [mb][MS]
-  double* fac = reinterpret_cast<double*>(Mp + (size_t)mb * MS);   // [mb][p + 1]
-  double* sd = fac + (size_t)mb * (p + 1);                          // [mb][3]
-  int* sctr = reinterpret_cast<int*>(sd + (size_t)mb * 3);          // [mb]
-  int s = ix.list3_rows[row];
-  int r = blockIdx.y;
+  double2* Lacc = smem2;                                 // [ncf]
+  double2* G = Lacc + ncf;                               // [8 RT][4 nw LEN], after the centers
+  double* A = reinterpret_cast<double*>(G);              // [32][AS]
+  double* seeds = A + 32 * AS;                           // [32][SD]
+  double* s_zr = seeds + 32 * SD;                        // [32] z / r^2
+  double* s_r2 = s_zr + 32;                              // [32] 1 / r^2
+  double* fac = s_r2 + 32;                               // [32][q + 1]
+  __shared__ int s_ctr[32], s_nb;
+  __shared__ int16_t s_slot[TRM_MAXSLOTS];
+  __shared__ uint8_t s_rowk[TRM_MAXROWS], s_rowl[TRM_MAXROWS];   // k; 2 l + part
+  const int s = ix.list3_rows[row];
+  const int r = blockIdx.y;
   if (!box_ok(g, s, err)) return;          // the whole cluster (one row) leaves
-  double rho_s = level_width(g, g.box_levels[s]);
+  const double rho_s = level_width(g, g.box_levels[s]);
   double cs[3];
   load_point<3>(g.box_centers, g.nboxes, s, cs);
-  for (int i = threadIdx.x; i < mb * (SS + MS); i += TRM_NT) S[i] = c2(0.0);
-  double2 acc[TRM_H];
+  for (int o = tid; o < ncf; o += blockDim.x) Lacc[o] = c2(0.0);
+  for (int k = tid; k <= q; k += blockDim.x)
+    for (int t = 0; t <= 2 * k; ++t) {
+      s_rowk[k * k + t] = (uint8_t)k;
+      s_rowl[k * k + t] = (uint8_t)(t == 0 ? 0 : t + 1);   // t = 2 l - 1 + part
+    }
+  // where S_N^M stands among the columns of all tasks
+  for (int o = tid; o < idx3(P + 1, 0); o += blockDim.x) {
+    int N, M, ts = 0;
+    decode3(o, N, M);
+    const int mg = M >> 2, nch = trm_chunks(P, mg, LEN), clen = (P - 4 * mg + nch) / nch;
+    for (int h = 0; h < mg; ++h) ts += trm_chunks(P, h, LEN);
+    const int ch = (N - 4 * mg) / clen;
+    s_slot[o] = (int16_t)(((ts + ch) * LEN + N - 4 * mg - ch * clen) * 4 + (M & 3));
+  }
+  const int e0 = ix.list3_rev_starts[row] + part, e1 = ix.list3_rev_starts[row + 1];
+  const int frow = lane >> 2, kq = lane & 3;
+  for (int R0 = 0; R0 < NQ; R0 += 8 * RT)
+    for (int t0 = 0; t0 < ntask; t0 += nw) {
+      // this warp's task: degrees n0 .. n0 + nn - 1 of M = 4 mg .. 4 mg + 3
+      int mg = 0, ch = t0 + warp, n0 = 0, nn = 0;
+      if (t0 + warp < ntask) {
+        int nch;
+        while (ch >= (nch = trm_chunks(P, mg, LEN))) {
+          ch -= nch;
+          ++mg;
+        }
+        const int clen = (P - 4 * mg + nch) / nch;       // degrees dealt evenly to the chunks
+        n0 = 4 * mg + ch * clen;
+        nn = min(clen, P + 1 - n0);
+      }
+      const int M = 4 * mg + (frow >> 1);
+      double acc[LEN][RT][2];
 #pragma unroll
-  for (int h = 0; h < TRM_H; ++h) acc[h] = c2(0.0);
-  int item = 0;                            // center batches dealt round-robin to the cluster
-  for (int e = ix.list3_rev_starts[row]; e < ix.list3_rev_starts[row + 1]; ++e) {
-    int b = ix.list3_rev_lists[e];
-    if (!box_ok(g, b, err)) continue;
-    int k0 = ix.box_center_starts[b], k1 = ix.box_center_starts[b + 1];
-    for (int kb = k0; kb < k1; kb += mb) {
-      if (item++ % CL != part) continue;
-      int nb = min(mb, k1 - kb);
-      __syncthreads();
-      if (threadIdx.x < nb) {
-        int ctr = ix.box_centers[kb + threadIdx.x];
-        bool ok = center_ok(g, ctr, err);
-        // a bad center contributes nothing: a unit vector for its table, zero factors
-        double cc[3] = {cs[0] - 1.0, cs[1], cs[2]};
-        double rho_c = 1.0;
-        if (ok) {
+      for (int i = 0; i < LEN; ++i)
+#pragma unroll
+        for (int t = 0; t < RT; ++t) acc[i][t][0] = acc[i][t][1] = 0.0;
+      // warp 0 walks the boxes of the reversed list and keeps the next batch's centers in
+      // registers, lane = center
+      int e = e0, k0 = 0, k1 = 0, nb = 0, ctr = -1;
+      double cc[3], rho_c = 1.0;
+      auto fetch = [&]() {
+        nb = 0;
+        ctr = -1;
+        while (nb < 32) {
+          if (k0 >= k1) {
+            if (e >= e1) break;
+            const int b = ix.list3_rev_lists[e];
+            e += CL;
+            if (!box_ok(g, b, err)) continue;
+            k0 = ix.box_center_starts[b];
+            k1 = ix.box_center_starts[b + 1];
+            continue;
+          }
+          const int n = min(32 - nb, k1 - k0);
+          if (lane >= nb && lane < nb + n) ctr = ix.box_centers[k0 + lane - nb];
+          nb += n;
+          k0 += n;
+        }
+        if (lane < nb && !center_ok(g, ctr, err)) ctr = -1;
+        // a bad center contributes nothing: zero rows of A, a unit vector for its seeds
+        cc[0] = cs[0] - rho_s;
+        cc[1] = cs[1];
+        cc[2] = cs[2];
+        if (ctr >= 0) {
           load_point<3>(g.centers, g.ncenters, ctr, cc);
           rho_c = g.expansion_radii[ctr];
         }
-        sctr[threadIdx.x] = ok ? ctr : -1;
-        for (int d = 0; d < 3; ++d) sd[threadIdx.x * 3 + d] = (cs[d] - cc[d]) / rho_c;
-        double ratio = rho_s / rho_c, f = ok ? 1.0 / rho_c : 0.0;
-        for (int j = 0; j <= p; ++j, f *= -ratio) fac[threadIdx.x * (p + 1) + j] = f;
-      }
-      __syncthreads();
-      for (int w = threadIdx.x; w < nb * (p + q + 1); w += TRM_NT) {
-        int ci = w / (p + q + 1), m = w - ci * (p + q + 1);
-        double x = sd[ci * 3], y = sd[ci * 3 + 1], z = sd[ci * 3 + 2];
-        double rinv2 = 1.0 / (x * x + y * y + z * z);
-        double2 a = c2(sqrt(rinv2));
-        for (int jj = 1; jj <= m; ++jj) a = cscale((2.0 * jj - 1) * rinv2, cmul(a, c2(x, y)));
-        double2 prev = c2(0.0);
-        double2* T = S + (size_t)ci * SS + q;
-        for (int n = m; n <= p + q; ++n) {
-          if (n > m) {
-            double2 bb = cscale(rinv2, csub(cscale((2.0 * n - 1) * z, a),
-                                            cscale((double)(n + m - 1) * (n - m - 1), prev)));
-            prev = a;
-            a = bb;
-          }
-          T[n * SW + m] = a;
-          if (m >= 1 && m <= q) T[n * SW - m] = (m & 1) ? c2(-a.x, a.y) : c2(a.x, -a.y);
+      };
+      if (warp == 0) fetch();
+      while (true) {
+        __syncthreads();                                 // the tables (or G) are free
+        if (warp == 0) {
+          s_ctr[lane] = ctr;
+          if (lane == 0) s_nb = nb;
+          const double ri = 1.0 / rho_s, ratio = rho_c * ri;
+          double f = ri;
+          for (int k = 0; k <= q; ++k, f *= ratio) fac[lane * (q + 1) + k] = f;
         }
-      }
-      for (int w = threadIdx.x; w < nb * ncq; w += TRM_NT) {
-        int ci = w / ncq, i = w - ci * ncq;
-        int ctr = sctr[ci];
-        int kk, l;
-        decode3(i, kk, l);
-        double2 v = ctr >= 0 ? cmp[((size_t)ctr * nrhs + r) * ncq + i] : c2(0.0);
-        double2* M = Mp + (size_t)ci * MS + q;
-        M[kk * MW + l] = v;
-        if (l > 0) M[kk * MW - l] = (l & 1) ? c2(-v.x, v.y) : c2(v.x, -v.y);
-      }
-      __syncthreads();
-      // task t = (half, o): output coefficient o over the batch's centers of one parity
+        __syncthreads();
+        const int n = s_nb;
+        if (n == 0) break;
+        if (warp == 0) {
+          const double ri = 1.0 / rho_s;
+          const double x = (cs[0] - cc[0]) * ri, y = (cs[1] - cc[1]) * ri, z = (cs[2] - cc[2]) * ri;
+          const double r2 = 1.0 / (x * x + y * y + z * z);
+          s_zr[lane] = z * r2;
+          s_r2[lane] = r2;
+          double2* sd = reinterpret_cast<double2*>(seeds + lane * SD);
+          const double2 u = c2(x * r2, y * r2);
+          double2 a = c2(sqrt(r2));
+          for (int m = 0; m < 4 * NG; ++m) {
+            sd[m] = m <= P ? a : c2(0.0);
+            a = cscale(2.0 * m + 1.0, cmul(a, u));
+          }
+          fetch();
+        }
+        if (warp > 0 || nw == 1) {
+          const int nt = nw == 1 ? 32 : 32 * (nw - 1);
+          for (int w = nw == 1 ? tid : tid - 32; w < 256 * RT; w += nt) {
+            const int c = w / (8 * RT), t = w - c * (8 * RT), R = R0 + t, ct = s_ctr[c];
+            double v = 0.0;
+            if (R < NQ && ct >= 0) {
+              const int k = s_rowk[R], l2 = s_rowl[R];
+              const double* m = reinterpret_cast<const double*>(
+                  cmp + ((size_t)ct * nrhs + r) * ncq + idx3(k, l2 >> 1));
+              v = fac[c * (q + 1) + k] * m[l2 & 1];
+            }
+            A[c * AS + t] = v;
+          }
+        }
+        __syncthreads();
+        if (nn > 0) {
+          for (int c = kq; c < n + kq; c += 4) {         // c < 32: zeros of A past the last center
+            const double seed = seeds[c * SD + 8 * mg + frow], zr = s_zr[c], r2 = s_r2[c];
+            double af[RT];
 #pragma unroll
-      for (int h = 0; h < TRM_H; ++h) {
-        const int t = threadIdx.x + h * TRM_NT;
-        if (t >= 2 * ncf) break;
-        const int half = t >= ncf ? 1 : 0, o = t - half * ncf;
-        int j, ii;
-        decode3(o, j, ii);
-        double2 a = acc[h];
-        for (int ci = half; ci < nb; ci += 2) {
-          const double2* M = Mp + (size_t)ci * MS + q;
-          const double2* T = S + (size_t)ci * SS + q;
-          double2 v = c2(0.0);
-          for (int kk = 0; kk <= q; ++kk) {
-            const double2* mrow = M + kk * MW;
-            const double2* trow = T + (kk + j) * SW + ii;
-            for (int l = -kk; l <= kk; ++l) v = cfma(mrow[l], trow[l], v);
+            for (int t = 0; t < RT; ++t) af[t] = A[c * AS + 8 * t + frow];
+            // S_{N+1} r^2 = (2 N + 1) z S_N - (N^2 - M^2) S_{N-1}, from S_M = seed
+            double cur = 0.0, prev = 0.0, d = 8 * mg + 1, bb = (4 * mg - M) * (4 * mg + M);
+            int N = 4 * mg;
+            auto step = [&]() {
+              const double nxt = d * (zr * cur) - bb * (r2 * prev);
+              prev = cur;
+              cur = nxt;
+              bb += d;
+              d += 2.0;
+              ++N;
+            };
+            while (N < n0) {
+              if (N == M) cur = seed;
+              step();
+            }
+#pragma unroll
+            for (int i = 0; i < LEN; ++i) {
+              if (i >= nn) break;
+              if (N == M) cur = seed;
+#pragma unroll
+              for (int t = 0; t < RT; ++t) trm_dmma(acc[i][t][0], acc[i][t][1], af[t], cur);
+              step();
+            }
           }
-          a = caxpy(fac[ci * (p + 1) + j], v, a);
         }
-        acc[h] = a;
+      }
+      __syncthreads();
+      // lane (frow, kq): row frow of each tile, both parts of M = 4 mg + kq
+      const int GW = 4 * nw * LEN;
+#pragma unroll
+      for (int i = 0; i < LEN; ++i)
+#pragma unroll
+        for (int t = 0; t < RT; ++t)
+          G[(8 * t + frow) * GW + (warp * LEN + i) * 4 + kq] = c2(acc[i][t][0], acc[i][t][1]);
+      __syncthreads();
+      // the terms of L that this pass holds
+      auto term = [&](int t, int N, int m, double2& v) {
+        const int w = s_slot[idx3(N, abs(m))] - t0 * LEN * 4;
+        if ((unsigned)w >= (unsigned)GW) return false;
+        v = G[t * GW + w];
+        if (m < 0) v = (m & 1) ? c2(-v.x, v.y) : c2(v.x, -v.y);
+        return true;
+      };
+      for (int o = tid; o < ncf; o += blockDim.x) {
+        int j, i;
+        decode3(o, j, i);
+        double2 sum = c2(0.0);
+        for (int t = 0; t < min(8 * RT, NQ - R0); ++t) {
+          const int k = s_rowk[R0 + t], l2 = s_rowl[R0 + t], l = l2 >> 1;
+          // a real: a (S^{l+i} + (-1)^l S^{i-l}); imaginary: i a (S^{l+i} - (-1)^l S^{i-l})
+          double2 v = c2(0.0), w;
+          if (term(t, k + j, l + i, w)) v = w;
+          if (l > 0 && term(t, k + j, i - l, w))
+            v = ((l ^ l2) & 1) ? csub(v, w) : cadd(v, w);
+          sum = cadd(sum, (l2 & 1) ? c2(-v.y, v.x) : v);
+        }
+        Lacc[o] = cadd(Lacc[o], (j & 1) ? c2(-sum.x, -sum.y) : sum);
       }
     }
-  }
-  // the two halves of each coefficient, then the cluster's CTAs, summed by rank 0 in a
-  // fixed order (distributed shared memory); the partials [2][ncf] reuse the tables'
-  // space (mb (SS + MS) >= 2 ncf for mb >= 2)
+  // the cluster's CTAs, summed by rank 0 in a fixed order (distributed shared memory)
   cg::cluster_group cl = cg::this_cluster();
-  double2* s_part = smem2;
-  __syncthreads();
-#pragma unroll
-  for (int h = 0; h < TRM_H; ++h) {
-    const int t = threadIdx.x + h * TRM_NT;
-    if (t < 2 * ncf) s_part[t] = acc[h];
-  }
   cl.sync();
   if (part == 0) {
     double2* L = locals + ((size_t)s * nrhs + r) * ncf;
-    for (int o = threadIdx.x; o < ncf; o += TRM_NT) {
-      double2 v = cadd(s_part[o], s_part[o + ncf]);
-      for (int qq = 1; qq < CL; ++qq) {
-        const double2* rp = cl.map_shared_rank(s_part, qq);
-        v = cadd(v, cadd(rp[o], rp[o + ncf]));
-      }
+    for (int o = tid; o < ncf; o += blockDim.x) {
+      double2 v = Lacc[o];
+      for (int qq = 1; qq < CL; ++qq) v = cadd(v, cl.map_shared_rank(Lacc, qq)[o]);
       L[o] = cadd(L[o], v);
     }
   }
@@ -785,30 +893,44 @@ cudaError_t launch_tr_l2qbxl(const qbxfmm_geometry& g, const qbxfmm_transpose_in
   return cudaGetLastError();
 }
 
+template <int CL, int RT>
+static cudaError_t tr_m2qbxl(const qbxfmm_geometry& g, const qbxfmm_transpose_index& ix, int p, int q,
+                             int nrhs, const double2* cmp, double2* locals, int32_t* err,
+                             cudaStream_t st)
+{
+  const int ncf = idx3(p + 1, 0), ncq = idx3(q + 1, 0), P = p + q, NG = P / 4 + 1;
+  int ntask = 0;
+  for (int m = 0; m < NG; ++m) ntask += trm_chunks(P, m, TRM_LEN<RT>);
+  const int npass = (ntask + TRM_NW - 1) / TRM_NW, nw = (ntask + npass - 1) / npass;
+  const size_t tabs = 32 * sizeof(double) * (size_t)((8 * RT + 4) + (8 * NG + 4) + 2 + (q + 1));
+  const size_t prod = (size_t)8 * RT * 4 * nw * TRM_LEN<RT> * sizeof(double2);
+  const size_t sh = ncf * sizeof(double2) + std::max(tabs, prod);
+  cudaError_t e = cudaFuncSetAttribute(k_tr_m2qbxl<CL, RT>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+  if (e != cudaSuccess) return e;
+  k_tr_m2qbxl<CL, RT><<<dim3(ix.nlist3_rows * CL, nrhs), 32 * nw, sh, st>>>(
+      g, ix, p, q, ncf, ncq, nrhs, ntask, cmp, locals, err);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_tr_m2qbxl(const qbxfmm_geometry& g, const qbxfmm_transpose_index& ix, int p,
                              int q, int nrhs, const double2* cmp, double2* locals, int32_t* err,
                              cudaStream_t st)
 {
   if (ix.nlist3_rows == 0) return cudaSuccess;
-  int ncf = idx3(p + 1, 0), ncq = idx3(q + 1, 0);
-  int mb = std::max(1, std::min(8, TRM_NT / (p + q + 1)));
-  if (2 * ncf > TRM_H * TRM_NT || mb < 2) return cudaErrorInvalidValue;
-  size_t sh = (size_t)mb * ((p + q + 1) * (p + 2 * q + 1) + (q + 1) * (2 * q + 1)) * sizeof(double2) +
-              (size_t)mb * (p + 4) * sizeof(double) + (size_t)mb * sizeof(int);
-  if (ix.nlist3_rows < TR_SPLIT_BELOW) {
-    cudaError_t e = cudaFuncSetAttribute(k_tr_m2qbxl<TR_CL>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    if (e != cudaSuccess) return e;
-    k_tr_m2qbxl<TR_CL><<<dim3(ix.nlist3_rows * TR_CL, nrhs), TRM_NT, sh, st>>>(
-        g, ix, p, q, ncf, ncq, nrhs, mb, cmp, locals, err);
-  } else {
-    cudaError_t e = cudaFuncSetAttribute(k_tr_m2qbxl<1>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    if (e != cudaSuccess) return e;
-    k_tr_m2qbxl<1><<<dim3(ix.nlist3_rows, nrhs), TRM_NT, sh, st>>>(g, ix, p, q, ncf, ncq, nrhs, mb,
-                                                              cmp, locals, err);
+  if (q > 8 || p > 21) return cudaErrorInvalidValue;
+  // tiles of 8 rows, dealt evenly to passes of at most 4
+  const int tiles = ((q + 1) * (q + 1) + 7) / 8, passes = (tiles + 3) / 4;
+  const bool split = ix.nlist3_rows < TR_SPLIT_BELOW;
+#define QBX_TRM(RT)                                                                \
+  case RT:                                                                         \
+    return split ? tr_m2qbxl<TR_CL, RT>(g, ix, p, q, nrhs, cmp, locals, err, st)   \
+                 : tr_m2qbxl<1, RT>(g, ix, p, q, nrhs, cmp, locals, err, st);
+  switch ((tiles + passes - 1) / passes) {
+    QBX_TRM(1) QBX_TRM(2) QBX_TRM(3) QBX_TRM(4)
+    default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
+#undef QBX_TRM
 }
 
 template <int Q>

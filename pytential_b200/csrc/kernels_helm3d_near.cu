@@ -18,8 +18,7 @@
 // A warp holds one octet of the chunk's targets x 4 sources: lane l evaluates the pair
 // (target l / 4, source l % 4), which is the A fragment of an FP64 tensor-core product
 // with the sources' strengths, columns (density, re / im), as in the M2L kernel.  The
-// products run on the tensor pipe beside the FP64 pipe, which bounds the kernel.  Source
-// tiles are double buffered with cp.async.
+// products run on the tensor pipe beside the FP64 pipe, which bounds the kernel.
 #include <algorithm>
 
 #include "../../include/qbxfmm_api.h"
@@ -31,7 +30,6 @@ namespace qbx {
 namespace {
 
 constexpr int NEAR_NT = 128;
-constexpr int NEAR_TS = 64;      // sources per tile, two tiles staged
 
 // C(i, u) / i! = 1 / (u! (i - u)!)
 constexpr double near_c(int i, int u)
@@ -74,22 +72,6 @@ QBX_D double near_w(int i, int U, int o, double X, const double* zp, const doubl
   return r;
 }
 
-QBX_D void near_cp16(void* dst, const void* src, bool on)
-{
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
-                   (unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src), "r"(on ? 16 : 0)
-               : "memory");
-}
-
-QBX_D void near_cp8(void* dst, const void* src)
-{
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(
-                   (unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src)
-               : "memory");
-}
-
 template <int Q, int NT, bool CUT>
 __global__ void __launch_bounds__(NEAR_NT)
 k_h3_near(qbxfmm_geometry g, HelmCoeffs hc, int nrhs, const double2* __restrict__ strengths,
@@ -97,19 +79,23 @@ k_h3_near(qbxfmm_geometry g, HelmCoeffs hc, int nrhs, const double2* __restrict_
 {
   constexpr int SS = 8 * NT + 4;                 // row stride of the strengths (doubles)
   constexpr int NR = 4 * NT;
-  constexpr int TILE = NEAR_TS * (SS + 6);       // strengths [TS][SS], y and nu [6][TS]
   extern __shared__ double2 smem2[];
-  double* tiles = reinterpret_cast<double*>(smem2);              // [2][TILE]
-  __shared__ int s_src[2][NEAR_TS];
+  double* S = reinterpret_cast<double*>(smem2);  // [NEAR_NT][SS]
+  __shared__ double2 s_a[NEAR_NT], s_b[NEAR_NT], s_c[NEAR_NT];   // (y0, y1), (y2, nu0), (nu1, nu2)
+  __shared__ int s_src[NEAR_NT];
   __shared__ int s_pref[MAXB + 1], s_start[MAXB];
   const int chunk = blockIdx.x, r0 = blockIdx.y * NR;
   const int itb = g.tsqbx_chunk_target_box[chunk];
   const int cnt = g.tsqbx_chunk_count[chunk], i0 = g.tsqbx_chunk_start[chunk];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = lane >> 2, kq = lane & 3;
-  const bool busy = 8 * warp < cnt;              // this warp's octet exists
-  bool active = 8 * warp + row < cnt;
-  const int pi = i0 + max(0, min(8 * warp + row, cnt - 1));
+  // with 1 or 2 octets of targets the four warps share an octet's sources: warp's octet, its
+  // part of the sources and the number of parts
+  const int noct = (cnt + 7) >> 3, parts = noct <= 2 ? 4 / max(noct, 1) : 1;
+  const int oct = warp / parts, part = warp - oct * parts;
+  const bool busy = oct < noct;
+  bool active = 8 * oct + row < cnt;
+  const int pi = i0 + max(0, min(8 * oct + row, cnt - 1));
   int t = g.tsqbx_targets[pi], ctr = g.tsqbx_centers[pi];
   if ((unsigned)ctr >= (unsigned)g.ncenters || (unsigned)t >= (unsigned)g.ntargets) {
     report(err, QBX_DEVERR_BAD_CENTER);
@@ -141,46 +127,35 @@ k_h3_near(qbxfmm_geometry g, HelmCoeffs hc, int nrhs, const double2* __restrict_
     h3_list_prefix(g, g.list1_lists, gb, nb, s_pref, s_start, err);
     __syncthreads();
     const int total = s_pref[nb];
-    // source indices of tile t; then its copies (positions, normals, strengths) by cp.async
-    auto index = [&](int t) {
-      const int v = t * NEAR_TS + threadIdx.x;
-      if (threadIdx.x < NEAR_TS)
-        s_src[t & 1][threadIdx.x] = v < total ? h3_stream_source(v, nb, s_pref, s_start) : -1;
-    };
-    auto fetch = [&](int t) {
-      double* S = tiles + (t & 1) * TILE;
-      double* Y = S + NEAR_TS * SS;
-      for (int e = threadIdx.x; e < NEAR_TS * NR; e += NEAR_NT) {
-        const int j = e & (NEAR_TS - 1), r = e / NEAR_TS, s = s_src[t & 1][j];
-        const bool on = s >= 0 && r0 + r < nrhs;
-        near_cp16(S + j * SS + 2 * r, strengths + (on ? (size_t)(r0 + r) * g.nsources + s : 0), on);
+    for (int base = 0; base < total; base += NEAR_NT) {
+      const int ns = min(NEAR_NT, total - base);
+      if ((int)threadIdx.x < ns) {
+        const int s = h3_stream_source(base + threadIdx.x, nb, s_pref, s_start);
+        double y[3], nv[3] = {0, 0, 0};
+        load_point<3>(g.sources, g.nsources, s, y);
+        if (dip) load_point<3>(g.source_normals, g.nsources, s, nv);
+        s_a[threadIdx.x] = c2(y[0], y[1]);
+        s_b[threadIdx.x] = c2(y[2], nv[0]);
+        s_c[threadIdx.x] = c2(nv[1], nv[2]);
+        s_src[threadIdx.x] = s;
+      } else {
+        s_src[threadIdx.x] = -1;
       }
-      for (int e = threadIdx.x; e < NEAR_TS * 6; e += NEAR_NT) {
-        const int j = e & (NEAR_TS - 1), d = e / NEAR_TS, s = s_src[t & 1][j];
-        const double* from = d < 3 ? g.sources + (size_t)d * g.nsources
-                                   : g.source_normals + (size_t)(d - 3) * g.nsources;
-        if (d < 3 || dip) near_cp8(Y + d * NEAR_TS + j, from + max(s, 0));
-      }
-      asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
-    const int ntile = (total + NEAR_TS - 1) / NEAR_TS;
-    if (ntile > 0) {
-      index(0);
-      index(1);
       __syncthreads();
-      fetch(0);
-    }
-    for (int tl = 0; tl < ntile; ++tl) {
-      const int ns = min(NEAR_TS, total - tl * NEAR_TS);
-      const double* S = tiles + (tl & 1) * TILE;
-      const double* Y = S + NEAR_TS * SS;
-      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-      __syncthreads();                           // tile tl is here, the other buffer is free
-      if (tl + 1 < ntile) fetch(tl + 1);
+      // strengths, sources fastest: runs of one box are contiguous
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        const int s = s_src[threadIdx.x];
+        double2 v = c2(0.0);
+        if (s >= 0 && r0 + r < nrhs) v = __ldg(strengths + (size_t)(r0 + r) * g.nsources + s);
+        *reinterpret_cast<double2*>(S + threadIdx.x * SS + 2 * r) = v;
+      }
+      __syncthreads();
       if (busy) {
-        for (int j0 = 0; j0 < ns; j0 += 4) {
+        for (int j0 = 4 * part; j0 < ns; j0 += 4 * parts) {
           const int j = j0 + kq;
-          const double b0 = Y[j] - cc[0], b1 = Y[NEAR_TS + j] - cc[1], b2 = Y[2 * NEAR_TS + j] - cc[2];
+          const double2 ya = s_a[j], yb = s_b[j], yc = s_c[j];
+          const double b0 = ya.x - cc[0], b1 = ya.y - cc[1], b2 = yb.x - cc[2];
           const double bs = b0 * b0 + b1 * b1 + b2 * b2;
           const double rho = rsqrt_h(bs), rho2 = rho * rho;
           const double x0 = hc.k * bs * rho, xi = kinv * rho;
@@ -195,9 +170,8 @@ k_h3_near(qbxfmm_geometry g, HelmCoeffs hc, int nrhs, const double2* __restrict_
           double2 hn = c2((sn - cs * x0) * xi * xi, -(sn * x0 + cs) * xi * xi);
           double bn = 0.0, an = 0.0;
           if (dip) {
-            const double n0 = Y[3 * NEAR_TS + j], n1 = Y[4 * NEAR_TS + j], n2 = Y[5 * NEAR_TS + j];
-            bn = b0 * n0 + b1 * n1 + b2 * n2;
-            an = a[0] * n0 + a[1] * n1 + a[2] * n2;
+            bn = b0 * yb.y + b1 * yc.x + b2 * yc.y;
+            an = a[0] * yb.y + a[1] * yc.x + a[2] * yc.y;
           }
           double2 vS = c2(0.0), vD = c2(0.0);
 #pragma unroll
@@ -219,18 +193,33 @@ k_h3_near(qbxfmm_geometry g, HelmCoeffs hc, int nrhs, const double2* __restrict_
           if (dip) K = cfma(kD, cscale(rho, vD), K);
           if (j >= ns || bs == 0.0) K = c2(0.0);
           const double* B = S + j * SS;
+          // columns (density, part): i sigma has (-im, re) there
+#pragma unroll
+          for (int n = 0; n < NT; ++n) h3_dmma(acc[n][0], acc[n][1], K.x, B[8 * n + row]);
 #pragma unroll
           for (int n = 0; n < NT; ++n) {
-            // columns (density, part): i sigma has (-im, re) there
             const double bx = B[8 * n + (row ^ 1)];
-            h3_dmma(acc[n][0], acc[n][1], K.x, B[8 * n + row]);
             h3_dmma(acc[n][0], acc[n][1], K.y, (row & 1) ? bx : -bx);
           }
         }
       }
-      __syncthreads();                           // (the copies of tile tl + 1 have their indices)
-      index(tl + 2);
+      __syncthreads();
     }
+  }
+  if (parts > 1) {             // (the last tile's barrier freed S) the parts in order
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+      *reinterpret_cast<double2*>(S + ((warp * NT + n) * 32 + lane) * 2) = c2(acc[n][0], acc[n][1]);
+    __syncthreads();
+    if (part > 0) return;
+    for (int w = 1; w < parts; ++w)
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        const double2 v =
+            *reinterpret_cast<const double2*>(S + (((warp + w) * NT + n) * 32 + lane) * 2);
+        acc[n][0] += v.x;
+        acc[n][1] += v.y;
+      }
   }
 #pragma unroll
   for (int n = 0; n < NT; ++n) {
@@ -245,7 +234,7 @@ template <int Q, int NT>
 cudaError_t near_launch(const qbxfmm_geometry& g, HelmCoeffs hc, int nrhs, const double2* s,
                         double2* pt, int32_t* err, cudaStream_t st)
 {
-  const size_t sh = (size_t)2 * NEAR_TS * (8 * NT + 4 + 6) * sizeof(double);
+  const size_t sh = (size_t)NEAR_NT * (8 * NT + 4) * sizeof(double);
   auto k = hc.taylor ? k_h3_near<Q, NT, true> : k_h3_near<Q, NT, false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
   if (e != cudaSuccess) return e;

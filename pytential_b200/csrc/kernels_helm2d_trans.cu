@@ -37,6 +37,7 @@ QBX_D void cp_async16_h2(void* dst, const void* src)
 constexpr int TR2_NT = 128;
 constexpr int TR2_PB = 16;                   // source boxes per batch
 constexpr int TR2_MAXP = 20;
+constexpr size_t TR2_FEW = 2 * 148;          // CTAs of 64 densities that leave the GPU idle
 constexpr int TR2_MT = (2 * TR2_MAXP + 1) / 8;
 
 // Plan tables: shift [level][8][4p + 1] (M2M from child position c into its parent of the
@@ -341,8 +342,20 @@ cudaError_t translate(const qbxfmm_geometry& g, double k, int p, int nrhs, int i
                       cudaStream_t st)
 {
   if (p > TR2_MAXP) return cudaErrorInvalidValue;
-  // more than 16 densities: each warp its own 16; else the warps deal the source boxes
-  if (nrhs > 16)
+  // More than 16 densities: each warp its own 16; else the warps deal the source boxes.  L2L
+  // has one source box, so its warps always split densities.  Where a level's CTAs leave the
+  // GPU idle, a CTA takes 16 densities instead of 64: its four warps M2M's children, or four
+  // densities each (65 to 33 us an M2M level, 75 to 14 an L2L level, of such levels at 64
+  // densities and order 20; larger levels are faster with 64, which share a table).
+  const bool few = (size_t)nb * ((nrhs + 63) / 64) < TR2_FEW;
+  if (KIND == 2) {
+    if (!few && nrhs > 32)
+      return translate_launch<KIND, 4, false>(g, k, p, nrhs, i0, nb, tab, ein, eout, err, st);
+    if (!few && nrhs > 16)
+      return translate_launch<KIND, 2, false>(g, k, p, nrhs, i0, nb, tab, ein, eout, err, st);
+    return translate_launch<KIND, 1, false>(g, k, p, nrhs, i0, nb, tab, ein, eout, err, st);
+  }
+  if (nrhs > 16 && !(KIND == 0 && few))
     return translate_launch<KIND, 4, false>(g, k, p, nrhs, i0, nb, tab, ein, eout, err, st);
   if (nrhs > 8) return translate_launch<KIND, 4, true>(g, k, p, nrhs, i0, nb, tab, ein, eout, err, st);
   if (nrhs > 4) return translate_launch<KIND, 2, true>(g, k, p, nrhs, i0, nb, tab, ein, eout, err, st);

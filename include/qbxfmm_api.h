@@ -79,6 +79,13 @@ int qbxfmm_workspace_sizes(const qbxfmm_plan* plan, size_t* sizes8);
 int qbxfmm_precompute_translations(const qbxfmm_plan* plan, const qbxfmm_workspace* ws,
                                    void* stream);
 
+/* One translation stage as qbxfmm_apply runs it, on ws->mpoles and ws->locals with
+ * ws->translations and ws->pair_scratch (either NULL: by pair, as the entries below):
+ * stage 0 coarsen_multipoles, 1 multipole_to_local, 2 refine_locals.  A stage reads and
+ * writes only its own buffers of ws; calls at the same time need their own pair_scratch. */
+int qbxfmm_translate_boxes(const qbxfmm_plan* plan, const qbxfmm_workspace* ws, int stage,
+                           void* stream);
+
 /* get_flat_strengths_from_densities + reorder_sources
  * (pytential/qbx/__init__.py:1075-1096; pytential/qbx/fmm.py:199-200).
  * density: [nrhs][nelements * nodes_per_element] stage-1, element-major. */

@@ -1210,6 +1210,21 @@ namespace {
 // precisions: they are latency-bound, a TF32 form would not be faster); M2L: split
 // TF32 in the mixed form.  `gemm`: the translation matrices of ws are built; T32:
 // their split-TF32 planes (mixed form), or NULL.
+// the matrix form of the translations (per-level orders run the stage entries, which truncate
+// level by level)
+bool use_matrices(const qbxfmm_plan* p, const qbxfmm_workspace* ws)
+{
+  return !p->h3 && p->trans_ok && ws->translations && ws->pair_scratch && !level_orders_on(p);
+}
+
+const uint32_t* tf32_planes(const qbxfmm_plan* p, const qbxfmm_workspace* ws, bool gemm)
+{
+  return (gemm && p->tf32_ok)
+             ? reinterpret_cast<const uint32_t*>((const double*)ws->translations +
+                                                 trans_matrix_bytes(p->tc) / sizeof(double))
+             : nullptr;
+}
+
 int run_m2m(const qbxfmm_plan* p, const qbxfmm_workspace* ws, const uint32_t* T32, bool gemm,
             void* stream)
 {
@@ -1276,6 +1291,19 @@ int run_l2l(const qbxfmm_plan* p, const qbxfmm_workspace* ws, const uint32_t* T3
 
 extern "C" {
 
+int qbxfmm_translate_boxes(const qbxfmm_plan* p, const qbxfmm_workspace* ws, int stage,
+                           void* stream)
+{
+  if (int rc = check_plan(p)) return rc;
+  if (!ws || stage < 0 || stage > 2 || (stage < 2 && !ws->mpoles) || (stage > 0 && !ws->locals))
+    return fail(QBXFMM_ERR_ARG, "translate_boxes: incomplete workspace or unknown stage");
+  const bool gemm = use_matrices(p, ws);
+  const uint32_t* T32 = tf32_planes(p, ws, gemm);
+  if (stage == 0) return run_m2m(p, ws, T32, gemm, stream);
+  if (stage == 1) return run_m2l(p, ws, T32, gemm, stream);
+  return run_l2l(p, ws, T32, gemm, stream);
+}
+
 int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_workspace* ws,
                  const void* density, void* out, void* stream)
 {
@@ -1286,9 +1314,7 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
     return fail(QBXFMM_ERR_ARG, "incomplete workspace");
   size_t sz[8];
   if (int rc = qbxfmm_workspace_sizes(p, sz)) return rc;
-  // (per-level orders run the stage entries, which truncate level by level)
-  const bool gemm = !p->h3 && p->trans_ok && ws->translations && ws->pair_scratch &&
-                    !level_orders_on(p);
+  const bool gemm = use_matrices(p, ws);
   if (p->h3) {
     if (!ws->translations)
       return fail(QBXFMM_ERR_ARG, "3D Helmholtz needs the translations buffer");
@@ -1309,10 +1335,7 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
   QBX_TRY(cudaMemsetAsync(ws->pot_tree, 0, sz[5], st), "apply: clear");
   if (ws->error_word) QBX_TRY(cudaMemsetAsync(ws->error_word, 0, sizeof(int32_t), st), "apply: clear");
   int rc;
-  const uint32_t* T32 = (gemm && p->tf32_ok)
-                            ? reinterpret_cast<const uint32_t*>((const double*)ws->translations +
-                                                                trans_matrix_bytes(p->tc) / sizeof(double))
-                            : nullptr;
+  const uint32_t* T32 = tf32_planes(p, ws, gemm);
   auto m2m = [&]() -> int { return run_m2m(p, ws, T32, gemm, stream); };
   auto m2l = [&]() -> int { return run_m2l(p, ws, T32, gemm, stream); };
   auto l2l = [&]() -> int { return run_l2l(p, ws, T32, gemm, stream); };

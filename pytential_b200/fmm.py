@@ -283,16 +283,16 @@ class B200QBXExpansionWrangler:
         self.plan = Plan(self.dgeo, tree_indep.spec, qbx_order, fmm_order, nrhs,
                          target_specific_qbx=self.using_tsqbx, fmm_backend=fmm_backend,
                          level_orders=level_orders)
+        # the translations' class matrices or tables, laid out once for the plan (the
+        # reference's translation-class data, pytential/qbx/fmm.py:155-161, 399-407)
+        sizes = self.plan.workspace_sizes()
+        per_level = needs_per_level_classes(tree_indep.spec)
         self._translations = None
-        if needs_per_level_classes(tree_indep.spec):
-            # the translation stages of this kernel run on precomputed matrices
-            sizes = self.plan.workspace_sizes()
-            self._translations = [torch.zeros(sz // 8 + 1, dtype=torch.float64,
-                                              device=self.device) for sz in sizes[6:]]
-            z = ctypes.c_void_p(0)
-            ws = abi.QBXFMMWorkspace(z, z, z, z, z, z, None,
-                                     ctypes.c_void_p(_ptr(self._translations[0])),
-                                     ctypes.c_void_p(_ptr(self._translations[1])))
+        self._scratch_words = None if per_level else sizes[7] // 8 + 1
+        if sizes[6] > 0:
+            self._translations = [torch.zeros(n, dtype=torch.float64, device=self.device)
+                                  for n in (sizes[6] // 8 + 1, 1)]
+            ws = self._translation_ws(None, None, self._translations[1])
             self.plan.call("qbxfmm_precompute_translations", ctypes.byref(ws), _stream_handle())
         self.traversal = geo_data.traversal()
         self.tree = self.traversal.tree
@@ -354,8 +354,31 @@ class B200QBXExpansionWrangler:
                        ctypes.c_void_p(_ptr(mp)), self._s())
         return mp
 
+    def _translation_ws(self, mpoles, locals_, scratch):
+        z = ctypes.c_void_p(0)
+        ptr = lambda t: z if t is None else ctypes.c_void_p(_ptr(t))  # noqa: E731
+        return abi.QBXFMMWorkspace(z, ptr(mpoles), ptr(locals_), z, z, z, None,
+                                   ptr(self._translations[0]), ptr(scratch))
+
+    def _translate(self, stage, mpoles=None, locals_=None):
+        """M2M (0), M2L (1) or L2L (2) with the plan's matrices, if there are any and memory
+        for the products of the pairs is left.  The scratch belongs to this call and its
+        stream."""
+        if self._translations is None or self._scratch_words is None:
+            return False
+        try:
+            scratch = torch.empty(self._scratch_words, dtype=torch.float64, device=self.device)
+        except torch.OutOfMemoryError:
+            return False
+        ws = self._translation_ws(mpoles, locals_, scratch)
+        ws.error_word = ctypes.cast(self._err(), ctypes.POINTER(ctypes.c_int32))
+        self.plan.call("qbxfmm_translate_boxes", ctypes.byref(ws), stage, self._s())
+        return True
+
     def coarsen_multipoles(self, actx, level_start_source_parent_box_nrs,
                            source_parent_boxes, mpoles):
+        if self._translate(0, mpoles=mpoles):
+            return mpoles
         self.plan.call("qbxfmm_coarsen_multipoles", ctypes.c_void_p(_ptr(mpoles)), self._s())
         return mpoles
 
@@ -369,6 +392,8 @@ class B200QBXExpansionWrangler:
     def multipole_to_local(self, actx, level_start_target_box_nrs, target_boxes,
                            starts, lists, mpole_exps):
         lo = self.local_expansion_zeros()
+        if self._translate(1, mpoles=mpole_exps, locals_=lo):
+            return lo
         self.plan.call("qbxfmm_multipole_to_local", ctypes.c_void_p(_ptr(mpole_exps)),
                        ctypes.c_void_p(_ptr(lo)), self._err(), self._s())
         return lo
@@ -389,6 +414,8 @@ class B200QBXExpansionWrangler:
 
     def refine_locals(self, actx, level_start_target_or_target_parent_box_nrs,
                       target_or_target_parent_boxes, local_exps):
+        if self._translate(2, locals_=local_exps):
+            return local_exps
         self.plan.call("qbxfmm_refine_locals", ctypes.c_void_p(_ptr(local_exps)), self._s())
         return local_exps
 

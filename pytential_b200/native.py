@@ -39,6 +39,7 @@ _STAGES = {
     "qbxfmm_assemble": [_vp, _vp, _vp, _vp],
     "qbxfmm_workspace_sizes": [ctypes.POINTER(ctypes.c_size_t)],
     "qbxfmm_precompute_translations": [ctypes.POINTER(abi.QBXFMMWorkspace), _vp],
+    "qbxfmm_translate_boxes": [ctypes.POINTER(abi.QBXFMMWorkspace), ctypes.c_int, _vp],
     "qbxfmm_apply": [ctypes.POINTER(abi.QBXFMMUpsample), ctypes.POINTER(abi.QBXFMMWorkspace),
                      _vp, _vp, _vp],
     "qbxfmm_apply_noalloc": [ctypes.POINTER(abi.QBXFMMUpsample), _vp, _vp, _vp],

@@ -80,11 +80,15 @@ def _translate(geo, k, p, kind, exps):
 @pytest.mark.parametrize("p,nrhs", [(1, 1), (3, 3), (4, 5), (7, 4), (8, 9), (10, 8), (12, 16),
                                     (15, 17), (16, 2), (19, 40), (20, 1), (20, 33)])
 @pytest.mark.parametrize("kind", ["up", "l2", "down"])
-def test_translations(p, nrhs, kind):
+@pytest.mark.parametrize("tables", [False, True])
+def test_translations(p, nrhs, kind, tables):
     k = 6.0
     d, geo = _geometry()
     spec = fmm.SourceKernelSpec(fmm.HelmholtzKernel(2, k), charge_coeff=-1j * k, dipole_coeff=1.0)
     w = _wrangler(geo, spec, 2, p, nrhs)
+    assert w._translations is not None
+    if not tables:
+        w._translations = None
     rng = np.random.default_rng(p)
     shape = (geo.tree().nboxes, nrhs, 2 * p + 1)
     e = rng.normal(size=shape) + 1j * rng.normal(size=shape)

@@ -89,8 +89,12 @@ def _close_by_degree(got, want, p):
 
 
 @pytest.mark.parametrize("p", [1, 10, 14, 15, 20])
-def test_translations_by_pair(p):
+@pytest.mark.parametrize("matrices", [False, True])
+def test_translations(p, matrices):
     w, o, s = _setup(2, p, 1.0, 0.0)
+    assert w._translations is not None
+    if not matrices:
+        w._translations = None
     mp = o.zeros_box_exps()
     o.stage("form_multipoles", s, mp)
     _close_by_degree(w.form_multipoles(None, None, None, [torch.from_numpy(s).cuda()]), mp, p)

@@ -98,6 +98,15 @@ cudaError_t launch_l2l_direct(const qbxfmm_geometry& g, const TransHost& th, con
 
 cudaError_t launch_form_strengths(const qbxfmm_geometry& g, const qbxfmm_upsample& up, int nrhs,
                                   const double* density, double* strengths, cudaStream_t st);
+// 2D Laplace (kernels_laplace2d.cu), reached through the launch_* of the same stages
+cudaError_t l2_launch_p2m(const qbxfmm_geometry& g, SourceCoeffs sc, int p, int nrhs,
+                          const double* s, double2* mp, cudaStream_t st);
+cudaError_t l2_launch_m2m(const qbxfmm_geometry& g, const int32_t* lvl_host, int p, int nrhs,
+                          double2* mp, cudaStream_t st);
+cudaError_t l2_launch_m2l(const qbxfmm_geometry& g, int p, int nrhs, const double2* mp, double2* lo,
+                          int32_t* err, cudaStream_t st);
+cudaError_t l2_launch_l2l(const qbxfmm_geometry& g, const int32_t* lvl_host, int p, int nrhs,
+                          double2* lo, cudaStream_t st);
 cudaError_t launch_p2m(const qbxfmm_geometry& g, SourceCoeffs sc, int p, int nrhs,
                        const double* s, double2* mp, cudaStream_t st);
 cudaError_t launch_m2m(const qbxfmm_geometry& g, const int32_t* lvl_host, int p, int nrhs,

@@ -105,10 +105,10 @@ QBX_D int stream_source(int v, int nb, const int* s_pref, const int* s_start)
 }
 
 // Stage sources [base, base + NT) of the stream into shared memory.
-template <int DIM, bool NORMALS>
+template <int DIM, bool NORMALS, int TN = NT>
 QBX_D void load_stream_tile(const qbxfmm_geometry& g, const double* __restrict__ st, int total,
                             int nb, int base, const int* s_pref, const int* s_start,
-                            double (*s_y)[NT], double (*s_n)[NT], double* s_q)
+                            double (*s_y)[TN], double (*s_n)[TN], double* s_q)
 {
   int v = base + threadIdx.x;
   if (v < total) {
@@ -138,9 +138,8 @@ QBX_D void load_stream_tile(const qbxfmm_geometry& g, const double* __restrict__
 constexpr int P2M_SUB = 16;
 constexpr int P2M_TS = P2M_SUB + 1;
 
-template <int DIM>
 __global__ void __launch_bounds__(NT)
-k_p2m(qbxfmm_geometry g, SourceCoeffs sc, int p, int ncf, int nrhs,
+k_p2m3(qbxfmm_geometry g, SourceCoeffs sc, int p, int ncf, int nrhs,
       const double* __restrict__ strengths, double2* __restrict__ mpoles)
 {
   constexpr int SUB = P2M_SUB;
@@ -154,7 +153,7 @@ k_p2m(qbxfmm_geometry g, SourceCoeffs sc, int p, int ncf, int nrhs,
   double rho = level_width(g, g.box_levels[b]);
   double rinv = 1.0 / rho;
   double c[3];
-  load_point<DIM>(g.box_centers, g.nboxes, b, c);
+  load_point<3>(g.box_centers, g.nboxes, b, c);
   int s0 = g.box_source_starts[b];
   int ns = g.box_source_counts_nonchild[b];
   const double* st = strengths + (size_t)r * g.nsources;
@@ -172,7 +171,7 @@ k_p2m(qbxfmm_geometry g, SourceCoeffs sc, int p, int ncf, int nrhs,
     valid[h] = ci < ncf;
     o_nm[h] = o_a[h] = o_b[h] = o_c[h] = 0;
     w_a[h] = w_b[h] = w_c[h] = 0.0;
-    if (DIM == 3 && valid[h]) {
+    if (valid[h]) {
       int n, m;
       decode3(ci, n, m);
       o_nm[h] = idx3(n, m) * TS;
@@ -191,46 +190,34 @@ k_p2m(qbxfmm_geometry g, SourceCoeffs sc, int p, int ncf, int nrhs,
     if (threadIdx.x < cnt) {
       int s = s0 + base + threadIdx.x;
       double y[3];
-      load_point<DIM>(g.sources, g.nsources, s, y);
+      load_point<3>(g.sources, g.nsources, s, y);
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) s_u[threadIdx.x][d] = (y[d] - c[d]) * rinv;
+      for (int d = 0; d < 3; ++d) s_u[threadIdx.x][d] = (y[d] - c[d]) * rinv;
       if (dip) {
         double nv[3];
-        load_point<DIM>(g.source_normals, g.nsources, s, nv);
+        load_point<3>(g.source_normals, g.nsources, s, nv);
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) s_n[threadIdx.x][d] = nv[d];
+        for (int d = 0; d < 3; ++d) s_n[threadIdx.x][d] = nv[d];
       }
       s_q[threadIdx.x] = __ldg(st + s);
     }
     __syncthreads();
-    if (DIM == 3) {
-      for (int w = threadIdx.x; w < cnt * (p + 1); w += NT) {
-        int m = w / cnt, j = w - m * cnt;
-        // column m of R for source j
-        double x = s_u[j][0], y = s_u[j][1], z = s_u[j][2];
-        double r2 = x * x + y * y + z * z;
-        double2 a = c2(1.0);
-        for (int k = 1; k <= m; ++k) a = cscale(0.5 * rcp(k), cmul(a, c2(x, y)));
-        double2* T = tab + j;
-        T[idx3(m, m) * TS] = a;
-        double2 prev = c2(0.0);
-        for (int n = m + 1; n <= p; ++n) {
-          double2 bb = cscale(rcp(n + m) * rcp(n - m),
-                              csub(cscale((2.0 * n - 1) * z, a), cscale(r2, prev)));
-          T[idx3(n, m) * TS] = bb;
-          prev = a;
-          a = bb;
-        }
-      }
-    } else {
-      for (int j = threadIdx.x; j < cnt; j += NT) {
-        double2 u = c2(s_u[j][0], s_u[j][1]);
-        double2* T = tab + j;
-        double2 a = c2(1.0);
-        for (int k = 0; k <= p; ++k) {
-          T[k * TS] = a;  // u^k
-          a = cmul(a, u);
-        }
+    for (int w = threadIdx.x; w < cnt * (p + 1); w += NT) {
+      int m = w / cnt, j = w - m * cnt;
+      // column m of R for source j
+      double x = s_u[j][0], y = s_u[j][1], z = s_u[j][2];
+      double r2 = x * x + y * y + z * z;
+      double2 a = c2(1.0);
+      for (int k = 1; k <= m; ++k) a = cscale(0.5 * rcp(k), cmul(a, c2(x, y)));
+      double2* T = tab + j;
+      T[idx3(m, m) * TS] = a;
+      double2 prev = c2(0.0);
+      for (int n = m + 1; n <= p; ++n) {
+        double2 bb = cscale(rcp(n + m) * rcp(n - m),
+                            csub(cscale((2.0 * n - 1) * z, a), cscale(r2, prev)));
+        T[idx3(n, m) * TS] = bb;
+        prev = a;
+        a = bb;
       }
     }
     __syncthreads();
@@ -239,38 +226,21 @@ k_p2m(qbxfmm_geometry g, SourceCoeffs sc, int p, int ncf, int nrhs,
       if (!valid[h]) continue;
       int ci = threadIdx.x + h * NT;
       double2 a = acc[h];
-      if (DIM == 3) {
-        for (int j = 0; j < cnt; ++j) {
-          const double2* T = tab + j;
-          double q = s_q[j];
-          a = caxpy(sc.cq * q, cconj(T[o_nm[h]]), a);
-          if (dip) {
-            double f = sc.cd * q * rinv;
-            double dx = s_n[j][0], dy = s_n[j][1], dz = s_n[j][2];
-            // conj(dz R_{n-1}^m + (dx+idy)/2 R_{n-1}^{m-1} - (dx-idy)/2 R_{n-1}^{m+1})
-            double2 tb_ = T[o_b[h]];
-            if (w_b[h] < 0) tb_ = c2(-tb_.x, tb_.y);
-            else tb_ = cscale(w_b[h], tb_);
-            double2 v = cscale(dz * w_a[h], T[o_a[h]]);
-            v = cfma(c2(0.5 * dx, 0.5 * dy), tb_, v);
-            v = cfma(c2(-0.5 * dx * w_c[h], 0.5 * dy * w_c[h]), T[o_c[h]], v);
-            a = caxpy(f, cconj(v), a);
-          }
-        }
-      } else {
-        int k = ci;
-        for (int j = 0; j < cnt; ++j) {
-          const double2* T = tab + j;
-          double q = s_q[j];
-          if (k == 0) {
-            a.x += sc.cq * q;
-          } else {
-            a = caxpy(-sc.cq * q * rcp(k), T[k * TS], a);
-            if (dip) {
-              double2 nu = c2(s_n[j][0], s_n[j][1]);
-              a = cfma(cscale(-sc.cd * q * rinv, nu), T[(k - 1) * TS], a);
-            }
-          }
+      for (int j = 0; j < cnt; ++j) {
+        const double2* T = tab + j;
+        double q = s_q[j];
+        a = caxpy(sc.cq * q, cconj(T[o_nm[h]]), a);
+        if (dip) {
+          double f = sc.cd * q * rinv;
+          double dx = s_n[j][0], dy = s_n[j][1], dz = s_n[j][2];
+          // conj(dz R_{n-1}^m + (dx+idy)/2 R_{n-1}^{m-1} - (dx-idy)/2 R_{n-1}^{m+1})
+          double2 tb_ = T[o_b[h]];
+          if (w_b[h] < 0) tb_ = c2(-tb_.x, tb_.y);
+          else tb_ = cscale(w_b[h], tb_);
+          double2 v = cscale(dz * w_a[h], T[o_a[h]]);
+          v = cfma(c2(0.5 * dx, 0.5 * dy), tb_, v);
+          v = cfma(c2(-0.5 * dx * w_c[h], 0.5 * dy * w_c[h]), T[o_c[h]], v);
+          a = caxpy(f, cconj(v), a);
         }
       }
       acc[h] = a;
@@ -289,9 +259,8 @@ k_p2m(qbxfmm_geometry g, SourceCoeffs sc, int p, int ncf, int nrhs,
 
 // {{{ M2M (coarsen_multipoles, fmm.py:451-455), one launch per parent level
 
-template <int DIM>
 __global__ void __launch_bounds__(NT)
-k_m2m(qbxfmm_geometry g, int p, int ncf, int nrhs, int i0, double2* __restrict__ mpoles)
+k_m2m3(qbxfmm_geometry g, int p, int ncf, int nrhs, int i0, double2* __restrict__ mpoles)
 {
   extern __shared__ double2 smem2[];
   double2* tab = smem2;          // [ncf] R table / powers
@@ -302,57 +271,34 @@ k_m2m(qbxfmm_geometry g, int p, int ncf, int nrhs, int i0, double2* __restrict__
   double rho_p = level_width(g, lev), rho_c = level_width(g, lev + 1);
   double ratio = rho_c / rho_p;
   double cp[3];
-  load_point<DIM>(g.box_centers, g.nboxes, b, cp);
+  load_point<3>(g.box_centers, g.nboxes, b, cp);
   double2 acc[2] = {c2(0.0), c2(0.0)};
-  const int nch = 1 << DIM;
+  const int nch = 1 << 3;
   for (int ci = 0; ci < nch; ++ci) {
     int ch = g.box_child_ids[(size_t)ci * g.nboxes + b];
     if (ch == 0 || g.box_source_counts_cumul[ch] == 0) continue;
     double cc[3], d[3];
-    load_point<DIM>(g.box_centers, g.nboxes, ch, cc);
+    load_point<3>(g.box_centers, g.nboxes, ch, cc);
 #pragma unroll
-    for (int k = 0; k < DIM; ++k) d[k] = (cc[k] - cp[k]) / rho_p;
+    for (int k = 0; k < 3; ++k) d[k] = (cc[k] - cp[k]) / rho_p;
     const double2* src = mpoles + ((size_t)ch * nrhs + r) * ncf;
     for (int i = threadIdx.x; i < ncf; i += NT) Min[i] = src[i];
-    if (DIM == 3) {
-      sh3_R_table(p, d[0], d[1], d[2], tab, threadIdx.x, NT);
-    } else if (threadIdx.x == 0) {
-      double2 t = c2(d[0], d[1]), a = c2(1.0);
-      for (int k = 0; k <= p; ++k) {
-        tab[k] = a;
-        a = cmul(a, t);
-      }
-    }
+    sh3_R_table(p, d[0], d[1], d[2], tab, threadIdx.x, NT);
     __syncthreads();
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       int o = threadIdx.x + h * NT;
       if (o >= ncf) break;
       double2 a = acc[h];
-      if (DIM == 3) {
-        int n, m;
-        decode3(o, n, m);
-        double rk = 1.0;
-        for (int k = 0; k <= n; ++k, rk *= ratio)
-          for (int l = -k; l <= k; ++l) {
-            int dm = m - l;
-            if (dm > n - k || -dm > n - k) continue;
-            a = cfmac(cscale(rk, sh3_get(Min, k, l)), sh3_get(tab, n - k, dm), a);
-          }
-      } else {
-        int l = o;
-        if (l == 0) {
-          a = cadd(a, Min[0]);
-        } else {
-          a = cfma(cscale(-rcp(l), Min[0]), tab[l], a);
-          double rk = ratio, bin = 1.0;  // C(l-1, k-1)
-          for (int k = 1; k <= l; ++k) {
-            a = cfma(cscale(rk * bin, Min[k]), tab[l - k], a);
-            rk *= ratio;
-            bin = bin * (l - k) * rcp(k);
-          }
+      int n, m;
+      decode3(o, n, m);
+      double rk = 1.0;
+      for (int k = 0; k <= n; ++k, rk *= ratio)
+        for (int l = -k; l <= k; ++l) {
+          int dm = m - l;
+          if (dm > n - k || -dm > n - k) continue;
+          a = cfmac(cscale(rk, sh3_get(Min, k, l)), sh3_get(tab, n - k, dm), a);
         }
-      }
       acc[h] = a;
     }
     __syncthreads();
@@ -504,69 +450,6 @@ k_m2l3(qbxfmm_geometry g, int p, int ncf, int nrhs, int pb_max, const double2* _
       double2 v = cadd(acc[h], red[o]);
       L[o] = caxpy((j & 1) ? -1.0 / rho : 1.0 / rho, v, L[o]);
     }
-  }
-}
-
-// 2D: L_0 = M_0 log t + sum_k M_k tau^-k,
-//     L_l = (-1)^(l+1) M_0 / (l tau^l) + (-1)^l tau^-l sum_k M_k C(k+l-1, l) tau^-k.
-__global__ void __launch_bounds__(NT)
-k_m2l2(qbxfmm_geometry g, int p, int ncf, int nrhs, const double2* __restrict__ mpoles,
-       double2* __restrict__ locals, int32_t* err)
-{
-  extern __shared__ double2 smem2[];
-  double2* Min = smem2;             // [ncf]
-  double2* tab = smem2 + ncf;       // [2p+2]
-  int i = blockIdx.x;
-  int tb = g.target_or_target_parent_boxes[i];
-  int r = blockIdx.y;
-  double rho = level_width(g, g.box_levels[tb]);
-  double ct[3];
-  load_point<2>(g.box_centers, g.nboxes, tb, ct);
-  double2 acc = c2(0.0);
-  int l0 = g.list2_starts[i], l1 = g.list2_starts[i + 1];
-  for (int li = l0; li < l1; ++li) {
-    int sb = g.list2_lists[li];
-    if ((unsigned)sb >= (unsigned)g.nboxes) {
-      report(err, QBX_DEVERR_BAD_BOX);
-      continue;
-    }
-    double cs[3];
-    load_point<2>(g.box_centers, g.nboxes, sb, cs);
-    double d0 = (ct[0] - cs[0]) / rho, d1 = (ct[1] - cs[1]) / rho;
-    const double2* src = mpoles + ((size_t)sb * nrhs + r) * ncf;
-    for (int q = threadIdx.x; q < ncf; q += NT) Min[q] = src[q];
-    if (threadIdx.x == 0) {
-      double2 tinv = cinv(c2(d0, d1)), a = tinv;
-      tab[0] = clog_(c2(d0 * rho, d1 * rho));
-      for (int k = 1; k <= 2 * p + 1; ++k) {
-        tab[k] = a;  // tau^-k
-        a = cmul(a, tinv);
-      }
-    }
-    __syncthreads();
-    int l = threadIdx.x;
-    if (l < ncf) {
-      if (l == 0) {
-        double2 s = cmul(Min[0], tab[0]);
-        for (int k = 1; k <= p; ++k) s = cfma(Min[k], tab[k], s);
-        acc = cadd(acc, s);
-      } else {
-        double2 s = c2(0.0);
-        double bin = 1.0;  // C(k+l-1, l) at k = 1
-        for (int k = 1; k <= p; ++k) {
-          s = cfma(cscale(bin, Min[k]), tab[k], s);
-          bin = bin * (k + l) * rcp(k);
-        }
-        double2 v = cscale(((l & 1) ? 1.0 : -1.0) * rcp(l), Min[0]);
-        v = cadd(v, cscale((l & 1) ? -1.0 : 1.0, s));
-        acc = cfma(v, tab[l], acc);
-      }
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x < ncf) {
-    double2* L = locals + ((size_t)tb * nrhs + r) * ncf;
-    L[threadIdx.x] = cadd(L[threadIdx.x], acc);
   }
 }
 
@@ -800,9 +683,8 @@ k_p2l3(qbxfmm_geometry g, SourceCoeffs sc, int p, int ncf, int nrhs,
 
 // {{{ L2L (refine_locals, fmm.py:519-523), one launch per child level
 
-template <int DIM>
 __global__ void __launch_bounds__(NT)
-k_l2l(qbxfmm_geometry g, int p, int ncf, int nrhs, int i0, double2* __restrict__ locals)
+k_l2l3(qbxfmm_geometry g, int p, int ncf, int nrhs, int i0, double2* __restrict__ locals)
 {
   extern __shared__ double2 smem2[];
   double2* tab = smem2;
@@ -814,44 +696,26 @@ k_l2l(qbxfmm_geometry g, int p, int ncf, int nrhs, int i0, double2* __restrict__
   double rho_p = level_width(g, lev - 1), rho_c = level_width(g, lev);
   double ratio = rho_c / rho_p;
   double cp[3], cc[3], d[3];
-  load_point<DIM>(g.box_centers, g.nboxes, par, cp);
-  load_point<DIM>(g.box_centers, g.nboxes, b, cc);
+  load_point<3>(g.box_centers, g.nboxes, par, cp);
+  load_point<3>(g.box_centers, g.nboxes, b, cc);
 #pragma unroll
-  for (int k = 0; k < DIM; ++k) d[k] = (cc[k] - cp[k]) / rho_p;
+  for (int k = 0; k < 3; ++k) d[k] = (cc[k] - cp[k]) / rho_p;
   const double2* src = locals + ((size_t)par * nrhs + r) * ncf;
   for (int q = threadIdx.x; q < ncf; q += NT) Lin[q] = src[q];
-  if (DIM == 3) {
-    sh3_R_table(p, d[0], d[1], d[2], tab, threadIdx.x, NT);
-  } else if (threadIdx.x == 0) {
-    double2 s = c2(d[0], d[1]), a = c2(1.0);
-    for (int k = 0; k <= p; ++k) {
-      tab[k] = a;
-      a = cmul(a, s);
-    }
-  }
+  sh3_R_table(p, d[0], d[1], d[2], tab, threadIdx.x, NT);
   __syncthreads();
   double2* L = locals + ((size_t)b * nrhs + r) * ncf;
   for (int o = threadIdx.x; o < ncf; o += NT) {
     double2 a = c2(0.0);
-    if (DIM == 3) {
-      int k, l;
-      decode3(o, k, l);
-      for (int n = k; n <= p; ++n)
-        for (int m = -n; m <= n; ++m) {
-          int dm = m - l;
-          if (dm > n - k || -dm > n - k) continue;
-          a = cfmac(sh3_get(Lin, n, m), sh3_get(tab, n - k, dm), a);
-        }
-      a = cscale(pow(ratio, (double)k), a);
-    } else {
-      int l = o;
-      double bin = 1.0;  // C(k, l)
-      for (int k = l; k <= p; ++k) {
-        a = cfma(cscale(bin, Lin[k]), tab[k - l], a);
-        bin = bin * (k + 1) * rcp(k + 1 - l);
+    int k, l;
+    decode3(o, k, l);
+    for (int n = k; n <= p; ++n)
+      for (int m = -n; m <= n; ++m) {
+        int dm = m - l;
+        if (dm > n - k || -dm > n - k) continue;
+        a = cfmac(sh3_get(Lin, n, m), sh3_get(tab, n - k, dm), a);
       }
-      a = cscale(pow(ratio, (double)l), a);
-    }
+    a = cscale(pow(ratio, (double)k), a);
     L[o] = cadd(L[o], a);
   }
 }
@@ -1604,17 +1468,22 @@ k_tsqbx3(qbxfmm_geometry g, SourceCoeffs sc, int nrhs, const double* __restrict_
   }
 }
 
-// 2D (lane = target)
-template <int Q, bool CHG, bool DIP>
-__global__ void __launch_bounds__(NT)
+constexpr size_t TS2_FEW = 4 * 148;
+
+// 2D (lane = target), W warps that share the sources: 16 where the chunks alone leave the GPU
+// idle, else 4.
+// 68 us with 4 warps at 1024 nodes, where it ran beside the box stages for longer than they took.
+template <int Q, bool CHG, bool DIP, int W>
+__global__ void __launch_bounds__(32 * W)
 k_tsqbx2(qbxfmm_geometry g, SourceCoeffs sc, int nrhs, const double* __restrict__ strengths,
         double* __restrict__ pot_tree, int32_t* err)
 {
-  __shared__ double s_y[3][NT];
-  __shared__ double s_n[3][NT];
-  __shared__ double s_q[NT];
+  constexpr int TN = 32 * W;
+  __shared__ double s_y[3][TN];
+  __shared__ double s_n[3][TN];
+  __shared__ double s_q[TN];
   __shared__ int s_pref[MAXB + 1], s_start[MAXB];
-  __shared__ double s_red[NW - 1][32];
+  __shared__ double s_red[W - 1][32];
   int chunk = blockIdx.x;
   int r = blockIdx.y;
   int itb = g.tsqbx_chunk_target_box[chunk];
@@ -1641,8 +1510,8 @@ k_tsqbx2(qbxfmm_geometry g, SourceCoeffs sc, int nrhs, const double* __restrict_
     list_prefix(g, g.list1_lists, gb, nb, s_pref, s_start, err);
     __syncthreads();
     int total = s_pref[nb];
-    for (int base = 0; base < total; base += NT) {
-      load_stream_tile<2, DIP>(g, st, total, nb, base, s_pref, s_start, s_y, s_n, s_q);
+    for (int base = 0; base < total; base += TN) {
+      load_stream_tile<2, DIP, TN>(g, st, total, nb, base, s_pref, s_start, s_y, s_n, s_q);
       __syncthreads();
       int jbeg = warp * 32, jend = min(jbeg + 32, total - base);
       if (active) {
@@ -1675,7 +1544,7 @@ k_tsqbx2(qbxfmm_geometry g, SourceCoeffs sc, int nrhs, const double* __restrict_
   if (warp > 0) s_red[warp - 1][lane] = acc;
   __syncthreads();
   if (warp == 0 && active) {
-    for (int w = 1; w < NW; ++w) acc += s_red[w - 1][lane];
+    for (int w = 1; w < W; ++w) acc += s_red[w - 1][lane];
     pot_tree[(size_t)r * g.ntargets + t] += acc;
   }
 }
@@ -1870,34 +1739,32 @@ cudaError_t launch_form_strengths(const qbxfmm_geometry& g, const qbxfmm_upsampl
   return cudaGetLastError();
 }
 
-template <int DIM>
-static cudaError_t p2m_(const qbxfmm_geometry& g, SourceCoeffs sc, int p, int nrhs,
+static cudaError_t p2m3(const qbxfmm_geometry& g, SourceCoeffs sc, int p, int nrhs,
                         const double* s, double2* mp, cudaStream_t st)
 {
-  int ncf = (int)ncoef_dim(DIM, p);
+  int ncf = (int)ncoef_dim(3, p);
   size_t sh = (size_t)P2M_TS * ncf * sizeof(double2);
   if (g.nsource_boxes == 0) return cudaSuccess;
-  cudaFuncSetAttribute(k_p2m<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-  k_p2m<DIM><<<dim3(g.nsource_boxes, grid_y(nrhs)), NT, sh, st>>>(g, sc, p, ncf, nrhs, s, mp);
+  cudaFuncSetAttribute(k_p2m3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+  k_p2m3<<<dim3(g.nsource_boxes, grid_y(nrhs)), NT, sh, st>>>(g, sc, p, ncf, nrhs, s, mp);
   return cudaGetLastError();
 }
 
 cudaError_t launch_p2m(const qbxfmm_geometry& g, SourceCoeffs sc, int p, int nrhs,
                        const double* s, double2* mp, cudaStream_t st)
 {
-  return g.dim == 3 ? p2m_<3>(g, sc, p, nrhs, s, mp, st) : p2m_<2>(g, sc, p, nrhs, s, mp, st);
+  return g.dim == 3 ? p2m3(g, sc, p, nrhs, s, mp, st) : l2_launch_p2m(g, sc, p, nrhs, s, mp, st);
 }
 
-template <int DIM>
-static cudaError_t m2m_(const qbxfmm_geometry& g, const int32_t* lvl_host, int p, int nrhs,
+static cudaError_t m2m3(const qbxfmm_geometry& g, const int32_t* lvl_host, int p, int nrhs,
                         double2* mp, cudaStream_t st)
 {
-  int ncf = (int)ncoef_dim(DIM, p);
+  int ncf = (int)ncoef_dim(3, p);
   size_t sh = 2 * (size_t)ncf * sizeof(double2);
   for (int lev = g.nlevels - 2; lev >= 0; --lev) {
     int i0 = lvl_host[lev], i1 = lvl_host[lev + 1];
     if (i1 <= i0) continue;
-    k_m2m<DIM><<<dim3(i1 - i0, grid_y(nrhs)), NT, sh, st>>>(g, p, ncf, nrhs, i0, mp);
+    k_m2m3<<<dim3(i1 - i0, grid_y(nrhs)), NT, sh, st>>>(g, p, ncf, nrhs, i0, mp);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -1907,24 +1774,20 @@ static cudaError_t m2m_(const qbxfmm_geometry& g, const int32_t* lvl_host, int p
 cudaError_t launch_m2m(const qbxfmm_geometry& g, const int32_t* lvl_host, int p, int nrhs,
                        double2* mp, cudaStream_t st)
 {
-  return g.dim == 3 ? m2m_<3>(g, lvl_host, p, nrhs, mp, st) : m2m_<2>(g, lvl_host, p, nrhs, mp, st);
+  return g.dim == 3 ? m2m3(g, lvl_host, p, nrhs, mp, st) : l2_launch_m2m(g, lvl_host, p, nrhs, mp, st);
 }
 
 cudaError_t launch_m2l(const qbxfmm_geometry& g, int p, int nrhs, const double2* mp, double2* lo,
                        int32_t* err, cudaStream_t st)
 {
   if (g.nttp_boxes == 0) return cudaSuccess;
-  int ncf = (int)ncoef_dim(g.dim, p);
-  if (g.dim == 3) {
-    size_t per = ((size_t)(2 * p + 1) * (3 * p + 1) + (size_t)(p + 1) * (2 * p + 1)) * sizeof(double2);
-    int pb = (int)std::min<size_t>(4, std::max<size_t>(1, (160 * 1024 - ncf * sizeof(double2)) / per));
-    size_t sh = pb * per + ncf * sizeof(double2);
-    cudaFuncSetAttribute(k_m2l3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    k_m2l3<<<dim3(g.nttp_boxes, grid_y(nrhs)), NT, sh, st>>>(g, p, ncf, nrhs, pb, mp, lo, err);
-  } else {
-    size_t sh = ((size_t)ncf + 2 * p + 2) * sizeof(double2);
-    k_m2l2<<<dim3(g.nttp_boxes, grid_y(nrhs)), NT, sh, st>>>(g, p, ncf, nrhs, mp, lo, err);
-  }
+  if (g.dim == 2) return l2_launch_m2l(g, p, nrhs, mp, lo, err, st);
+  const int ncf = (int)ncoef_dim(3, p);
+  size_t per = ((size_t)(2 * p + 1) * (3 * p + 1) + (size_t)(p + 1) * (2 * p + 1)) * sizeof(double2);
+  int pb = (int)std::min<size_t>(4, std::max<size_t>(1, (160 * 1024 - ncf * sizeof(double2)) / per));
+  size_t sh = pb * per + ncf * sizeof(double2);
+  cudaFuncSetAttribute(k_m2l3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+  k_m2l3<<<dim3(g.nttp_boxes, grid_y(nrhs)), NT, sh, st>>>(g, p, ncf, nrhs, pb, mp, lo, err);
   return cudaGetLastError();
 }
 
@@ -1972,16 +1835,15 @@ cudaError_t launch_p2l(const qbxfmm_geometry& g, SourceCoeffs sc, int p, int nrh
                       : p2l3<false>(g, sc, p, nrhs, s, lo, err, st);
 }
 
-template <int DIM>
-static cudaError_t l2l_(const qbxfmm_geometry& g, const int32_t* lvl_host, int p, int nrhs,
+static cudaError_t l2l3(const qbxfmm_geometry& g, const int32_t* lvl_host, int p, int nrhs,
                         double2* lo, cudaStream_t st)
 {
-  int ncf = (int)ncoef_dim(DIM, p);
+  int ncf = (int)ncoef_dim(3, p);
   size_t sh = 2 * (size_t)ncf * sizeof(double2);
   for (int lev = 1; lev < g.nlevels; ++lev) {
     int i0 = lvl_host[lev], i1 = lvl_host[lev + 1];
     if (i1 <= i0) continue;
-    k_l2l<DIM><<<dim3(i1 - i0, grid_y(nrhs)), NT, sh, st>>>(g, p, ncf, nrhs, i0, lo);
+    k_l2l3<<<dim3(i1 - i0, grid_y(nrhs)), NT, sh, st>>>(g, p, ncf, nrhs, i0, lo);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -1991,7 +1853,7 @@ static cudaError_t l2l_(const qbxfmm_geometry& g, const int32_t* lvl_host, int p
 cudaError_t launch_l2l(const qbxfmm_geometry& g, const int32_t* lvl_host, int p, int nrhs,
                        double2* lo, cudaStream_t st)
 {
-  return g.dim == 3 ? l2l_<3>(g, lvl_host, p, nrhs, lo, st) : l2l_<2>(g, lvl_host, p, nrhs, lo, st);
+  return g.dim == 3 ? l2l3(g, lvl_host, p, nrhs, lo, st) : l2_launch_l2l(g, lvl_host, p, nrhs, lo, st);
 }
 
 cudaError_t launch_eval_direct(const qbxfmm_geometry& g, SourceCoeffs sc, int nrhs,
@@ -2169,9 +2031,18 @@ static cudaError_t tsqbx_q(const qbxfmm_geometry& g, SourceCoeffs sc, int nrhs, 
     else if (sc.cd != 0.0) k_tsqbx3<Q, false, true><<<grid, NT, 0, st>>>(g, sc, nrhs, s, pt, err);
     else k_tsqbx3<Q, true, false><<<grid, NT, 0, st>>>(g, sc, nrhs, s, pt, err);
   } else {
-    if (sc.cq != 0.0 && sc.cd != 0.0) k_tsqbx2<Q, true, true><<<grid, NT, 0, st>>>(g, sc, nrhs, s, pt, err);
-    else if (sc.cd != 0.0) k_tsqbx2<Q, false, true><<<grid, NT, 0, st>>>(g, sc, nrhs, s, pt, err);
-    else k_tsqbx2<Q, true, false><<<grid, NT, 0, st>>>(g, sc, nrhs, s, pt, err);
+    const bool few = (size_t)g.ntsqbx_chunks * nrhs < TS2_FEW;
+    auto launch = [&](auto wide) {
+      constexpr int W = decltype(wide)::value;
+      if (sc.cq != 0.0 && sc.cd != 0.0)
+        k_tsqbx2<Q, true, true, W><<<grid, 32 * W, 0, st>>>(g, sc, nrhs, s, pt, err);
+      else if (sc.cd != 0.0)
+        k_tsqbx2<Q, false, true, W><<<grid, 32 * W, 0, st>>>(g, sc, nrhs, s, pt, err);
+      else
+        k_tsqbx2<Q, true, false, W><<<grid, 32 * W, 0, st>>>(g, sc, nrhs, s, pt, err);
+    };
+    if (few) launch(std::integral_constant<int, 16>());
+    else launch(std::integral_constant<int, NW>());
   }
   return cudaGetLastError();
 }

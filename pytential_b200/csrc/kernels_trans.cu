@@ -25,6 +25,7 @@
 #include <array>
 #include <cstdlib>
 #include <map>
+#include <type_traits>
 #include <vector>
 
 #include <cooperative_groups.h>
@@ -35,8 +36,6 @@ namespace qbx {
 namespace {
 
 constexpr int NT = 128;
-constexpr int NTILE = 32;            // max columns (pair x rhs) per CTA
-constexpr int XS = NTILE + 4;        // padded X row stride (conflict-free B fragments)
 
 QBX_D void dmma_8x8x4(double& d0, double& d1, double a, double b)
 {
@@ -111,47 +110,56 @@ k_trans_build(int kind, int p, int ncf, int rp, int kp, int nclasses, const int3
 
 // {{{ GEMM
 
-constexpr int KC = 32;               // K chunk staged per step
-constexpr int TSTR = KC + 4;         // padded T-chunk row stride (== 4 mod 16 doubles)
+// C = T X for one group (class), one tile of 16 MI rows and one of 64 columns (pair x rhs):
+// four warps of 8 MI x 32, operands in four cp.async stages of 16 k, k-contiguous with a row
+// stride of 20 doubles (4 mod 16), free of bank conflicts as fragments.  A class symmetry
+// permutes and negates parts of coefficients: of X when a fragment is read, of C in the
+// epilogue.  If pair_dst is given the result is added (x scale) into the destination box's
+// expansion (each destination occurs once per launch), else stored into
+// cpair[pair * nrhs + r][0..rp).
+// The form before (32 columns, operands staged between two barriers per 32 k, one row
+// fragment loaded per product) took 4.53 ms for the M2L of 307 200 nodes at order 12 and
+// 0.222 ms of 19 200 at order 10; this 3.35 and 0.191.
+constexpr int GN = 64, GK = 16, GST = 4, GS = GK + 4;
 
-// C = T X for one group (class) and one tile of columns (pair x rhs).  Warps are
-// arranged NWN (column tiles of 8) x NWM (row groups); each warp holds MTW m-tiles
-// of 8 rows x one 8-column tile in registers.  T and X are streamed in K chunks of
-// KC through shared memory.  If pair_dst is given the result is added (x scale)
-// into the destination box's expansion (each destination occurs once per launch),
-// else stored into cpair[pair * nrhs + r][0..rp).
-template <int MTW>
+template <int MI>
+constexpr int gemm_stage() { return (16 * MI + GN) * GS; }
+
+QBX_D void cp_async16_zfill(void* dst, const void* src, bool on)
+{
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(on ? 16 : 0)
+               : "memory");
+}
+
+template <int MI>
 __global__ void __launch_bounds__(NT)
-k_trans_gemm(int ncf, int rp, int kp, int nrhs, int nwm, const double* __restrict__ T,
-             int mat_base, int mat_mod, const int32_t* __restrict__ cls_code,
-             const int32_t* __restrict__ group_starts, int g0,
+k_trans_gemm(int ncf, int rp, int kp, int nrhs, const double* __restrict__ T, int mat_mod,
+             const int32_t* __restrict__ cls_code, const int32_t* __restrict__ group_starts, int g0,
              const int32_t* __restrict__ pair_src, const int32_t* __restrict__ pair_dst,
              const double2* __restrict__ ein, double2* __restrict__ eout, double scale,
              double* __restrict__ cpair, int32_t* err, int nboxes)
 {
-  extern __shared__ double sm[];
-  const int nwn = 4 / nwm;
-  const int ntile = 8 * nwn;
-  double* Ts = sm;                          // [rp][TSTR]
-  double* Xs = sm + (size_t)rp * TSTR;      // [KC][XS]
-  __shared__ int s_src[NTILE];
-  int grp = g0 + blockIdx.y;
-  int p0 = group_starts[grp], p1 = group_starts[grp + 1];
-  int ncol = (p1 - p0) * nrhs;
-  int c0 = blockIdx.x * ntile;
+  constexpr int GM = 16 * MI;
+  extern __shared__ double2 smem2[];
+  double* sm = reinterpret_cast<double*>(smem2);       // [GST]{A [GM][GS], B [GN][GS]}
+  __shared__ int s_src[GN];
+  __shared__ uint8_t s_opi[M2L_SYM_MAXR], s_opo[M2L_SYM_MAXR];
+  const int grp = g0 + blockIdx.z;
+  const int p0 = group_starts[grp], ncol = (group_starts[grp + 1] - p0) * nrhs;
+  const int c0 = blockIdx.x * GN, m0 = blockIdx.y * GM;
   if (c0 >= ncol) return;
-  int mat = mat_base + (mat_mod > 0 ? (grp % mat_mod) : grp), sym = 0;
+  int mat = mat_mod > 0 ? grp % mat_mod : grp, sym = 0;
   if (cls_code) {
     const int code = cls_code[grp];
-    mat = mat_base + (code >> 4);
+    mat = code >> 4;
     sym = code & 15;
   }
-  const double* Tg = T + (size_t)mat * rp * kp;
-  const int R = 2 * ncf;
-  __shared__ uint8_t s_opi[M2L_SYM_MAXR], s_opo[M2L_SYM_MAXR];
-  if (sym) m2l_sym_tables(sym, R, s_opi, s_opo, threadIdx.x, NT);
-  for (int j = threadIdx.x; j < ntile; j += NT) {
-    int c = c0 + j;
+  const int R = 2 * ncf, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (sym) m2l_sym_tables(sym, R, s_opi, s_opo, tid, NT);
+  for (int j = tid; j < GN; j += NT) {
+    const int c = c0 + j;
     int src = -1;
     if (c < ncol) {
       src = pair_src[p0 + c / nrhs];
@@ -162,105 +170,119 @@ k_trans_gemm(int ncf, int rp, int kp, int nrhs, int nwm, const double* __restric
     }
     s_src[j] = src;
   }
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int g = lane >> 2, tq = lane & 3;
-  int wn = warp % nwn, wm = warp / nwn;
-  int mt = rp / 8;
-  int mtw = (mt + nwm - 1) / nwm;
-  int mbeg = wm * mtw;
-  mt = min(mt, mbeg + mtw);                 // the rows from there on are the next group's
-  double acc[MTW][2];
+  __syncthreads();
+  // this thread's 16-byte pieces of a chunk: rows / columns tid / 8 + 16 i, k = 2 (tid % 8)
+  const double* Tg = T + (size_t)mat * rp * kp;
+  const int kk = 2 * (tid & 7), rb = tid >> 3;
+  const double* bp[GN / 16];
+  bool bon[GN / 16];
 #pragma unroll
-  for (int i = 0; i < MTW; ++i) acc[i][0] = acc[i][1] = 0.0;
-  for (int kc = 0; kc < kp; kc += KC) {
-    int kw = min(KC, kp - kc);
-    __syncthreads();
-    // 16-byte loads and stores: kp, kc, kw, TSTR, R and every matrix offset are even
-    constexpr int KH = KC / 2;
-    for (int e = threadIdx.x; e < rp * KH; e += NT) {
-      const int row = e / KH, col = 2 * (e - row * KH);
-      const double2 v = col < kw
-          ? __ldg(reinterpret_cast<const double2*>(Tg + (size_t)row * kp + kc + col)) : c2(0.0);
-      *reinterpret_cast<double2*>(Ts + row * TSTR + col) = v;
-    }
-    for (int e = threadIdx.x; e < ntile * KH; e += NT) {
-      const int j = e / KH, k = 2 * (e - j * KH);
-      const int src = s_src[j];
-      double v0 = 0.0, v1 = 0.0;
-      if (src >= 0 && k < kw && kc + k < R) {
-        const int r = (c0 + j) % nrhs, kg = kc + k;
-        const double2 z = __ldg(ein + ((size_t)src * nrhs + r) * ncf + (kg >> 1));
-        if (sym) {
-          const int o0 = s_opi[kg], o1 = s_opi[kg + 1];
-          v0 = (o0 & 1) ? z.y : z.x;
-          v1 = (o1 & 1) ? z.x : z.y;
-          if (o0 & 2) v0 = -v0;
-          if (o1 & 2) v1 = -v1;
-        } else {
-          v0 = z.x;
-          v1 = z.y;
-        }
-      }
-      Xs[k * XS + j] = v0;
-      Xs[(k + 1) * XS + j] = v1;
-    }
-    __syncthreads();
-    for (int k0 = 0; k0 < kw; k0 += 4) {
-      double b = Xs[(k0 + tq) * XS + wn * 8 + g];
+  for (int i = 0; i < GN / 16; ++i) {
+    const int src = s_src[rb + 16 * i];
+    bon[i] = src >= 0;
+    bp[i] = reinterpret_cast<const double*>(
+                ein + ((size_t)(bon[i] ? src : 0) * nrhs + (c0 + rb + 16 * i) % nrhs) * ncf) + kk;
+  }
+  const double* ap = Tg + (size_t)(m0 + rb) * kp + kk;
+  const int nk = (R + GK - 1) / GK;
+  auto fetch = [&](int ck) {
+    if (ck < nk) {
+      double* A = sm + (ck % GST) * gemm_stage<MI>();
+      double* B = A + GM * GS;
+      const bool in = ck * GK + kk < R;                  // kp >= R; the rest is zero
 #pragma unroll
-      for (int i = 0; i < MTW; ++i) {
-        int mi = mbeg + i;
-        if (mi < mt) {
-          double a = Ts[(mi * 8 + g) * TSTR + k0 + tq];
-          dmma_8x8x4(acc[i][0], acc[i][1], a, b);
-        }
+      for (int i = 0; i < MI; ++i) {
+        const bool on = in && m0 + rb + 16 * i < rp;
+        cp_async16_zfill(A + (rb + 16 * i) * GS + kk, on ? ap + (size_t)16 * i * kp + ck * GK : Tg, on);
       }
+#pragma unroll
+      for (int i = 0; i < GN / 16; ++i) {
+        const bool on = in && bon[i];
+        cp_async16_zfill(B + (rb + 16 * i) * GS + kk, on ? bp[i] + ck * GK : Tg, on);
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  const int row = lane >> 2, tq = lane & 3, wm = warp & 1, wn = warp >> 1;
+  double acc[MI][4][2];
+#pragma unroll
+  for (int i = 0; i < MI; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  for (int i = 0; i < GST - 1; ++i) fetch(i);
+  for (int ck = 0; ck < nk; ++ck) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(GST - 2) : "memory");
+    __syncthreads();
+    fetch(ck + GST - 1);                                 // into the stage read last round
+    const double* A = sm + (ck % GST) * gemm_stage<MI>() + (wm * 8 * MI + row) * GS + tq;
+    const double* B = sm + (ck % GST) * gemm_stage<MI>() + (GM + wn * 32 + row) * GS;
+    const int kw = R - ck * GK;
+#pragma unroll
+    for (int k0 = 0; k0 < GK; k0 += 4) {
+      if (k0 >= kw) break;
+      double a[MI], b[4];
+#pragma unroll
+      for (int i = 0; i < MI; ++i) a[i] = A[i * 8 * GS + k0];
+      int k = k0 + tq, neg = 0;
+      if (sym && k < kw) {
+        const int o = s_opi[ck * GK + k];
+        k ^= o & 1;
+        neg = (o & 2) << 30;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const double x = B[j * 8 * GS + k];
+        b[j] = __hiloint2double(__double2hiint(x) ^ neg, __double2loint(x));
+      }
+#pragma unroll
+      for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
     }
   }
-  // epilogue: acc[i][v] = C[row = (mbeg + i) * 8 + g][col = wn * 8 + 2 tq + v]; with a
-  // class symmetry, its output map first (the other half of row's coefficient, row ^ 1,
+  // acc[i][j][v] = C[row m0 + (wm MI + i) 8 + row][column c0 + wn 32 + 8 j + 2 tq + v]; with a
+  // class symmetry, its output map first (the other part of the row's coefficient, row ^ 1,
   // is in lane ^ 4)
   if (sym) {
 #pragma unroll
-    for (int v = 0; v < 2; ++v)
+    for (int i = 0; i < MI; ++i) {
+      const int rr = m0 + (wm * MI + i) * 8 + row, op = rr < R ? s_opo[rr] : 0;
 #pragma unroll
-      for (int i = 0; i < MTW; ++i) {
-        const double other = __shfl_xor_sync(0xffffffffu, acc[i][v], 4);
-        const int row = (mbeg + i) * 8 + g;
-        if (mbeg + i < mt && row < R) {
-          const int op = s_opo[row];
-          const double w = (op & 1) ? other : acc[i][v];
-          acc[i][v] = (op & 2) ? -w : w;
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          const double other = __shfl_xor_sync(0xffffffffu, acc[i][j][v], 4);
+          const double w = (op & 1) ? other : acc[i][j][v];
+          acc[i][j][v] = (op & 2) ? -w : w;
         }
-      }
-  }
-#pragma unroll
-  for (int v = 0; v < 2; ++v) {
-    int j = wn * 8 + 2 * tq + v;
-    int c = c0 + j;
-    if (c >= ncol) continue;
-    int pr = p0 + c / nrhs, r = c % nrhs;
-    if (pair_dst) {
-      int dst = pair_dst[pr];
-      if ((unsigned)dst >= (unsigned)nboxes) {
-        report(err, QBX_DEVERR_BAD_BOX);
-        continue;
-      }
-      double* y = reinterpret_cast<double*>(eout + ((size_t)dst * nrhs + r) * ncf);
-#pragma unroll
-      for (int i = 0; i < MTW; ++i) {
-        int row = (mbeg + i) * 8 + g;
-        if (mbeg + i < mt && row < R) y[row] += scale * acc[i][v];
-      }
-    } else {
-      double* y = cpair + ((size_t)pr * nrhs + r) * rp;
-#pragma unroll
-      for (int i = 0; i < MTW; ++i) {
-        int row = (mbeg + i) * 8 + g;
-        if (mbeg + i < mt) y[row] = acc[i][v];
-      }
     }
   }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      const int c = c0 + wn * 32 + j * 8 + 2 * tq + v;
+      if (c >= ncol) continue;
+      const int pr = p0 + c / nrhs, r = c % nrhs;
+      double* y = cpair + ((size_t)pr * nrhs + r) * rp;
+      if (pair_dst) {
+        const int dst = pair_dst[pr];
+        if ((unsigned)dst >= (unsigned)nboxes) {
+          report(err, QBX_DEVERR_BAD_BOX);
+          continue;
+        }
+        y = reinterpret_cast<double*>(eout + ((size_t)dst * nrhs + r) * ncf);
+      }
+#pragma unroll
+      for (int i = 0; i < MI; ++i) {
+        const int rr = m0 + (wm * MI + i) * 8 + row;
+        if (pair_dst) {
+          if (rr < R) y[rr] += scale * acc[i][j][v];
+        } else if (rr < rp) {
+          y[rr] = acc[i][j][v];
+        }
+      }
+    }
 }
 
 // Tiled form for large matrices (3D Helmholtz M2M / L2L): CTA tile of 64 rows x 64 columns
@@ -279,14 +301,6 @@ constexpr int GT_M = 64, GT_N = 64, GT_K = 16, GT_ST = 4;
 constexpr int GT_S = GT_K + 4;               // row stride of a staged operand (doubles)
 constexpr int GT_STAGE = (GT_M + GT_N) * GT_S;
 constexpr int GT_CS = GT_N + 4;              // row stride of the result tile (doubles)
-
-QBX_D void cp_async16_zfill(void* dst, const void* src, bool on)
-{
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
-                   (unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src), "r"(on ? 16 : 0)
-               : "memory");
-}
 
 template <bool SUM>
 __global__ void __launch_bounds__(NT)
@@ -643,16 +657,7 @@ size_t trans_scratch_bytes(const TransCfg& c, int npairs, int nrhs)
   return (size_t)(npairs > 0 ? npairs : 1) * nrhs * c.rp * sizeof(double);
 }
 
-static size_t gemm_smem(int rp) { return ((size_t)rp * TSTR + (size_t)KC * XS) * sizeof(double); }
-
-// warp arrangement: nwm row groups so that each warp holds <= 24 m-tiles
-static int gemm_nwm(int rp)
-{
-  int mt = rp / 8;
-  return mt <= 24 ? 1 : (mt <= 48 ? 2 : 4);
-}
-
-bool trans_supported(const TransCfg& c) { return c.rp / 8 <= 96 && gemm_smem(c.rp) <= 200 * 1024; }
+bool trans_supported(const TransCfg& c) { return c.rp <= 672; }
 
 M2LSymClasses m2l_symmetry_classes(int nclasses, const std::vector<int32_t>& offs)
 {
@@ -721,28 +726,31 @@ static cudaError_t gemm_launch(const qbxfmm_geometry& g, const TransCfg& c, int 
                                double scale, double* cpair, int32_t* err, cudaStream_t st)
 {
   if (ngroups <= 0 || maxcols <= 0) return cudaSuccess;
-  int ncf = c.ncf, rp = c.rp, kp = c.kp;
-  size_t sh = gemm_smem(rp);
-  int nwm = gemm_nwm(rp);
-  int ntile = 8 * (4 / nwm);
-  int mtw = (rp / 8 + nwm - 1) / nwm;
-  dim3 grid((maxcols + ntile - 1) / ntile, ngroups);
-  const double* Tb = T + mat_base * (size_t)rp * kp;
-#define QBX_GEMM_CASE(W)                                                                        \
-  if (mtw <= W) {                                                                               \
-    cudaFuncSetAttribute(k_trans_gemm<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh); \
-    k_trans_gemm<W><<<grid, NT, sh, st>>>(ncf, rp, kp, nrhs, nwm, Tb, 0, mat_mod, cls_code,     \
-                                          group_starts_dev, g0, pair_src, pair_dst, ein, eout,  \
-                                          scale, cpair, err, g.nboxes);                         \
-    return cudaGetLastError();                                                                  \
+  // the tile height with the fewest rows past the end, the tallest of those
+  const int mt = (c.rp + 7) / 8;
+  int mi = 3;
+  auto rows = [&](int m) { return (mt + 2 * m - 1) / (2 * m) * 2 * m; };
+  for (int m = 4; m <= 6; ++m)
+    if (rows(m) <= rows(mi)) mi = m;
+  const double* Tb = T + mat_base * (size_t)c.rp * c.kp;
+  auto launch = [&](auto height) {
+    constexpr int MI = decltype(height)::value;
+    const size_t sh = (size_t)GST * gemm_stage<MI>() * sizeof(double);
+    cudaError_t e = cudaFuncSetAttribute(k_trans_gemm<MI>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+    if (e != cudaSuccess) return e;
+    const dim3 grid((maxcols + GN - 1) / GN, (c.rp + 16 * MI - 1) / (16 * MI), ngroups);
+    k_trans_gemm<MI><<<grid, NT, sh, st>>>(c.ncf, c.rp, c.kp, nrhs, Tb, mat_mod, cls_code,
+                                           group_starts_dev, g0, pair_src, pair_dst, ein, eout, scale,
+                                           cpair, err, g.nboxes);
+    return cudaGetLastError();
+  };
+  switch (mi) {
+    case 3: return launch(std::integral_constant<int, 3>());
+    case 4: return launch(std::integral_constant<int, 4>());
+    case 5: return launch(std::integral_constant<int, 5>());
+    default: return launch(std::integral_constant<int, 6>());
   }
-  QBX_GEMM_CASE(8)
-  QBX_GEMM_CASE(12)
-  QBX_GEMM_CASE(16)
-  QBX_GEMM_CASE(20)
-  QBX_GEMM_CASE(24)
-#undef QBX_GEMM_CASE
-  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_m2l_gemm(const qbxfmm_geometry& g, const TransHost& th, const TransCfg& c,

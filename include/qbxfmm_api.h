@@ -79,6 +79,17 @@ int qbxfmm_workspace_sizes(const qbxfmm_plan* plan, size_t* sizes8);
 int qbxfmm_precompute_translations(const qbxfmm_plan* plan, const qbxfmm_workspace* ws,
                                    void* stream);
 
+/* One GMRES iteration after w = A r (pytential/linalg/gmres.py:224-299) for `ndens` vectors of
+ * n float64 (complex128: is_complex) entries: twice, w is orthogonalized against the kept
+ * images images[0..count) in turn and v, starting from r, gets the same combination of the
+ * preimages, both divided by |w|; then d = <w, r>, r_new = r - d w (unless NULL), x += d v.
+ * w_in is not changed.  active: ndens bytes on the device; a density with 0 gets w = v = 0
+ * and d = 0.  images, preimages: host arrays of device pointers.  No two outputs, and no
+ * output and input, may overlap. */
+int qbxfmm_gmres_step(int is_complex, int ndens, long long n, int count, const void* const* images,
+                      const void* const* preimages, const void* w_in, const void* r, void* w,
+                      void* v, const unsigned char* active, void* r_new, void* x, void* stream);
+
 /* One translation stage as qbxfmm_apply runs it, on ws->mpoles and ws->locals with
  * ws->translations and ws->pair_scratch (either NULL: by pair, as the entries below):
  * stage 0 coarsen_multipoles, 1 multipole_to_local, 2 refine_locals.  A stage reads and

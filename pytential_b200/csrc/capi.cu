@@ -1291,6 +1291,21 @@ int run_l2l(const qbxfmm_plan* p, const qbxfmm_workspace* ws, const uint32_t* T3
 
 extern "C" {
 
+int qbxfmm_gmres_step(int is_complex, int ndens, long long n, int count, const void* const* images,
+                      const void* const* preimages, const void* w_in, const void* r, void* w,
+                      void* v, const unsigned char* active, void* r_new, void* x, void* stream)
+{
+  if (ndens < 0 || n < 0 || count < 0) return fail(QBXFMM_ERR_ARG, "gmres_step: negative size");
+  if (ndens == 0 || n == 0) return QBXFMM_OK;
+  if (!w_in || !r || !w || !v || !active || !x || (count > 0 && (!images || !preimages)))
+    return fail(QBXFMM_ERR_ARG, "gmres_step: null argument");
+  if (ndens > 65535) return fail(QBXFMM_ERR_UNSUPPORTED, "gmres_step: more than 65535 densities");
+  QBX_TRY(launch_gmres_step(is_complex != 0, ndens, n, count, images, preimages, w_in, r, w, v,
+                            active, r_new, x, S(stream)),
+          "gmres_step");
+  return QBXFMM_OK;
+}
+
 int qbxfmm_translate_boxes(const qbxfmm_plan* p, const qbxfmm_workspace* ws, int stage,
                            void* stream)
 {

@@ -98,6 +98,11 @@ cudaError_t launch_l2l_direct(const qbxfmm_geometry& g, const TransHost& th, con
 
 cudaError_t launch_form_strengths(const qbxfmm_geometry& g, const qbxfmm_upsample& up, int nrhs,
                                   const double* density, double* strengths, cudaStream_t st);
+// one GMRES iteration's orthogonalization against `count` images and update, for nd densities
+// of n entries (complex128 or float64)
+cudaError_t launch_gmres_step(bool cplx, int nd, long long n, int count, const void* const* a,
+                              const void* const* e, const void* win, const void* r, void* w, void* v,
+                              const uint8_t* active, void* rnew, void* x, cudaStream_t st);
 // 2D Laplace (kernels_laplace2d.cu), reached through the launch_* of the same stages
 cudaError_t l2_launch_p2m(const qbxfmm_geometry& g, SourceCoeffs sc, int p, int nrhs,
                           const double* s, double2* mp, cudaStream_t st);

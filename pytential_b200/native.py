@@ -66,6 +66,8 @@ _STAGES = {
 # every symbol include/qbxfmm_api.h declares
 # entries that take no plan
 _FREE = {
+    "qbxfmm_gmres_step": [_int, _int, ctypes.c_longlong, _int, ctypes.POINTER(_vp),
+                          ctypes.POINTER(_vp), _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "qbxfmm_laplace3d_grad_direct": [_int, _vp, _vp, _int, _vp, _vp, _vp],
     "qbxfmm_laplace3d_grad_direct_f32": [_int, _vp, _vp, _int, _vp, _vp, _vp],
     "qbxfmm_laplace3d_qbx_matrix": [_int, _vp, _vp, ctypes.c_double, ctypes.c_double, _int, _vp,

@@ -255,55 +255,6 @@ QBX_D double2 h3_e2p(const double2* E, int p, bool local, double k, double s, co
   return acc;
 }
 
-// M2P over list 3: CTA per chunk of <= 32 non-QBX targets (lane = target), the warps
-// split the list-3 boxes and stage each multipole in their own shared slice.
-__global__ void __launch_bounds__(NT)
-k_h3_eval_multipoles(qbxfmm_geometry g, HelmCoeffs hc, int p, int nrhs,
-                     const double2* __restrict__ mpoles, double2* __restrict__ pot, int32_t* err)
-{
-  extern __shared__ double2 smem2[];
-  const int ncf = (p + 1) * (p + 1);
-  double2* rec = smem2;                                  // [(p+1)(p+2)/2]
-  int nrec = (p + 1) * (p + 2) / 2;
-  __shared__ double2 s_red[NW - 1][32];
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double2* M = smem2 + nrec + (size_t)warp * ncf;
-  h3_rec_table(p, rec, threadIdx.x, NT);
-  __syncthreads();
-  int chunk = blockIdx.x;
-  int r = blockIdx.y;
-  int itb = g.nonqbx_chunk_target_box[chunk];
-  int t = g.nonqbx_chunk_start[chunk] + lane;
-  bool active = lane < g.nonqbx_chunk_count[chunk];
-  double x[3] = {0, 0, 0};
-  if (active) load_point<3>(g.nonqbx_targets, g.nfiltered_targets, t, x);
-  double2 acc = c2(0.0);
-  for (int li = g.list3_starts[itb] + warp; li < g.list3_starts[itb + 1]; li += NW) {
-    int sb = g.list3_lists[li];
-    if ((unsigned)sb >= (unsigned)g.nboxes) {
-      report(err, QBX_DEVERR_BAD_BOX);
-      continue;
-    }
-    __syncwarp();
-    const double2* src = mpoles + ((size_t)sb * nrhs + r) * ncf;
-    for (int q = lane; q < ncf; q += 32) M[q] = src[q];
-    __syncwarp();
-    if (!active) continue;
-    double cs[3];
-    load_point<3>(g.box_centers, g.nboxes, sb, cs);
-    double s = h3_scale(hc.k, level_width(g, g.box_levels[sb]));
-    acc = cadd(acc, h3_e2p(M, p, false, hc.k, s, cs, x, rec));
-  }
-  __syncthreads();
-  if (warp > 0) s_red[warp - 1][lane] = acc;
-  __syncthreads();
-  if (warp == 0 && active) {
-    for (int w = 1; w < NW; ++w) acc = cadd(acc, s_red[w - 1][lane]);
-    double2* P = pot + (size_t)r * g.nfiltered_targets + t;
-    *P = cadd(*P, acc);
-  }
-}
-
 // L2P: one thread per non-QBX target, its own box's local expansion
 __global__ void __launch_bounds__(NT)
 k_h3_eval_locals(qbxfmm_geometry g, HelmCoeffs hc, int p, int nrhs,
@@ -1680,17 +1631,6 @@ cudaError_t h3_launch_eval_direct(const qbxfmm_geometry& g, HelmCoeffs hc, int n
   if (g.nnonqbx_chunks == 0) return cudaSuccess;
   k_h3_eval_direct<<<dim3(g.nnonqbx_chunks * H3_PSPLIT, gridy(nrhs)), NT, 0, st>>>(g, hc, nrhs, s,
                                                                                   pot, err);
-  return cudaGetLastError();
-}
-
-cudaError_t h3_launch_eval_multipoles(const qbxfmm_geometry& g, HelmCoeffs hc, int p, int nrhs,
-                                      const double2* mp, double2* pot, int32_t* err, cudaStream_t st)
-{
-  if (g.nnonqbx_chunks == 0) return cudaSuccess;
-  size_t sh = ((size_t)(p + 1) * (p + 2) / 2 + (size_t)NW * (p + 1) * (p + 1)) * sizeof(double2);
-  cudaFuncSetAttribute(k_h3_eval_multipoles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-  k_h3_eval_multipoles<<<dim3(g.nnonqbx_chunks, gridy(nrhs)), NT, sh, st>>>(g, hc, p, nrhs, mp, pot,
-                                                                            err);
   return cudaGetLastError();
 }
 

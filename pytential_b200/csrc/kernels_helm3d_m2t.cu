@@ -52,11 +52,13 @@ __host__ __device__ constexpr size_t m2t_warp_smem(int pf, int q)
 // inner index = column), whose B fragment is the box's M_{n,+-m} of 8 densities: DG
 // groups of 8 densities (MMA), or DG densities by plain multiply-adds and a sum over
 // the four lanes at the end.
-template <int Q, int DG, bool MMA>
+// OFF: M2P at the non-QBX targets (eval_multipoles), each its own center, Q = 0.
+template <int Q, int DG, bool MMA, bool OFF>
 __global__ void __launch_bounds__(M2T_NT, 3)
 k_h3_m2t(qbxfmm_geometry g, HelmCoeffs hc, int pf, int nrhs, const double2* __restrict__ mpoles,
-         double2* __restrict__ pot_tree, int32_t* err)
+         double2* __restrict__ pot, int32_t* err)
 {
+  static_assert(!OFF || Q == 0);
   extern __shared__ double2 smem2[];
   const int ncf = (pf + 1) * (pf + 1);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -69,27 +71,33 @@ k_h3_m2t(qbxfmm_geometry g, HelmCoeffs hc, int pf, int nrhs, const double2* __re
   double2* E = H + lane;                                         // [i][lane]
   constexpr int NWARP = M2T_NT / 32, OCT = QBXFMM_CENTER_CHUNK / M2T_TG;
   const int chunk = blockIdx.x / OCT, oct = blockIdx.x - chunk * OCT;
-  const int itb = g.tsqbx_chunk_target_box[chunk];
-  const int cnt = g.tsqbx_chunk_count[chunk];
+  const int itb = (OFF ? g.nonqbx_chunk_target_box : g.tsqbx_chunk_target_box)[chunk];
+  const int cnt = (OFF ? g.nonqbx_chunk_count : g.tsqbx_chunk_count)[chunk];
   if (oct * M2T_TG >= cnt) return;
   const int l0 = g.list3_starts[itb], l1 = g.list3_starts[itb + 1];
   if (l1 <= l0) return;
   h3_rec_table(pf, rec, threadIdx.x, M2T_NT);
   __syncthreads();
   const int ti = oct * M2T_TG + tg;
-  const int pi = g.tsqbx_chunk_start[chunk] + min(ti, cnt - 1);
+  const int pi = (OFF ? g.nonqbx_chunk_start : g.tsqbx_chunk_start)[chunk] + min(ti, cnt - 1);
   bool active = ti < cnt;
-  int t = g.tsqbx_targets[pi], ctr = g.tsqbx_centers[pi];
-  if ((unsigned)ctr >= (unsigned)g.ncenters || (unsigned)t >= (unsigned)g.ntargets) {
-    report(err, QBX_DEVERR_BAD_CENTER);
-    active = false;
-    t = ctr = 0;
-  }
-  double cc[3], a[3];
-  load_point<3>(g.centers, g.ncenters, ctr, cc);
-  load_point<3>(g.targets, g.ntargets, t, a);
+  int t = pi;
+  double cc[3], a[3] = {0.0, 0.0, 0.0};
+  if (OFF) {
+    load_point<3>(g.nonqbx_targets, g.nfiltered_targets, t, cc);
+  } else {
+    t = g.tsqbx_targets[pi];
+    int ctr = g.tsqbx_centers[pi];
+    if ((unsigned)ctr >= (unsigned)g.ncenters || (unsigned)t >= (unsigned)g.ntargets) {
+      report(err, QBX_DEVERR_BAD_CENTER);
+      active = false;
+      t = ctr = 0;
+    }
+    load_point<3>(g.centers, g.ncenters, ctr, cc);
+    load_point<3>(g.targets, g.ntargets, t, a);
 #pragma unroll
-  for (int d = 0; d < 3; ++d) a[d] -= cc[d];
+    for (int d = 0; d < 3; ++d) a[d] -= cc[d];
+  }
   const int r0 = blockIdx.y * (MMA ? 8 * DG : DG);
   double gw[Q + 1];
   m2t_taylor_weights<Q>(hc.taylor != 0, hc.k * sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]), gw);
@@ -313,39 +321,51 @@ k_h3_m2t(qbxfmm_geometry g, HelmCoeffs hc, int pf, int nrhs, const double2* __re
     if (!active || r >= nrhs || (!MMA && kq != 0)) continue;
     double2 v = red[d * 32 + lane];
     for (int w = 1; w < NWARP; ++w) v = cadd(v, red[(w * NV + d) * 32 + lane]);
-    double2* P = pot_tree + (size_t)r * g.ntargets + t;
+    double2* P = pot + (size_t)r * (OFF ? g.nfiltered_targets : g.ntargets) + t;
     *P = cadd(*P, v);
   }
 }
 
-template <int Q, int DG, bool MMA>
+template <int Q, int DG, bool MMA, bool OFF>
 cudaError_t m2t_launch(const qbxfmm_geometry& g, HelmCoeffs hc, int pf, int nrhs,
                        const double2* mp, double2* pot, int32_t* err, cudaStream_t st)
 {
   constexpr int ND = MMA ? 8 * DG : DG;
   const size_t scratch = std::max(m2t_warp_smem(pf, Q), (size_t)(MMA ? 2 * DG : DG) * 32);
   const size_t sh = ((size_t)(pf + 1) * (pf + 2) / 2 + (M2T_NT / 32) * scratch) * sizeof(double2);
-  cudaError_t e = cudaFuncSetAttribute(k_h3_m2t<Q, DG, MMA>,
+  cudaError_t e = cudaFuncSetAttribute(k_h3_m2t<Q, DG, MMA, OFF>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
   if (e != cudaSuccess) return e;
-  dim3 grid(g.ntsqbx_chunks * (QBXFMM_CENTER_CHUNK / M2T_TG), (nrhs + ND - 1) / ND);
-  k_h3_m2t<Q, DG, MMA><<<grid, M2T_NT, sh, st>>>(g, hc, pf, nrhs, mp, pot, err);
+  const int chunks = OFF ? g.nnonqbx_chunks : g.ntsqbx_chunks;
+  dim3 grid(chunks * (QBXFMM_CENTER_CHUNK / M2T_TG), (nrhs + ND - 1) / ND);
+  k_h3_m2t<Q, DG, MMA, OFF><<<grid, M2T_NT, sh, st>>>(g, hc, pf, nrhs, mp, pot, err);
   return cudaGetLastError();
 }
 
-template <int Q>
+template <int Q, bool OFF = false>
 cudaError_t m2t_q(const qbxfmm_geometry& g, HelmCoeffs hc, int pf, int nrhs, const double2* mp,
                   double2* pot, int32_t* err, cudaStream_t st)
 {
   // a tensor-core group of 8 densities costs as much as 8 plain ones: plain for the few
-  if (nrhs > 8) return m2t_launch<Q, 2, true>(g, hc, pf, nrhs, mp, pot, err, st);
-  if (nrhs > 4) return m2t_launch<Q, 1, true>(g, hc, pf, nrhs, mp, pot, err, st);
-  if (nrhs > 2) return m2t_launch<Q, 4, false>(g, hc, pf, nrhs, mp, pot, err, st);
-  if (nrhs > 1) return m2t_launch<Q, 2, false>(g, hc, pf, nrhs, mp, pot, err, st);
-  return m2t_launch<Q, 1, false>(g, hc, pf, nrhs, mp, pot, err, st);
+  if (nrhs > 8) return m2t_launch<Q, 2, true, OFF>(g, hc, pf, nrhs, mp, pot, err, st);
+  if (nrhs > 4) return m2t_launch<Q, 1, true, OFF>(g, hc, pf, nrhs, mp, pot, err, st);
+  if (nrhs > 2) return m2t_launch<Q, 4, false, OFF>(g, hc, pf, nrhs, mp, pot, err, st);
+  if (nrhs > 1) return m2t_launch<Q, 2, false, OFF>(g, hc, pf, nrhs, mp, pot, err, st);
+  return m2t_launch<Q, 1, false, OFF>(g, hc, pf, nrhs, mp, pot, err, st);
 }
 
 }  // namespace
+
+// Bound by the FP64 pipe at the ladder's recurrences.  One warp per chunk and list-3 quarter
+// with the whole ladder in one lane per target took 825 us for 1500 points beside 24 300
+// nodes at order 15 (too few warps); 555 us here.
+cudaError_t h3_launch_eval_multipoles(const qbxfmm_geometry& g, HelmCoeffs hc, int p, int nrhs,
+                                      const double2* mp, double2* pot, int32_t* err, cudaStream_t st)
+{
+  if (g.nnonqbx_chunks == 0) return cudaSuccess;
+  if (p > H3_MAXP) return cudaErrorInvalidValue;
+  return m2t_q<0, true>(g, hc, p, nrhs, mp, pot, err, st);
+}
 
 bool h3_m2t_wins(const qbxfmm_geometry& g)
 {

@@ -1229,17 +1229,14 @@ int run_m2m(const qbxfmm_plan* p, const qbxfmm_workspace* ws, const uint32_t* T3
             void* stream)
 {
   cudaStream_t st = S(stream);
-  if (gemm && trans_mv_supported(p->tc))
-    QBX_TRY(launch_m2m_mv(p->geo, p->th, p->tc, p->kern.nrhs, (const double*)ws->translations,
-                          (double2*)ws->mpoles, ws->error_word, st),
-            "coarsen_multipoles (matrix form)");
-  else if (T32)
+  // the mixed form's matrices up to order 14 are no larger than its FP32 tiles: FP64 there too
+  if (T32 && !trans_small(p->tc))
     QBX_TRY(launch_m2m_gemm_mixed(p->geo, p->th, p->tc, p->kern.nrhs, T32, (double2*)ws->mpoles,
                                   (double*)ws->pair_scratch, ws->error_word, st),
             "coarsen_multipoles (split TF32)");
   else if (gemm)
-    QBX_TRY(launch_m2m_gemm(p->geo, p->th, p->tc, p->kern.nrhs, (const double*)ws->translations,
-                            (double2*)ws->mpoles, (double*)ws->pair_scratch, ws->error_word, st),
+    QBX_TRY(launch_m2m_direct(p->geo, p->th, p->tc, p->kern.nrhs, (const double*)ws->translations,
+                              (double2*)ws->mpoles, ws->error_word, st),
             "coarsen_multipoles (matrix form)");
   else
     return coarsen(p, p->h2_npairs > 0 ? ws->translations : nullptr, ws->mpoles, stream);
@@ -1270,17 +1267,14 @@ int run_l2l(const qbxfmm_plan* p, const qbxfmm_workspace* ws, const uint32_t* T3
             void* stream)
 {
   cudaStream_t st = S(stream);
-  if (gemm && trans_mv_supported(p->tc))
-    QBX_TRY(launch_l2l_mv(p->geo, p->th, p->tc, p->kern.nrhs, (const double*)ws->translations,
-                          (double2*)ws->locals, ws->error_word, st),
-            "refine_locals (matrix form)");
-  else if (T32)
+  // the mixed form's matrices up to order 14 are no larger than its FP32 tiles: FP64 there too
+  if (T32 && !trans_small(p->tc))
     QBX_TRY(launch_l2l_gemm_mixed(p->geo, p->th, p->tc, p->kern.nrhs, T32, (double2*)ws->locals,
                                   ws->error_word, st),
             "refine_locals (split TF32)");
   else if (gemm)
-    QBX_TRY(launch_l2l_gemm(p->geo, p->th, p->tc, p->kern.nrhs, (const double*)ws->translations,
-                            (double2*)ws->locals, ws->error_word, st),
+    QBX_TRY(launch_l2l_direct(p->geo, p->th, p->tc, p->kern.nrhs, (const double*)ws->translations,
+                              (double2*)ws->locals, ws->error_word, st),
             "refine_locals (matrix form)");
   else
     return refine(p, p->h2_npairs > 0 ? ws->translations : nullptr, ws->locals, stream);

@@ -53,16 +53,7 @@ cudaError_t launch_trans_build(const TransCfg& c, int nm2l, const int32_t* offs,
 cudaError_t launch_m2l_gemm(const qbxfmm_geometry& g, const TransHost& th, const TransCfg& c,
                             int nrhs, const double* T, const TransAux& aux, const double2* mp,
                             double2* lo, double* cpair, int32_t* err, cudaStream_t st);
-cudaError_t launch_m2m_gemm(const qbxfmm_geometry& g, const TransHost& th, const TransCfg& c,
-                            int nrhs, const double* T, double2* mp, double* cpair, int32_t* err,
-                            cudaStream_t st);
-bool trans_mv_supported(const TransCfg& c);
-cudaError_t launch_m2m_mv(const qbxfmm_geometry& g, const TransHost& th, const TransCfg& c,
-                          int nrhs, const double* T, double2* mp, int32_t* err, cudaStream_t st);
-cudaError_t launch_l2l_mv(const qbxfmm_geometry& g, const TransHost& th, const TransCfg& c,
-                          int nrhs, const double* T, double2* lo, int32_t* err, cudaStream_t st);
-cudaError_t launch_l2l_gemm(const qbxfmm_geometry& g, const TransHost& th, const TransCfg& c,
-                            int nrhs, const double* T, double2* lo, int32_t* err, cudaStream_t st);
+bool trans_small(const TransCfg& c);   // up to order 14
 cudaError_t launch_trans_reduce_m2l(const qbxfmm_geometry& g, const TransCfg& c, int nrhs,
                                     const double* cpair, double2* lo, cudaStream_t st);
 cudaError_t launch_trans_reduce_m2m(const qbxfmm_geometry& g, const TransHost& th, const TransCfg& c,

@@ -10,9 +10,10 @@
 // real (2 ncoeff) x (2 ncoeff) matrix T acting on interleaved (re, im) vectors.
 //
 //   k_trans_build  : one CTA per class, T from the harmonic table of the class vector
-//   k_trans_gemm   : one CTA per (class, 32 pairs x rhs): C = T X with X the gathered
-//                    source expansions; T and X staged in shared memory
+//   k_trans_gemm   : M2L, a CTA per (class, rows, 64 pairs x rhs): C = T X with X the
+//                    gathered source expansions
 //   k_trans_reduce : deterministic sum of each output box's pair results (list order)
+//   k_trans_gemm_pipe : M2M and L2L, a launch per level
 //
 // M2L classes related by a lattice symmetry (quarter turns about z, y and z
 // reflections) share the matrix of their canonical offset: the GEMM applies the
@@ -114,9 +115,7 @@ k_trans_build(int kind, int p, int ncf, int rp, int kp, int nclasses, const int3
 // four warps of 8 MI x 32, operands in four cp.async stages of 16 k, k-contiguous with a row
 // stride of 20 doubles (4 mod 16), free of bank conflicts as fragments.  A class symmetry
 // permutes and negates parts of coefficients: of X when a fragment is read, of C in the
-// epilogue.  If pair_dst is given the result is added (x scale) into the destination box's
-// expansion (each destination occurs once per launch), else stored into
-// cpair[pair * nrhs + r][0..rp).
+// epilogue.  The result is stored into cpair[pair * nrhs + r][0..rp).
 // The form before (32 columns, operands staged between two barriers per 32 k, one row
 // fragment loaded per product) took 4.53 ms for the M2L of 307 200 nodes at order 12 and
 // 0.222 ms of 19 200 at order 10; this 3.35 and 0.191.
@@ -135,10 +134,9 @@ QBX_D void cp_async16_zfill(void* dst, const void* src, bool on)
 
 template <int MI>
 __global__ void __launch_bounds__(NT)
-k_trans_gemm(int ncf, int rp, int kp, int nrhs, const double* __restrict__ T, int mat_mod,
-             const int32_t* __restrict__ cls_code, const int32_t* __restrict__ group_starts, int g0,
-             const int32_t* __restrict__ pair_src, const int32_t* __restrict__ pair_dst,
-             const double2* __restrict__ ein, double2* __restrict__ eout, double scale,
+k_trans_gemm(int ncf, int rp, int kp, int nrhs, const double* __restrict__ T,
+             const int32_t* __restrict__ cls_code, const int32_t* __restrict__ group_starts,
+             const int32_t* __restrict__ pair_src, const double2* __restrict__ ein,
              double* __restrict__ cpair, int32_t* err, int nboxes)
 {
   constexpr int GM = 16 * MI;
@@ -146,11 +144,11 @@ k_trans_gemm(int ncf, int rp, int kp, int nrhs, const double* __restrict__ T, in
   double* sm = reinterpret_cast<double*>(smem2);       // [GST]{A [GM][GS], B [GN][GS]}
   __shared__ int s_src[GN];
   __shared__ uint8_t s_opi[M2L_SYM_MAXR], s_opo[M2L_SYM_MAXR];
-  const int grp = g0 + blockIdx.z;
+  const int grp = blockIdx.z;
   const int p0 = group_starts[grp], ncol = (group_starts[grp + 1] - p0) * nrhs;
   const int c0 = blockIdx.x * GN, m0 = blockIdx.y * GM;
   if (c0 >= ncol) return;
-  int mat = mat_mod > 0 ? grp % mat_mod : grp, sym = 0;
+  int mat = grp, sym = 0;
   if (cls_code) {
     const int code = cls_code[grp];
     mat = code >> 4;
@@ -265,27 +263,15 @@ k_trans_gemm(int ncf, int rp, int kp, int nrhs, const double* __restrict__ T, in
       if (c >= ncol) continue;
       const int pr = p0 + c / nrhs, r = c % nrhs;
       double* y = cpair + ((size_t)pr * nrhs + r) * rp;
-      if (pair_dst) {
-        const int dst = pair_dst[pr];
-        if ((unsigned)dst >= (unsigned)nboxes) {
-          report(err, QBX_DEVERR_BAD_BOX);
-          continue;
-        }
-        y = reinterpret_cast<double*>(eout + ((size_t)dst * nrhs + r) * ncf);
-      }
 #pragma unroll
       for (int i = 0; i < MI; ++i) {
         const int rr = m0 + (wm * MI + i) * 8 + row;
-        if (pair_dst) {
-          if (rr < R) y[rr] += scale * acc[i][j][v];
-        } else if (rr < rp) {
-          y[rr] = acc[i][j][v];
-        }
+        if (rr < rp) y[rr] = acc[i][j][v];
       }
     }
 }
 
-// Tiled form for large matrices (3D Helmholtz M2M / L2L): CTA tile of 64 rows x 64 columns
+// Tiled form of M2M / L2L: CTA tile of 64 rows x 64 columns
 // (box x rhs), K streamed in chunks of 16 through a cp.async pipeline of GT_ST stages (the
 // synchronous form waited for two rounds of global loads per chunk: 8.8 us of 140 us a
 // launch); warp (wm, wn) owns 32 x 32 of the tile as 4 x 4 m8n8 accumulators.  Both
@@ -482,136 +468,6 @@ k_trans_reduce(int ncf, int rp, int nrhs, const int32_t* __restrict__ boxes, int
 
 // {{{ M2M / L2L as matrix-vector products (small matrices)
 
-// group g of a pair: group_starts[g] <= pr < group_starts[g + 1], g in [g0, g0 + 8)
-QBX_D int pair_group(const int32_t* __restrict__ group_starts, int g0, int pr)
-{
-  int grp = g0;
-  while (grp + 1 < g0 + 8 && group_starts[grp + 1] <= pr) ++grp;
-  return grp;
-}
-
-// y[row] += sum_k T[row][k] x[k] over one matrix, rows row0 and row0 + NT; x in
-// shared memory (kp doubles, zero-padded).  Eight row loads are issued before their
-// products, so that a thread keeps 128 bytes of the (L2-resident) matrix in flight.
-QBX_D void mv_rows(const double* __restrict__ Tm, int kp, int R, const double* x, double* acc2,
-                   int row0)
-{
-  const int n2 = kp / 2;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    int row = row0 + h * NT;
-    if (row >= R) break;
-    const double2* tr = reinterpret_cast<const double2*>(Tm + (size_t)row * kp);
-    const double2* xv = reinterpret_cast<const double2*>(x);
-    double a[4] = {0.0, 0.0, 0.0, 0.0};
-    int k2 = 0;
-    for (; k2 + 8 <= n2; k2 += 8) {
-      double2 t[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) t[u] = __ldg(tr + k2 + u);
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        double2 xx = xv[k2 + u];
-        a[u & 3] = fma(t[u].x, xx.x, a[u & 3]);
-        a[u & 3] = fma(t[u].y, xx.y, a[u & 3]);
-      }
-    }
-    for (; k2 < n2; ++k2) {
-      double2 t0 = __ldg(tr + k2), x0 = xv[k2];
-      a[0] = fma(t0.x, x0.x, a[0]);
-      a[1] = fma(t0.y, x0.y, a[1]);
-    }
-    acc2[h] += (a[0] + a[1]) + (a[2] + a[3]);
-  }
-}
-
-// M2M of one level: a cluster of eight CTAs per source parent box (i = i0 +
-// blockIdx.x / 8, density blockIdx.y); CTA c multiplies child slot c's multipole by
-// its (child position) matrix, and CTA 0 adds the eight products into the parent in
-// a fixed order through distributed shared memory.
-__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(NT)
-k_trans_m2m_mv(int ncf, int rp, int kp, int nrhs, const double* __restrict__ T, size_t mat_base,
-               int mat_mod, const int32_t* __restrict__ group_starts, int g0,
-               const int32_t* __restrict__ parents, int i0, const int32_t* __restrict__ par_starts,
-               const int32_t* __restrict__ par_pairs, const int32_t* __restrict__ pair_src,
-               double2* __restrict__ mp, int32_t* err, int nboxes)
-{
-  extern __shared__ double xs[];   // [kp] child multipole, then [2 NT] product rows
-  double* res = xs + kp;
-  cg::cluster_group cl = cg::this_cluster();
-  int i = i0 + blockIdx.x / 8;
-  int slot = blockIdx.x & 7;
-  int r = blockIdx.y;
-  int q0 = par_starts[i];
-  int nch = min(par_starts[i + 1] - q0, 8);
-  const int R = 2 * ncf;
-  double acc[2] = {0.0, 0.0};
-  if (slot < nch) {
-    int pr = par_pairs[q0 + slot];
-    int src = pair_src[pr];
-    int grp = pair_group(group_starts, g0, pr);
-    bool ok = (unsigned)src < (unsigned)nboxes;
-    if (!ok && threadIdx.x == 0) report(err, QBX_DEVERR_BAD_BOX);
-    const double* x = reinterpret_cast<const double*>(mp + ((size_t)(ok ? src : 0) * nrhs + r) * ncf);
-    for (int k = threadIdx.x; k < kp; k += NT) xs[k] = (ok && k < R) ? x[k] : 0.0;
-    __syncthreads();
-    int mat = (int)mat_base + (mat_mod > 0 ? grp % mat_mod : grp);
-    mv_rows(T + (size_t)mat * rp * kp, kp, R, xs, acc, threadIdx.x);
-  }
-  res[threadIdx.x] = acc[0];
-  res[threadIdx.x + NT] = acc[1];
-  cl.sync();
-  if (slot == 0) {
-    int parent = parents[i];
-    if ((unsigned)parent >= (unsigned)nboxes) {
-      if (threadIdx.x == 0) report(err, QBX_DEVERR_BAD_BOX);
-    } else {
-      double s0 = 0.0, s1 = 0.0;
-      for (int q = 0; q < nch; ++q) {
-        const double* rq = cl.map_shared_rank(res, q);
-        s0 += rq[threadIdx.x];
-        s1 += rq[threadIdx.x + NT];
-      }
-      double* y = reinterpret_cast<double*>(mp + ((size_t)parent * nrhs + r) * ncf);
-      if (threadIdx.x < R) y[threadIdx.x] += s0;
-      if (threadIdx.x + NT < R) y[threadIdx.x + NT] += s1;
-    }
-  }
-  cl.sync();
-}
-
-// L2L of one level: CTA per (parent, child) pair p0 + blockIdx.x of the level's
-// eight groups; child local += T_{child position} parent local.
-__global__ void __launch_bounds__(NT)
-k_trans_l2l_mv(int ncf, int rp, int kp, int nrhs, const double* __restrict__ T, size_t mat_base,
-               int mat_mod, const int32_t* __restrict__ group_starts, int g0,
-               const int32_t* __restrict__ pair_src, const int32_t* __restrict__ pair_dst,
-               double2* __restrict__ lo, int32_t* err, int nboxes)
-{
-  extern __shared__ double xs[];   // [kp]
-  int pr = group_starts[g0] + blockIdx.x;
-  int r = blockIdx.y;
-  int grp = pair_group(group_starts, g0, pr);
-  int src = pair_src[pr], dst = pair_dst[pr];
-  if ((unsigned)src >= (unsigned)nboxes || (unsigned)dst >= (unsigned)nboxes) {
-    if (threadIdx.x == 0) report(err, QBX_DEVERR_BAD_BOX);
-    return;
-  }
-  const int R = 2 * ncf;
-  const double* x = reinterpret_cast<const double*>(lo + ((size_t)src * nrhs + r) * ncf);
-  for (int k = threadIdx.x; k < kp; k += NT) xs[k] = k < R ? x[k] : 0.0;
-  __syncthreads();
-  double acc[2] = {0.0, 0.0};
-  int mat = (int)mat_base + (mat_mod > 0 ? grp % mat_mod : grp);
-  mv_rows(T + (size_t)mat * rp * kp, kp, R, xs, acc, threadIdx.x);
-  double* y = reinterpret_cast<double*>(lo + ((size_t)dst * nrhs + r) * ncf);
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    int row = threadIdx.x + h * NT;
-    if (row < R) y[row] += acc[h];
-  }
-}
-
 // }}}
 
 // {{{ launchers
@@ -718,31 +574,26 @@ cudaError_t launch_trans_build(const TransCfg& c, int nm2l, const int32_t* offs,
   return cudaGetLastError();
 }
 
-static cudaError_t gemm_launch(const qbxfmm_geometry& g, const TransCfg& c, int nrhs, const double* T,
-                               size_t mat_base, int mat_mod, const int32_t* cls_code,
-                               const int32_t* group_starts_dev,
-                               int g0, int ngroups, int maxcols, const int32_t* pair_src,
-                               const int32_t* pair_dst, const double2* ein, double2* eout,
-                               double scale, double* cpair, int32_t* err, cudaStream_t st)
+static cudaError_t m2l_products(const qbxfmm_geometry& g, const TransCfg& c, int nrhs,
+                                const double* T, const int32_t* cls_code, int maxcols,
+                                const double2* mp, double* cpair, int32_t* err, cudaStream_t st)
 {
-  if (ngroups <= 0 || maxcols <= 0) return cudaSuccess;
+  if (maxcols <= 0) return cudaSuccess;
   // the tile height with the fewest rows past the end, the tallest of those
   const int mt = (c.rp + 7) / 8;
   int mi = 3;
   auto rows = [&](int m) { return (mt + 2 * m - 1) / (2 * m) * 2 * m; };
   for (int m = 4; m <= 6; ++m)
     if (rows(m) <= rows(mi)) mi = m;
-  const double* Tb = T + mat_base * (size_t)c.rp * c.kp;
   auto launch = [&](auto height) {
     constexpr int MI = decltype(height)::value;
     const size_t sh = (size_t)GST * gemm_stage<MI>() * sizeof(double);
     cudaError_t e = cudaFuncSetAttribute(k_trans_gemm<MI>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
     if (e != cudaSuccess) return e;
-    const dim3 grid((maxcols + GN - 1) / GN, (c.rp + 16 * MI - 1) / (16 * MI), ngroups);
-    k_trans_gemm<MI><<<grid, NT, sh, st>>>(c.ncf, c.rp, c.kp, nrhs, Tb, mat_mod, cls_code,
-                                           group_starts_dev, g0, pair_src, pair_dst, ein, eout, scale,
-                                           cpair, err, g.nboxes);
+    const dim3 grid((maxcols + GN - 1) / GN, (c.rp + 16 * MI - 1) / (16 * MI), g.m2l_nclasses);
+    k_trans_gemm<MI><<<grid, NT, sh, st>>>(c.ncf, c.rp, c.kp, nrhs, T, cls_code, g.m2l_class_starts,
+                                           g.m2l_pair_src, mp, cpair, err, g.nboxes);
     return cudaGetLastError();
   };
   switch (mi) {
@@ -758,51 +609,10 @@ cudaError_t launch_m2l_gemm(const qbxfmm_geometry& g, const TransHost& th, const
                             double2* lo, double* cpair, int32_t* err, cudaStream_t st)
 {
   if (g.m2l_nclasses == 0) return cudaSuccess;
-  cudaError_t e = gemm_launch(g, c, nrhs, T, 0, 0, aux.cls_code, g.m2l_class_starts, 0,
-                              g.m2l_nclasses, th.m2l_max_pairs * nrhs, g.m2l_pair_src, nullptr, mp,
-                              nullptr, 1.0, cpair, err, st);
+  cudaError_t e = m2l_products(g, c, nrhs, T, aux.cls_code, th.m2l_max_pairs * nrhs, mp, cpair, err,
+                               st);
   if (e != cudaSuccess) return e;
   return launch_trans_reduce_m2l(g, c, nrhs, cpair, lo, st);
-}
-
-cudaError_t launch_m2m_gemm(const qbxfmm_geometry& g, const TransHost& th, const TransCfg& c,
-                            int nrhs, const double* T, double2* mp, double* cpair, int32_t* err,
-                            cudaStream_t st)
-{
-  const int nch = 8;
-  for (int lev = g.nlevels - 2; lev >= 0; --lev) {
-    int g0 = lev * nch;
-    int maxp = th.m2m_level_max_group[lev];
-    if (maxp == 0) continue;
-    cudaError_t e = gemm_launch(g, c, nrhs, T, c.m2m_base, c.m2m_mat_mod, nullptr, g.m2m_group_starts, g0,
-                                nch, maxp * nrhs, g.m2m_pair_src, nullptr, mp, nullptr, 1.0, cpair,
-                                err, st);
-    if (e != cudaSuccess) return e;
-    int i0 = th.lvl_source_parent[lev], i1 = th.lvl_source_parent[lev + 1];
-    if (i1 > i0)
-      k_trans_reduce<<<dim3(i1 - i0, nrhs), NT, 0, st>>>(c.ncf, c.rp, nrhs, g.source_parent_boxes,
-                                                         i0, g.m2m_par_pair_starts, g.m2m_par_pairs,
-                                                         cpair, mp, 0, g.box_levels, g.root_extent);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
-}
-
-cudaError_t launch_l2l_gemm(const qbxfmm_geometry& g, const TransHost& th, const TransCfg& c,
-                            int nrhs, const double* T, double2* lo, int32_t* err, cudaStream_t st)
-{
-  const int nch = 8;
-  for (int lev = 1; lev < g.nlevels; ++lev) {
-    int g0 = lev * nch;
-    int maxp = th.l2l_level_max_group[lev];
-    if (maxp == 0) continue;
-    cudaError_t e = gemm_launch(g, c, nrhs, T, c.l2l_base, c.m2m_mat_mod, nullptr, g.l2l_group_starts, g0,
-                                nch, maxp * nrhs, g.l2l_pair_src, g.l2l_pair_dst, lo, lo, 1.0,
-                                nullptr, err, st);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
 }
 
 cudaError_t launch_trans_reduce_m2l(const qbxfmm_geometry& g, const TransCfg& c, int nrhs,
@@ -881,42 +691,7 @@ cudaError_t launch_l2l_direct(const qbxfmm_geometry& g, const TransHost& th, con
 }
 
 
-bool trans_mv_supported(const TransCfg& c) { return 2 * c.ncf <= 2 * NT && c.kp % 2 == 0; }
-
-// M2M level by level as matrix-vector products, eight CTAs per parent (small matrices)
-cudaError_t launch_m2m_mv(const qbxfmm_geometry& g, const TransHost& th, const TransCfg& c,
-                          int nrhs, const double* T, double2* mp, int32_t* err, cudaStream_t st)
-{
-  size_t sh = ((size_t)c.kp + 2 * NT) * sizeof(double);
-  for (int lev = g.nlevels - 2; lev >= 0; --lev) {
-    int i0 = th.lvl_source_parent[lev], i1 = th.lvl_source_parent[lev + 1];
-    if (i1 <= i0) continue;
-    k_trans_m2m_mv<<<dim3(8 * (i1 - i0), nrhs), NT, sh, st>>>(
-        c.ncf, c.rp, c.kp, nrhs, T, c.m2m_base, c.m2m_mat_mod, g.m2m_group_starts, lev * 8,
-        g.source_parent_boxes, i0, g.m2m_par_pair_starts, g.m2m_par_pairs, g.m2m_pair_src, mp, err,
-        g.nboxes);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
-}
-
-// L2L level by level, CTA per (parent, child) pair
-cudaError_t launch_l2l_mv(const qbxfmm_geometry& g, const TransHost& th, const TransCfg& c,
-                          int nrhs, const double* T, double2* lo, int32_t* err, cudaStream_t st)
-{
-  size_t sh = (size_t)c.kp * sizeof(double);
-  for (int lev = 1; lev < g.nlevels; ++lev) {
-    int n = th.l2l_level_pairs[lev];
-    if (n == 0) continue;
-    k_trans_l2l_mv<<<dim3(n, nrhs), NT, sh, st>>>(c.ncf, c.rp, c.kp, nrhs, T, c.l2l_base,
-                                                  c.m2m_mat_mod, g.l2l_group_starts, lev * 8,
-                                                  g.l2l_pair_src, g.l2l_pair_dst, lo, err, g.nboxes);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
-}
+bool trans_small(const TransCfg& c) { return c.ncf <= NT; }
 
 // }}}
 

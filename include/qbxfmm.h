@@ -200,13 +200,14 @@ typedef struct qbxfmm_workspace {
   void* strengths;    /* [nrhs][nsources] tree order */
   void* mpoles;       /* [nboxes][nrhs][ncoeff(fmm_order)] complex128 */
   void* locals;       /* [nboxes][nrhs][ncoeff(fmm_order)] complex128 */
-  void* qbx_exps;     /* [ncenters][nrhs][ncoeff(qbx_order)] complex128 */
+  void* qbx_exps;     /* [ncenters][nrhs][ncoeff(qbx_order)] complex128; not formed by a
+                         Helmholtz apply that takes the far field straight to the targets */
   void* pot_nonqbx;   /* [nrhs][nfiltered_targets] */
   void* pot_tree;     /* [nrhs][ntargets] */
   int32_t* error_word;/* one int32, set by kernels that meet an out-of-range index */
-  void* translations; /* translation-class matrices (filled by
-                         qbxfmm_precompute_translations); NULL selects the
-                         per-pair translation kernels */
+  void* translations; /* translation-class matrices, or the translation tables of a
+                         Helmholtz plan (filled by qbxfmm_precompute_translations);
+                         NULL selects the per-pair translation kernels */
   void* pair_scratch; /* per-pair translation results, reduced per output box */
 } qbxfmm_workspace;
 

@@ -228,6 +228,15 @@ def algorithmic_flops(arrays: dict, scalars: dict, dim: int, complex_: bool, pf:
 # }}}
 
 
+def helmholtz3d_m2l_rotation_flops(scalars: dict, arrays: dict, p: int, nrhs: int) -> int:
+    """Real multiply-adds (x 2) of the 3D Helmholtz M2L as rotation, coaxial translation and
+    rotation back, sums and differences over +-m apart: per (pair, density) and order n
+    (n + 1)^2 + n^2 real entries on complex values twice, complex entries once."""
+    npairs = int(arrays["list2_starts"][scalars["nttp_boxes"]])
+    s = sum((n + 1) ** 2 + n ** 2 for n in range(p + 1))
+    return 2 * 8 * s * npairs * nrhs
+
+
 # {{{ apply-level roofline
 
 #: stages bounded by HBM bandwidth (the rest by the FP64 pipe), as classified for the

@@ -224,7 +224,6 @@ k_p2m3(qbxfmm_geometry g, SourceCoeffs sc, int p, int ncf, int nrhs,
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       if (!valid[h]) continue;
-      int ci = threadIdx.x + h * NT;
       double2 a = acc[h];
       for (int j = 0; j < cnt; ++j) {
         const double2* T = tab + j;
@@ -1118,9 +1117,8 @@ k_m2qbxl3(qbxfmm_geometry g, int pf, int ncf, int nrhs, const double2* __restric
   constexpr int NC = (Q + 1) * (Q + 2) / 2;
   extern __shared__ double2 smem2[];
   const int NMP = pf + Q + 1;                          // columns m'
-  const int TSZ = NMP * (pf + 1) * (Q + 1) * 2;        // [m'][n][i]{T1, T2}
   double2* Ms = smem2;                                 // [ncf] the box's multipole, rho_s^n
-  double2* T = Ms + ncf;                               // [TSZ]
+  double2* T = Ms + ncf;                               // [NMP m'][pf + 1 n][Q + 1 i]{T1, T2}
   double2* red = T;                                    // [NW][32][NC] after the last box
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int chunk = blockIdx.x / MZ, zpart = blockIdx.x - chunk * MZ;

@@ -15,6 +15,8 @@
 #include "common.cuh"
 #include "kernels.h"
 
+#include <utility>
+
 #include <cooperative_groups.h>
 namespace cg = cooperative_groups;
 
@@ -57,6 +59,9 @@ k_gmres_step(GmresImages im, int count, int nsweep, bool first, bool norm, bool 
              const uint8_t* __restrict__ active, T* __restrict__ rnew, T* __restrict__ x)
 {
   cg::cluster_group cl = cg::this_cluster();
+  // no CTA writes to another's shared memory before all have started; the loads of w and v
+  // run meanwhile
+  auto started = cl.barrier_arrive();
   __shared__ T s_warp[GM_W], s_part[2][GM_CL];
   const int rank = cl.block_rank(), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const size_t off = (size_t)blockIdx.y * n;
@@ -81,6 +86,17 @@ k_gmres_step(GmresImages im, int count, int nsweep, bool first, bool norm, bool 
     else return v[off + at(k)];
   };
   const T zero = gm_scale(0.0, T());
+  each([&](int k) {
+    const bool in = at(k) < n;
+    if constexpr (E > 0) {
+      wr[k] = in ? (first ? win : w)[off + at(k)] : zero;
+      vr[k] = in ? (first ? r : v)[off + at(k)] : zero;
+    } else if (first && in) {
+      W(k) = win[off + at(k)];
+      V(k) = r[off + at(k)];
+    }
+  });
+  cl.barrier_wait(std::move(started));
   int par = 0;
   auto reduce = [&](T s) {
 #pragma unroll
@@ -99,16 +115,6 @@ k_gmres_step(GmresImages im, int count, int nsweep, bool first, bool norm, bool 
     par ^= 1;
     return t;
   };
-  each([&](int k) {
-    const bool in = at(k) < n;
-    if constexpr (E > 0) {
-      wr[k] = in ? (first ? win : w)[off + at(k)] : zero;
-      vr[k] = in ? (first ? r : v)[off + at(k)] : zero;
-    } else if (first && in) {
-      W(k) = win[off + at(k)];
-      V(k) = r[off + at(k)];
-    }
-  });
   auto fetch = [&](const void* p) {
     if constexpr (E > 0) {
 #pragma unroll

@@ -9,7 +9,9 @@
 // densities and 6224 nodes took 0.9 ms beside an operator of 1 ms.  Here a cluster of eight
 // CTAs holds a density's w and v in registers (up to 16384 entries, else in L2), the next
 // image is loaded during a reduction, and a reduction is one exchange through distributed
-// shared memory, summed in a fixed order: one launch an iteration.
+// shared memory, summed in a fixed order: one launch an iteration.  Above 16384 entries a step
+// reads and writes w and v as well, and eight SMs a density are few: the caller (gmres.py) takes
+// the tensor operations where they are faster.
 // 25 iterations with 7 densities of 6224 nodes: 48.6 -> 28.0 ms, 25 of them in the operator.
 #include "../../include/qbxfmm_api.h"
 #include "common.cuh"

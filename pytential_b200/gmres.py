@@ -12,7 +12,8 @@ device.  A density stops changing once its residual meets the tolerance.
 
 On a GPU the orthogonalization and the updates of an iteration are one kernel launch
 (``qbxfmm_gmres_step``), which takes plain contiguous float64 or complex128 tensors
-outside of autograd; anything else goes through the tensor operations below.
+outside of autograd; anything else, and few densities of very many unknowns, goes through
+the tensor operations below.
 """
 
 from __future__ import annotations
@@ -57,6 +58,18 @@ def _plain(*tensors):
         and not torch._C._functorch.is_functorch_wrapped_tensor(t)
         and torch.autograd.forward_ad.unpack_dual(t).tangent is None
         for t in tensors) and t0.shape[0] <= 65535
+
+
+def _step_wins(nd, n):
+    """Whether the kernel is faster than the tensor operations.  It gives a density eight
+    SMs, which wait on one another at every inner product; the tensor operations use the
+    whole GPU but read and write every vector at every step.  Kernel against operations,
+    float64 and complex128, 2 to 40 kept images, 1 to 64 densities: 6224 unknowns 37-374
+    against 410-3933 us, 65 536 (the slowest for the kernel: 4 densities, 40 images, float64)
+    2.5 against 3.2 ms; 131 072, 40 images: 1 density 3.9-5.8 against 3.3-4.1 ms, 64 densities
+    9.4-14.7 against 13.9-28.6; 307 200, 40 images: 1 density 11.1-13.5 against 3.3-4.1 ms, 16
+    16.4-22.3 against 8.3-17.5, 64 21.7-34.8 against 30.9-64.0."""
+    return n <= 65536 or nd >= 64
 
 
 def _step(Ae, e, w, r, x, active, update_r):
@@ -154,7 +167,7 @@ def gmres(op, rhs: torch.Tensor, restart: int | None = None, tol: float | None =
 
         w = op(r)
         recalc_r = (iteration + 1) % 10 == 0
-        if _plain(w, r, x, *Ae[:orth_count], *e[:orth_count]):
+        if _step_wins(nd, rhs.shape[1]) and _plain(w, r, x, *Ae[:orth_count], *e[:orth_count]):
             Ae[k], e[k], r, x = _step(Ae[:orth_count], e[:orth_count], w, r, x, active_dev,
                                       not recalc_r)
             k += 1

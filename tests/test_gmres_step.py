@@ -49,3 +49,21 @@ def test_step(n, nd, count, dtype, update_r):
     for a, b in zip(got, want):
         scale = max(float(b.abs().max()), 1.0)
         assert float((a - b).abs().max()) <= 1e-11 * scale
+
+
+@pytest.mark.parametrize("n,nd,kernel", [(65536, 1, True), (65537, 1, False), (65537, 63, False),
+                                         (65537, 64, True)])
+def test_few_densities_of_many_unknowns(n, nd, kernel, monkeypatch):
+    """The kernel's eight SMs a density are for moderate sizes or many densities; the solve
+    is the same either way."""
+    calls = []
+    step = mod._step
+    monkeypatch.setattr(mod, "_step", lambda *a: calls.append(1) or step(*a))
+    g = torch.Generator(device="cuda").manual_seed(n)
+    diag = 1.0 + torch.rand(n, generator=g, dtype=torch.float64, device="cuda")
+    b = torch.randn(nd, n, generator=g, dtype=torch.float64, device="cuda")
+    res = mod.gmres(lambda v: diag * v, b, tol=1e-10, restart=30, maxiter=60)
+    assert bool(calls) == kernel
+    # |A x - b| <= 1e-10 |b| and A >= 1
+    err = torch.linalg.norm(res.solution - b / diag, dim=1) / torch.linalg.norm(b, dim=1)
+    assert float(err.max()) <= 1.01e-10

@@ -11,7 +11,7 @@
 //
 // Bessel functions: J_0..J_N by Miller's backward recurrence normalized with
 // J_0 + 2 sum_k J_2k = 1; Y_0, Y_1 from the CUDA math library (y0, y1) below x = 8 and
-// their Neumann series above, where the library's error is absolute (5e-12);
+// Hankel's form above, where the library's error is absolute (5e-12);
 // Y_{n+1} = (2n/x) Y_n - Y_{n-1} (stable upward).
 #pragma once
 
@@ -22,9 +22,51 @@ namespace qbx {
 // first index of Miller's recurrence for orders up to nmax and arguments up to nmax
 QBX_D int miller_start(int nmax) { return 2 * ((nmax + 16 + (int)sqrt(40.0 * nmax)) / 2); }
 
-// Y_0 and Y_1 at x > 0; from x = 8 on by Abramowitz & Stegun 9.1.88 and 9.1.89 over Miller's
-// J_k: (pi/2) Y_0 = (ln(x/2) + gamma) J_0 - 2 sum_k (-1)^k J_2k / k, (pi/2) Y_1 = (ln(x/2) +
-// gamma - 1) J_1 - J_0 / x - sum_k (-1)^k (2k+1) J_{2k+1} / (k (k+1))
+// P_0, Q_0 x / 8, P_1, Q_1 x / 8 of Hankel's form of H_0 and H_1 (Abramowitz & Stegun
+// 9.2.5-9.2.6) in powers of z = (8/x)^2, x >= 8: Chebyshev expansions computed from the
+// integrals that define them, cut at degree 12 (tests/golden/make_hankel_pq.py)
+static __constant__ double c_hankel_pq[4][13] = {
+    {  // P0
+     1, -0.0010986328124988106, 2.7380883622028302e-05, -2.183917912860027e-06,
+     3.6202014961341726e-07, -1.0230381069471657e-07, 4.3424496202719202e-08, -2.4257416747728671e-08,
+     1.4955669741118411e-08, -8.4244019168030117e-09, 3.6616327747651667e-09, -1.029775376082398e-09,
+     1.3657578771623472e-10,
+    },
+    {  // Q0
+     -0.015624999999999997, 0.00014305114745956593, -6.9307861041698743e-06, 8.2384278024370908e-07,
+     -1.8162568982031541e-07, 6.4007335210559721e-08, -3.2323578736828035e-08, 2.0507328469913932e-08,
+     -1.3732461399427442e-08, 8.1281000911352184e-09, -3.6388968690144927e-09, 1.0424810644356815e-09,
+     -1.3997455046895388e-10,
+    },
+    {  // P1
+     1, 0.0018310546874986088, -3.5203993240441122e-05, 2.5809940497456218e-06,
+     -4.1029067171084456e-07, 1.1307836608916155e-07, -4.7219294565271443e-08, 2.6096037687254697e-08,
+     -1.5984079019861392e-08, 8.9706334212754281e-09, -3.8918385551293495e-09, 1.0937431701070939e-09,
+     -1.4506440493278205e-10,
+    },
+    {  // Q1
+     0.046874999999999993, -0.00020027160644386617, 8.4709608075089276e-06, -9.5058801055065598e-07,
+     2.0299488931624851e-07, -7.0110464104389147e-08, 3.4932506905851458e-08, -2.1971335618931054e-08,
+     1.4637445489481168e-08, -8.6385753180392068e-09, 3.8609338134006537e-09, -1.1049507975258166e-09,
+     1.482618472437025e-10,
+    },
+};
+
+QBX_D double hankel_pq(int f, double z)
+{
+  double r = c_hankel_pq[f][12];
+#pragma unroll
+  for (int i = 11; i >= 0; --i) r = fma(r, z, c_hankel_pq[f][i]);
+  return r;
+}
+
+// Y_0 and Y_1 at x > 0; from x = 8 on, where the library's error is absolute,
+//   Y_0 = sqrt(2 / (pi x)) (P_0 sin(x - pi/4) + Q_0 cos(x - pi/4)), Y_1 alike from x - 3 pi/4,
+// with the phases' sines and cosines as sums of sin x and cos x: 50 multiply-adds beside one
+// sincos, no more than the library's.  (Their Neumann series over the J_k of a recurrence of
+// its own took M2P from 110 to 207 us, M2QBXL from 401 to 681 and P2QBXL from 573 to 1572 of a
+// 1024-node boundary with 100 points, k 20; with this form 109,
+// 384 and 510.)
 QBX_D void bessel_y01(double x, double& Y0, double& Y1)
 {
   if (x < 8.0) {
@@ -32,32 +74,12 @@ QBX_D void bessel_y01(double x, double& Y0, double& Y1)
     Y1 = y1(x);
     return;
   }
-  const double xinv = 1.0 / x;
-  double fp1 = 0.0, f = 1e-200, sum = 0.0, a = 0.0, b = 0.0;
-  for (int k = miller_start((int)x); k > 0; --k) {
-    const int m = k >> 1;
-    const double t = m & 1 ? -f : f;
-    if (!(k & 1)) {
-      sum += 2.0 * f;
-      a += t / m;
-    } else if (m > 0) {
-      b += t * (2 * m + 1) / ((double)m * (m + 1));
-    }
-    const double fm1 = 2.0 * k * xinv * f - fp1;
-    fp1 = f;
-    f = fm1;
-    if (fabs(f) > 1e200) {
-      f *= 1e-200;
-      fp1 *= 1e-200;
-      sum *= 1e-200;
-      a *= 1e-200;
-      b *= 1e-200;
-    }
-  }
-  const double norm = 1.0 / (sum + f), J0 = f * norm, J1 = fp1 * norm;
-  const double L = log(0.5 * x) + 0.57721566490153286061, c = 0.63661977236758134308;  // 2 / pi
-  Y0 = c * (L * J0 - 2.0 * a * norm);
-  Y1 = c * ((L - 1.0) * J1 - xinv * J0 - b * norm);
+  double s, c;
+  sincos(x, &s, &c);
+  const double w = 8.0 / x, z = w * w, a = 0.56418958354775628695 * sqrt(0.125 * w);   // 1 / sqrt(pi x)
+  const double d = s - c, e = s + c;
+  Y0 = a * (hankel_pq(0, z) * d + w * hankel_pq(1, z) * e);
+  Y1 = a * (w * hankel_pq(3, z) * d - hankel_pq(2, z) * e);
 }
 
 // J[0..N], Y[0..N] (Y only if want_y) at x > 0.

@@ -69,12 +69,12 @@ struct qbxfmm_plan {
   // branch, on a high-priority stream)
   cudaStream_t side[3] = {nullptr, nullptr, nullptr};
   cudaEvent_t ev_fork = nullptr, ev_mpoles = nullptr, ev_near = nullptr, ev_p2l = nullptr,
-              ev_qbx = nullptr;
+              ev_qbx = nullptr, ev_m2p = nullptr;
   ~qbxfmm_plan()
   {
     for (cudaStream_t s : side)
       if (s) cudaStreamDestroy(s);
-    for (cudaEvent_t e : {ev_fork, ev_mpoles, ev_near, ev_p2l, ev_qbx})
+    for (cudaEvent_t e : {ev_fork, ev_mpoles, ev_near, ev_p2l, ev_qbx, ev_m2p})
       if (e) cudaEventDestroy(e);
     if (lorders_dev) cudaFree(lorders_dev);
   }
@@ -568,7 +568,8 @@ int qbxfmm_plan_create(const qbxfmm_kernel* kernel, const qbxfmm_geometry* geome
   for (int i = 0; i < 3 && e == cudaSuccess; ++i)
     e = cudaStreamCreateWithPriority(&p->side[i], cudaStreamNonBlocking,
                                      i == 2 ? prio_greatest : prio_least);
-  for (cudaEvent_t* ev : {&p->ev_fork, &p->ev_mpoles, &p->ev_near, &p->ev_p2l, &p->ev_qbx})
+  for (cudaEvent_t* ev : {&p->ev_fork, &p->ev_mpoles, &p->ev_near, &p->ev_p2l, &p->ev_qbx,
+                          &p->ev_m2p})
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     delete p;
@@ -1352,17 +1353,23 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
   // that several stages add into is written by one stream at a time:
   //   caller's stream: strengths, P2M, M2M | M2L, L2L | L2P | L2QBXL, QBXL2P, assembly
   //   side[0]:         P2P, target-specific near field | M2T, M2P
-  //   side[1]:         P2L
+  //   side[1]:         P2L; with `apart` P2P | M2P here and not on side[0]
   //   side[2]:         P2QBXL | M2QBXL (unless M2T takes its place)
-  // with events: fork after the strengths; M2P and M2QBXL wait for M2M; M2L waits
-  // for P2L (both add into the locals); L2P and QBXL2P wait for side[0]
-  // (pot_nonqbx, pot_tree); L2QBXL waits for side[2] (the QBX expansions).  Every
+  // with events: fork after the strengths; M2P, M2T and M2QBXL wait for M2M; M2L waits
+  // for P2L (both add into the locals); L2P waits for M2P (pot_nonqbx), QBXL2P for side[0]
+  // (pot_tree); L2QBXL waits for side[2] (the QBX expansions).  Every
   // stage adds into its outputs, so the order of the writers of one buffer does not
   // matter, only that they do not overlap.
+  // `apart`: the 2D Helmholtz kernels are chains of Bessel recurrences over few CTAs, whose
+  // times on one stream add up, so the two potentials have a stream each.  One density, apply
+  // with P2P, near field, M2T and M2P in a row on side[0] against this: 2400 nodes, 100 points
+  // 1.08 -> 0.78 ms, 1000 points 1.90 -> 1.22; 8000 nodes, 5000 points 1.20 -> 1.04.
+  const bool apart = p->helm && !p->h3;
   void* s1 = p->side[0];
   void* s2 = p->side[1];
   void* s3 = p->side[2];
   cudaStream_t side1 = p->side[0], side2 = p->side[1], side3 = p->side[2];
+  cudaStream_t side_p = apart ? side2 : side1;          // of the non-QBX targets
   const bool tsqbx = p->kern.target_specific_qbx != 0;
   bool forked = false;
   // on an error, join the side streams before returning, so that a stream capture
@@ -1393,7 +1400,7 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
   forked = true;
   QBX_STEP(qbxfmm_form_locals(p, ws->strengths, ws->locals, ws->error_word, s2));
   QBX_CUDA_STEP(cudaEventRecord(p->ev_p2l, side2), "apply: P2L event");
-  QBX_STEP(qbxfmm_eval_direct(p, ws->strengths, ws->pot_nonqbx, ws->error_word, s1));
+  QBX_STEP(qbxfmm_eval_direct(p, ws->strengths, ws->pot_nonqbx, ws->error_word, side_p));
   if (tsqbx) {
     QBX_STEP(qbxfmm_eval_target_specific_qbx_locals(p, ws->strengths, ws->pot_tree, ws->error_word, s1));
   } else {
@@ -1418,13 +1425,16 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
                                 p->kern.nrhs, false, (const double2*)ws->mpoles,
                                 (double2*)ws->pot_tree, ws->error_word, side1),
                   "apply: multipoles to QBX targets");
-  QBX_STEP(qbxfmm_eval_multipoles(p, ws->mpoles, ws->pot_nonqbx, ws->error_word, s1));
+  if (apart) QBX_CUDA_STEP(cudaStreamWaitEvent(side2, p->ev_mpoles, 0), "apply: multipole event");
+  QBX_STEP(qbxfmm_eval_multipoles(p, ws->mpoles, ws->pot_nonqbx, ws->error_word, side_p));
+  QBX_CUDA_STEP(cudaEventRecord(p->ev_m2p, side_p), "apply: M2P event");
   QBX_CUDA_STEP(cudaEventRecord(p->ev_near, side1), "apply: near-field event");
   QBX_CUDA_STEP(cudaStreamWaitEvent(st, p->ev_p2l, 0), "apply: join P2L");
   QBX_STEP(m2l());
   QBX_STEP(l2l());
-  QBX_CUDA_STEP(cudaStreamWaitEvent(st, p->ev_near, 0), "apply: join near field");
+  QBX_CUDA_STEP(cudaStreamWaitEvent(st, p->ev_m2p, 0), "apply: join M2P");
   QBX_STEP(qbxfmm_eval_locals(p, ws->locals, ws->pot_nonqbx, stream));
+  QBX_CUDA_STEP(cudaStreamWaitEvent(st, p->ev_near, 0), "apply: join near field");
   QBX_CUDA_STEP(cudaStreamWaitEvent(st, p->ev_qbx, 0), "apply: join QBX expansions");
   forked = false;
 #undef QBX_STEP

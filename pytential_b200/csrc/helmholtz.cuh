@@ -65,8 +65,8 @@ QBX_D double hankel_pq(int f, double z)
 // with the phases' sines and cosines as sums of sin x and cos x: 50 multiply-adds beside one
 // sincos, no more than the library's.  (Their Neumann series over the J_k of a recurrence of
 // its own took M2P from 110 to 207 us, M2QBXL from 401 to 681 and P2QBXL from 573 to 1572 of a
-// 1024-node boundary with 100 points, k 20; with this form 109,
-// 384 and 510.)
+// 1024-node boundary with 100 points, k 20; with this form 109, 384
+// and 510.)
 QBX_D void bessel_y01(double x, double& Y0, double& Y1)
 {
   if (x < 8.0) {

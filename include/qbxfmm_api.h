@@ -75,7 +75,8 @@ int qbxfmm_workspace_sizes(const qbxfmm_plan* plan, size_t* sizes8);
 
 /* Build the translation-class matrices of M2L / M2M / L2L into ws->translations
  * (the reference's translation-class precompute, pytential/qbx/fmm.py:155-161,
- * 399-407).  Once per plan and workspace, before qbxfmm_apply. */
+ * 399-407).  Once per plan and workspace, before qbxfmm_apply.  Enqueued on `stream`: a caller
+ * that applies on another one orders the two. */
 int qbxfmm_precompute_translations(const qbxfmm_plan* plan, const qbxfmm_workspace* ws,
                                    void* stream);
 

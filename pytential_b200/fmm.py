@@ -40,6 +40,13 @@ def _stream_handle(stream: torch.cuda.Stream | None = None):
     return ctypes.c_void_p(s.cuda_stream)
 
 
+def _finish_setup(device):
+    """Wait for what a constructor has enqueued on its stream (zero fills, the translations'
+    tables): the object may be called on any other stream, and inside a capture, which could
+    not wait for an event recorded outside of it."""
+    torch.cuda.current_stream(device).synchronize()
+
+
 # {{{ kernels
 
 @dataclass(frozen=True)
@@ -298,6 +305,7 @@ class B200QBXExpansionWrangler:
         self.tree = self.traversal.tree
         self.error_word = torch.zeros(1, dtype=torch.int32, device=self.device)
         self._reorder = _IdentityUpsampler(self.dgeo.nsources, self.device)
+        _finish_setup(self.device)
 
     # {{{ buffers
 
@@ -602,6 +610,7 @@ class QBXApply:
         self.nuser_targets = self.dgeo.nuser_targets
         self.dtype = torch.complex128 if spec.is_complex else torch.float64
         self._graph = None
+        _finish_setup(self.device)
 
     def new_output(self):
         return torch.empty(self.nrhs, self.nuser_targets, dtype=self.dtype, device=self.device)

@@ -284,7 +284,7 @@ class QBXTransposeApply:
 
         from .fmm import (PRECISION_FP64, B200QBXExpansionWrangler,
                           B200TreeIndependentDataForWrangler, DeviceGeometry, Plan, _ptr,
-                          _stream_handle)
+                          _finish_setup, _stream_handle)
         from .fmm import LaplaceKernel, SourceKernelSpec
         plan = apply.plan
         spec = plan.spec
@@ -356,6 +356,7 @@ class QBXTransposeApply:
         self._cm = torch.zeros(max(nc, 1), nrhs, self.ncq, dtype=torch.complex128, device=dev)
         self._grad = (torch.zeros(nrhs, 3, self.nsources, dtype=torch.float64, device=dev)
                       if self.has_dipole else None)
+        _finish_setup(dev)
 
     def _inputs(self, r):
         """Tree-target values and the non-QBX ones (the exchanged-role strengths)."""

@@ -92,9 +92,11 @@ int qbxfmm_gmres_step(int is_complex, int ndens, long long n, int count, const v
                       void* v, const unsigned char* active, void* r_new, void* x, void* stream);
 
 /* One translation stage as qbxfmm_apply runs it, on ws->mpoles and ws->locals with
- * ws->translations and ws->pair_scratch (either NULL: by pair, as the entries below):
- * stage 0 coarsen_multipoles, 1 multipole_to_local, 2 refine_locals.  A stage reads and
- * writes only its own buffers of ws; calls at the same time need their own pair_scratch. */
+ * ws->translations (NULL: by pair, as the entries below):
+ * stage 0 coarsen_multipoles, 1 multipole_to_local, 2 refine_locals.  Stage 1, and stage 0 of
+ * a mixed-precision plan above order 14, use ws->pair_scratch too (NULL: by pair); the others
+ * need none.  A stage reads and writes only its own buffers of ws; calls at the same time
+ * need their own pair_scratch. */
 int qbxfmm_translate_boxes(const qbxfmm_plan* plan, const qbxfmm_workspace* ws, int stage,
                            void* stream);
 

@@ -1207,17 +1207,22 @@ int qbxfmm_precompute_translations(const qbxfmm_plan* p, const qbxfmm_workspace*
 
 namespace {
 
-// M2M / L2L: the FP64 matrix-vector kernels whenever the matrices are small (both
-// precisions: they are latency-bound, a TF32 form would not be faster); M2L: split
-// TF32 in the mixed form.  `gemm`: the translation matrices of ws are built; T32:
-// their split-TF32 planes (mixed form), or NULL.
-// the matrix form of the translations (per-level orders run the stage entries, which truncate
-// level by level)
-bool use_matrices(const qbxfmm_plan* p, const qbxfmm_workspace* ws)
+// the translation matrices of ws are built (per-level orders run the stage entries, which
+// truncate level by level)
+bool have_matrices(const qbxfmm_plan* p, const qbxfmm_workspace* ws)
 {
-  return !p->h3 && p->trans_ok && ws->translations && ws->pair_scratch && !level_orders_on(p);
+  return !p->h3 && p->trans_ok && ws->translations && !level_orders_on(p);
 }
 
+// stages whose matrix form goes by the pairs' products in ws->pair_scratch: M2L (1), and M2M (0)
+// in split TF32
+bool needs_pair_scratch(const qbxfmm_plan* p, int stage)
+{
+  return stage == 1 || (stage == 0 && p->tf32_ok && !trans_small(p->tc));
+}
+
+// The translations below: `gemm`: by matrices; T32: the matrices' split-TF32 planes (mixed
+// form), or NULL.
 const uint32_t* tf32_planes(const qbxfmm_plan* p, const qbxfmm_workspace* ws, bool gemm)
 {
   return (gemm && p->tf32_ok)
@@ -1307,7 +1312,7 @@ int qbxfmm_translate_boxes(const qbxfmm_plan* p, const qbxfmm_workspace* ws, int
   if (int rc = check_plan(p)) return rc;
   if (!ws || stage < 0 || stage > 2 || (stage < 2 && !ws->mpoles) || (stage > 0 && !ws->locals))
     return fail(QBXFMM_ERR_ARG, "translate_boxes: incomplete workspace or unknown stage");
-  const bool gemm = use_matrices(p, ws);
+  const bool gemm = have_matrices(p, ws) && (ws->pair_scratch || !needs_pair_scratch(p, stage));
   const uint32_t* T32 = tf32_planes(p, ws, gemm);
   if (stage == 0) return run_m2m(p, ws, T32, gemm, stream);
   if (stage == 1) return run_m2l(p, ws, T32, gemm, stream);
@@ -1324,7 +1329,7 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
     return fail(QBXFMM_ERR_ARG, "incomplete workspace");
   size_t sz[8];
   if (int rc = qbxfmm_workspace_sizes(p, sz)) return rc;
-  const bool gemm = use_matrices(p, ws);
+  const bool gemm = have_matrices(p, ws) && ws->pair_scratch;
   if (p->h3) {
     if (!ws->translations)
       return fail(QBXFMM_ERR_ARG, "3D Helmholtz needs the translations buffer");

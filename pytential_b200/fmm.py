@@ -369,15 +369,18 @@ class B200QBXExpansionWrangler:
                                    ptr(self._translations[0]), ptr(scratch))
 
     def _translate(self, stage, mpoles=None, locals_=None):
-        """M2M (0), M2L (1) or L2L (2) with the plan's matrices, if there are any and memory
-        for the products of the pairs is left.  The scratch belongs to this call and its
-        stream."""
+        """M2M (0), M2L (1) or L2L (2) with the plan's matrices or tables, if there are any and,
+        for M2L, memory for the products of the pairs is left.  That scratch belongs to this
+        call and its stream."""
         if self._translations is None or self._scratch_words is None:
             return False
-        try:
-            scratch = torch.empty(self._scratch_words, dtype=torch.float64, device=self.device)
-        except torch.OutOfMemoryError:
-            return False
+        scratch = None
+        if stage == 1:
+            try:
+                scratch = torch.empty(self._scratch_words, dtype=torch.float64,
+                                      device=self.device)
+            except torch.OutOfMemoryError:
+                return False
         ws = self._translation_ws(mpoles, locals_, scratch)
         ws.error_word = ctypes.cast(self._err(), ctypes.POINTER(ctypes.c_int32))
         self.plan.call("qbxfmm_translate_boxes", ctypes.byref(ws), stage, self._s())

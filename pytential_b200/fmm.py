@@ -297,8 +297,13 @@ class B200QBXExpansionWrangler:
         self._translations = None
         self._scratch_words = None if per_level else sizes[7] // 8 + 1
         if sizes[6] > 0:
-            self._translations = [torch.zeros(n, dtype=torch.float64, device=self.device)
-                                  for n in (sizes[6] // 8 + 1, 1)]
+            try:
+                self._translations = [torch.zeros(n, dtype=torch.float64, device=self.device)
+                                      for n in (sizes[6] // 8 + 1, 1)]
+            except torch.OutOfMemoryError:
+                if per_level:           # its translation stages have no other form
+                    raise
+        if self._translations is not None:
             ws = self._translation_ws(None, None, self._translations[1])
             self.plan.call("qbxfmm_precompute_translations", ctypes.byref(ws), _stream_handle())
         self.traversal = geo_data.traversal()

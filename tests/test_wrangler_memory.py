@@ -51,3 +51,17 @@ def test_products_of_pairs(problem, monkeypatch):
     assert "qbxfmm_multipole_to_local" in [n for n, _ in names]
     # the same sums in another order
     assert float((got - want).abs().max() / want.abs().max()) < 1e-13
+
+
+def test_matrices(problem, monkeypatch):
+    """Without memory for the matrices the wrangler translates by pair."""
+    geo, spec, want = problem
+    sizes = fmm.Plan.workspace_sizes
+    monkeypatch.setattr(fmm.Plan, "workspace_sizes",
+                        lambda self: [*sizes(self)[:6], 8 * NEVER, *sizes(self)[7:]])
+    names = _calls(monkeypatch)
+    w = _wrangler(geo, spec)
+    got = _drive(geo, w)
+    names = [n for n, _ in names]
+    assert "qbxfmm_precompute_translations" not in names and "qbxfmm_translate_boxes" not in names
+    assert float((got - want).abs().max() / want.abs().max()) < 1e-13

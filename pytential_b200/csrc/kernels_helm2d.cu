@@ -97,10 +97,9 @@ QBX_D double2 hbar(const double2* Z, int N, int m)
 
 // {{{ strengths (complex density)
 
-// One thread per tree source and up to FS_RB densities: a source's interpolation row (a
+// One thread per tree source and up to RB densities: a source's interpolation row (a
 // strided read of the matrix) serves all of them.
-constexpr int FS_RB = 8;
-
+template <int RB>
 __global__ void __launch_bounds__(256)
 k_h2_form_strengths(int nsources, int ndofs, int npe, int nqpe, int nrhs,
                     const double* __restrict__ U, const double* __restrict__ qw,
@@ -108,24 +107,24 @@ k_h2_form_strengths(int nsources, int ndofs, int npe, int nqpe, int nrhs,
                     const double2* __restrict__ density, double2* __restrict__ out)
 {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int r0 = blockIdx.y * FS_RB, nr = min(FS_RB, nrhs - r0);
+  const int r0 = blockIdx.y * RB, nr = min(RB, nrhs - r0);
   if (t >= nsources) return;
   const int j = __ldg(user_source_ids + t);
   const int e = j / nqpe;
   const double* u = U + (size_t)(j - e * nqpe) * npe;
   const double2* d = density + (size_t)r0 * ndofs + (size_t)e * npe;
-  double2 acc[FS_RB];
+  double2 acc[RB];
 #pragma unroll
-  for (int r = 0; r < FS_RB; ++r) acc[r] = c2(0.0);
+  for (int r = 0; r < RB; ++r) acc[r] = c2(0.0);
   for (int i = 0; i < npe; ++i) {
     const double w = __ldg(u + i);
 #pragma unroll
-    for (int r = 0; r < FS_RB; ++r)
+    for (int r = 0; r < RB; ++r)
       if (r < nr) acc[r] = caxpy(w, __ldg(d + (size_t)r * ndofs + i), acc[r]);
   }
   const double w = __ldg(qw + j);
 #pragma unroll
-  for (int r = 0; r < FS_RB; ++r)
+  for (int r = 0; r < RB; ++r)
     if (r < nr) out[(size_t)(r0 + r) * nsources + t] = cscale(w, acc[r]);
 }
 
@@ -1057,11 +1056,16 @@ static size_t zsh(int p) { return (size_t)(2 * (p + 1) + 1); }
 cudaError_t h2_launch_form_strengths(const qbxfmm_geometry& g, const qbxfmm_upsample& up, int nrhs,
                                      const double2* density, double2* strengths, cudaStream_t st)
 {
-  dim3 grid((g.nsources + 255) / 256, (nrhs + FS_RB - 1) / FS_RB);
-  k_h2_form_strengths<<<grid, 256, 0, st>>>(g.nsources, up.nelements * up.nodes_per_element,
-                                            up.nodes_per_element, up.quad_nodes_per_element, nrhs,
-                                            up.matrix, up.quad_weights, g.user_source_ids, density,
-                                            strengths);
+  // densities a thread: 8 for much work, 1 where threads are few (us for 1 / 4 / 8 of them: 4096
+  // sources, 8 densities 4.7 / 6.6 / 11.1; 9600, 4 densities 6.8 / 6.6 / 9.7; 25 600, 16 densities
+  // 29.3 / 13.3 / 14.4; 64 000, 6 densities 29.1 / 15.9 / 13.6; 131 072, 64 densities 542 / 202 / 178)
+  const long long work = (long long)g.nsources * nrhs;
+  const int rb = nrhs == 1 || work < 36000 ? 1 : work < 400000 ? 4 : 8;
+  auto k = rb == 1 ? k_h2_form_strengths<1> : rb == 4 ? k_h2_form_strengths<4> : k_h2_form_strengths<8>;
+  const dim3 grid((g.nsources + 255) / 256, (nrhs + rb - 1) / rb);
+  k<<<grid, 256, 0, st>>>(g.nsources, up.nelements * up.nodes_per_element, up.nodes_per_element,
+                          up.quad_nodes_per_element, nrhs, up.matrix, up.quad_weights,
+                          g.user_source_ids, density, strengths);
   return cudaGetLastError();
 }
 

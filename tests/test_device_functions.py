@@ -85,3 +85,27 @@ def test_y01_against_scipy():
     for nu, y in ((0, y0), (1, y1)):
         ref = hankel1(nu, x)
         assert np.all(np.abs(y - ref.imag) <= 1e-13 * np.abs(ref)), nu
+
+
+def _rsqrt_arguments():
+    rng = np.random.default_rng(0)
+    # every upper word of [1, 4) (the approximation reads no more of x), lower words at
+    # random; then all binades of the normal range
+    top = np.arange(2 << 20, dtype=np.uint64) + (np.uint64(1023) << np.uint64(20))
+    dense = (top << np.uint64(32) | rng.integers(0, 1 << 32, top.size, dtype=np.uint64)).view(float)
+    e = rng.integers(-1022, 1024, 1 << 20)
+    return np.concatenate([dense, np.ldexp(rng.uniform(1, 2, e.size), e)])
+
+
+@pytest.mark.gpu
+def test_rsqrt():
+    x = _rsqrt_arguments()
+    seed, h, lib = _call("device_rsqrt", x, 3)
+    xl = x.astype(np.longdouble)
+    root = np.sqrt(xl)
+    assert float(np.abs(seed * root - 1).max()) <= 2.0 ** -18.4
+    # the third-order step leaves 2.5 |seed error|^3 < 2^-54; x y, 1 - (x y) y, y e and the
+    # last sum are rounded: below 2 units in the last place, like the library's
+    ulp = np.spacing((1 / root).astype(float))
+    assert float(np.abs((h - 1 / root) / ulp).max()) <= 2.0
+    assert float(np.abs((h - lib) / ulp).max()) <= 3.0

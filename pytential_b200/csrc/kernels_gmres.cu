@@ -199,7 +199,7 @@ cudaError_t step(int nd, long long n, int count, const void* const* a, const voi
                  const T* win, const T* r, T* w, T* v, const uint8_t* active, T* rnew, T* x,
                  cudaStream_t st)
 {
-  const long long per = n / (GM_CL * GM_NT) + 1;
+  const long long per = (n + GM_CL * GM_NT - 1) / (GM_CL * GM_NT);
   const dim3 grid(GM_CL, nd);
   auto launch = [&](int j0, int cnt, int nsweep, bool first, bool norm, bool last) {
     GmresImages im;

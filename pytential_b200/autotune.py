@@ -77,9 +77,25 @@ def _time_stage(ap, entry, reps, flush):
     return statistics.median(ms)
 
 
+def _run_by_apply(ap) -> set:
+    """The knobs of stages that the apply itself runs: in FP64 with the target-specific near
+    field it takes list-3 multipoles (in the sumpy truncation box locals too) straight to the
+    QBX targets, unless those are many beside the centers (``h3_m2t_wins``)."""
+    s, plan = ap.dgeo.scalars, ap.plan
+    run = set(KNOBS)
+    if not plan.target_specific_qbx:
+        run.discard("tsqbx_densities")
+    elif plan.precision == 0 and 0 < s["ntsqbx_chunks"] <= 8 * s["nqbx_chunks"]:
+        run.discard("m2qbxl_densities")
+        if plan.fmm_backend == "sumpy":
+            run.discard("l2qbxl_densities")
+    return run
+
+
 def autotune(ap, reps: int = 3, knobs=None, flush_bytes: int = 256 << 20) -> dict:
     """Pick the densities per CTA of each knob of ``ap`` (a 3D Helmholtz
-    :class:`~pytential_b200.fmm.QBXApply`) by timing the candidates; the apply's
+    :class:`~pytential_b200.fmm.QBXApply`) by timing the candidates: of the stages that
+    the apply runs, or of ``knobs``; the apply's
     workspace is overwritten (run it again afterwards).  Returns ``{"choice": ...,
     "ms": {knob: {candidate: ms}}}``."""
     spec = ap.plan.spec
@@ -92,7 +108,7 @@ def autotune(ap, reps: int = 3, knobs=None, flush_bytes: int = 256 << 20) -> dic
         if flush_bytes else None
     choice = get_tuning(ap.plan)
     timings = {}
-    for knob in knobs or KNOBS:
+    for knob in knobs or [k for k in KNOBS if k in _run_by_apply(ap)]:
         entry, cands, mixed_only = KNOBS[knob]
         if knob == "tsqbx_densities" and not ap.plan.target_specific_qbx:
             continue

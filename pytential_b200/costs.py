@@ -63,47 +63,6 @@ def p2p_pairs(arrays: dict, scalars: dict) -> int:
     return int((nt * nsrc).sum())
 
 
-def apply_launch_count(scalars: dict, arrays: dict, matrices: bool = False,
-                       tsqbx: bool = False, m2m_by_parent: bool = True) -> int:
-    """Kernels of this library launched by one qbxfmm_apply (3D matrix-form
-    translations when ``matrices``: M2M as one matrix-vector launch per level when
-    ``m2m_by_parent`` (the FP64 form), else products + reduction; target-specific
-    near field when ``tsqbx``)."""
-    nl = scalars["nlevels"]
-    lsp = arrays["level_start_source_parent_box_nrs"]
-    lttp = arrays["level_start_ttp_box_nrs"]
-    nch = 2 ** scalars["dim"]
-    n = 1                                                   # strengths
-    n += scalars["nsource_boxes"] > 0                       # P2M
-    if matrices:
-        mg = arrays["m2m_group_starts"]
-        lg = arrays["l2l_group_starts"]
-        for lev in range(nl - 1):
-            if mg[(lev + 1) * nch] > mg[lev * nch]:
-                n += 1                                      # M2M products
-                if not m2m_by_parent:
-                    n += lsp[lev + 1] > lsp[lev]            # M2M reduction
-        n += 2 * (scalars["m2l_nclasses"] > 0)              # M2L products + reduction
-        n += sum(1 for lev in range(1, nl) if lg[(lev + 1) * nch] > lg[lev * nch])  # L2L
-    else:
-        n += sum(1 for lev in range(nl - 1) if lsp[lev + 1] > lsp[lev])   # M2M
-        n += scalars["nttp_boxes"] > 0                      # M2L
-        n += sum(1 for lev in range(1, nl) if lttp[lev + 1] > lttp[lev])  # L2L
-    nf = scalars["nnonqbx_chunks"] > 0
-    n += nf                                                 # P2P
-    n += nf                                                 # M2P
-    n += scalars["nttp_boxes"] > 0                          # P2L
-    n += nf                                                 # L2P
-    if tsqbx:
-        n += scalars["ntsqbx_chunks"] > 0                   # target-specific near field
-    else:
-        n += scalars["nqbx_chunks"] > 0                     # P2QBXL
-    n += scalars["nqbx_chunks"] > 0                         # M2QBXL
-    n += 2 * (scalars["nglobal_qbx_centers"] > 0)           # L2QBXL, QBXL2P
-    n += (scalars["ntargets"] > 0) + (scalars["nfiltered_targets"] > 0)  # assembly
-    return int(n)
-
-
 def tsqbx_flops_per_pair(dim: int, q: int, charge: bool, dipole: bool) -> int:
     """Target-specific near field per (target, source) pair: prelude 15 (b = s - c,
     |b|^2, 1/|b|, cos), per order n Legendre and derivative recurrences 9 and

@@ -136,10 +136,10 @@ k_h2_form_strengths(int nsources, int ndofs, int npe, int nqpe, int nrhs,
 //   P2M: W(m) = cq conj(Z_m) + kd (conj(nu) conj(Z_{m-1}) - nu conj(Z_{m+1})),  Z = J
 //   P2L: W(m) = cq Hb_m + kd (conj(nu) Hb_{m-1} - nu Hb_{m+1})
 // (kd = (k/2) cd) do not depend on the density, so a box is a (2p+1) x nsrc times
-// nsrc x rhs complex product.  One CTA per (box, tile of RW * TR right-hand sides),
-// thread t: right-hand sides rl + RW j
-// (rl = t % RW, j < TR) and coefficients mg + G i (mg = t / RW, G = NT / RW); SUB sources per stage: Bessel tables one per
-// thread, then W and the strengths tile in shared memory.
+// nsrc x rhs complex product.  One CTA per (box, tile of RW * TR right-hand sides), thread t:
+// right-hand sides rl + RW j (rl = t % RW, j < TR) and coefficients mg + G i (mg = t / RW,
+// G = NT / RW); SUB sources per stage: Bessel tables one per thread, then W and the strengths
+// tile in shared memory.
 template <bool LOCAL, int RW, int TR>
 __global__ void __launch_bounds__(NT)
 k_h2_p2e(qbxfmm_geometry g, HelmCoeffs hc, int p, int nrhs, const double2* __restrict__ strengths,
@@ -1108,7 +1108,6 @@ cudaError_t h2_launch_p2l(const qbxfmm_geometry& g, HelmCoeffs hc, int p, int nr
   return h2_p2e<true>(g, hc, p, nrhs, g.nttp_boxes, s, lo, err, st);
 }
 
-// right-hand-side tiling of the translation kernels: (lanes over rhs, rhs per lane)
 cudaError_t h2_launch_eval_direct(const qbxfmm_geometry& g, HelmCoeffs hc, int nrhs,
                                   const double2* s, double2* pot, int32_t* err, cudaStream_t st)
 {

@@ -466,10 +466,6 @@ k_trans_reduce(int ncf, int rp, int nrhs, const int32_t* __restrict__ boxes, int
 
 // }}}
 
-// {{{ M2M / L2L as matrix-vector products (small matrices)
-
-// }}}
-
 // {{{ launchers
 
 static void dims_from_ncf(int ncf, int& rp, int& kp)

@@ -51,6 +51,9 @@ def _plain(*tensors):
     t0 = tensors[0]
     if not t0.is_cuda or t0.dtype not in (torch.float64, torch.complex128):
         return False
+    # modes that see every operation (counters, recorders, tracers) would miss the kernel's
+    if torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack() > 0:
+        return False
     return all(
         type(t) is torch.Tensor and t.shape == t0.shape and t.dtype == t0.dtype
         and t.device == t0.device and t.is_contiguous() and not t.is_conj() and not t.is_neg()

@@ -672,9 +672,12 @@ def run_b200(args):
         kt = stage_times(torch, ap, K, flush)
         scal, arr = ap.dgeo.scalars, ap.dgeo.host_arrays
         alg = costs.algorithmic_flops(arr, scal, 3, True, wl.fmm_order, wl.qbx_order, count)
-        # (M2L: the products of its rotations, fewer than the dense count)
+        # (M2L: the products of its rotations, fewer than the dense count; near field: the
+        # series once for all densities)
         alg["multipole_to_local"] = costs.helmholtz3d_m2l_rotation_flops(scal, arr, wl.fmm_order,
                                                                          count)
+        alg["eval_target_specific_qbx_locals"] = costs.helmholtz3d_near_flops(
+            scal, arr, wl.qbx_order, count)
         in_apply = {k: v for k, v in kt.items() if k not in NOT_IN_APPLY}
         dom = max(in_apply, key=in_apply.get)
         fp64_peak = measure_fp64_peak(torch, dev)

@@ -196,6 +196,13 @@ def helmholtz3d_m2l_rotation_flops(scalars: dict, arrays: dict, p: int, nrhs: in
     return 2 * 8 * s * npairs * nrhs
 
 
+def helmholtz3d_near_flops(scalars: dict, arrays: dict, q: int, nrhs: int) -> int:
+    """The 3D Helmholtz target-specific near field as its kernel needs it: per (target,
+    source) pair a series of q + 1 complex terms once for all densities, then one complex
+    product per density."""
+    return tsqbx_pairs(arrays, scalars) * 8 * (q + 1 + nrhs)
+
+
 # {{{ apply-level roofline
 
 #: stages bounded by HBM bandwidth (the rest by the FP64 pipe), as classified for the

@@ -1368,7 +1368,7 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
   // `apart`: the 2D Helmholtz kernels are chains of Bessel recurrences over few CTAs, whose
   // times on one stream add up, so the two potentials have a stream each.  One density, apply
   // with P2P, near field, M2T and M2P in a row on side[0] against this: 2400 nodes, 100 points
-  // 1.08 -> 0.78 ms, 1000 points 1.90 -> 1.22; 8000 nodes, 5000 points 1.20 -> 1.04.
+  // 1.15 -> 0.67 ms, 1000 points 1.91 -> 1.16; 8000 nodes, 5000 points 1.28 -> 1.02.
   const bool apart = p->helm && !p->h3;
   void* s1 = p->side[0];
   void* s2 = p->side[1];

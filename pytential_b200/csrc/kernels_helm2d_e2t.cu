@@ -203,12 +203,12 @@ cudaError_t e2t_q(const qbxfmm_geometry& g, double k, int p, int nrhs, const dou
 // the expansions are faster.  That line lies higher where no other targets' P2P and M2P take
 // the GPU meanwhile.  Apply with the expansions against this form, q 5, p 20, k 20, chunks of
 // the starfish at 64, 150, 220, 300, 500 and 700 elements (84, 216, 326, 414, 733, 1081):
-//   no other targets, 2 densities: 308 / 380, 461 / 586, 562 / 734, 549 / 693, 892 / 970,
-//   1098 / 932 us; 16 densities: 354 / 416, 527 / 634, 793 / 812, 964 / 900, 1527 / 1443,
-//   1901 / 1638 us;
-//   30 others, 1 density: 682 / 766, 682 / 794, 746 / 764, 1047 / 979 us; 100 others, 150
-//   elements: 1 density 1034 / 776, 2 820 / 786, 4 845 / 866, 8 1051 / 1001 us; 30 others, 16
-//   densities: 899 / 976, 851 / 982, 1024 / 958, 1471 / 1378 us.
+//   no other targets, 2 densities: 303 / 360, 444 / 563, 562 / 704, 536 / 666, 875 / 945,
+//   1107 / 980 us; 16 densities: 344 / 435, 558 / 665, 804 / 837, 950 / 988, 1529 / 1499,
+//   1910 / 1716 us;
+//   30 others, the first four: 1 density 613 / 672, 573 / 744, 615 / 735, 959 / 903 us, 16
+//   densities 833 / 968, 786 / 1012, 942 / 1010, 1409 / 1312 us; 100 others, 150 elements:
+//   1 density 802 / 697, 2 728 / 692, 4 772 / 765, 8 970 / 904 us.
 bool h2_e2t_wins(const qbxfmm_geometry& g, int nrhs)
 {
   const int ctas_per_sm = g.nnonqbx_chunks == 0 ? (nrhs <= 4 ? 5 : 2) : (nrhs == 1 ? 1 : 2);

@@ -23,7 +23,7 @@
 //
 // Each output (a box expansion, a source value) has one writer: the kernels gather
 // over the reversed lists of qbxfmm_transpose_index (M2QBXL^T and P2QBXL^T, when the
-// rows are too few to fill the GPU, with a cluster of TR_CL CTAs per row whose partial
+// rows are too few to fill the GPU, with a cluster of CTAs per row whose partial
 // sums rank 0 adds in rank order through distributed shared memory), so results do not
 // depend on scheduling.  The box stages of the transpose are the library's own P2M / M2M /
 // M2L / M2P / P2L / L2L / L2P / P2P on the exchanged-role geometry.
@@ -41,7 +41,7 @@ namespace qbx {
 namespace {
 
 constexpr int NT = 128;
-constexpr int TR_CL = 8;      // CTAs per row (a cluster) in M2QBXL^T and P2QBXL^T when
+constexpr int TR_CL = 8;      // CTAs per row (a cluster) in P2QBXL^T when
                               // the rows alone would not fill the GPU
 constexpr int TR_SPLIT_BELOW = 4 * 148;   // rows below which a row is split
 // M2QBXL^T: warps per CTA; rows of the product (qbx_order <= 8)
@@ -922,11 +922,18 @@ cudaError_t launch_tr_m2qbxl(const qbxfmm_geometry& g, const qbxfmm_transpose_in
   if (q > 8 || p > 21) return cudaErrorInvalidValue;
   // tiles of 8 rows, dealt evenly to passes of at most 4
   const int tiles = ((q + 1) * (q + 1) + 7) / 8, passes = (tiles + 3) / 4;
-  const bool split = ix.nlist3_rows < TR_SPLIT_BELOW;
-#define QBX_TRM(RT)                                                                \
-  case RT:                                                                         \
-    return split ? tr_m2qbxl<TR_CL, RT>(g, ix, p, q, nrhs, cmp, locals, err, st)   \
-                 : tr_m2qbxl<1, RT>(g, ix, p, q, nrhs, cmp, locals, err, st);
+  // CTAs per row: each pays for its batches' tables and for every pass, so a row is split only
+  // where the rows do not fill the GPU (two CTAs an SM), and not further than that.  The whole
+  // transpose with 1 / 2 / 4 / 8 CTAs a row: 70 rows (q 5, p 10) 0.70 / 0.48 / 0.41 / 0.44 ms, 208
+  // 1.35 / 1.09 / 1.01 / 1.06; 291 (q 6, p 10) 1.99 / 1.95 / 2.18 / 2.75, 420 2.19 / 2.19 / 2.54 /
+  // 3.32, 543 2.29 / 2.54 / 2.75 / 3.63, 727 2.42 / 2.71 / 3.16.
+  const long long rows = (long long)ix.nlist3_rows * nrhs;
+  const int cl = rows < 222 ? 4 : rows < 518 ? 2 : 1;          // 1.5 and 3.5 rows an SM
+#define QBX_TRM(RT)                                                                    \
+  case RT:                                                                             \
+    return cl == 4   ? tr_m2qbxl<4, RT>(g, ix, p, q, nrhs, cmp, locals, err, st)       \
+           : cl == 2 ? tr_m2qbxl<2, RT>(g, ix, p, q, nrhs, cmp, locals, err, st)       \
+                     : tr_m2qbxl<1, RT>(g, ix, p, q, nrhs, cmp, locals, err, st);
   switch ((tiles + passes - 1) / passes) {
     QBX_TRM(1) QBX_TRM(2) QBX_TRM(3) QBX_TRM(4)
     default: return cudaErrorInvalidValue;

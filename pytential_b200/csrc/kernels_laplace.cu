@@ -318,10 +318,10 @@ k_m2m3(qbxfmm_geometry g, int p, int ncf, int nrhs, int i0, double2* __restrict_
 // list-2 pairs: the singular-harmonic tables (rows 0..2p, columns -p..2p) and the
 // multipoles (rows 0..p, columns -p..p) are expanded into zero-padded dense arrays
 // in shared memory, so the inner product is branch-free.  Each output's sum is
-// split over two threads (k ranges with about equal term counts); each thread takes up to
-// M2L3_H of the 2 ncf jobs (462 at order 20).
-constexpr int M2L3_H = 4;
-__global__ void __launch_bounds__(NT)
+// split over two threads (k ranges with about equal term counts); each of the TN >= ncf threads
+// takes up to two of the 2 ncf jobs.
+template <int TN>
+__global__ void __launch_bounds__(TN)
 k_m2l3(qbxfmm_geometry g, int p, int ncf, int nrhs, int pb_max, const double2* __restrict__ mpoles,
        double2* __restrict__ locals, int32_t* err)
 {
@@ -341,7 +341,7 @@ k_m2l3(qbxfmm_geometry g, int p, int ncf, int nrhs, int pb_max, const double2* _
   double ct[3];
   load_point<3>(g.box_centers, g.nboxes, tb, ct);
 
-  for (int q = threadIdx.x; q < pb_max * (SS + MS); q += NT) smem2[q] = c2(0.0);
+  for (int q = threadIdx.x; q < pb_max * (SS + MS); q += TN) smem2[q] = c2(0.0);
 
   // k split point: first half takes rows 0..ksplit-1
   int ksplit = 0;
@@ -349,9 +349,9 @@ k_m2l3(qbxfmm_geometry g, int p, int ncf, int nrhs, int pb_max, const double2* _
     int half = (p + 1) * (p + 1) / 2, cum = 0;
     while (ksplit <= p && cum + ksplit <= half) cum += 2 * ksplit + 1, ++ksplit;
   }
-  double2 acc[M2L3_H];
+  double2 acc[2];
 #pragma unroll
-  for (int h = 0; h < M2L3_H; ++h) acc[h] = c2(0.0);
+  for (int h = 0; h < 2; ++h) acc[h] = c2(0.0);
   int l0 = g.list2_starts[i], l1 = g.list2_starts[i + 1];
   for (int lb = l0; lb < l1; lb += pb_max) {
     int nbat = min(pb_max, l1 - lb);
@@ -371,7 +371,7 @@ k_m2l3(qbxfmm_geometry g, int p, int ncf, int nrhs, int pb_max, const double2* _
     }
     __syncthreads();
     // S tables: one thread per (pair, column m in 0..2p); negative columns by symmetry
-    for (int w = threadIdx.x; w < nbat * (2 * p + 1); w += NT) {
+    for (int w = threadIdx.x; w < nbat * (2 * p + 1); w += TN) {
       int b = w / (2 * p + 1), m = w - b * (2 * p + 1);
       double2* S = Spad + (size_t)b * SS;
       if (s_sb[b] < 0) {
@@ -398,7 +398,7 @@ k_m2l3(qbxfmm_geometry g, int p, int ncf, int nrhs, int pb_max, const double2* _
       }
     }
     // M tables
-    for (int w = threadIdx.x; w < nbat * ncf; w += NT) {
+    for (int w = threadIdx.x; w < nbat * ncf; w += TN) {
       int b = w / ncf, c = w - b * ncf;
       int k, l;
       decode3(c, k, l);
@@ -410,8 +410,8 @@ k_m2l3(qbxfmm_geometry g, int p, int ncf, int nrhs, int pb_max, const double2* _
     }
     __syncthreads();
 #pragma unroll
-    for (int h = 0; h < M2L3_H; ++h) {
-      int job = threadIdx.x + h * NT;
+    for (int h = 0; h < 2; ++h) {
+      int job = threadIdx.x + h * TN;
       if (job >= 2 * ncf) break;
       int o = job >> 1, half = job & 1;
       int j, ii;
@@ -433,15 +433,15 @@ k_m2l3(qbxfmm_geometry g, int p, int ncf, int nrhs, int pb_max, const double2* _
   // combine the two halves of each output
   __syncthreads();
 #pragma unroll
-  for (int h = 0; h < M2L3_H; ++h) {
-    int job = threadIdx.x + h * NT;
+  for (int h = 0; h < 2; ++h) {
+    int job = threadIdx.x + h * TN;
     if (job < 2 * ncf && (job & 1)) red[job >> 1] = acc[h];
   }
   __syncthreads();
   double2* L = locals + ((size_t)tb * nrhs + r) * ncf;
 #pragma unroll
-  for (int h = 0; h < M2L3_H; ++h) {
-    int job = threadIdx.x + h * NT;
+  for (int h = 0; h < 2; ++h) {
+    int job = threadIdx.x + h * TN;
     if (job < 2 * ncf && !(job & 1)) {
       int o = job >> 1;
       int j, ii;
@@ -1805,8 +1805,14 @@ cudaError_t launch_m2l(const qbxfmm_geometry& g, int p, int nrhs, const double2*
   size_t per = ((size_t)(2 * p + 1) * (3 * p + 1) + (size_t)(p + 1) * (2 * p + 1)) * sizeof(double2);
   int pb = (int)std::min<size_t>(4, std::max<size_t>(1, (160 * 1024 - ncf * sizeof(double2)) / per));
   size_t sh = pb * per + ncf * sizeof(double2);
-  cudaFuncSetAttribute(k_m2l3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-  k_m2l3<<<dim3(g.nttp_boxes, grid_y(nrhs)), NT, sh, st>>>(g, p, ncf, nrhs, pb, mp, lo, err);
+  // 128 threads up to order 14; at most 231 coefficients.  With up to four jobs a thread on 128
+  // threads the apply by pair of 43 200 nodes took 25.9 ms at order 15 (a third round for 16
+  // jobs), 18.4 here; 10 800 nodes: order 12 3.50 and 3.36 ms, order 20 13.5 and 9.6.
+  const int tn = std::max(NT, (ncf + 31) / 32 * 32);
+  auto k = tn == 128 ? k_m2l3<128> : tn == 160 ? k_m2l3<160> : tn == 192 ? k_m2l3<192>
+         : tn == 224 ? k_m2l3<224> : k_m2l3<256>;
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+  k<<<dim3(g.nttp_boxes, grid_y(nrhs)), tn, sh, st>>>(g, p, ncf, nrhs, pb, mp, lo, err);
   return cudaGetLastError();
 }
 

@@ -1343,7 +1343,8 @@ int qbxfmm_apply(const qbxfmm_plan* p, const qbxfmm_upsample* up, const qbxfmm_w
   // to the QBX targets, and the box locals too (then no QBX expansions are formed) except in
   // the spherical-wave truncation in 3D
   const bool direct = p->helm && !p->mixed && p->kern.target_specific_qbx != 0;
-  const bool m2t = direct && (p->h3 ? h3_m2t_wins(p->geo) : h2_e2t_wins(p->geo, p->kern.nrhs));
+  const bool m2t = direct && (p->h3 ? h3_m2t_wins(p->geo) : h2_e2t_wins(p->geo, p->kern.fmm_order,
+                                                                  p->kern.qbx_order, p->kern.nrhs));
   const bool l2t = m2t && (!p->h3 || p->hc.taylor);
   if (!l2t) QBX_TRY(cudaMemsetAsync(ws->qbx_exps, 0, sz[3], st), "apply: clear");
   QBX_TRY(cudaMemsetAsync(ws->pot_nonqbx, 0, sz[4], st), "apply: clear");

@@ -165,7 +165,9 @@ cudaError_t h2_launch_p2qbxl(const qbxfmm_geometry& g, HelmCoeffs hc, int q, int
 cudaError_t h2_launch_e2t(const qbxfmm_geometry& g, double k, int p, int q, int nrhs,
                           bool from_local, const double2* exps, double2* pot_tree, int32_t* err,
                           cudaStream_t st);
-bool h2_e2t_wins(const qbxfmm_geometry& g, int nrhs);
+bool h2_e2t_wins(const qbxfmm_geometry& g, int p, int q, int nrhs);
+// whether the M2QBXL / L2QBXL kernels of these orders and densities can run
+bool h2_m2qbxl_fits(int pf, int q, int nrhs);
 cudaError_t h2_launch_m2qbxl(const qbxfmm_geometry& g, HelmCoeffs hc, int pf, int q, int nrhs,
                              const double2* mp, double2* qe, int32_t* err, cudaStream_t st);
 cudaError_t h2_launch_l2qbxl(const qbxfmm_geometry& g, HelmCoeffs hc, int pf, int q, int nrhs,

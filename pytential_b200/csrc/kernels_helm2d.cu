@@ -1141,12 +1141,17 @@ static cudaError_t h2_p2qbxl_q(const qbxfmm_geometry& g, HelmCoeffs hc, int nrhs
   return cudaGetLastError();
 }
 
+// Bessel tables of cw centers and E2Q_LB boxes, coefficients of rc densities
+static size_t h2_e2qbxl_smem(int pf, int q, int rc, int cw)
+{
+  return ((size_t)E2Q_LB * cw * (2 * (pf + q) + 1) + (size_t)rc * (2 * pf + 1)) * sizeof(double2);
+}
+
 template <int Q, bool FROM_LOCAL, int RW, int TR, int CW>
 static cudaError_t h2_e2qbxl_rt(const qbxfmm_geometry& g, HelmCoeffs hc, int pf, int nrhs,
                                 const double2* e, double2* qe, int32_t* err, cudaStream_t st)
 {
-  size_t sh = ((size_t)E2Q_LB * CW * (2 * (pf + Q) + 1) + (size_t)RW * TR * (2 * pf + 1)) *
-              sizeof(double2);
+  const size_t sh = h2_e2qbxl_smem(pf, Q, RW * TR, CW);
   cudaError_t ce = cudaFuncSetAttribute(k_h2_e2qbxl<Q, FROM_LOCAL, RW, TR, CW>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
   if (ce != cudaSuccess) return ce;
@@ -1163,6 +1168,13 @@ static cudaError_t h2_e2qbxl_qf(const qbxfmm_geometry& g, HelmCoeffs hc, int pf,
   if (nrhs <= 4) return h2_e2qbxl_rt<Q, FROM_LOCAL, 4, 1, 32>(g, hc, pf, nrhs, e, qe, err, st);
   if (nrhs <= 32) return h2_e2qbxl_rt<Q, FROM_LOCAL, 32, 1, 4>(g, hc, pf, nrhs, e, qe, err, st);
   return h2_e2qbxl_rt<Q, FROM_LOCAL, 32, 2, 4>(g, hc, pf, nrhs, e, qe, err, st);
+}
+
+// whether a CTA of that shape fits the shared memory (up to 4 densities, whose CTAs hold 32
+// centers: up to pf + q = 27)
+bool h2_m2qbxl_fits(int pf, int q, int nrhs)
+{
+  return h2_e2qbxl_smem(pf, q, nrhs == 1 ? 1 : 4, nrhs <= 4 ? 32 : 4) <= 227 * 1024;
 }
 
 template <int Q>

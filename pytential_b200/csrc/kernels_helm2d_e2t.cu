@@ -201,18 +201,24 @@ cudaError_t e2t_q(const qbxfmm_geometry& g, double k, int p, int nrhs, const dou
 // Less work than the expansions, but after the near field, which writes the same potential,
 // where M2QBXL runs beside it: with few chunks the apply is as long as its longest stream, and
 // the expansions are faster.  That line lies higher where no other targets' P2P and M2P take
-// the GPU meanwhile.  Apply with the expansions against this form, q 5, p 20, k 20, chunks of
-// the starfish at 64, 150, 220, 300, 500 and 700 elements (84, 216, 326, 414, 733, 1081):
-//   no other targets, 2 densities: 303 / 360, 444 / 563, 562 / 704, 536 / 666, 875 / 945,
-//   1107 / 980 us; 16 densities: 344 / 435, 558 / 665, 804 / 837, 950 / 988, 1529 / 1499,
-//   1910 / 1716 us;
-//   30 others, the first four: 1 density 613 / 672, 573 / 744, 615 / 735, 959 / 903 us, 16
-//   densities 833 / 968, 786 / 1012, 942 / 1010, 1409 / 1312 us; 100 others, 150 elements:
-//   1 density 802 / 697, 2 728 / 692, 4 772 / 765, 8 970 / 904 us.
-bool h2_e2t_wins(const qbxfmm_geometry& g, int nrhs)
+// the GPU meanwhile, and where the expansions are little work, nrhs (2q + 1) (2p + 1).  Apply of
+// the starfish with the expansions against this form, us:
+//   no other targets, 296 chunks: q 3, p 15, 16 densities 537 / 656; q 6, p 20, 64: 1352 / 1300;
+//   414 chunks, q 5, p 20: 2 densities 536 / 666, 16 950 / 988, 64 1852 / 1659; 634: 2 760 / 824,
+//   8 1061 / 993, 16 1261 / 1261; 733: 2 875 / 945, 16 1529 / 1499; q 1, p 4, 64 1052 / 1332; q 3,
+//   p 15, 16 1002 / 1058, 64 2033 / 1874; 1446: q 1, p 4, 16 1115 / 1088; q 6, p 20, 1 1775 / 1323;
+//   30 others, q 5, p 20, 84, 216, 326 and 414 chunks: 1 density 613 / 672, 573 / 744, 615 / 735,
+//   959 / 903, 16 densities 833 / 968, 786 / 1012, 942 / 1010, 1409 / 1312; 100 others, 216: 1
+//   density 802 / 697, 2 728 / 692, 8 970 / 904; 1000 others, 300 chunks, orders 0 to 8: 0.99 to
+//   1.10 times the other.
+bool h2_e2t_wins(const qbxfmm_geometry& g, int p, int q, int nrhs)
 {
-  const int ctas_per_sm = g.nnonqbx_chunks == 0 ? (nrhs <= 4 ? 5 : 2) : (nrhs == 1 ? 1 : 2);
-  return g.ntsqbx_chunks >= ctas_per_sm * 148 &&
+  if (g.ntsqbx_chunks == 0) return false;
+  if (!h2_m2qbxl_fits(p, q, nrhs)) return true;
+  const long long work = (long long)nrhs * (2 * q + 1) * (2 * p + 1);
+  const int per_sm = g.nnonqbx_chunks > 0 ? (nrhs == 1 ? 1 : 2)
+                                          : work >= 20000 ? 2 : work >= 3500 ? 4 : 5;
+  return g.ntsqbx_chunks >= per_sm * 148 &&
          g.ntsqbx_chunks <= g.nqbx_chunks * (nrhs >= 4 ? 4 : 1);
 }
 

@@ -30,7 +30,8 @@ def _geometry(kind, nel):
 
 
 @pytest.mark.parametrize("kind,nel,nrhs,direct,q,p,k", [
-    ("surface", 250, 4, False, 3, 12, 12.0), ("surface", 250, 5, True, 8, 20, 20.0),
+    ("surface", 250, 4, False, 3, 12, 12.0), ("surface", 250, 60, True, 5, 20, 20.0),
+    ("surface", 440, 5, False, 4, 12, 12.0), ("surface", 500, 9, True, 6, 16, 20.0),
     ("surface", 600, 4, True, 5, 20, 20.0), ("surface", 600, 1, True, 0, 1, 3.0),
     ("points", 60, 1, False, 4, 15, 10.0), ("points", 110, 1, True, 5, 20, 15.0),
     ("points", 110, 2, False, 2, 9, 10.0), ("points", 230, 2, True, 6, 16, 15.0),
@@ -40,7 +41,9 @@ def _geometry(kind, nel):
 def test_both_sides_of_the_rule(kind, nel, nrhs, direct, q, p, k):
     d, geo = _geometry(kind, nel)
     s, _ = abi.geometry_arrays(geo)
-    per_sm = ((5 if nrhs <= 4 else 2) if s["nnonqbx_chunks"] == 0 else (1 if nrhs == 1 else 2))
+    work = nrhs * (2 * q + 1) * (2 * p + 1)
+    per_sm = ((2 if work >= 20000 else 4 if work >= 3500 else 5) if s["nnonqbx_chunks"] == 0
+              else (1 if nrhs == 1 else 2))
     assert direct == (per_sm * 148 <= s["ntsqbx_chunks"]
                       <= s["nqbx_chunks"] * (4 if nrhs >= 4 else 1))
     spec = fmm.SourceKernelSpec(fmm.HelmholtzKernel(2, k), charge_coeff=-1j * k, dipole_coeff=1.0)
@@ -60,3 +63,20 @@ def test_both_sides_of_the_rule(kind, nel, nrhs, direct, q, p, k):
     # a captured apply runs the same kernels in the same order
     ap.capture()
     assert torch.equal(ap.replay(x), u)
+
+
+@pytest.mark.parametrize("kind,nel", [("surface", 40), ("points", 60), ("many", 160)])
+@pytest.mark.parametrize("nrhs", [1, 4])
+def test_orders_whose_expansions_do_not_fit(kind, nel, nrhs):
+    """Orders 8 and 20 with up to 4 densities, whose M2QBXL needs more shared memory than there
+    is: straight to the targets, however few they are; with 6 densities it fits."""
+    d, geo = _geometry(kind, nel)
+    k = 9.0
+    spec = fmm.SourceKernelSpec(fmm.HelmholtzKernel(2, k), charge_coeff=-1j * k, dipole_coeff=1.0)
+    rng = np.random.default_rng(5)
+    x = torch.from_numpy(rng.normal(size=(6, d.ndofs)) + 1j * rng.normal(size=(6, d.ndofs))).cuda()
+    ap = fmm.QBXApply(geo, spec, 8, 20, nrhs=nrhs)
+    u = ap(x[:nrhs])
+    ap.check_error_word()
+    v = fmm.QBXApply(geo, spec, 8, 20, nrhs=6)(x)[:nrhs]
+    assert float((u - v).abs().max() / v.abs().max()) < 5e-12

@@ -201,23 +201,27 @@ cudaError_t e2t_q(const qbxfmm_geometry& g, double k, int p, int nrhs, const dou
 // Less work than the expansions, but after the near field, which writes the same potential,
 // where M2QBXL runs beside it: with few chunks the apply is as long as its longest stream, and
 // the expansions are faster.  That line lies higher where no other targets' P2P and M2P take
-// the GPU meanwhile, and where the expansions are little work, nrhs (2q + 1) (2p + 1).  Apply of
-// the starfish with the expansions against this form, us:
-//   no other targets, 296 chunks: q 3, p 15, 16 densities 537 / 656; q 6, p 20, 64: 1352 / 1300;
-//   414 chunks, q 5, p 20: 2 densities 536 / 666, 16 950 / 988, 64 1852 / 1659; 634: 2 760 / 824,
-//   8 1061 / 993, 16 1261 / 1261; 733: 2 875 / 945, 16 1529 / 1499; q 1, p 4, 64 1052 / 1332; q 3,
-//   p 15, 16 1002 / 1058, 64 2033 / 1874; 1446: q 1, p 4, 16 1115 / 1088; q 6, p 20, 1 1775 / 1323;
-//   30 others, q 5, p 20, 84, 216, 326 and 414 chunks: 1 density 613 / 672, 573 / 744, 615 / 735,
-//   959 / 903, 16 densities 833 / 968, 786 / 1012, 942 / 1010, 1409 / 1312; 100 others, 216: 1
-//   density 802 / 697, 2 728 / 692, 8 970 / 904; 1000 others, 300 chunks, orders 0 to 8: 0.99 to
-//   1.10 times the other.
+// the GPU meanwhile, and where the expansions are little work: up to four densities, whose
+// M2QBXL wastes no lanes, and low orders, by (2q + 1) (2p + 1) a density.  Time of the starfish's
+// apply with the expansions over this form's:
+//   no other targets, 350, 414, 498, 600, 680, 724, 759 and 964 chunks: 7 densities q 5, p 20
+//   0.98 0.99 1.04 1.09 1.11 1.11 1.18 1.16; q 4, p 18 0.83 0.95 0.97 0.98 1.06 1.02 1.17 1.18;
+//   q 3, p 15 0.82 0.90 0.94 0.96 0.99 0.95 1.10 1.06; q 1, p 6 0.85 0.82 0.86 0.87 0.91 0.86 0.96
+//   1.06; 16 densities q 6, p 18 0.94 0.99 1.02 1.02 1.06 1.02 1.09 1.11; 64 densities, 296 and
+//   733 chunks: q 6, p 20 1.04 1.21, q 3, p 15 0.94 1.08, q 2, p 8 0.91 0.92; 4 densities, q 5,
+//   p 20, 414, 634, 733 and 1081: 0.81 0.90 0.94 1.13;
+//   30 others, q 5, p 20, 84, 216, 326 and 414 chunks: 1 density 0.91 0.77 0.84 1.06, 16 0.86
+//   0.78 0.93 1.07; 100 others, 216: 1 density 1.15, 2 1.05, 8 1.07; 1000 others, 300 chunks,
+//   orders 0 to 8: 0.99 to 1.10.
 bool h2_e2t_wins(const qbxfmm_geometry& g, int p, int q, int nrhs)
 {
   if (g.ntsqbx_chunks == 0) return false;
   if (!h2_m2qbxl_fits(p, q, nrhs)) return true;
-  const long long work = (long long)nrhs * (2 * q + 1) * (2 * p + 1);
-  const int per_sm = g.nnonqbx_chunks > 0 ? (nrhs == 1 ? 1 : 2)
-                                          : work >= 20000 ? 2 : work >= 3500 ? 4 : 5;
+  const int work = (2 * q + 1) * (2 * p + 1);
+  int per_sm = 5;
+  if (g.nnonqbx_chunks > 0) per_sm = nrhs == 1 ? 1 : 2;
+  else if (nrhs > 4 && work >= 400) per_sm = nrhs > 32 ? 2 : 3;
+  else if (nrhs > 32 && work >= 160) per_sm = 4;
   return g.ntsqbx_chunks >= per_sm * 148 &&
          g.ntsqbx_chunks <= g.nqbx_chunks * (nrhs >= 4 ? 4 : 1);
 }

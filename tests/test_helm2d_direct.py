@@ -31,7 +31,8 @@ def _geometry(kind, nel):
 
 @pytest.mark.parametrize("kind,nel,nrhs,direct,q,p,k", [
     ("surface", 250, 4, False, 3, 12, 12.0), ("surface", 250, 60, True, 5, 20, 20.0),
-    ("surface", 440, 5, False, 4, 12, 12.0), ("surface", 500, 9, True, 6, 16, 20.0),
+    ("surface", 250, 9, False, 5, 20, 20.0), ("surface", 440, 5, True, 6, 16, 20.0),
+    ("surface", 440, 33, True, 3, 15, 12.0), ("surface", 440, 32, False, 3, 15, 12.0),
     ("surface", 600, 4, True, 5, 20, 20.0), ("surface", 600, 1, True, 0, 1, 3.0),
     ("points", 60, 1, False, 4, 15, 10.0), ("points", 110, 1, True, 5, 20, 15.0),
     ("points", 110, 2, False, 2, 9, 10.0), ("points", 230, 2, True, 6, 16, 15.0),
@@ -41,9 +42,13 @@ def _geometry(kind, nel):
 def test_both_sides_of_the_rule(kind, nel, nrhs, direct, q, p, k):
     d, geo = _geometry(kind, nel)
     s, _ = abi.geometry_arrays(geo)
-    work = nrhs * (2 * q + 1) * (2 * p + 1)
-    per_sm = ((2 if work >= 20000 else 4 if work >= 3500 else 5) if s["nnonqbx_chunks"] == 0
-              else (1 if nrhs == 1 else 2))
+    work = (2 * q + 1) * (2 * p + 1)
+    if s["nnonqbx_chunks"] > 0:
+        per_sm = 1 if nrhs == 1 else 2
+    elif nrhs > 4 and work >= 400:
+        per_sm = 2 if nrhs > 32 else 3
+    else:
+        per_sm = 4 if nrhs > 32 and work >= 160 else 5
     assert direct == (per_sm * 148 <= s["ntsqbx_chunks"]
                       <= s["nqbx_chunks"] * (4 if nrhs >= 4 else 1))
     spec = fmm.SourceKernelSpec(fmm.HelmholtzKernel(2, k), charge_coeff=-1j * k, dipole_coeff=1.0)
